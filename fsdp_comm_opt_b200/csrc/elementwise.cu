@@ -1,6 +1,5 @@
 // Memory-bound training ops for sm_100a: RMSNorm (+ residual add) forward/backward, RoPE, SwiGLU
-// forward/backward, cross-entropy with in-place gradient, int8 absmax quantise/dequantise and
-// fused AdamW.  Every kernel moves 16-byte vectors, keeps fp32 math in registers and touches each
+// forward/backward, cross-entropy with in-place gradient and fused AdamW.  Every kernel moves 16-byte vectors, keeps fp32 math in registers and touches each
 // HBM byte once per pass.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -439,10 +438,6 @@ __global__ void __launch_bounds__(1024) ce_kernel(__nv_bfloat16* __restrict__ lo
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// int8 absmax quantisation.  Packed buffer: word0 = fp32 scale, word1 = absmax bits (scratch),
-// bytes [16, 16+n) = int8 payload.
-// ---------------------------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
@@ -451,46 +446,6 @@ template <typename T> __device__ __forceinline__ T from_f(float v);
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half(v); }
-
-template <typename T>
-__global__ void __launch_bounds__(256) absmax_kernel(const T* __restrict__ x, int64_t n, uint32_t* __restrict__ hdr) {
-  float m = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
-    m = fmaxf(m, fabsf(to_f<T>(x[i])));
-  m = warp_max(m);
-  __shared__ float red[8];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; ++i) m = fmaxf(m, red[i]);
-    atomicMax(hdr + 1, __float_as_uint(m));  // non-negative floats order like their bit patterns
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) quant_kernel(const T* __restrict__ x, int64_t n, uint8_t* __restrict__ out) {
-  const float absmax = __uint_as_float(reinterpret_cast<const uint32_t*>(out)[1]);
-  const float scale = fmaxf(absmax / 127.f, 1e-8f);
-  if (blockIdx.x == 0 && threadIdx.x == 0) reinterpret_cast<float*>(out)[0] = scale;
-  int8_t* q = reinterpret_cast<int8_t*>(out + 16);
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-    const float r = rintf(to_f<T>(x[i]) / scale);
-    q[i] = (int8_t)fminf(fmaxf(r, -127.f), 127.f);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict__ gathered, int64_t stride,
-                                                      int world, int64_t n, T* __restrict__ out) {
-  const int64_t total = (int64_t)world * n;
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
-    const int r = (int)(i / n);
-    const int64_t k = i - (int64_t)r * n;
-    const uint8_t* slot = gathered + r * stride;
-    const float scale = reinterpret_cast<const float*>(slot)[0];
-    out[i] = from_f<T>((float)reinterpret_cast<const int8_t*>(slot + 16)[k] * scale);
-  }
-}
 
 // ---------------------------------------------------------------------------------------------
 // AdamW (decoupled weight decay), one launch per shard
@@ -715,41 +670,6 @@ int zc_ce_fwd_bwd_ld(void* logits, const int64_t* labels, float* row_loss, const
 int zc_ce_fwd_bwd(void* logits, const int64_t* labels, float* row_loss, const float* inv_count, int64_t T, int V,
                   int ignore_index, cudaStream_t st) {
   return zc_ce_fwd_bwd_ld(logits, labels, row_loss, inv_count, T, V, V, ignore_index, st);
-}
-
-int zc_quant_int8(const void* x, int64_t n, int dtype, void* out, cudaStream_t st) {
-  cudaMemsetAsync(out, 0, 16, st);
-  if (n == 0) return zc::launch_status();
-  const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)zc::sm_count() * 16);
-  if (dtype == 0) {
-    zc::absmax_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)x, n, (uint32_t*)out);
-    zc::quant_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)x, n, (uint8_t*)out);
-  } else if (dtype == 1) {
-    zc::absmax_kernel<float><<<grid, 256, 0, st>>>((const float*)x, n, (uint32_t*)out);
-    zc::quant_kernel<float><<<grid, 256, 0, st>>>((const float*)x, n, (uint8_t*)out);
-  } else if (dtype == 2) {
-    zc::absmax_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, n, (uint32_t*)out);
-    zc::quant_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, n, (uint8_t*)out);
-  } else {
-    return ERR_UNSUPPORTED;
-  }
-  return zc::launch_status();
-}
-
-int zc_dequant_int8(const void* gathered, int64_t stride, int world, int64_t n, int dtype, void* out,
-                    cudaStream_t st) {
-  const int64_t total = (int64_t)world * n;
-  if (total == 0) return 0;
-  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
-  if (dtype == 0)
-    zc::dequant_kernel<bf16><<<grid, 256, 0, st>>>((const uint8_t*)gathered, stride, world, n, (bf16*)out);
-  else if (dtype == 1)
-    zc::dequant_kernel<float><<<grid, 256, 0, st>>>((const uint8_t*)gathered, stride, world, n, (float*)out);
-  else if (dtype == 2)
-    zc::dequant_kernel<__half><<<grid, 256, 0, st>>>((const uint8_t*)gathered, stride, world, n, (__half*)out);
-  else
-    return ERR_UNSUPPORTED;
-  return zc::launch_status();
 }
 
 // The library's health word of the current device (0 = healthy): set by a fused collective whose

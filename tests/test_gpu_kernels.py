@@ -265,6 +265,28 @@ def test_int8_quant_kernels():
         assert (out[r * n:(r + 1) * n].float() - xs[r].float()).abs().max() <= scale * 1.01
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("n,world", [(1, 1), (7, 3), (16, 2), (4099, 5), (1 << 19, 2), ((1 << 19) + 9, 3)])
+def test_int8_vector_paths_and_their_edges(n, world, dt):
+    """One-launch and three-launch quantiser, output rows at every alignment of the dequantiser."""
+    torch.manual_seed(n)
+    buf = torch.zeros(world, quant.packed_bytes(n), dtype=torch.uint8, device=DEV)
+    xs = [(torch.randn(n, device=DEV) * 0.02).to(dt) for _ in range(world)]
+    for r in range(world):
+        quant.quantize_pack(xs[r], buf[r])
+    out = torch.full((world * n + 8,), 7.0, dtype=dt, device=DEV)
+    quant.dequantize_unpack(buf, n, out[:world * n])
+    assert bool((out[world * n:] == 7.0).all())
+    for r in range(world):
+        scale = buf[r, :4].view(torch.float32)
+        assert torch.allclose(scale, (xs[r].float().abs().max() / 127).clamp_min(1e-8).reshape(1))
+        q = buf[r, 16:16 + n].view(torch.int8).float()
+        # the approximate division may round a quotient that lies on a half the other way
+        assert (q - xs[r].float() / scale).abs().max() <= 0.5 + 1e-4
+        assert torch.equal(out[r * n:(r + 1) * n], (q * scale).to(dt))
+        assert not buf[r, 16 + n:].any()
+
+
 @pytest.mark.parametrize("pdt,sdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
 def test_fused_adamw_kernel(pdt, sdt):
     torch.manual_seed(5)
