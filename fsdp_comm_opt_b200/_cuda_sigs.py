@@ -56,15 +56,15 @@ def declare(lib) -> None:
     # tensor cores
     _sig(lib, "zc_umma_selftest", P, P, P, I, I, I, P, P)
     _sig(lib, "zc_attn_fwd", P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, L, L, L, F, P)
-    _sig(lib, "zc_attn_bwd", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P)
+    _sig(lib, "zc_attn_bwd", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P, P)
     _sig(lib, "zc_attn_status_read_and_clear")
     _sig(lib, "zc_attn_fwd_ws", P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, L, L, L, F, P)
     _sig(lib, "zc_attn_ws_status_read_and_clear")
-    _sig(lib, "zc_attn_bwd_ws", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P)
+    _sig(lib, "zc_attn_bwd_ws", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P, P)
     _sig(lib, "zc_attn_bwd_ws_status_read_and_clear")
     _sig(lib, "zc_attn_fwd_2q", P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, L, L, L, F, P)
     _sig(lib, "zc_attn_fwd_2q_status_read_and_clear")
-    _sig(lib, "zc_attn_bwd_kt", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P)
+    _sig(lib, "zc_attn_bwd_kt", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P, P)
     _sig(lib, "zc_gemm_bf16", P, P, P, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm", P, P, P, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm_ld", P, P, P, L, L, L, L, L, L, I, I, I, P)

@@ -104,6 +104,12 @@ def launch_count() -> int:
     return _LAUNCHES
 
 
+def add_launches(n: int) -> None:
+    """Count ``n`` launches that a replayed graph makes."""
+    global _LAUNCHES
+    _LAUNCHES += n
+
+
 def reset_launch_count() -> None:
     global _LAUNCHES
     _LAUNCHES = 0

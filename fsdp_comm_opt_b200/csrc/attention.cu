@@ -453,8 +453,6 @@ __global__ void __launch_bounds__(256) attn_dq_convert_kernel(const float* __res
 // per-device scratch that persists across calls: status word and the fp32 dQ accumulator
 struct AttnScratch {
   int* status = nullptr;
-  float* dq_acc = nullptr;
-  size_t dq_bytes = 0;
 };
 static AttnScratch g_scratch[64];
 
@@ -516,7 +514,7 @@ int zc_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
                 float* delta, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv, int D, int64_t qs0,
                 int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,
                 int64_t vs2, int64_t dqs0, int64_t dqs1, int64_t dqs2, int64_t dks0, int64_t dks1, int64_t dks2,
-                int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, cudaStream_t st) {
+                int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, float* dq_acc, cudaStream_t st) {
   using namespace zc;
   if ((D != 64 && D != 128) || Hq % Hkv) return ERR_UNSUPPORTED;
   if ((qs1 | qs2 | ks1 | ks2 | vs1 | vs2 | qs0 | ks0 | vs0 | dqs1 | dqs2 | dks1 | dks2 | dvs1 | dvs2 | dqs0 | dks0 | dvs0) % 8)
@@ -526,16 +524,10 @@ int zc_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
   cudaGetDevice(&dev);
   AttnScratch& sc = g_scratch[dev];
   const size_t need = (size_t)B * S * Hq * D * sizeof(float);
-  if (sc.dq_bytes < need) {
-    // grown only when a larger problem appears; stream-ordered so earlier launches keep their buffer
-    if (sc.dq_acc) cudaFreeAsync(sc.dq_acc, st);
-    if (cudaMallocAsync(&sc.dq_acc, need, st) != cudaSuccess) { sc.dq_acc = nullptr; sc.dq_bytes = 0; return (int)cudaGetLastError(); }
-    sc.dq_bytes = need;
-  }
-  cudaMemsetAsync(sc.dq_acc, 0, need, st);
+  cudaMemsetAsync(dq_acc, 0, need, st);
   AttnBwdParams p;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
-  p.dout = (const __nv_bfloat16*)dout; p.lse = lse; p.delta = delta; p.dq_acc = sc.dq_acc;
+  p.dout = (const __nv_bfloat16*)dout; p.lse = lse; p.delta = delta; p.dq_acc = dq_acc;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.qs0 = qs0; p.qs1 = qs1; p.qs2 = qs2; p.ks0 = ks0; p.ks1 = ks1; p.ks2 = ks2; p.vs0 = vs0; p.vs1 = vs1; p.vs2 = vs2;
@@ -557,7 +549,7 @@ int zc_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
     if (!attr[1]) { cudaFuncSetAttribute(attn_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr[1] = true; }
     attn_bwd_kernel<64><<<grid, 128, smem, st>>>(p);
   }
-  attn_dq_convert_kernel<<<cgrid, 256, 0, st>>>(sc.dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
+  attn_dq_convert_kernel<<<cgrid, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
   return launch_status();
 }
 

@@ -342,8 +342,6 @@ static bool make_map4_f32(CUtensorMap* m, const void* base, int D, int H, int S,
 
 struct Scratch {
   int* status = nullptr;
-  float* dq_acc = nullptr;
-  size_t dq_bytes = 0;
 };
 static Scratch g_scratch[64];
 static long long* g_trace = nullptr;
@@ -832,12 +830,13 @@ int zc_attn_bwd_ws_status_read_and_clear() {
   return v;
 }
 
-// Same argument list as zc_attn_bwd.
+// Same argument list as zc_attn_bwd: `dq_acc` is the fp32 accumulator of dQ, B * Hq * D * (S rounded up to 4)
+// floats that the launcher clears.
 int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                    float* delta, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv, int D, int64_t qs0,
                    int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,
                    int64_t vs2, int64_t dqs0, int64_t dqs1, int64_t dqs2, int64_t dks0, int64_t dks1, int64_t dks2,
-                   int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, cudaStream_t st) {
+                   int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, float* dq_acc, cudaStream_t st) {
   using namespace zc;
   using namespace zc::bws;
   if ((D != 64 && D != 128) || Hq % Hkv) return ERR_UNSUPPORTED;
@@ -856,20 +855,15 @@ int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, c
     cudaMemset(sc.status, 0, sizeof(int));
   }
   const size_t need = (size_t)B * S * Hq * D * sizeof(float);
-  if (sc.dq_bytes < need) {
-    if (sc.dq_acc) cudaFreeAsync(sc.dq_acc, st);
-    if (cudaMallocAsync(&sc.dq_acc, need, st) != cudaSuccess) { sc.dq_acc = nullptr; sc.dq_bytes = 0; return (int)cudaGetLastError(); }
-    sc.dq_bytes = need;
-  }
-  cudaMemsetAsync(sc.dq_acc, 0, need, st);
+  cudaMemsetAsync(dq_acc, 0, need, st);
   CUtensorMap mq, mk, mv, mdo, mdq;
   if (!make_map4(&mq, q, D, Hq, S, B, qs0, qs1, qs2) || !make_map4(&mk, k, D, Hkv, S, B, ks0, ks1, ks2) ||
       !make_map4(&mv, v, D, Hkv, S, B, vs0, vs1, vs2) ||
       !make_map4(&mdo, dout, D, Hq, S, B, (int64_t)S * Hq * D, (int64_t)Hq * D, D) ||
-      !make_map4_f32(&mdq, sc.dq_acc, D, Hq, S, B))
+      !make_map4_f32(&mdq, dq_acc, D, Hq, S, B))
     return ERR_BAD_ARG;
   BwdParams p;
-  p.lse = lse; p.delta = delta; p.dq_acc = sc.dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
+  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.dks0 = dks0; p.dks1 = dks1; p.dks2 = dks2; p.dvs0 = dvs0; p.dvs1 = dvs1; p.dvs2 = dvs2;
   p.scale = scale; p.status = sc.status; p.trace = nullptr;
@@ -887,7 +881,7 @@ int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, c
     attn_bwd_ws_kernel<64><<<grid, 320, smem, st>>>(mq, mk, mv, mdo, mdq, p);
   }
   const int cgrid = (int)std::min<int64_t>((rows * (D / 4) + 255) / 256, (int64_t)sm_count() * 16);
-  dq_convert_kernel<<<cgrid, 256, 0, st>>>(sc.dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
+  dq_convert_kernel<<<cgrid, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
   return launch_status();
 }
 
@@ -903,12 +897,12 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
                    float* delta, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv, int D, int64_t qs0,
                    int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,
                    int64_t vs2, int64_t dqs0, int64_t dqs1, int64_t dqs2, int64_t dks0, int64_t dks1, int64_t dks2,
-                   int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, cudaStream_t st) {
+                   int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, float* dq_acc, cudaStream_t st) {
   using namespace zc;
   using namespace zc::bws;
   if (D != 128)
     return zc_attn_bwd_ws(q, k, v, o, dout, lse, delta, dq, dk, dv, B, S, Hq, Hkv, D, qs0, qs1, qs2, ks0, ks1, ks2, vs0,
-                          vs1, vs2, dqs0, dqs1, dqs2, dks0, dks1, dks2, dvs0, dvs1, dvs2, scale, st);
+                          vs1, vs2, dqs0, dqs1, dqs2, dks0, dks1, dks2, dvs0, dvs1, dvs2, scale, dq_acc, st);
   if (Hq % Hkv) return ERR_UNSUPPORTED;
   if ((qs1 | qs2 | ks1 | ks2 | vs1 | vs2 | qs0 | ks0 | vs0 | dqs1 | dqs2 | dks1 | dks2 | dvs1 | dvs2 | dqs0 | dks0 | dvs0) % 8)
     return ERR_UNSUPPORTED;
@@ -926,20 +920,15 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
   }
   const int Sp = (S + 3) & ~3;  // row stride of the transposed accumulator: a multiple of 16 bytes
   const size_t need = (size_t)B * Hq * D * Sp * sizeof(float);
-  if (sc.dq_bytes < need) {
-    if (sc.dq_acc) cudaFreeAsync(sc.dq_acc, st);
-    if (cudaMallocAsync(&sc.dq_acc, need, st) != cudaSuccess) { sc.dq_acc = nullptr; sc.dq_bytes = 0; return (int)cudaGetLastError(); }
-    sc.dq_bytes = need;
-  }
-  cudaMemsetAsync(sc.dq_acc, 0, need, st);
+  cudaMemsetAsync(dq_acc, 0, need, st);
   CUtensorMap mq, mk, mv, mdo, mdq;
   if (!make_map4(&mq, q, D, Hq, S, B, qs0, qs1, qs2, bkt::QB) || !make_map4(&mk, k, D, Hkv, S, B, ks0, ks1, ks2) ||
       !make_map4(&mv, v, D, Hkv, S, B, vs0, vs1, vs2) ||
       !make_map4(&mdo, dout, D, Hq, S, B, (int64_t)S * Hq * D, (int64_t)Hq * D, D, bkt::QB) ||
-      !make_map_dq_t(&mdq, sc.dq_acc, D, Hq, S, Sp, B))
+      !make_map_dq_t(&mdq, dq_acc, D, Hq, S, Sp, B))
     return ERR_BAD_ARG;
   BwdParams p;
-  p.lse = lse; p.delta = delta; p.dq_acc = sc.dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
+  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.dks0 = dks0; p.dks1 = dks1; p.dks2 = dks2; p.dvs0 = dvs0; p.dvs1 = dvs1; p.dvs2 = dvs2;
   p.scale = scale; p.status = sc.status; p.trace = g_trace;
@@ -952,7 +941,7 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
   const int nkb = (S + 127) / 128;
   bkt::attn_bwd_kt_kernel<<<nkb * Hkv * B, 352, smem, st>>>(mq, mk, mv, mdo, mdq, p, nkb);
   dq_convert_t_kernel<<<dim3((S + 31) / 32, D / 64, B * Hq), dim3(32, 8), 0, st>>>(
-      sc.dq_acc, (__nv_bfloat16*)dq, S, Sp, Hq, D, dqs0, dqs1, dqs2);
+      dq_acc, (__nv_bfloat16*)dq, S, Sp, Hq, D, dqs0, dqs1, dqs2);
   return launch_status();
 }
 

@@ -21,7 +21,8 @@
 // producer thread fetches the next index and publishes it to every role of both CTAs through a small
 // ring in shared memory), so a cluster that starts late, or not at all for a while, because another
 // kernel (a collective running beside the GEMM) holds its SMs simply takes fewer units; with a
-// static round-robin the whole GEMM would wait for that cluster's share.
+// static round-robin the whole GEMM would wait for that cluster's share.  (Launches recorded into a CUDA
+// graph, which only a one-rank step makes, and those with no second round use the static order.)
 // Units: whole tiles first, then the tiles of the last, partial wave are split
 // along K into `split` slices each, so that all clusters stay busy to the end.  A slice writes its
 // fp32 partial sums to a workspace and a small second kernel adds the slices and rounds to bf16.
@@ -159,7 +160,8 @@ struct Params {
   int full_tiles;      // tiles computed whole; the remaining tiles are split along K
   int split;           // K slices per tail tile (1: no tile is split)
   int* status;
-  unsigned* counter;   // [0] units handed out beyond the first round, [1] clusters finished; both 0 at launch
+  unsigned* counter;   // [0] units handed out beyond the first round, [1] clusters finished; both 0 at launch;
+                       // null: unit i of cluster c is c + i * clusters
 };
 
 // Tile order.  The clusters running at one time work on consecutive tile indices; walking bands of
@@ -291,7 +293,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           // fetch the i-th unit and publish it to both CTAs
           const uint32_t slot = i & (SCHED - 1), sph = (i / SCHED) & 1;
           if (!(ok = wait_bar_cluster(smem_u32(&sched_empty[slot]), sph ^ 1, &s_abort))) break;
-          u = (i == 0) ? cluster_id : n_clusters + (int)atomicAdd(p.counter, 1u);
+          u = (i == 0 || !p.counter) ? cluster_id + (int)i * n_clusters : n_clusters + (int)atomicAdd(p.counter, 1u);
           sched_u[slot] = u;
           st_shared_cluster_u32(su_c1 + 4 * slot, (uint32_t)u);
           mbar_arrive(&sched_full[slot]);
@@ -453,7 +455,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   // neither CTA may leave (or free its TMEM) while the pair's MMAs can still touch its memory
   cluster_sync_all();
   if (warp == 1) tmem_dealloc(tm, 2 * BN);
-  if (tid == 0 && rank == 0) {
+  if (tid == 0 && rank == 0 && p.counter) {
     // the last cluster to finish puts the counters back to zero for the next launch that uses this slot
     if (atomicAdd(p.counter + 1, 1u) == (unsigned)n_clusters - 1u) {
       p.counter[0] = 0u;
@@ -637,10 +639,6 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
   static const int forced_split = getenv("ZC_GEMM_SPLIT") ? atoi(getenv("ZC_GEMM_SPLIT")) : -1;
   p.group_m = forced_gm > 0 ? forced_gm : 8;
   p.status = status;
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    p.counter = ds.counters + 2 * (ds.next_slot++ % COUNTER_SLOTS);
-  }
   const int64_t tiles = m_tiles * n_tiles;
   const int64_t k_blocks = (K + BK - 1) / BK;
   const int clusters = (int)std::min<int64_t>(tiles, ds.clusters);
@@ -655,6 +653,14 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
   }
   p.split = split;
   p.full_tiles = (int)(split > 1 ? tiles - rem : tiles);
+  // Counters only where a second round is handed out, and not in a launch that is being recorded: a
+  // replayed launch would keep its slot for good, next to launches of other streams that take slots in turn.
+  p.counter = nullptr;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (tiles > clusters && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    p.counter = ds.counters + 2 * (ds.next_slot++ % COUNTER_SLOTS);
+  }
   p.partial = nullptr;
   if (split > 1) {
     const size_t need = (size_t)rem * split * BM * BN;

@@ -25,6 +25,7 @@ from .ops.adamw import FusedAdamW
 from .ops.loss import unit_loss_grad
 from .parallel.flat_shard import FlatShardEngine, FlatShardPlan
 from .parallel.fsdp import FSDPPlan, apply_fsdp, make_hook_factories
+from .parallel.step_graph import StepGraphs
 
 
 @dataclass
@@ -47,6 +48,7 @@ class EngineConfig:
     error_feedback: bool = True
     time_collectives: bool = False  # flat only: CUDA-event timing of every collective
     reshard_after_forward: object = "auto"   # flat only: True | False | "auto" (see FlatShardPlan)
+    step_graphs: bool = True        # flat on one rank: replay forward and backward as CUDA graphs (parallel/step_graph.py)
 
 
 def build_sharded(cfg: EngineConfig, device: torch.device):
@@ -92,29 +94,65 @@ class TrainEngine:
         self.lr_scheduler = torch.optim.lr_scheduler.CosineAnnealingLR(self.optimizer, T_max=1000,
                                                                        eta_min=cfg.lr * 1e-2)
         self.global_step = 0
+        self._graphs = None
+        if (cfg.step_graphs and self.flat is not None and self.flat.cuda and self.flat.world == 1
+                and not cfg.time_collectives):
+            self._graphs = StepGraphs(self.model, self.flat, self.model_config)
+        self._loss_host = self._loss_ready = None
+        if device.type == "cuda":
+            self._loss_host = torch.empty((), dtype=torch.float32, pin_memory=True)
+            self._loss_ready = torch.cuda.Event()
 
-    def step_on_device(self, input_ids: torch.Tensor) -> torch.Tensor:
-        """One optimizer step on a batch already on the device; returns the loss tensor."""
+    def _forward_backward(self, input_ids: torch.Tensor) -> torch.Tensor:
+        """Loss of the batch (host or device ids), with the gradients in place.  The tensor may be a buffer
+        that the next call overwrites."""
+        if self._graphs is not None:
+            loss = self._graphs.run(input_ids)
+            if loss is not None:
+                return loss
+        if input_ids.device != self.device:
+            input_ids = input_ids.to(self.device, non_blocking=True)
         if self.flat is not None:
             self.flat.begin_step()
             out = self.model(input_ids=input_ids, labels=input_ids)
             self.flat.backward(out.loss)
-            self.flat.optimizer_step(self.optimizer, self.lr_scheduler)
         else:
             self.model.unshard()
             out = self.model(input_ids=input_ids, labels=input_ids)
             with unit_loss_grad():
                 out.loss.backward()
+        return out.loss.detach()
+
+    def _update(self) -> None:
+        if self.flat is not None:
+            self.flat.optimizer_step(self.optimizer, self.lr_scheduler)
+        else:
             self.optimizer.step()
             self.lr_scheduler.step()
             self.optimizer.zero_grad(set_to_none=True)
         self.global_step += 1
-        return out.loss.detach()
+
+    def step_on_device(self, input_ids: torch.Tensor) -> torch.Tensor:
+        """One optimizer step on a batch already on the device; returns the loss tensor."""
+        loss = self._forward_backward(input_ids)
+        if self._graphs is not None and self._graphs.owns(loss):
+            loss = loss.clone()
+        self._update()
+        return loss
 
     def step(self, input_ids_host: torch.Tensor) -> float:
-        """Host batch in, loss out: H2D copy, one optimizer step, D2H read of the loss."""
-        ids = input_ids_host.to(self.device, non_blocking=True)
-        return float(self.step_on_device(ids).item())
+        """Host batch in, loss out: H2D copy, one optimizer step, D2H read of the loss.  The loss is
+        read as soon as the backward pass has produced the gradients: the optimizer update is already
+        enqueued behind it and runs while the caller prepares its next batch."""
+        loss = self._forward_backward(input_ids_host)
+        if self._loss_host is None or loss.device.type != "cuda":
+            self._update()
+            return float(loss.item())
+        self._loss_host.copy_(loss, non_blocking=True)
+        self._loss_ready.record()
+        self._update()
+        self._loss_ready.synchronize()
+        return float(self._loss_host)
 
     def comm_report(self) -> dict:
         """What the collectives of this engine actually ran on (see ``parallel.fsdp.comm_report``)."""

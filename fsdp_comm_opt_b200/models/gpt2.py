@@ -96,7 +96,7 @@ class GPT2ForCausalLM(nn.Module):
         x, m = t.wte(input_ids), t.wpe(pos)[None].expand(B, S, -1)   # the position add runs in the first norm
         for blk in t.h:
             if self.activation_checkpointing and torch.is_grad_enabled():
-                x, m = checkpoint(blk, x, m, use_reentrant=False)
+                x, m = checkpoint(blk, x, m, use_reentrant=False, preserve_rng_state=False)
             else:
                 x, m = blk(x, m)
         x, _ = gpt2_ops.add_layer_norm(x, m, t.ln_f.weight, t.ln_f.bias, t.ln_f.eps)

@@ -133,7 +133,7 @@ class LlamaForCausalLM(nn.Module):
         x, delta = self.model.embed_tokens(input_ids), None
         for layer in self.model.layers:
             if self.activation_checkpointing and torch.is_grad_enabled():
-                x, delta = checkpoint(layer, x, delta, use_reentrant=False)
+                x, delta = checkpoint(layer, x, delta, use_reentrant=False, preserve_rng_state=False)
             else:
                 x, delta = layer(x, delta)
         x = self.model.norm(x, delta)

@@ -102,6 +102,8 @@ class _Attention(torch.autograd.Function):
         dqkv = torch.empty_like(qkv)
         dq, dk, dv = dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]
         delta = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
+        # fp32 accumulator of dQ: allocated per call, so that calls on other streams and recorded graphs own theirs
+        dq_acc = torch.empty(B * Hq * D * ((S + 3) // 4 * 4), dtype=torch.float32, device=qkv.device)
         lib = _lib.cuda()
         # default: key-row kernel (64-query iterations, pipelined); ZC_ATTN_BWD=ws / simple select
         # the earlier warp-specialised and single-role kernels
@@ -110,7 +112,7 @@ class _Attention(torch.autograd.Function):
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
             delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, Hq, Hkv, D,
             *_strides(q), *_strides(k), *_strides(v), *_strides(dq), *_strides(dk), *_strides(dv),
-            float(ctx.scale), _lib.stream_ptr(qkv.device)), "zc_attn_bwd")
+            float(ctx.scale), dq_acc.data_ptr(), _lib.stream_ptr(qkv.device)), "zc_attn_bwd")
         return _Attention._unrope(ctx, dqkv), None, None, None, None, None
 
     @staticmethod
