@@ -23,8 +23,11 @@ def declare(lib) -> None:
     _sig(lib, "zc_v2_encode_nibble", P, L, P, P, P)
     _sig(lib, "zc_v2_decode_nibble", P, P, L, P, P)
     _sig(lib, "zc_v2_decode_ctas", P, P, L, P, I, P)
-    _sig(lib, "zc_v1_encode_split", P, L, P, P, I, P, P, P, P, P, L, P)
-    _sig(lib, "zc_v1_encode_fused", P, L, P, I, P, P, P, L, P, P, L, P)
+    _sig(lib, "zc_v1_encode_split", P, L, P, P, I, P, P, P, P, P, P, L, P)
+    _sig(lib, "zc_v1_totals_words", L, I)
+    if hasattr(lib, "zc_v1_totals_words"):
+        lib.zc_v1_totals_words.restype = L
+    _sig(lib, "zc_v1_encode_fused", P, L, P, I, P, P, P, L, P, P, P, L, P)
     _sig(lib, "zc_v1_decode_split", P, P, P, P, I, L, P, P, P, L, L, P)
     _sig(lib, "zc_v1_decode_fused", P, P, P, I, L, P, L, L, P)
     _sig(lib, "zc_v1_base_from_std", P, L, P, P)

@@ -552,7 +552,9 @@ int adamw_launch(void* p, void* g, void* m, void* v, int64_t n, float lr, float 
                                       reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15) == 0);
   if (vec) {
     const int64_t nvec = n / 8;
-    const int grid = (int)std::min<int64_t>((nvec + 255) / 256, (int64_t)sm_count() * 8);
+    // a few dozen CTAs per SM that follow one another in address order: 10^9 elements take 2301 us, 2424 with one
+    // wave whose CTAs stride through seven buffers at their own pace
+    const int grid = (int)std::min<int64_t>((nvec + 511) / 512, (int64_t)sm_count() * 64);
     adamw_vec_kernel<TP, TG, TS><<<grid, 256, 0, st>>>((TP*)p, (TG*)g, (TS*)m, (TS*)v, nvec, lr, b1, b2, eps, wd,
                                                         bc1, rs, zg, guard);
   } else {
@@ -645,7 +647,7 @@ int zc_swiglu_fwd(const void* gu, void* out, int64_t T, int F, cudaStream_t st) 
   if (F % 8) return ERR_UNSUPPORTED;
   const int64_t total = T * (F / 8);
   if (total == 0) return 0;
-  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
+  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 128);
   zc::swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const bf16*)gu, (bf16*)out, T, F);
   return zc::launch_status();
 }
@@ -654,7 +656,7 @@ int zc_swiglu_bwd(const void* gu, const void* dy, void* dgu, int64_t T, int F, c
   if (F % 8) return ERR_UNSUPPORTED;
   const int64_t total = T * (F / 8);
   if (total == 0) return 0;
-  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
+  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 128);
   zc::swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const bf16*)gu, (const bf16*)dy, (bf16*)dgu, T, F);
   return zc::launch_status();
 }

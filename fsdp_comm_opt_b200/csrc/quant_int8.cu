@@ -243,7 +243,9 @@ int dequantise(const uint8_t* gathered, int64_t stride, int world, int64_t n, vo
   const bool ok = ((reinterpret_cast<uintptr_t>(gathered) | (uintptr_t)stride) & 15) == 0 &&
                   reinterpret_cast<uintptr_t>(out) % sizeof(T) == 0;
   const int64_t units = (n + 7) / 8;
-  const int64_t most = std::max<int64_t>(1, (int64_t)sm_count() * 8 / world);
+  // 32 CTAs per SM (four waves): 108 us for the eight ranks above, 121 with one wave, which reads too many pages
+  // at a time
+  const int64_t most = std::max<int64_t>(1, (int64_t)sm_count() * 32 / world);
   if (ok) {
     const dim3 grid((unsigned)std::min<int64_t>((units + THREADS - 1) / THREADS, most), world);
     dequant_kernel<T><<<grid, THREADS, 0, st>>>(gathered, stride, n, (T*)out);

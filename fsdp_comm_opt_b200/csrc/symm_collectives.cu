@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(256, 3) symm_all_gather_kernel(const AgArgs a)
     unsigned long long pushed = 0;
     uint32_t hint = 0xFFFFFFFFu;  // window of the previous chunk this warp encoded
     int hint_esc = 0;
+    const V2Lane vl(lane);
     for (long long g = blockIdx.x; g < ngroups; g += a.push_ctas) {
       for (int it = 0; it < gc / 8; ++it) {
         const long long c = g * gc + it * 8 + warp;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(256, 3) symm_all_gather_kernel(const AgArgs a)
         LaneSplit s;
         split_lane(li, s);
         const uint32_t hdr = WIRE == 2 ? v2_encode_chunk_nibble(s, srec[warp] - 1024, lane)
-                                       : v2_encode_chunk_hint<false>(s, srec[warp] - 1024, lane, hint, hint_esc);
+                                       : v2_encode_chunk_hint<false>(s, srec[warp] - 1024, lane, vl, hint, hint_esc);
         __syncwarp();
         const int used = v2_record_bytes(hdr);
         if (!ZC_SLOT_OK(L, c, used, a.local, L.rank)) {
@@ -456,6 +457,7 @@ __global__ void __launch_bounds__(256, 2) symm_reduce_scatter_kernel(const RsArg
     unsigned long long pushed = 0;
     uint32_t hint = 0xFFFFFFFFu;
     int hint_esc = 0;
+    const V2Lane vl(lane);
     // work item = (destination, group); destinations interleaved so all links are busy
     const long long items = ngroups * (L.world - 1);
     for (long long i = blockIdx.x; i < items; i += a.push_ctas) {
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(256, 2) symm_reduce_scatter_kernel(const RsArg
         LaneSplit s;
         split_lane(li, s);
         const uint32_t hdr = WIRE == 2 ? v2_encode_chunk_nibble(s, srec[warp] - 1024, lane)
-                                       : v2_encode_chunk_hint<false>(s, srec[warp] - 1024, lane, hint, hint_esc);
+                                       : v2_encode_chunk_hint<false>(s, srec[warp] - 1024, lane, vl, hint, hint_esc);
         __syncwarp();
         const int used = v2_record_bytes(hdr);
         if (!ZC_SLOT_OK(L, c, used, a.local, q)) {

@@ -137,6 +137,55 @@ def test_v1_gather_protocol_unpad_and_unpad_v():
     assert torch.equal(bits(out2), bits(torch.cat(xs[::-1])))
 
 
+@pytest.mark.parametrize("orig,works,off,base", [(4095, 3, 0, 116), (4097, 9, 1, 116), (33000, 5, 3, 130), (20001, 2, 7, 252),
+                                                (5_000_003, 3, 5, 116), (9_000_001, 1, 8, 118)])
+def test_v1_packed_works_at_any_alignment(orig, works, off, base):
+    """Works packed back to back at odd element offsets (loads and stores cut out of 16-byte pieces), several
+    chunks per warp, outliers from none to all: bytes equal to the scalar codec's, round trip into a buffer that
+    starts ``off`` elements in."""
+    torch.manual_seed(orig)
+    x = torch.cat([torch.zeros(off, dtype=torch.bfloat16, device=DEV)] + [
+        torch.cat([gauss(orig - orig // 4, seed=w), rand_bits(orig // 4, seed=w)]) for w in range(works)])[off:]
+    per = codec.pad_to_block(orig)
+
+    def encode(v):
+        dev = v.device
+        n_8 = torch.full((works,), per, dtype=torch.int32, device=dev)
+        on = torch.full((works,), orig, dtype=torch.int32, device=dev)
+        bases = torch.full((256,), base, dtype=torch.int32, device=dev)
+        det = torch.zeros(works * codec.v1_det_bytes(per), dtype=torch.uint8, device=dev)
+        esc = torch.zeros(works * codec.align128(per), dtype=torch.uint8, device=dev)
+        gc = torch.zeros(works, dtype=torch.int32, device=dev)
+        hz.compress_split_store_pad(v, n_8, on, bases, det, torch.zeros(works * per, dtype=torch.uint8, device=dev), esc,
+                                    gc, works * per, works)
+        return n_8, det, esc, gc
+
+    n_8, det, esc, gc = encode(x)
+    _, detc, escc, gcc = encode(x.cpu())
+    assert torch.equal(gc.cpu(), gcc) and torch.equal(det.cpu(), detc)
+    at = 0
+    for c in gcc.tolist():
+        assert torch.equal(esc[at:at + c].cpu(), escc[at:at + c])
+        at += codec.align128(c)
+    out = torch.full((off + works * orig + 16,), 3.0, dtype=torch.bfloat16, device=DEV)
+    out_off = torch.tensor([off + w * orig for w in range(works)], dtype=torch.int32, device=DEV)
+    on = torch.full((works,), orig, dtype=torch.int32, device=DEV)
+    hz.decompress_split_store_unpad_v(det, esc, n_8, gc, out_off, on, out, works * per, works)
+    assert torch.equal(bits(out[off:off + works * orig]), bits(x))
+    assert bool((out[:off] == 3.0).all()) and bool((out[off + works * orig:] == 3.0).all())
+
+
+@pytest.mark.parametrize("n", [1, 7, 4095, 4096, 100_001, 3_000_003])
+def test_v1_base_statistic_sizes(n):
+    for scale in (0.02, 3.0):
+        x = gauss(n, seed=n) * (scale / 0.02)
+        got = torch.zeros(1, dtype=torch.int32, device=DEV)
+        codec.v1_base_from_std(x, got)
+        std = x.double().std().item() if n > 1 else 0.0
+        want = math.floor(math.log2(max(std, 1e-30)) - 5.35 + 127.0)
+        assert int(got) == min(max(want, 0), 255)
+
+
 def test_v1_pad_variant_and_fused_layout():
     origs = [100, 4096, 7168, 1]
     xs = [rand_bits(o, seed=i) for i, o in enumerate(origs)]
