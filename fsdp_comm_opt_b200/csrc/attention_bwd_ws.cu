@@ -1,6 +1,5 @@
-// Causal GQA attention backward for sm_100a.  Two kernels: the warp-specialised kernel below (head
-// dimension 64, and 128 with ZC_ATTN_BWD=ws) and, further down, the key-row kernel that is the default
-// for head dimension 128.
+// Causal GQA attention backward for sm_100a.  Two kernels: the warp-specialised kernel below
+// (ZC_ATTN_BWD=ws) and, further down, the key-row kernel that is the default.
 //
 // One CTA (320 threads) per (128-key block, kv head, batch); it loops over the query heads of the
 // group and over the query blocks at or below the diagonal, with dK and dV accumulating in TMEM.
@@ -21,6 +20,7 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "attn_sm100.cuh"
 #include "launch_util.h"
 #include "umma.cuh"
 
@@ -83,7 +83,6 @@ struct BwdParams {
   int64_t dks0, dks1, dks2, dvs0, dvs1, dvs2;
   float scale;
   int* status;
-  long long* trace;  // null, or [3][256][8] SM-clock stamps written by CTA 0 of the key-row kernel
 };
 
 template <int D>
@@ -344,7 +343,6 @@ struct Scratch {
   int* status = nullptr;
 };
 static Scratch g_scratch[64];
-static long long* g_trace = nullptr;
 
 __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ o,
                                                     const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
@@ -387,409 +385,411 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
   }
 }
 
-// fp32 accumulator kept transposed, [B, H, D, Sp] (queries contiguous, Sp = S rounded up to 4 so
-// that every stride is a multiple of 16 bytes), viewed as (S, D, H, B); box = 32 queries x 128 dims
-static bool make_map_dq_t(CUtensorMap* m, const void* base, int D, int H, int S, int Sp, int B) {
-  EncodeFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[4] = {(cuuint64_t)S, (cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)Sp * 4, (cuuint64_t)D * Sp * 4, (cuuint64_t)H * D * Sp * 4};
-  cuuint32_t box[4] = {32, (cuuint32_t)D, 1, 1};
-  cuuint32_t el[4] = {1, 1, 1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, strides, box, el,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) fprintf(stderr, "[zc_attn_bwd] transposed fp32 tensor map failed (%d)\n", (int)r);
-  return r == CUDA_SUCCESS;
-}
-
-// acc [B, H, D, Sp] fp32 -> dq [B, S, H, D] bf16 (element strides s_b, s_s, s_h): tiles of 32 queries
-// x 64 dims transposed through shared memory (128-byte rows on both sides);
-// grid (ceil(S/32), D/64, B*H), block (32, 8)
-__global__ void __launch_bounds__(256) dq_convert_t_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                                           int S, int Sp, int H, int D, int64_t s_b, int64_t s_s,
-                                                           int64_t s_h) {
-  __shared__ float tile[64][33];
-  const int q0 = blockIdx.x * 32, d0 = blockIdx.y * 64;
-  const int b = blockIdx.z / H, h = blockIdx.z % H;
-  const float* src = acc + ((int64_t)blockIdx.z * D + d0) * Sp + q0;
-  const bool qok = q0 + (int)threadIdx.x < S;
+// delta[b, h, s] = sum_d o * dout and the cleared fp32 accumulator of dQ in one pass: D / 8 threads a (row, head), 16
+// bytes of each input and 32 of the accumulator a thread.  Bound by HBM; 4096 x 32 x 128: 20.5 us, with a warp a
+// (row, head), four-byte loads and a memset 28.5 + 12.2.
+template <int D>
+__global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
+                                                         float* __restrict__ delta, float4* __restrict__ dq_acc, int S,
+                                                         int Hq, int64_t total) {
+  constexpr int T = D / 8;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  float acc = 0.f;
+  if (i < total * T) {
+    const uint4 a = __ldg(o + i), g = __ldg(dout + i);
+    dq_acc[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    dq_acc[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-  for (int dy = threadIdx.y; dy < 64; dy += 8) tile[dy][threadIdx.x] = qok ? src[(int64_t)dy * Sp + threadIdx.x] : 0.f;
-  __syncthreads();
-#pragma unroll
-  for (int qy = threadIdx.y; qy < 32; qy += 8) {
-    if (q0 + qy < S) {
-      const __nv_bfloat162 v = __floats2bfloat162_rn(tile[2 * threadIdx.x][qy], tile[2 * threadIdx.x + 1][qy]);
-      *reinterpret_cast<__nv_bfloat162*>(dq + b * s_b + (int64_t)(q0 + qy) * s_s + h * s_h + d0 + 2 * threadIdx.x) = v;
+    for (int k = 0; k < 4; ++k) {
+      const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&av[k]));
+      const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv[k]));
+      acc += x.x * y.x + x.y * y.y;
     }
   }
+#pragma unroll
+  for (int k = T / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+  if (i < total * T && threadIdx.x % T == 0) {
+    const int64_t row = i / T, bs = row / Hq, b = bs / S;
+    delta[(b * Hq + row % Hq) * S + bs % S] = acc;
+  }
+}
+
+// acc [rows, Hq, D] fp32 -> dq bf16 (16-byte aligned, element strides multiples of 8): eight elements a thread.
+// Bound by HBM; 4096 x 32 x 128: 24 us with four elements and 64-bit divisions a thread, 13 so.
+template <int D>
+__global__ void __launch_bounds__(256) dq_convert8_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+                                                          int64_t units, uint32_t Hq, int64_t s_bs, int64_t s_h) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= units) return;
+  const float4 a = __ldcs(acc + 2 * i), c = __ldcs(acc + 2 * i + 1);
+  const uint32_t rh = (uint32_t)(i / (D / 8)), r = rh / Hq, h = rh - r * Hq;
+  uint4 v;
+  __nv_bfloat162 p0 = __floats2bfloat162_rn(a.x, a.y), p1 = __floats2bfloat162_rn(a.z, a.w);
+  __nv_bfloat162 p2 = __floats2bfloat162_rn(c.x, c.y), p3 = __floats2bfloat162_rn(c.z, c.w);
+  v.x = *reinterpret_cast<uint32_t*>(&p0);
+  v.y = *reinterpret_cast<uint32_t*>(&p1);
+  v.z = *reinterpret_cast<uint32_t*>(&p2);
+  v.w = *reinterpret_cast<uint32_t*>(&p3);
+  *reinterpret_cast<uint4*>(dq + r * s_bs + h * s_h + (i % (D / 8)) * 8) = v;
 }
 
 }  // namespace bws
 
 // =================================================================================================
-// Key-row ("transposed") backward for head dimension 128: the default.
+// Key-row ("transposed") backward, head dimensions 64 and 128: the default.
 //
-// The kernel above keeps one Q/dO tile in flight and spends most of an iteration waiting (loads,
-// then MMAs, then the element-wise pass, then the dQ drain, one after the other).  This one works on
-// 64 queries per iteration and computes everything with the KEY index on the TMEM lane axis:
-//   S^T  = K  Q^T   (128 keys x 64 queries)        dP^T = V dO^T
-//   P^T  = exp2(S^T c - lse[q]),  dS^T = P^T (dP^T - delta[q]) scale      (bf16, K-major A tiles)
-//   dV  += P^T dO,  dK += dS^T Q                   (accumulate in TMEM over all iterations)
-//   dQ^T = K^T dS^T (128 dims x 64 queries)        -> staged in shared memory as it is and added by
-//                                                     bulk tensor reductions to an fp32 accumulator
-//                                                     that is kept transposed ([B, Hq, D, S])
-// so a 64-query tile is half the size (two Q/dO stages, two P^T/dS^T stages and the dQ staging
-// buffer fit beside K and V in 224 KB) and no operand needs a transpose.  The S^T/dP^T accumulators
-// are read into registers at once and released before the arithmetic, so the tensor core computes
-// iteration i+1's scores during iteration i's element-wise pass, and iteration i's dQ^T is drained
-// while iteration i+1's MMAs run.
-// TMEM (512 columns): dK 128 | dV 128 | S^T 64 | dP^T 64 | dQ^T 2 x 64.
+// One CTA (512 threads) per (128-key block, kv head, batch); 128 queries an iteration, with the KEY index on the
+// TMEM lanes:
+//   S^T  = K Q^T,  dP^T = V dO^T                     (128 keys x 128 queries each)
+//   P^T  = exp2(S^T c - lse[q])                      bf16 into TMEM, over the scores that it came from
+//   dS^T = P^T (dP^T - delta[q]) scale               bf16 into shared memory
+//   dV  += P^T dO (A from TMEM),  dK += dS^T Q       (accumulate in TMEM over all iterations)
+//   dQ   = dS K                                      (dS^T read MN-major; at head dimension 128 over dP^T)
+// Roles, by warpgroup (registers are moved with setmaxnreg, 48 + 2 x 152 + 160 = the launch's 4 x 128 a thread):
+//   0     warp 0: TMA producer (K, V once, then Q two iterations ahead and dO one or two), warp 1: MMA issuer,
+//         warp 2: lse and delta of the iteration's queries into shared memory
+//   1, 2  P^T and dS^T; a thread owns a key row and 64 of the queries
+//   3     drains dQ: TMEM -> registers -> 16 KB pieces of 32 dimensions in shared memory -> bulk tensor reduction
+//         into the fp32 accumulator [B, S, Hq, D]
+// Order of the MMAs: dV(i), S(i+1), dQ(i), dK(i), dP(i+1): the exponentials of i+1 run beside dQ(i) and dK(i), dS(i+1)
+// beside dV(i+1) and S(i+2), the drain of dQ(i) beside dK(i).  (At head dimension 64, where dQ has columns of its own,
+// dP(i+1) ahead of dQ(i) was slower: 1927 against 1754 us for 2 x 8192 keys and 25 heads.)
+// What bounds it: the issue of the MMAs, which take 70 to 110 clocks each whatever their width (an operand's bytes
+// move at about 70 B per clock from shared memory), 40 of them an iteration at head dimension 128 and 32 at 64.  With 64
+// queries an iteration and P^T in shared memory it was 64 for the same work.  16384 keys, 32 / 8 heads of 128: 7200 ->
+// 4884 us; 8 x 1024 keys, 25 heads of 64: 259 -> 180.
 // CTAs are numbered heaviest first (key block 0 has the most query blocks below the diagonal).
 namespace bkt {
 using namespace bws;
 
-// Phase stamps for kernel development: compiled in only with -DZC_PHASE_TRACE
-#ifdef ZC_PHASE_TRACE
-#define ZC_BTRACE(slot, i, k)                                                                      \
-  do {                                                                                             \
-    if (p.trace && blockIdx.x == 0 && (i) < 256) p.trace[((slot) * 256 + (i)) * 8 + (k)] = clock64(); \
-  } while (0)
-#else
-#define ZC_BTRACE(slot, i, k) \
-  do {                        \
-  } while (0)
-#endif
+template <int D>
+struct Cfg {
+  static constexpr int TILE = 128 * D * 2;               // K, V, Q or dO
+  static constexpr int DO_STAGES = D == 128 ? 1 : 2;
+  static constexpr bool ALIAS = D == 128;                // dQ takes the columns of dP^T
+  static constexpr int TILES = 4 + DO_STAGES;            // K, V, 2 Q, dO
+  static constexpr int DS = TILES * TILE, STAGE = DS + 32768, STAT = STAGE + 32768, BARS = STAT + 2048;
+  static constexpr int SMEM = BARS + 256;
+  static constexpr int TM_S = 0, TM_DP = 128, TM_DK = 256, TM_DV = 256 + D, TM_DQ = ALIAS ? TM_DP : 256 + 2 * D;
+};
+struct Bars {
+  uint64_t kv_full, q_full[2], q_empty[2], do_full[2], do_empty[2], s_full, dp_full, p_full, ds_full, dv_done, dq_full,
+      dq_empty, stat_full[2], stat_empty[2], all_done;
+  uint32_t tmem_base;
+  int abort;
+};
+static_assert(sizeof(Bars) <= 256, "the barriers' space");
 
-constexpr int QB = 64;  // queries per iteration
-
-// barrier over `nthreads` threads that also ORs a predicate: every participant gets the same answer,
-// so all compute threads leave the loop at the same barrier when one of them timed out
-__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
-  uint32_t r;
+// MMAs whose shared-memory operands are given by the low words of their descriptors: 1024 bytes between groups of eight
+// rows, SWIZZLE_128B and the sm_100 version field are the same for all of this kernel's
+constexpr uint32_t DESC_HI = (1024 >> 4) | 1u << 14 | 2u << 29;
+__device__ __forceinline__ void mma_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 p, %3, 0;\n"
-      "bar.red.or.pred q, %1, %2, p;\n"
-      "selp.u32 %0, 1, 0, q;\n"
-      "}\n"
-      : "=r"(r)
-      : "r"(id), "r"(nthreads), "r"((uint32_t)pred)
+      ".reg .pred p;\n"
+      ".reg .b64 da, db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "mov.b64 da, {%1, %5};\n"
+      "mov.b64 db, {%2, %5};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+      "}\n" ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(DESC_HI)
       : "memory");
-  return r != 0;
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t tmem_a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b64 db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "mov.b64 db, {%2, %5};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+      "}\n" ::"r"(d), "r"(tmem_a), "r"(b), "r"(idesc), "r"(accumulate), "n"(DESC_HI)
+      : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
 
-__global__ void __launch_bounds__(352, 1) attn_bwd_kt_kernel(const __grid_constant__ CUtensorMap mapQ,
+template <int D>
+__global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_constant__ CUtensorMap mapQ,
                                                              const __grid_constant__ CUtensorMap mapK,
                                                              const __grid_constant__ CUtensorMap mapV,
                                                              const __grid_constant__ CUtensorMap mapdO,
                                                              const __grid_constant__ CUtensorMap mapdQ,
-                                                             const BwdParams p, const int nkb) {
-  constexpr int D = 128;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;                 // [128 keys x 128] bf16, two 64-column slabs of 16 KB
-  uint8_t* sV = smem + 32768;
-  uint8_t* sQ = smem + 65536;         // 2 stages x [64 queries x 128], two slabs of 8 KB each
-  uint8_t* sdO = smem + 98304;        // 2 stages
-  uint8_t* sP = smem + 131072;        // 2 stages x [128 keys x 64 queries] bf16 (one slab)
-  uint8_t* sdS = smem + 163840;       // 2 stages
-  uint8_t* sStage = smem + 196608;    // dQ staging: per query half, [128 dims x 32 queries] fp32, swizzled
-  __shared__ uint64_t kv_full, qdo_full[2], qdo_empty[2], sdp_full, sdp_empty, pds_full[2], pds_empty[2], dq_full[2],
-      dq_empty[2];
-  __shared__ uint32_t tmem_base;
-  __shared__ volatile int s_abort;
-  __shared__ __align__(16) float s_stat[2][128];  // per stage: lse * log2(e) of the 64 queries, then their delta * scale
+                                                             const BwdParams p) {
+  using C = Cfg<D>;
+  // No static shared memory: the dynamic part starts at the (1024-byte aligned) beginning of the block's window
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) {
+    if (threadIdx.x == 0) atomicExch(p.status, 9);
+    return;
+  }
+  uint8_t* sK = smem;  // [128 keys x D] bf16, D / 64 column slabs of 16 KB
+  uint8_t* sV = smem + C::TILE;
+  uint8_t* sQ = smem + 2 * C::TILE;
+  uint8_t* sdO = smem + 4 * C::TILE;
+  uint8_t* sdS = smem + C::DS;        // [128 keys x 128 queries] bf16, two slabs of 64 queries
+  uint8_t* sStage = smem + C::STAGE;  // 2 x [128 queries x 32 dims] fp32
+  float* s_stat = reinterpret_cast<float*>(smem + C::STAT);  // per stage: -lse * log2(e) of 128 queries, their -delta * scale
+  Bars& m = *reinterpret_cast<Bars*>(smem + C::BARS);
+  volatile int* s_abort = &m.abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per_jb = p.Hkv * p.B;
   const int jb = blockIdx.x / per_jb;
   const int hk = (blockIdx.x % per_jb) % p.Hkv, b = (blockIdx.x % per_jb) / p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int k0 = jb * 128;
-  const int nq64 = (p.S + QB - 1) / QB;
-  const int nqi = nq64 - 2 * jb;  // query blocks at or below this key block's diagonal
-  const int iters = group * nqi;
-  (void)nkb;
+  const int nqb = (p.S + 127) / 128;
+  const int iters = group * (nqb - jb);  // query blocks at or below this key block's diagonal
   if (tid == 0) {
-    mbar_init(&kv_full, 1);
-    mbar_init(&sdp_full, 1);
-    mbar_init(&sdp_empty, 1);
+    mbar_init(&m.kv_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
-      mbar_init(&pds_full[i], 1);
-      mbar_init(&pds_empty[i], 1);
-      mbar_init(&dq_full[i], 1);
-      mbar_init(&dq_empty[i], 1);
+      mbar_init(&m.q_full[i], 1);
+      mbar_init(&m.q_empty[i], 1);
+      mbar_init(&m.do_full[i], 1);
+      mbar_init(&m.do_empty[i], 1);
+      mbar_init(&m.stat_full[i], 1);
+      mbar_init(&m.stat_empty[i], 8);
     }
+    mbar_init(&m.s_full, 1);
+    mbar_init(&m.dp_full, 1);
+    mbar_init(&m.p_full, 8);
+    mbar_init(&m.ds_full, 8);
+    mbar_init(&m.dv_done, 1);
+    mbar_init(&m.dq_full, 1);
+    mbar_init(&m.dq_empty, 4);
+    mbar_init(&m.all_done, 1);
     mbar_fence_init();
-    s_abort = 0;
+    m.abort = 0;
   }
   if (warp == 1) {
-    tmem_alloc(&tmem_base, 512);
+    tmem_alloc(&m.tmem_base, 512);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tm_dk = tmem_base, tm_dv = tmem_base + 128, tm_st = tmem_base + 256, tm_dp = tmem_base + 320,
-                 tm_dq = tmem_base + 384;
+  const uint32_t tm = m.tmem_base;
+  // bounded wait: parked in hardware, woken when the phase completes, given up after two seconds or when another role
+  // raised the abort flag
+  auto role_wait = [&](uint64_t* bar, uint32_t parity) -> bool { return mbar_wait_parked(bar, parity, s_abort); };
 
-  // bounded wait of the single-thread roles: parked in hardware, woken when the phase completes,
-  // given up after two seconds or when another role raised the abort flag
-  auto role_wait = [&](uint64_t* bar, uint32_t parity) -> bool { return mbar_wait_parked(bar, parity, &s_abort); };
-
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(&kv_full, 2 * 32768);
+  if (warp < 4) {
+    regs_dec<48>();
+    if (warp == 0 && lane == 0) {
+      mbar_expect_tx(&m.kv_full, 2 * C::TILE);
 #pragma unroll
-      for (int sl = 0; sl < 2; ++sl) {
-        tma_load_4d(sK + sl * 16384, &mapK, &kv_full, sl * 64, hk, k0, b);
-        tma_load_4d(sV + sl * 16384, &mapV, &kv_full, sl * 64, hk, k0, b);
+      for (int sl = 0; sl < D / 64; ++sl) {
+        tma_load_4d(sK + sl * 16384, &mapK, &m.kv_full, sl * 64, hk, k0, b);
+        tma_load_4d(sV + sl * 16384, &mapV, &m.kv_full, sl * 64, hk, k0, b);
       }
-      int h = hk * group, ib = 2 * jb;
+      int h = hk * group, ib = jb;
       for (int i = 0; i < iters; ++i) {
-        const int st = i & 1;
-        const int q0 = ib * QB;
-        if (!role_wait(&qdo_empty[st], ((i >> 1) & 1) ^ 1)) { s_abort = 1; break; }
-        mbar_expect_tx(&qdo_full[st], 2 * 16384);
+        const int sq = i & 1, sd = i % C::DO_STAGES;
+        if (!role_wait(&m.q_empty[sq], ((i >> 1) & 1) ^ 1)) { *s_abort = 1; break; }
+        mbar_expect_tx(&m.q_full[sq], C::TILE);
 #pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-          tma_load_4d(sQ + st * 16384 + sl * 8192, &mapQ, &qdo_full[st], sl * 64, h, q0, b);
-          tma_load_4d(sdO + st * 16384 + sl * 8192, &mapdO, &qdo_full[st], sl * 64, h, q0, b);
-        }
-        if (++ib == nq64) { ib = 2 * jb; ++h; }
+        for (int sl = 0; sl < D / 64; ++sl)
+          tma_load_4d(sQ + sq * C::TILE + sl * 16384, &mapQ, &m.q_full[sq], sl * 64, h, ib * 128, b);
+        if (!role_wait(&m.do_empty[sd], ((i / C::DO_STAGES) & 1) ^ 1)) { *s_abort = 1; break; }
+        mbar_expect_tx(&m.do_full[sd], C::TILE);
+#pragma unroll
+        for (int sl = 0; sl < D / 64; ++sl)
+          tma_load_4d(sdO + sd * C::TILE + sl * 16384, &mapdO, &m.do_full[sd], sl * 64, h, ib * 128, b);
+        if (++ib == nqb) { ib = jb; ++h; }
       }
-    }
-  } else if (warp == 1 || warp == 10) {
-    if (lane == 0) {
-      const uint32_t id_st = idesc_bf16(128, QB, MAJOR_K, MAJOR_K);     // S^T, dP^T
-      const uint32_t id_kv = idesc_bf16(128, D, MAJOR_K, MAJOR_MN);     // dV, dK
-      const uint32_t id_dq = idesc_bf16(128, QB, MAJOR_MN, MAJOR_MN);   // dQ^T
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO), aP = smem_u32(sP),
-                     adS = smem_u32(sdS);
-      // Operand descriptors at offset 0, built once; an MMA adds (byte offset >> 4) to the start-address
-      // field (shared memory is below 256 KB, the 14-bit field never carries).  The S^T / dP^T / dQ^T
-      // MMAs are 32 clocks of tensor work each: the issuing thread cannot afford to build two
-      // descriptors between them.
-      const uint64_t dK_k = smem_desc(aK, 16, 1024), dV_k = smem_desc(aV, 16, 1024);       // K-major, 16 KB slabs
-      const uint64_t dQ_k = smem_desc(aQ, 16, 1024), ddO_k = smem_desc(adO, 16, 1024);     // K-major, 8 KB slabs
-      const uint64_t dP_k = smem_desc(aP, 16, 1024), ddS_k = smem_desc(adS, 16, 1024);     // K-major A operands
-      const uint64_t ddO_mn = smem_desc(adO, 8192, 1024), dQ_mn = smem_desc(aQ, 8192, 1024);  // MN-major B operands
-      const uint64_t dK_mn = smem_desc(aK, 16384, 1024), ddS_mn = smem_desc(adS, 8192, 1024);
-      auto off128 = [](int k) { return (uint64_t)(((k >> 2) * 16384 + (k & 3) * 32) >> 4); };
-      auto off64 = [](int k) { return (uint64_t)(((k >> 2) * 8192 + (k & 3) * 32) >> 4); };
-      bool ok = role_wait(&kv_full, 0);
-      // Two issuers: a tcgen05.mma takes about a hundred cycles to issue whatever its width, so the
-      // 32 MMAs of an iteration are split between warp 1 (S^T, dP^T) and warp 10 (dV, dK, dQ^T).
-      if (warp == 1) {
-        for (int i = 0; i < iters && ok; ++i) {
-          const int st = i & 1;
-          ZC_BTRACE(1, i, 0);
-          if (!(ok = role_wait(&qdo_full[st], (i >> 1) & 1))) break;
-          ZC_BTRACE(1, i, 1);
-          if (i > 0 && !(ok = role_wait(&sdp_empty, (i - 1) & 1))) break;
+    } else if (warp == 1 && lane == 0) {
+      const uint32_t id_s = idesc_bf16(128, 128, MAJOR_K, MAJOR_K);    // S^T, dP^T
+      const uint32_t id_kv = idesc_bf16(128, D, MAJOR_K, MAJOR_MN);    // dV, dK
+      const uint32_t id_dq = idesc_bf16(128, D, MAJOR_MN, MAJOR_MN);   // dQ
+      // Operand descriptors at offset 0; an MMA adds (byte offset >> 4) to the start-address field (shared memory is
+      // below 256 KB, the 14-bit field never carries).  K-major: 16 KB slabs of 64 elements; MN-major: the same slabs.
+      uint32_t dK_k = (uint32_t)smem_desc(smem_u32(sK), 16, 1024), dV_k = (uint32_t)smem_desc(smem_u32(sV), 16, 1024);
+      uint32_t dQ_k = (uint32_t)smem_desc(smem_u32(sQ), 16, 1024), ddO_k = (uint32_t)smem_desc(smem_u32(sdO), 16, 1024);
+      uint32_t ddS_k = (uint32_t)smem_desc(smem_u32(sdS), 16, 1024);
+      constexpr uint32_t MN = ((16384 - 16) >> 4) << 16;  // added, K-major -> MN-major: the slab stride
+      auto off_k = [](int k) { return (uint32_t)(((k >> 2) * 16384 + (k & 3) * 32) >> 4); };
+      auto off_mn = [](int k) { return (uint32_t)((k * 2048) >> 4); };
+      auto issue_s = [&](int i) {  // S^T(i)
+        const uint32_t dq = dQ_k + (uint32_t)((i & 1) * (C::TILE >> 4));
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) mma_ss(tm + C::TM_S, dK_k + off_k(k), dq + off_k(k), id_s, k != 0);
+        mma_commit(&m.s_full);
+      };
+      auto issue_dp = [&](int i) {  // dP^T(i)
+        const uint32_t dd = ddO_k + (uint32_t)((i % C::DO_STAGES) * (C::TILE >> 4));
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) mma_ss(tm + C::TM_DP, dV_k + off_k(k), dd + off_k(k), id_s, k != 0);
+        mma_commit(&m.dp_full);
+      };
+      auto run = [&]() -> bool {
+        if (!role_wait(&m.kv_full, 0) || !role_wait(&m.q_full[0], 0)) return false;
+        tc_fence_after_sync();
+        issue_s(0);
+        if (!role_wait(&m.do_full[0], 0)) return false;
+        tc_fence_after_sync();
+        issue_dp(0);
+        for (int i = 0; i < iters; ++i) {
+          // the sums with constants are made where they are used, not kept over the loop in registers that are not there
+          asm volatile("" : "+r"(dK_k), "+r"(dV_k), "+r"(dQ_k), "+r"(ddO_k), "+r"(ddS_k));
+          const int sq = i & 1, sd = i % C::DO_STAGES;
+          if (!role_wait(&m.p_full, i & 1)) return false;
           tc_fence_after_sync();
-          ZC_BTRACE(1, i, 2);
-          const uint64_t stg = (uint64_t)(st * (16384 >> 4));
-#pragma unroll
-          for (int k = 0; k < D / 16; ++k) mma_bf16(tm_st, dK_k + off128(k), dQ_k + stg + off64(k), id_st, k != 0);
-#pragma unroll
-          for (int k = 0; k < D / 16; ++k) mma_bf16(tm_dp, dV_k + off128(k), ddO_k + stg + off64(k), id_st, k != 0);
-          mma_commit(&sdp_full);
-          ZC_BTRACE(1, i, 3);
-        }
-      } else {
-        for (int i = 0; i < iters && ok; ++i) {
-          const int st = i & 1, ph = (i >> 1) & 1;
-          // pds_full(i) also tells that S^T(i) and dP^T(i) have completed (the compute threads read
-          // them before writing P^T and dS^T), so this thread's commits cover every reader of Q/dO
-          ZC_BTRACE(2, i, 0);
-          if (!(ok = role_wait(&pds_full[st], ph))) break;
-          ZC_BTRACE(2, i, 1);
-          if (!(ok = role_wait(&dq_empty[st], ph ^ 1))) break;
-          tc_fence_after_sync();
-          ZC_BTRACE(2, i, 2);
-          const uint64_t stg = (uint64_t)(st * (16384 >> 4));
-          // dV += P^T dO and dK += dS^T Q: A = [128 keys x 64 queries] K-major, B = [64 queries x 128] MN-major
-#pragma unroll
-          for (int k = 0; k < QB / 16; ++k)
-            mma_bf16(tm_dv, dP_k + stg + (uint64_t)((k * 32) >> 4), ddO_mn + stg + (uint64_t)((k * 2048) >> 4), id_kv,
-                     (i | k) != 0);
-#pragma unroll
-          for (int k = 0; k < QB / 16; ++k)
-            mma_bf16(tm_dk, ddS_k + stg + (uint64_t)((k * 32) >> 4), dQ_mn + stg + (uint64_t)((k * 2048) >> 4), id_kv,
-                     (i | k) != 0);
-          // dQ^T = K^T dS^T: A = K read MN-major (M = head dim), B = dS^T read MN-major (N = queries)
+          // dV += P^T dO: the thread that owns queries [64 g, 64 g + 64) keeps its P at column 64 g
+          const uint32_t dd = (ddO_k + MN) + (uint32_t)(sd * (C::TILE >> 4));
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            mma_bf16(tm_dq + st * QB, dK_mn + (uint64_t)((k * 2048) >> 4), ddS_mn + stg + (uint64_t)((k * 2048) >> 4),
-                     id_dq, k != 0);
-          mma_commit(&dq_full[st]);
-          mma_commit(&pds_empty[st]);
-          mma_commit(&qdo_empty[st]);
-          ZC_BTRACE(2, i, 3);
-        }
-      }
-      if (!ok) s_abort = 1;
-    }
-  } else {
-    const int ct = tid - 64;               // 0..255
-    const int quarter = warp & 3;          // TMEM lane quarter this warp may access
-    const int half = (warp - 2) >> 2;      // which 32 of the 64 query columns
-    const int r = quarter * 32 + lane;     // key row of the tile == TMEM lane (head dim index for dQ^T)
-    const int key = k0 + r;
-    const uint32_t lane_base = (uint32_t)(quarter * 32);
-    const int c0 = half * 32;
-    const float sl2 = p.scale * LOG2E;
-    // threads 0..63 fetch lse, 64..127 fetch delta of the next iteration's queries (one value each)
-    auto fetch = [&](int h, int ib, bool valid) -> float {
-      if (ct >= 128 || !valid) return 0.f;
-      const int q = ib * QB + (ct & 63);
-      if (q >= p.S) return 0.f;
-      const int64_t idx = ((int64_t)b * p.Hq + h) * p.S + q;
-      return ct < 64 ? __ldg(p.lse + idx) * LOG2E : __ldg(p.delta + idx) * p.scale;
-    };
-    // (head, 64-query block) of the current and of the previous iteration, advanced without divisions
-    int cur_h = hk * group, cur_ib = 2 * jb, prev_h = 0, prev_q0 = 0;
-    float pre = fetch(cur_h, cur_ib, iters > 0);
-    bool fail = false, aborted = false;
-    for (int i = 0; i <= iters; ++i) {
-      if (i < iters) {
-        const int st = i & 1, ph = (i >> 1) & 1;
-        // ---- A: scores and dP of this thread's key row into registers, then release the accumulators
-        if (tid == 64) ZC_BTRACE(0, i, 0);
-        if (!mbar_wait_parked(&sdp_full, i & 1, &s_abort)) fail = true;
-        tc_fence_after_sync();
-        if (tid == 64) ZC_BTRACE(0, i, 1);
-        uint32_t rs[32], rp[32];
-        tmem_ld32(tmem_addr(tm_st, lane_base, c0), rs);
-        tmem_ld32(tmem_addr(tm_dp, lane_base, c0), rp);
-        if (ct < 128) s_stat[st][ct] = pre;
-        tmem_ld_wait();
-        tc_fence_before_sync();
-        if (named_bar_or(1, 256, fail || s_abort)) { aborted = true; break; }
-        if (tid == 64) mbar_arrive(&sdp_empty);
-        __syncwarp();
-        if (tid == 64) ZC_BTRACE(0, i, 2);
-        {
-          int nh = cur_h, nib = cur_ib + 1;
-          if (nib == nq64) { nib = 2 * jb; ++nh; }
-          pre = fetch(nh, nib, i + 1 < iters);
-        }
-        // ---- B: P^T and dS^T ------------------------------------------------------------------
-        const int q0 = cur_ib * QB;
-        const bool diag = (q0 < k0 + 128) || (q0 + QB > p.S) || (k0 + 128 > p.S);
-        const float4* st_l = reinterpret_cast<const float4*>(&s_stat[st][c0]);
-        const float4* st_d = reinterpret_cast<const float4*>(&s_stat[st][64 + c0]);
-        uint32_t pk[16], dk_[16];
-        // two copies of the loop, so that blocks away from the diagonal carry no masking
-        // instructions at all (predicated-off instructions still take issue slots)
-        auto elementwise = [&](auto masked) {
-#pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const float4 l4 = st_l[g], d4 = st_d[g];
-            const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-            const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-            float e[4], ds[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const int c = g * 4 + t;
-              float ev = exp2f(__uint_as_float(rs[c]) * sl2 - ls[t]);
-              if (decltype(masked)::value) {
-                const int q = q0 + c0 + c;
-                if (key > q || key >= p.S || q >= p.S) ev = 0.f;
-              }
-              e[t] = ev;
-              ds[t] = ev * fmaf(__uint_as_float(rp[c]), p.scale, -dl[t]);
-            }
-            pk[2 * g] = pack_bf16(e[0], e[1]);
-            pk[2 * g + 1] = pack_bf16(e[2], e[3]);
-            dk_[2 * g] = pack_bf16(ds[0], ds[1]);
-            dk_[2 * g + 1] = pack_bf16(ds[2], ds[3]);
+            mma_ts(tm + C::TM_DV, tm + C::TM_S + (uint32_t)((k >> 2) * 64 + (k & 3) * 8), dd + off_mn(k), id_kv, (i | k) != 0);
+          mma_commit(&m.dv_done);
+          mma_commit(&m.do_empty[sd]);
+          if (i + 1 < iters) {  // S^T(i+1) overwrites P^T(i)
+            if (!role_wait(&m.q_full[(i + 1) & 1], ((i + 1) >> 1) & 1) || !role_wait(&m.dv_done, i & 1)) return false;
+            tc_fence_after_sync();
+            issue_s(i + 1);
           }
-        };
-        if (diag) elementwise(std::true_type{});
-        else elementwise(std::false_type{});
-        if (tid == 64) ZC_BTRACE(0, i, 3);
-        if (!mbar_wait_parked(&pds_empty[st], ph ^ 1, &s_abort)) fail = true;  // MMAs of iteration i-2 have read this stage
-        if (tid == 64) ZC_BTRACE(0, i, 4);
-        uint8_t* tp = sP + st * 16384;
-        uint8_t* td = sdS + st * 16384;
+          if (!role_wait(&m.ds_full, i & 1)) return false;
+          if (!C::ALIAS && i > 0 && !role_wait(&m.dq_empty, (i - 1) & 1)) return false;
+          tc_fence_after_sync();
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          *reinterpret_cast<uint4*>(tp + sw128_off(r, half * 4 + j)) =
-              make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-          *reinterpret_cast<uint4*>(td + sw128_off(r, half * 4 + j)) =
-              make_uint4(dk_[4 * j], dk_[4 * j + 1], dk_[4 * j + 2], dk_[4 * j + 3]);
+          for (int k = 0; k < 8; ++k)
+            mma_ss(tm + C::TM_DQ, (ddS_k + MN) + off_mn(k), (dK_k + MN) + off_mn(k), id_dq, k != 0);
+          mma_commit(&m.dq_full);
+          const uint32_t dq = (dQ_k + MN) + (uint32_t)(sq * (C::TILE >> 4));
+#pragma unroll
+          for (int k = 0; k < 8; ++k) mma_ss(tm + C::TM_DK, ddS_k + off_k(k), dq + off_mn(k), id_kv, (i | k) != 0);
+          mma_commit(&m.q_empty[sq]);
+          if (i + 1 < iters) {  // at head dimension 128 dP^T(i+1) overwrites dQ(i)
+            if (!role_wait(&m.do_full[(i + 1) % C::DO_STAGES], ((i + 1) / C::DO_STAGES) & 1)) return false;
+            if (C::ALIAS && !role_wait(&m.dq_empty, i & 1)) return false;
+            tc_fence_after_sync();
+            issue_dp(i + 1);
+          }
         }
-        fence_proxy_async_smem();
-        if (tid == 64) bulk_wait_read0();  // the previous dQ reduction has read the staging buffer
-        __syncwarp();
-        if (named_bar_or(2, 256, fail || s_abort)) { aborted = true; break; }
-        if (tid == 64) mbar_arrive(&pds_full[st]);
-        __syncwarp();
-        if (tid == 64) ZC_BTRACE(0, i, 5);
-      } else {
-        if (tid == 64) bulk_wait_read0();
-        __syncwarp();
-        if (named_bar_or(1, 256, fail || s_abort)) { aborted = true; break; }
-      }
-      if (i > 0) {
-        // ---- C: drain dQ^T of iteration i-1 (its MMAs ran during this iteration's phases A and B)
-        const int j = i - 1, sj = j & 1;
-        if (!mbar_wait_parked(&dq_full[sj], (j >> 1) & 1, &s_abort)) fail = true;
-        tc_fence_after_sync();
-        if (tid == 64) ZC_BTRACE(0, i, 6);
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm_dq + sj * QB, lane_base, c0), rr);
-        tmem_ld_wait();
-        // this thread holds dQ^T[dim r][query c0 .. c0+31]: 128 contiguous bytes of row r of the
-        // staging slab of its query half ([128 dims x 32 queries] fp32, 128-byte swizzle), which is
-        // also the layout of the accumulator ([B, Hq, D, S]: queries contiguous), so the drain is
-        // eight 16-byte stores per thread and no transpose
-        uint8_t* slab = sStage + half * 16384;
+        mma_commit(&m.all_done);
+        return true;
+      };
+      if (!run()) *s_abort = 1;
+    } else if (warp == 2) {
+      int h = hk * group, ib = jb;
+      for (int i = 0; i < iters; ++i) {
+        const int st = i & 1;
+        const int64_t row = ((int64_t)b * p.Hq + h) * p.S;
+        float vl[4], vd[4];
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
-          *reinterpret_cast<uint4*>(slab + sw128_off(r, t)) =
-              make_uint4(rr[4 * t], rr[4 * t + 1], rr[4 * t + 2], rr[4 * t + 3]);
-        fence_proxy_async_smem();
-        tc_fence_before_sync();
-        if (named_bar_or(3, 256, fail || s_abort)) { aborted = true; break; }
-        if (tid == 64) {
-#pragma unroll
-          for (int t = 0; t < 2; ++t) tma_reduce_add_4d(&mapdQ, sStage + t * 16384, prev_q0 + t * 32, 0, prev_h, b);
-          bulk_commit();
-          mbar_arrive(&dq_empty[sj]);
-          ZC_BTRACE(0, i, 7);
+        for (int k = 0; k < 4; ++k) {
+          // queries past the end: P = exp2(0 - inf) = 0
+          const int q = ib * 128 + lane * 4 + k;
+          vl[k] = q < p.S ? -__ldg(p.lse + row + q) * LOG2E : -CUDART_INF_F;
+          vd[k] = q < p.S ? -__ldg(p.delta + row + q) * p.scale : 0.f;
         }
+        const bool ok = role_wait(&m.stat_empty[st], ((i >> 1) & 1) ^ 1);
+        if (!__all_sync(0xffffffffu, ok)) { *s_abort = 1; break; }
+        float4* dst = reinterpret_cast<float4*>(s_stat + st * 256);
+        dst[lane] = make_float4(vl[0], vl[1], vl[2], vl[3]);
+        dst[32 + lane] = make_float4(vd[0], vd[1], vd[2], vd[3]);
         __syncwarp();
+        if (lane == 0) mbar_arrive(&m.stat_full[st]);
+        if (++ib == nqb) { ib = jb; ++h; }
       }
-      prev_h = cur_h;
-      prev_q0 = cur_ib * QB;
-      if (++cur_ib == nq64) { cur_ib = 2 * jb; ++cur_h; }
     }
-    if (tid == 64) bulk_wait0();
-    __syncwarp();
-    if (aborted) s_abort = 1;
-    if (!aborted) {
-      // every MMA into dK / dV has completed: dq_full of the last iteration was committed after them
+  } else if (warp < 12) {
+    regs_inc<152>();
+    const int quarter = warp & 3;          // TMEM lane quarter this warp may access
+    const int half = (warp - 4) >> 2;      // which 64 of the 128 query columns
+    const int r = quarter * 32 + lane;     // key row of the tile == TMEM lane
+    const uint32_t lane_base = (uint32_t)(quarter * 32);
+    const int c0 = half * 64;
+    const uint64_t sl22 = pack2(p.scale * LOG2E, p.scale * LOG2E), scale2 = pack2(p.scale, p.scale);
+    int ib = jb;
+    bool fail = false;
+    for (int i = 0; i < iters; ++i) {
+      const int st = i & 1;
+      fail = !mbar_wait_parked(&m.stat_full[st], (i >> 1) & 1, s_abort) || !mbar_wait_parked(&m.s_full, i & 1, s_abort);
+      if (__any_sync(0xffffffffu, fail || *s_abort)) { fail = true; break; }
+      tc_fence_after_sync();
+      uint32_t e[2][32];
+      tmem_ld32(tmem_addr(tm + C::TM_S, lane_base, c0), e[0]);
+      tmem_ld32(tmem_addr(tm + C::TM_S, lane_base, c0 + 32), e[1]);
+      tmem_ld_wait();
+      const ulonglong2* nl = reinterpret_cast<const ulonglong2*>(s_stat + st * 256 + c0);        // pairs of floats
+      const ulonglong2* nd = reinterpret_cast<const ulonglong2*>(s_stat + st * 256 + 128 + c0);
+#pragma unroll
+      for (int g = 0; g < 16; ++g) {
+        const ulonglong2 l4 = nl[g];
+        uint32_t* v = &e[g >> 3][(g & 7) * 4];
+        float x[4];
+        unpack2(fma2(pack2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl22, l4.x), x[0], x[1]);
+        unpack2(fma2(pack2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl22, l4.y), x[2], x[3]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = __float_as_uint(exp2f(x[k]));
+      }
+      if (ib == jb) {  // the block on the diagonal; keys past the end of the sequence lie below it
+#pragma unroll
+        for (int c = 0; c < 64; ++c)
+          if (r > c0 + c) e[c >> 5][c & 31] = 0u;
+      }
+      uint32_t pk[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        pk[c] = pack_bf16(__uint_as_float(e[c >> 4][(c & 15) * 2]), __uint_as_float(e[c >> 4][(c & 15) * 2 + 1]));
+      tmem_st32(tmem_addr(tm + C::TM_S, lane_base, c0), pk);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m.p_full);
+      __syncwarp();
+      // dp_full(i) also tells that dQ(i-1) and dK(i-1), issued before it, have read dS^T(i-1)
+      fail = !mbar_wait_parked(&m.dp_full, i & 1, s_abort);
+      if (__any_sync(0xffffffffu, fail || *s_abort)) { fail = true; break; }
+      tc_fence_after_sync();
+      uint8_t* slab = sdS + half * 16384;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t dp[32];
+        tmem_ld32(tmem_addr(tm + C::TM_DP, lane_base, c0 + c * 32), dp);
+        tmem_ld_wait();
+        uint32_t ds[16];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const ulonglong2 d4 = nd[c * 8 + g];
+          float x[4];
+          unpack2(mul2(pack2(__uint_as_float(e[c][4 * g]), __uint_as_float(e[c][4 * g + 1])),
+                       fma2(pack2(__uint_as_float(dp[4 * g]), __uint_as_float(dp[4 * g + 1])), scale2, d4.x)), x[0], x[1]);
+          unpack2(mul2(pack2(__uint_as_float(e[c][4 * g + 2]), __uint_as_float(e[c][4 * g + 3])),
+                       fma2(pack2(__uint_as_float(dp[4 * g + 2]), __uint_as_float(dp[4 * g + 3])), scale2, d4.y)), x[2], x[3]);
+          ds[2 * g] = pack_bf16(x[0], x[1]);
+          ds[2 * g + 1] = pack_bf16(x[2], x[3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<uint4*>(slab + sw128_off(r, c * 4 + j)) =
+              make_uint4(ds[4 * j], ds[4 * j + 1], ds[4 * j + 2], ds[4 * j + 3]);
+      }
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&m.ds_full);
+        mbar_arrive(&m.stat_empty[st]);
+      }
+      __syncwarp();
+      if (++ib == nqb) ib = jb;
+    }
+    if (!fail) fail = !mbar_wait_parked(&m.all_done, 0, s_abort);
+    if (__any_sync(0xffffffffu, fail)) {
+      *s_abort = 1;
+    } else {
+      tc_fence_after_sync();
+      const int key = k0 + r;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
-        const uint32_t tmx = which ? tm_dv : tm_dk;
+        const uint32_t tmx = tm + (which ? C::TM_DV : C::TM_DK);
         __nv_bfloat16* dst = which ? p.dv + b * p.dvs0 + (int64_t)key * p.dvs1 + hk * p.dvs2
                                    : p.dk + b * p.dks0 + (int64_t)key * p.dks1 + hk * p.dks2;
 #pragma unroll 1
-        for (int c = half * 64; c < half * 64 + 64; c += 32) {
+        for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
           uint32_t rr[32];
           tmem_ld32(tmem_addr(tmx, lane_base, c), rr);
           tmem_ld_wait();
@@ -807,11 +807,62 @@ __global__ void __launch_bounds__(352, 1) attn_bwd_kt_kernel(const __grid_consta
         }
       }
     }
+  } else {
+    regs_inc<160>();
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;     // query row of the tile == TMEM lane
+    const uint32_t lane_base = (uint32_t)(quarter * 32);
+    int h = hk * group, ib = jb;
+    bool fail = false;
+    for (int i = 0; i < iters; ++i) {
+      fail = !mbar_wait_parked(&m.dq_full, i & 1, s_abort) || *s_abort;
+      // all four warps leave together: they share the named barriers below
+      if (named_bar_or(1, 128, fail)) { fail = true; break; }
+      tc_fence_after_sync();
+      uint32_t rr[D / 32][32];
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) tmem_ld32(tmem_addr(tm + C::TM_DQ, lane_base, c * 32), rr[c]);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m.dq_empty);
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint8_t* buf = sStage + (c & 1) * 16384;
+        if (tid == 384) bulk_wait_read<1>();  // the reduction before the last one has read this buffer
+        named_bar_sync(2, 128);
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+          *reinterpret_cast<uint4*>(buf + sw128_off(r, t)) =
+              make_uint4(rr[c][4 * t], rr[c][4 * t + 1], rr[c][4 * t + 2], rr[c][4 * t + 3]);
+        fence_proxy_async_smem();
+        named_bar_sync(3, 128);
+        if (tid == 384) {
+          tma_reduce_add_4d(&mapdQ, buf, c * 32, h, ib * 128, b);
+          bulk_commit();
+        }
+      }
+      __syncwarp();
+      if (++ib == nqb) { ib = jb; ++h; }
+    }
+    if (tid == 384) bulk_wait0();
+    if (fail) *s_abort = 1;
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && s_abort) atomicExch(p.status, 6);
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if (tid == 0 && *s_abort) atomicExch(p.status, 6);
+  if (warp == 1) tmem_dealloc(tm, 512);
+}
+
+template <int D>
+static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
+                  const CUtensorMap& mdq, const BwdParams& p, cudaStream_t st) {
+  using C = Cfg<D>;
+  if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    return launch_status();
+  attn_bwd_kt_kernel<D><<<(p.S + 127) / 128 * p.Hkv * p.B, 512, C::SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+  return launch_status();
 }
 
 }  // namespace bkt
@@ -866,7 +917,7 @@ int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, c
   p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.dks0 = dks0; p.dks1 = dks1; p.dks2 = dks2; p.dvs0 = dvs0; p.dvs1 = dvs1; p.dvs2 = dvs2;
-  p.scale = scale; p.status = sc.status; p.trace = nullptr;
+  p.scale = scale; p.status = sc.status;
   const int64_t rows = (int64_t)B * S * Hq;
   delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                    delta, B, S, Hq, D);
@@ -885,14 +936,7 @@ int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, c
   return launch_status();
 }
 
-#ifdef ZC_PHASE_TRACE
-// Development builds only: a device buffer of 3 * 256 * 8 int64 (or null) that CTA 0 of later key-row
-// launches fills with SM-clock stamps of its phases.
-void zc_attn_bwd_kt_set_trace(void* buf) { zc::bws::g_trace = (long long*)buf; }
-#endif
-
-// Same argument list as zc_attn_bwd.  Head dimension 128 runs the key-row kernel; 64 falls back to
-// zc_attn_bwd_ws.
+// Same argument list as zc_attn_bwd: the key-row kernel.
 int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                    float* delta, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv, int D, int64_t qs0,
                    int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,
@@ -900,10 +944,7 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
                    int64_t dvs0, int64_t dvs1, int64_t dvs2, float scale, float* dq_acc, cudaStream_t st) {
   using namespace zc;
   using namespace zc::bws;
-  if (D != 128)
-    return zc_attn_bwd_ws(q, k, v, o, dout, lse, delta, dq, dk, dv, B, S, Hq, Hkv, D, qs0, qs1, qs2, ks0, ks1, ks2, vs0,
-                          vs1, vs2, dqs0, dqs1, dqs2, dks0, dks1, dks2, dvs0, dvs1, dvs2, scale, dq_acc, st);
-  if (Hq % Hkv) return ERR_UNSUPPORTED;
+  if ((D != 64 && D != 128) || Hq % Hkv) return ERR_UNSUPPORTED;
   if ((qs1 | qs2 | ks1 | ks2 | vs1 | vs2 | qs0 | ks0 | vs0 | dqs1 | dqs2 | dks1 | dks2 | dvs1 | dvs2 | dqs0 | dks0 | dvs0) % 8)
     return ERR_UNSUPPORTED;
   if (dqs0 != (int64_t)S * dqs1) return ERR_UNSUPPORTED;
@@ -918,30 +959,36 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
     if (cudaMalloc(&sc.status, sizeof(int)) != cudaSuccess) return ERR_BAD_ARG;
     cudaMemset(sc.status, 0, sizeof(int));
   }
-  const int Sp = (S + 3) & ~3;  // row stride of the transposed accumulator: a multiple of 16 bytes
-  const size_t need = (size_t)B * Hq * D * Sp * sizeof(float);
-  cudaMemsetAsync(dq_acc, 0, need, st);
   CUtensorMap mq, mk, mv, mdo, mdq;
-  if (!make_map4(&mq, q, D, Hq, S, B, qs0, qs1, qs2, bkt::QB) || !make_map4(&mk, k, D, Hkv, S, B, ks0, ks1, ks2) ||
+  if (!make_map4(&mq, q, D, Hq, S, B, qs0, qs1, qs2) || !make_map4(&mk, k, D, Hkv, S, B, ks0, ks1, ks2) ||
       !make_map4(&mv, v, D, Hkv, S, B, vs0, vs1, vs2) ||
-      !make_map4(&mdo, dout, D, Hq, S, B, (int64_t)S * Hq * D, (int64_t)Hq * D, D, bkt::QB) ||
-      !make_map_dq_t(&mdq, dq_acc, D, Hq, S, Sp, B))
+      !make_map4(&mdo, dout, D, Hq, S, B, (int64_t)S * Hq * D, (int64_t)Hq * D, D) ||
+      !make_map4_f32(&mdq, dq_acc, D, Hq, S, B))
     return ERR_BAD_ARG;
   BwdParams p;
   p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.dks0 = dks0; p.dks1 = dks1; p.dks2 = dks2; p.dvs0 = dvs0; p.dvs1 = dvs1; p.dvs2 = dvs2;
-  p.scale = scale; p.status = sc.status; p.trace = g_trace;
-  const int64_t rows = (int64_t)B * S * Hq;
-  delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
-                                                                   delta, B, S, Hq, D);
-  const int smem = 7 * 32768 + 1024;
-  static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(bkt::attn_bwd_kt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr = true; }
-  const int nkb = (S + 127) / 128;
-  bkt::attn_bwd_kt_kernel<<<nkb * Hkv * B, 352, smem, st>>>(mq, mk, mv, mdo, mdq, p, nkb);
-  dq_convert_t_kernel<<<dim3((S + 31) / 32, D / 64, B * Hq), dim3(32, 8), 0, st>>>(
-      dq_acc, (__nv_bfloat16*)dq, S, Sp, Hq, D, dqs0, dqs1, dqs2);
+  p.scale = scale; p.status = sc.status;
+  const int64_t rows = (int64_t)B * S * Hq, units = rows * (D / 8);
+  const unsigned ugrid = (unsigned)((units + 255) / 256);
+  if (reinterpret_cast<uintptr_t>(o) & 15) {  // a saved output that came back from a hook at an odd address
+    cudaMemsetAsync(dq_acc, 0, (size_t)rows * D * sizeof(float), st);
+    delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+                                                                     delta, B, S, Hq, D);
+  } else if (D == 128) {
+    delta_zero_kernel<128><<<ugrid, 256, 0, st>>>((const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
+  } else {
+    delta_zero_kernel<64><<<ugrid, 256, 0, st>>>((const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
+  }
+  const int rc = D == 128 ? bkt::launch<128>(mq, mk, mv, mdo, mdq, p, st) : bkt::launch<64>(mq, mk, mv, mdo, mdq, p, st);
+  if (rc) return rc;
+  if ((reinterpret_cast<uintptr_t>(dq) & 15) || rows >= (1ll << 32))
+    dq_convert_kernel<<<(unsigned)(sm_count() * 16), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
+  else if (D == 128)
+    dq_convert8_kernel<128><<<ugrid, 256, 0, st>>>((const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
+  else
+    dq_convert8_kernel<64><<<ugrid, 256, 0, st>>>((const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
   return launch_status();
 }
 

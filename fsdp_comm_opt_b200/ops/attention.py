@@ -3,9 +3,8 @@
 Layout: one packed projection ``[B, S, Hq + 2*Hkv, D]`` (q heads, then k heads, then v heads),
 output ``[B, S, Hq, D]`` contiguous; the backward returns one packed gradient of the same shape,
 so the qkv projection's backward reads it without a concatenation.
-CUDA tensors run the sm_100a flash-style kernels (``zc_attn_fwd_2q`` / ``zc_attn_bwd_kt`` for head
-dimension 128, ``zc_attn_fwd_ws`` / ``zc_attn_bwd_ws`` for 64: online softmax, log-sum-exp saved for
-the backward, no S x S tensor in memory); CPU tensors run fp32 matmul/softmax.  The reference reaches PyTorch SDPA through HF attention modules.
+CUDA tensors run the sm_100a flash-style kernels (``zc_attn_fwd_2q`` / ``zc_attn_bwd_kt``, head
+dimensions 64 and 128: online softmax, log-sum-exp saved for the backward, no S x S tensor in memory); CPU tensors run fp32 matmul/softmax.  The reference reaches PyTorch SDPA through HF attention modules.
 """
 from __future__ import annotations
 
@@ -103,9 +102,9 @@ class _Attention(torch.autograd.Function):
         dq, dk, dv = dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]
         delta = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
         # fp32 accumulator of dQ: allocated per call, so that calls on other streams and recorded graphs own theirs
-        dq_acc = torch.empty(B * Hq * D * ((S + 3) // 4 * 4), dtype=torch.float32, device=qkv.device)
+        dq_acc = torch.empty(B * Hq * D * S, dtype=torch.float32, device=qkv.device)
         lib = _lib.cuda()
-        # default: key-row kernel (64-query iterations, pipelined); ZC_ATTN_BWD=ws / simple select
+        # default: key-row kernel (128 x 128 iterations, pipelined); ZC_ATTN_BWD=ws / simple select
         # the earlier warp-specialised and single-role kernels
         bwd = {"simple": lib.zc_attn_bwd, "ws": lib.zc_attn_bwd_ws}.get(_BWD_IMPL, lib.zc_attn_bwd_kt)
         _lib.check(bwd(

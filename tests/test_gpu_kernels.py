@@ -404,6 +404,34 @@ def test_attention_fwd_bwd(B, S, Hq, Hkv, D, impl, monkeypatch):
     assert torch.allclose(qkv.grad.float(), qf.grad, atol=3e-2, rtol=3e-2), err
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1, 1, 1), (2, 65, 2, 1), (1, 127, 3, 3), (1, 129, 4, 1), (3, 256, 2, 2),
+                                        (1, 257, 8, 2), (1, 769, 2, 2), (2, 1024, 25, 25)])
+def test_attention_at_the_edges_of_key_and_query_tiles(B, S, Hq, Hkv, D):
+    """One, a part of one, exactly one and one more than a tile of 128 (and a pair of tiles); scores that rise
+    along the sequence in the last heads, so that the accumulator is rescaled at both head sizes.  The bound:
+    bf16 probabilities and score gradients (2^-9 relative each) summed over a row, against the result's norm."""
+    torch.manual_seed(S * D)
+    qkv = torch.randn(B, S, Hq + 2 * Hkv, D, device=DEV) * 0.5
+    qkv[:, :, Hq - 1] = 1.0
+    qkv[:, :, Hq + Hkv - 1] += torch.linspace(-2.0, 2.0, S, device=DEV)[None, :, None]
+    qkv = qkv.bfloat16().requires_grad_()
+    o = attention.causal_attention(qkv, Hq, Hkv)
+    g = torch.randn_like(o)
+    (dqkv,) = torch.autograd.grad(o, qkv, g)
+    torch.cuda.synchronize()
+    assert attention.status_read_and_clear() == 0
+    qf = qkv.detach().double().requires_grad_()
+    q, k, v = (t.transpose(1, 2) for t in qf.split([Hq, Hkv, Hkv], 2))
+    k, v = (t.repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    p = torch.matmul(q, k.transpose(2, 3)) / D ** 0.5
+    p = p.masked_fill(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("-inf")).softmax(-1)
+    ref = torch.matmul(p, v).transpose(1, 2)
+    (dref,) = torch.autograd.grad(ref, qf, g.double())
+    assert ((o - ref).norm() / ref.norm()).item() < 6e-3
+    assert ((dqkv - dref).norm() / dref.norm()).item() < 1e-2
+
+
 @pytest.mark.parametrize("impl", ["2q+kt", "ws+ws"])
 def test_attention_rising_scores_rescale_the_accumulator(impl, monkeypatch):
     """Keys whose scores grow along the sequence raise the running row maximum again and again, so
