@@ -21,6 +21,9 @@
 // TMEM (512 columns allocated): S_0 64 | S_1 64 | O_0 128 | O_1 128 | P: tile t, block parity u at
 // 384 + (2 t + u) * 32 (64 keys as 32 columns).
 // Shared memory: Q 2 x 32 KB, K/V ring 4 x (16 + 16) KB.
+// What bounds it: the issue of the MMAs, about 90 clocks each at 64 columns.  Blocks of 128 keys (fewer, wider MMAs) leave
+// no TMEM for P beside the scores, a tile's block becomes one chain, and that was no faster: 16384 keys, 32 heads 2155 us
+// with the tiles taking turns at the exponentials, 2396 with two threads a row, 2135 as it is.
 // CTAs are numbered heaviest first (the last 256 queries see the most keys).  Every wait is
 // bounded; a timed-out role raises a CTA-wide abort flag, the CTA frees its TMEM and returns, and the
 // launcher's status word reports it.
@@ -31,9 +34,11 @@
 #include "attn_common.cuh"
 #include "launch_util.h"
 
-extern "C" int zc_attn_fwd_ws(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S, int Hq,
-                              int Hkv, int D, int64_t qs0, int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1,
-                              int64_t ks2, int64_t vs0, int64_t vs1, int64_t vs2, float scale, cudaStream_t st);
+namespace zc {
+int attn_fwd_d64(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S, int Hq, int Hkv,
+                 int64_t qs0, int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,
+                 int64_t vs2, float scale, int* status, cudaStream_t st);  // attention_fwd_d64.cu
+}
 
 namespace zc {
 namespace fwd2q {
@@ -364,32 +369,33 @@ int zc_attn_fwd_2q_status_read_and_clear() {
 void zc_attn_fwd_2q_set_trace(void* buf) { zc::fwd2q::g_trace = (long long*)buf; }
 #endif
 
-// Same argument list as zc_attn_fwd_ws.  Head dimension 128 runs the two-tile kernel; 64 falls back
-// to zc_attn_fwd_ws.
+// Same argument list as zc_attn_fwd_ws.  Head dimension 128 runs the two-tile kernel, 64 the one of
+// attention_fwd_d64.cu.
 int zc_attn_fwd_2q(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S, int Hq, int Hkv,
                    int D, int64_t qs0, int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0,
                    int64_t vs1, int64_t vs2, float scale, cudaStream_t st) {
   using namespace zc;
   using namespace zc::fwd2q;
-  if (D != 128)
-    return zc_attn_fwd_ws(q, k, v, o, lse, B, S, Hq, Hkv, D, qs0, qs1, qs2, ks0, ks1, ks2, vs0, vs1, vs2, scale, st);
-  if (Hq % Hkv) return ERR_UNSUPPORTED;
+  if ((D != 64 && D != 128) || Hq % Hkv) return ERR_UNSUPPORTED;
   if ((qs0 | qs1 | qs2 | ks0 | ks1 | ks2 | vs0 | vs1 | vs2) % 8) return ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15)
     return ERR_UNSUPPORTED;
   int dev = 0;
   cudaGetDevice(&dev);
   cudaSetDevice(dev);  // binds the primary context on autograd worker threads (tensor-map encoder needs it)
+  int* status = status_word(dev);
+  if (!status) return ERR_BAD_ARG;
+  if (D == 64)
+    return attn_fwd_d64(q, k, v, o, lse, B, S, Hq, Hkv, qs0, qs1, qs2, ks0, ks1, ks2, vs0, vs1, vs2, scale, status, st);
   CUtensorMap mq, mk, mv;
   if (!make_map_bshd(&mq, q, D, Hq, S, B, qs0, qs1, qs2, 128) || !make_map_bshd(&mk, k, D, Hkv, S, B, ks0, ks1, ks2, KB) ||
       !make_map_bshd(&mv, v, D, Hkv, S, B, vs0, vs1, vs2, KB))
     return ERR_BAD_ARG;
   Params p;
   p.o = (__nv_bfloat16*)o; p.lse = lse; p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.scale = scale;
-  p.status = status_word(dev);
+  p.status = status;
   p.ncb = (S + 255) / 256;
   p.trace = g_trace;
-  if (!p.status) return ERR_BAD_ARG;
   const int smem = 65536 + STAGES * 32768 + 1024;
   static bool attr = false;
   if (!attr) { cudaFuncSetAttribute(attn_fwd_2q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr = true; }
