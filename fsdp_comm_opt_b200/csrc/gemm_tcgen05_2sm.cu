@@ -53,7 +53,9 @@ constexpr int THREADS = 192;
 constexpr int A_BYTES = BM_CTA * BK * 2;  // 16 KB
 constexpr int B_BYTES = BN_CTA * BK * 2;  // 16 KB
 constexpr int STAGE = A_BYTES + B_BYTES;
-constexpr int MAX_SPLIT = 4;
+constexpr int MAX_SPLIT = 4;          // slices of a tail tile
+constexpr int MAX_SPLIT_SINGLE = 16;  // slices of a product that has fewer tiles than clusters
+constexpr int SINGLE_MIN_KB = 8;      // K blocks of such a slice at least
 constexpr int SCHED = 4;       // slots of the unit-index ring
 constexpr int COUNTER_SLOTS = 256;
 
@@ -474,6 +476,7 @@ __global__ void __launch_bounds__(256) gemm_2sm_fixup_kernel(const Params p, int
     const int row = i / (BN / 8), c8 = i % (BN / 8);
     if ((int64_t)mi * BM + row >= p.M || (int64_t)ni * BN + c8 * 8 >= p.N) continue;
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
     for (int s = 0; s < p.split; ++s) {
       const float4* src = reinterpret_cast<const float4*>(base + (int64_t)s * (BM * BN) + row * BN + c8 * 8);
       const float4 x = src[0], y = src[1];
@@ -571,6 +574,31 @@ static int max_clusters(int smem) {
   return std::min(n, sm_count() / 2);
 }
 
+// K slices of a product whose tiles leave at least half of the clusters idle (a layer of a small model, or few
+// tokens): it is cut along K altogether, so that about every cluster has a slice.  A slice has at least SINGLE_MIN_KB
+// K blocks: below that the fp32 partials and the second launch cost what the shorter K loop saves.
+static int single_split(int64_t tiles, int64_t k_blocks, int clusters) {
+  if (tiles <= 0 || tiles * 2 > clusters) return 1;
+  const int64_t want = std::min<int64_t>(std::min<int64_t>(clusters / tiles, MAX_SPLIT_SINGLE), k_blocks / SINGLE_MIN_KB);
+  if (want < 2) return 1;
+  const int64_t per = (k_blocks + want - 1) / want;
+  return (int)((k_blocks + per - 1) / per);  // no empty slice
+}
+
+static int init_state(DeviceState& ds, int smem) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (!ds.ready) {
+    int c = max_clusters<MAJOR_K, MAJOR_K>(smem);
+    c = std::min(c, max_clusters<MAJOR_K, MAJOR_MN>(smem));
+    c = std::min(c, max_clusters<MAJOR_MN, MAJOR_MN>(smem));
+    ds.clusters = c;
+    if (cudaMalloc(&ds.counters, 2 * COUNTER_SLOTS * sizeof(unsigned)) != cudaSuccess) return ERR_BAD_ARG;
+    cudaMemset(ds.counters, 0, 2 * COUNTER_SLOTS * sizeof(unsigned));
+    ds.ready = true;
+  }
+  return 0;
+}
+
 }  // namespace g2
 }  // namespace zc
 
@@ -587,9 +615,11 @@ int* zc_gemm_status_word();  // gemm_tcgen05.cu: the current device's GEMM statu
 // (zc_gemm_status_read_and_clear; code 8 = a bounded wait of this kernel expired).
 // `bias`: null, or N bf16 values (16-byte aligned) added to every row of the product before it is rounded
 // (and before the old C is added when `accumulate` is set).
-int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
-                          int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate,
-                          cudaStream_t st) {
+// `ws`: null, or `ws_bytes` of device memory (16-byte aligned) of the caller's for the fp32 partial sums of a product
+// that zc_gemm_2sm_split_bytes names a size for; without it such a product is not split.
+int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
+                        int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate, void* ws,
+                        int64_t ws_bytes, cudaStream_t st) {
   ZC_NVTX_RANGE("zc_gemm_bf16_2sm");
   if (reinterpret_cast<uintptr_t>(bias) & 15) return zc::ERR_UNSUPPORTED;
   using namespace zc;
@@ -619,18 +649,7 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
   if (!ok) return ERR_BAD_ARG;
   const int smem = STAGES * STAGE + 1024;
   DeviceState& ds = g_state[dev];
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    if (!ds.ready) {
-      int c = max_clusters<MAJOR_K, MAJOR_K>(smem);
-      c = std::min(c, max_clusters<MAJOR_K, MAJOR_MN>(smem));
-      c = std::min(c, max_clusters<MAJOR_MN, MAJOR_MN>(smem));
-      ds.clusters = c;
-      if (cudaMalloc(&ds.counters, 2 * COUNTER_SLOTS * sizeof(unsigned)) != cudaSuccess) return ERR_BAD_ARG;
-      cudaMemset(ds.counters, 0, 2 * COUNTER_SLOTS * sizeof(unsigned));
-      ds.ready = true;
-    }
-  }
+  if (const int rc = init_state(ds, smem)) return rc;
   Params p;
   p.C = (__nv_bfloat16*)C; p.M = M; p.N = N; p.K = K; p.ldc = ldc;
   p.bias = (const __nv_bfloat16*)bias;
@@ -645,14 +664,23 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
   // Tail: the tiles of the last, partial wave are cut into K slices so that every cluster has one
   // unit of about the same length to finish with.
   const int64_t rem = tiles % clusters;
-  int split = 1;
+  int split = 1, grid_clusters = clusters;
   if (rem > 0 && tiles > clusters) {
     split = (int)std::min<int64_t>(std::min<int64_t>(clusters / rem, MAX_SPLIT), k_blocks / 8);
     if (forced_split >= 0) split = std::min(forced_split, MAX_SPLIT);
     if (split < 2 || rem * 10 > (int64_t)clusters * 8) split = 1;  // a nearly full last wave is left alone
   }
+  int64_t rem_tiles = rem;
+  const int single = ws ? single_split(tiles, k_blocks, ds.clusters) : 1;
+  if (single > 1 && ws_bytes >= tiles * single * (int64_t)(BM * BN * sizeof(float))) {
+    split = single;
+    rem_tiles = tiles;
+    grid_clusters = (int)(tiles * split);
+  } else {
+    ws = nullptr;
+  }
   p.split = split;
-  p.full_tiles = (int)(split > 1 ? tiles - rem : tiles);
+  p.full_tiles = (int)(split > 1 ? tiles - rem_tiles : tiles);
   // Counters only where a second round is handed out, and not in a launch that is being recorded: a
   // replayed launch would keep its slot for good, next to launches of other streams that take slots in turn.
   p.counter = nullptr;
@@ -662,7 +690,9 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
     p.counter = ds.counters + 2 * (ds.next_slot++ % COUNTER_SLOTS);
   }
   p.partial = nullptr;
-  if (split > 1) {
+  if (split > 1 && ws) {
+    p.partial = (float*)ws;
+  } else if (split > 1) {
     const size_t need = (size_t)rem * split * BM * BN;
     std::lock_guard<std::mutex> lock(g_mutex);
     if (ds.partial_elems < need) {
@@ -679,16 +709,34 @@ int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bia
     }
     p.partial = ds.partial;
   }
-  const dim3 grid(2 * clusters);
+  const dim3 grid(2 * grid_clusters);
   if (a_major == MAJOR_K && b_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_K><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   else if (a_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   else gemm_2sm_kernel<MAJOR_MN, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   int rc = launch_status();
   if (rc == 0 && p.split > 1) {
-    gemm_2sm_fixup_kernel<<<dim3(16, (unsigned)rem), 256, 0, st>>>(p, (int)m_tiles, (int)n_tiles);
+    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)rem_tiles), 256, 0, st>>>(p, (int)m_tiles, (int)n_tiles);
     rc = launch_status();
   }
   return rc;
+}
+
+int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
+                          int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate,
+                          cudaStream_t st) {
+  return zc_gemm_bf16_2sm_ws(A, B, C, bias, M, N, K, lda, ldb, ldc, trans_a, trans_b, accumulate, nullptr, 0, st);
+}
+
+// Bytes of the workspace with which zc_gemm_bf16_2sm_ws splits an M x N x K product along K; 0 when it does not.
+int64_t zc_gemm_2sm_split_bytes(int64_t M, int64_t N, int64_t K) {
+  using namespace zc;
+  using namespace zc::g2;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (M <= 0 || N <= 0 || K <= 0 || dev < 0 || dev >= 64 || init_state(g_state[dev], STAGES * STAGE + 1024)) return 0;
+  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int split = single_split(tiles, (K + BK - 1) / BK, g_state[dev].clusters);
+  return split > 1 ? tiles * split * (int64_t)(BM * BN * sizeof(float)) : 0;
 }
 
 int zc_gemm_bf16_2sm_ld(const void* A, const void* B, void* C, int64_t M, int64_t N, int64_t K, int64_t lda,

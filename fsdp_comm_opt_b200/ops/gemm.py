@@ -20,6 +20,9 @@ import torch
 
 from .. import _lib
 
+# above this a product's 256 x 256 tiles occupy more than half of the 74 pairs of SMs: it is not split along K
+_SPLIT_MAX_OUT = 37 * 256 * 256
+
 _BACKEND = os.environ.get("ZC_GEMM_BACKEND", "auto")
 
 
@@ -87,10 +90,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
         if kind == "2sm":
             fused_bias = (bias is not None and bias.dtype == torch.bfloat16 and bias.is_contiguous()
                           and bias.numel() == N and bias.data_ptr() % 16 == 0)
-            _lib.check(lib.zc_gemm_bf16_2sm_bias(
+            # fp32 partial sums of a product that is split along K: this call's own, so that no other stream shares them
+            ws_bytes = lib.zc_gemm_2sm_split_bytes(M, N, K) if M * N <= _SPLIT_MAX_OUT else 0
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device) if ws_bytes else None
+            _lib.check(lib.zc_gemm_bf16_2sm_ws(
                 a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if fused_bias else None, M, N, K,
                 a.stride(0), b.stride(0), out.stride(0), int(trans_a), int(trans_b), int(accumulate),
-                _lib.stream_ptr(a.device)), "zc_gemm_bf16_2sm")
+                ws.data_ptr() if ws is not None else None, ws_bytes, _lib.stream_ptr(a.device)), "zc_gemm_bf16_2sm")
             if bias is not None and not fused_bias:
                 out.add_(bias.to(out.dtype))
         else:

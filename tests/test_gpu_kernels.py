@@ -610,6 +610,35 @@ def test_tcgen05_gemm_three_forms(backend, M, N, K):
         gemm.set_backend("auto")
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 128, 1024), (512, 256, 8192), (1024, 1024, 4096), (200, 137, 1096), (300, 520, 17 * 64),
+                                   (2048, 1024, 1023), (256, 9472, 1024), (256, 9728, 1024)])
+def test_gemm_split_along_k_when_tiles_are_few(M, N, K):
+    """The smallest product, one slice of 8 K blocks each, a K that does not divide into equal slices, ragged M / N / K,
+    and the last size that is split (37 tiles) beside the first that is not.  Each is rounded once from fp32 sums: half
+    a bf16 unit (2^-9) at most per value, so the relative error in the 2-norm is below 2^-9 plus the sums' 1e-5."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(K)
+    pad = (K + 7) // 8 * 8
+    x = torch.randn(M, pad, device=DEV).bfloat16()[:, :K]
+    w = torch.randn(N, pad, device=DEV).bfloat16()[:, :K]
+    bias = torch.randn(N, device=DEV).bfloat16()
+    y = gemm.gemm(x, w, False, True, bias=bias)
+    dw = gemm.gemm(x, x, True, False) if K <= 4096 else None          # K x K, summed over the M rows
+    acc = y.clone() if N % 8 == 0 else None
+    if acc is not None:
+        gemm.gemm(x, w, False, True, out=acc, accumulate=True)
+    torch.cuda.synchronize()
+    assert _lib.cuda().zc_gemm_status_read_and_clear() == 0
+    ref = x.double() @ w.double().t()
+    assert ((y.double() - (ref + bias.double())).norm() / ref.norm()).item() < 2 ** -9 + 1e-5
+    if dw is not None:
+        rw = x.double().t() @ x.double()
+        assert ((dw.double() - rw).norm() / rw.norm()).item() < 2 ** -9 + 1e-5
+    if acc is not None:
+        assert ((acc.double() - (ref + y.double())).norm() / ref.norm()).item() < 2 ** -8 + 1e-5
+
+
 def test_gemm_with_leading_dimensions_and_odd_sizes():
     """Operands and results that are slices of wider buffers, and M / N / K that are not multiples of 8
     (GPT-2's vocabulary): the two-SM kernel takes row strides, zero-fills what lies outside a slice and
