@@ -68,6 +68,7 @@ def declare(lib) -> None:
     _sig(lib, "zc_attn_fwd_2q", P, P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, L, L, L, F, P)
     _sig(lib, "zc_attn_fwd_2q_status_read_and_clear")
     _sig(lib, "zc_attn_bwd_kt", P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, *([L] * 18), F, P, P)
+    _sig(lib, "zc_embedding_grad", P, P, P, L, L, L, I, P)
     _sig(lib, "zc_gemm_bf16", P, P, P, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm", P, P, P, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm_ld", P, P, P, L, L, L, L, L, L, I, I, I, P)

@@ -17,7 +17,7 @@ import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
 from ..ops import attention as attn_ops
-from ..ops import gemm, loss as loss_ops, norm, rope, swiglu
+from ..ops import embedding, gemm, loss as loss_ops, norm, rope, swiglu
 from .config import ModelConfig
 
 
@@ -54,6 +54,9 @@ class Embedding(nn.Embedding):
 
     def reset_parameters(self):
         nn.init.normal_(self.weight, mean=0.0, std=self.init_std)
+
+    def forward(self, input_ids: torch.Tensor) -> torch.Tensor:
+        return embedding.embedding(input_ids, self.weight)
 
 
 class Linear(nn.Module):

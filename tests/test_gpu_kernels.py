@@ -575,6 +575,34 @@ def test_linear_with_bias_in_the_gemm_epilogue(T, K, N):
     assert torch.allclose(w.grad.float(), wf.grad, atol=2e-2 * float(wf.grad.abs().max()), rtol=3e-2)
 
 
+# ------------------------------------------------------------------ embedding gradient
+@pytest.mark.parametrize("n,dim,rows,accumulate", [(1, 8, 5, False), (31, 256, 64, True), (1025, 1600, 300, False),
+                                                   (4096, 2056, 50257, True), (8192, 64, 3, False), (8192, 16, 1, True)])
+def test_embedding_gradient_in_the_flat_buffer(n, dim, rows, accumulate):
+    """One position, repeated ids (8192 positions of one row), widths below, at and past a block's 2048 columns, an old
+    gradient to add to.  fp32 sums of m bf16 terms rounded once: 2^-9 relative plus m 2^-24 of the terms' magnitudes."""
+    from fsdp_comm_opt_b200.ops.embedding import embedding
+
+    torch.manual_seed(n)
+    w = torch.nn.Parameter(torch.randn(rows, dim, device=DEV).bfloat16())
+    w.main_grad = torch.randn(rows, dim, device=DEV).bfloat16()
+    w.main_grad_written = accumulate
+    old = w.main_grad.double() * accumulate
+    ids = torch.randint(0, rows, (n,), device=DEV)
+    out = embedding(ids, w)
+    assert torch.equal(out, w.detach()[ids])
+    g = torch.randn(n, dim, device=DEV).bfloat16()
+    out.backward(g)
+    assert w.grad is None and w.main_grad_written
+    ref = old.index_add(0, ids, g.double())
+    mag = old.abs().index_add(0, ids, g.double().abs())
+    assert ((w.main_grad.double() - ref).abs() <= ref.abs() * 2 ** -8 + mag * n * 2 ** -24 + 1e-30).all()
+    hook = w.register_hook(lambda t: None)     # a hook on the table still sees its gradient
+    embedding(ids, w).backward(g)
+    assert w.grad is not None
+    hook.remove()
+
+
 # ------------------------------------------------------------------ GEMM
 @pytest.mark.parametrize("backend,M,N,K", [
     ("tcgen05", 128, 128, 128), ("tcgen05", 256, 512, 384), ("tcgen05", 4096, 1536, 1024), ("tcgen05", 384, 256, 4096),
