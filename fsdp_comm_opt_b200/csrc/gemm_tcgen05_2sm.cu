@@ -55,7 +55,8 @@ constexpr int B_BYTES = BN_CTA * BK * 2;  // 16 KB
 constexpr int STAGE = A_BYTES + B_BYTES;
 constexpr int MAX_SPLIT = 4;          // slices of a tail tile
 constexpr int MAX_SPLIT_SINGLE = 16;  // slices of a product that has fewer tiles than clusters
-constexpr int SINGLE_MIN_KB = 8;      // K blocks of such a slice at least
+constexpr int SINGLE_MIN_KB = 8;      // K blocks of such a slice at least,
+constexpr int SINGLE_MIN_SAVED = 20;  // and fewer K blocks one after the other than in the whole product
 constexpr int SCHED = 4;       // slots of the unit-index ring
 constexpr int COUNTER_SLOTS = 256;
 
@@ -575,13 +576,14 @@ static int max_clusters(int smem) {
 }
 
 // K slices of a product whose tiles leave at least half of the clusters idle (a layer of a small model, or few
-// tokens): it is cut along K altogether, so that about every cluster has a slice.  A slice has at least SINGLE_MIN_KB
-// K blocks: below that the fp32 partials and the second launch cost what the shorter K loop saves.
+// tokens): it is cut along K altogether, so that about every cluster has a slice.  A K block
+// takes 0.25 to 0.3 us there, the fp32 partials and the pass that adds them 4 to 5 us: SINGLE_MIN_SAVED.
 static int single_split(int64_t tiles, int64_t k_blocks, int clusters) {
   if (tiles <= 0 || tiles * 2 > clusters) return 1;
   const int64_t want = std::min<int64_t>(std::min<int64_t>(clusters / tiles, MAX_SPLIT_SINGLE), k_blocks / SINGLE_MIN_KB);
   if (want < 2) return 1;
   const int64_t per = (k_blocks + want - 1) / want;
+  if (k_blocks - per < SINGLE_MIN_SAVED) return 1;
   return (int)((k_blocks + per - 1) / per);  // no empty slice
 }
 
