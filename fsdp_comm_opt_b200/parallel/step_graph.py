@@ -70,6 +70,14 @@ class StepGraphs:
         saved = c.n_layers * block if not self.model.activation_checkpointing else c.n_layers * 2 * c.d_model + block
         return 2 * tokens * (saved + c.vocab_size + 6 * c.ffn)
 
+    def _host_bound(self, tokens: int) -> bool:
+        """Whether the launches (about 23 a layer and 20 beside the layers, 28 us each) are more than a tenth of the GPU's
+        work (products at 1.4 PFLOP/s, 14 bytes an element for the update).  Below that a replay has nothing to save, and
+        recorded GEMMs hand their tiles out in a fixed order: a 34B layer at 4096 tokens took 29.0 ms eagerly and
+        29.9 replayed (a twentieth), a 13B layer at 2048 tokens 7.4 and 7.2 (a sixth)."""
+        n = self.cfg.num_params()
+        return 10 * 28e-6 * (23 * self.cfg.n_layers + 20) > 6 * n * tokens / 1.4e15 + 14 * n / 6e12
+
     # -- run ---------------------------------------------------------------------------------------
     def owns(self, loss: torch.Tensor) -> bool:
         return any(r.loss is loss for r in self._recorded.values())
@@ -95,7 +103,8 @@ class StepGraphs:
                 return None
             free, _ = torch.cuda.mem_get_info(self.flat.device)
             free += torch.cuda.memory_reserved(self.flat.device) - torch.cuda.memory_allocated(self.flat.device)
-            if self._activation_bytes(ids.numel()) > min(self.MAX_BYTES, self.MAX_FREE_FRACTION * free):
+            if (not self._host_bound(ids.numel())
+                    or self._activation_bytes(ids.numel()) > min(self.MAX_BYTES, self.MAX_FREE_FRACTION * free)):
                 if len(self._refused) > 256:
                     self._refused.clear()
                 self._refused.add(shape)
