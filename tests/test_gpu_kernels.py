@@ -299,6 +299,28 @@ def test_cross_entropy_fwd_bwd(V):
     assert torch.allclose(work.grad.float(), lf.grad, atol=2e-4, rtol=2e-2)
 
 
+@pytest.mark.parametrize("V", [8, 36864, 36871, 36872, 73719, 73720, 100001])
+def test_cross_entropy_at_the_edges_of_its_clusters(V):
+    """The longest row of one and of two CTAs, the first that needs more, ragged rows whose label lies among the
+    last V % 8 columns, in the first and the last share, masked logits, a row that is ignored.  fp32 against 64 bits: the loss to 1e-5, the
+    gradient to half a bf16 unit (2^-9) of its value plus fp32 sums' 1e-5."""
+    torch.manual_seed(V)
+    T, ld = 7, (V + 7) // 8 * 8 + 8
+    buf = (torch.randn(T, ld, device=DEV) * 2).bfloat16()
+    buf[3, :V // 2] = float("-inf")                 # masked logits, whole threads' shares of them
+    labels = torch.tensor([0, V - 1, V // 8 * 8 - 1, V // 2, -100, max(0, V - 2), V // 4 * 3], device=DEV)
+    lf = buf[:, :V].double().requires_grad_()
+    ref = F.cross_entropy(lf, labels, ignore_index=-100)
+    ref.backward()
+    work = buf.clone()
+    logits = work[:, :V].requires_grad_()
+    out = loss.cross_entropy(logits, labels)
+    (grad,) = torch.autograd.grad(out, logits)
+    assert abs(out.item() - ref.item()) <= 1e-5 * max(1.0, ref.item())
+    assert ((grad.double() - lf.grad).abs() <= lf.grad.abs() * (2 ** -8 + 1e-5) + 1e-12).all()
+    assert (work[:, V:] == 0).all()
+
+
 def test_int8_quant_kernels():
     torch.manual_seed(4)
     n, world = 100003, 3
