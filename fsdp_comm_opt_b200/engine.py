@@ -98,10 +98,7 @@ class TrainEngine:
         if (cfg.step_graphs and self.flat is not None and self.flat.cuda and self.flat.world == 1
                 and not cfg.time_collectives):
             self._graphs = StepGraphs(self.model, self.flat, self.model_config)
-        self._loss_host = self._loss_ready = None
-        if device.type == "cuda":
-            self._loss_host = torch.empty((), dtype=torch.float32, pin_memory=True)
-            self._loss_ready = torch.cuda.Event()
+        self._loss_host = torch.empty((), dtype=torch.float32, pin_memory=True) if device.type == "cuda" else None
 
     def _forward_backward(self, input_ids: torch.Tensor) -> torch.Tensor:
         """Loss of the batch (host or device ids), with the gradients in place.  The tensor may be a buffer
@@ -141,17 +138,16 @@ class TrainEngine:
         return loss
 
     def step(self, input_ids_host: torch.Tensor) -> float:
-        """Host batch in, loss out: H2D copy, one optimizer step, D2H read of the loss.  The loss is
-        read as soon as the backward pass has produced the gradients: the optimizer update is already
-        enqueued behind it and runs while the caller prepares its next batch."""
+        """Host batch in, loss out: H2D copy, one optimizer step, D2H read of the loss.  On return the whole step,
+        the optimizer update included, has finished on the device: parameters and moments may be read from any
+        stream.  The loss is copied ahead of the update, so that its way to the host is not waited for apart."""
         loss = self._forward_backward(input_ids_host)
         if self._loss_host is None or loss.device.type != "cuda":
             self._update()
             return float(loss.item())
         self._loss_host.copy_(loss, non_blocking=True)
-        self._loss_ready.record()
         self._update()
-        self._loss_ready.synchronize()
+        torch.cuda.current_stream(loss.device).synchronize()
         return float(self._loss_host)
 
     def comm_report(self) -> dict:

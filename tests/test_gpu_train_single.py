@@ -80,3 +80,26 @@ def _graph_worker(rank, world, family):
 @pytest.mark.parametrize("family", ["llama", "gpt2", "ckpt"])
 def test_replayed_steps_equal_eager_steps(family):
     run_ranks(_graph_worker, 1, backend="nccl", args=(family,))
+
+
+def _finished_worker(rank, world, graphs):
+    import dataclasses
+
+    import torch
+
+    from fsdp_comm_opt_b200.engine import EngineConfig, TrainEngine
+    from fsdp_comm_opt_b200.models import get_config
+
+    # 2.6e8 table elements: the update takes about 0.6 ms, far longer than the way from the loss to the caller
+    cfg = dataclasses.replace(get_config("tiny"), vocab_size=512_000)
+    eng = TrainEngine(EngineConfig(model=cfg, seed=3, step_graphs=graphs), torch.device("cuda", 0))
+    ids = torch.randint(0, cfg.vocab_size, (1, 64)).pin_memory()
+    for _ in range(5):
+        eng.step(ids)
+        assert torch.cuda.current_stream().query()
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_a_step_has_finished_when_it_returns(graphs):
+    """Parameters and moments may be read from another stream as soon as ``step`` is back."""
+    run_ranks(_finished_worker, 1, backend="nccl", args=(graphs,))
