@@ -17,10 +17,15 @@ _TABLES: dict = {}
 def cached_tables(seq_len: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:
     """fp32 cos/sin tables, cached per (seq_len, head_dim, theta, device).  Modules fetch them here
     instead of receiving them as forward arguments: FSDP2's mixed-precision policy casts floating
-    point forward inputs to the parameter dtype, which would silently turn the tables into bf16."""
+    point forward inputs to the parameter dtype, which would silently turn the tables into bf16.
+
+    Tables that are made while a CUDA graph is recorded live in the graph's memory, which other graphs
+    of its pool write to: they belong to the recording alone and are not cached."""
     key = (int(seq_len), int(head_dim), float(theta), str(device))
     t = _TABLES.get(key)
     if t is None:
+        if torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing():
+            return rope_tables(seq_len, head_dim, theta, device)
         if len(_TABLES) > 16:
             _TABLES.clear()
         t = _TABLES[key] = rope_tables(seq_len, head_dim, theta, device)

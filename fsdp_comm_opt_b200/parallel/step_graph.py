@@ -124,6 +124,9 @@ class StepGraphs:
         rec = _Recorded()
         rec.key = key
         rec.ids = torch.zeros(shape, dtype=torch.int64, device=dev)
+        # the cached tables that the recorded launches read: made ahead of the recording, outside the graphs' memory
+        rec.keep = (rope.cached_tables(shape[1], self.cfg.head_dim, self.cfg.rope_theta, rec.ids.device)
+                    if self.cfg.family == "llama" else None)
         rec.graph = torch.cuda.CUDAGraph()
         if self._stream is None:
             self._stream = torch.cuda.Stream(dev)
@@ -144,5 +147,4 @@ class StepGraphs:
         cur.wait_stream(self._stream)
         rec.launches = _lib.launch_count() - before
         _lib.add_launches(-rec.launches)  # recorded, not run
-        rec.keep = list(rope._TABLES.values())  # the cached tables that the recorded launches read
         return rec

@@ -103,3 +103,52 @@ def _finished_worker(rank, world, graphs):
 def test_a_step_has_finished_when_it_returns(graphs):
     """Parameters and moments may be read from another stream as soon as ``step`` is back."""
     run_ranks(_finished_worker, 1, backend="nccl", args=(graphs,))
+
+
+def _engines(family="llama", act_ckpt=False, **changes):
+    """The same small model with and without recorded steps."""
+    import dataclasses
+
+    import torch
+
+    from fsdp_comm_opt_b200.engine import EngineConfig, TrainEngine
+    from fsdp_comm_opt_b200.models import get_config
+
+    cfg = dataclasses.replace(get_config("gpt2-tiny" if family == "gpt2" else "tiny"), vocab_size=1024, **changes)
+    dev = torch.device("cuda", 0)
+    return [TrainEngine(EngineConfig(model=cfg, lr=1e-3, seed=3, step_graphs=g, act_ckpt=act_ckpt), dev) for g in (True, False)]
+
+
+def _same_steps(a, b, shapes, seed=1):
+    import torch
+
+    g = torch.Generator().manual_seed(seed)
+    for i, shape in enumerate(shapes):
+        ids = torch.randint(0, a.model_config.vocab_size, shape, generator=g).pin_memory()
+        la, lb = a.step(ids), b.step(ids)
+        assert abs(la - lb) < 2e-3 * abs(lb), (i, shape, la, lb)        # dQ is summed in any order
+
+
+def _many_lengths_worker(rank, world):
+    import torch
+
+    from fsdp_comm_opt_b200.ops import rope
+
+    a, b = _engines()
+    # a long shape is recorded; a short one is seen twice; so many other lengths that the table cache is emptied; the
+    # short one is recorded; the long one is replayed over whatever the short recording left in their common memory
+    _same_steps(a, b, [(2, 512)] * 4 + [(2, 96)] * 2 + [(1, 101 + 3 * i) for i in range(18)] + [(2, 96), (2, 512)])
+    assert len(a._graphs._recorded) == 2 and any(key[0] == 96 for key in rope._TABLES)
+    segments = torch.cuda.memory_snapshot()
+    for (seq, dim, theta, dev), tables in rope._TABLES.items():
+        for t, r in zip(tables, rope.rope_tables(seq, dim, theta, dev)):
+            (segment,) = [s for s in segments if 0 <= t.data_ptr() - s["address"] < s["total_size"]]
+            assert segment["segment_pool_id"] == (0, 0), f"the table of {seq} lies in the graphs' memory"
+            assert torch.equal(t, r), seq
+    _same_steps(a, b, [(1, 96), (2, 96), (1, 512)])                     # eager and replayed readers of the tables
+    # twenty lengths with two batch sizes, each often enough to be recorded
+    _same_steps(a, b, [(1 + i % 2, 64 + 8 * (i // 2 % 20)) for i in range(160)])
+
+
+def test_steps_of_many_lengths_equal_eager_steps():
+    run_ranks(_many_lengths_worker, 1, backend="nccl")
