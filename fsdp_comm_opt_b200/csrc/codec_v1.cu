@@ -185,9 +185,11 @@ __global__ void __launch_bounds__(128, 8) v1_encode_kernel(
       *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(pack + i);
     // the unfinished piece is written too, and once more as a whole by the next chunk with outliers
     for (int i = full + lane; i < have; i += 32) dst[i] = pack[i];
+    // Only the bytes of that piece move to the front: the next chunk's outliers are stored right behind them, by other
+    // lanes and with nothing in between that orders the two.
     const uint8_t v = pack[whole + (lane & 15)];
     __syncwarp();
-    if (lane < 16) pack[lane] = v;
+    if (lane < have - whole) pack[lane] = v;
     run += total;
   }
   if (lane == 0) totals[blockIdx.x * 4 + warp] = run;

@@ -175,6 +175,31 @@ def test_v1_packed_works_at_any_alignment(orig, works, off, base):
     assert bool((out[:off] == 3.0).all()) and bool((out[off + works * orig:] == 3.0).all())
 
 
+@pytest.mark.parametrize("step", [1, 7, 15, 16, 17, 31, 33, 1000])
+def test_v1_outliers_that_leave_an_unfinished_piece(step):
+    """Chunks of 0, step, 2 step, ... outliers, at random lanes: the unfinished 16-byte piece that a warp carries into its
+    next chunk has every length, and the next chunk's outliers start behind it.  Enough chunks for dozens per warp."""
+    n = 16 << 20
+    g = torch.Generator(device=DEV).manual_seed(step)
+    c = torch.arange(n // 1024, device=DEV)
+    per = (c * step) % 1025
+    order = torch.rand(n // 1024, 1024, generator=g, device=DEV).argsort(1)
+    exponent = torch.where(order < per[:, None], torch.randint(1, 116, (n // 1024, 1024), generator=g, device=DEV), 118)
+    x = (exponent << 7).to(torch.int16).view(torch.bfloat16).reshape(-1).contiguous()
+
+    def encode(v):
+        dev = v.device
+        n_8, bases = torch.full((1,), n, dtype=torch.int32, device=dev), torch.full((256,), 116, dtype=torch.int32, device=dev)
+        det, esc = (torch.zeros(m, dtype=torch.uint8, device=dev) for m in (codec.v1_det_bytes(n), n))
+        gc = torch.zeros(1, dtype=torch.int32, device=dev)
+        hz.compress_split_store(v, n_8, bases, det, torch.zeros(n, dtype=torch.uint8, device=dev), esc, gc, 1)
+        return det.cpu(), esc.cpu(), int(gc)
+
+    det, esc, count = encode(x)
+    detc, escc, countc = encode(x.cpu())
+    assert count == countc == int(per.sum()) and torch.equal(det, detc) and torch.equal(esc[:count], escc[:count])
+
+
 @pytest.mark.parametrize("n", [1, 7, 4095, 4096, 100_001, 3_000_003])
 def test_v1_base_statistic_sizes(n):
     for scale in (0.02, 3.0):
