@@ -29,6 +29,9 @@ enum : int { LAYOUT_SPLIT = 0, LAYOUT_FUSED = 1 };
 // The works' ranges are numbered one work after the other; range r covers `cnt` chunks from `c0` on, `part`
 // of them per warp.
 constexpr int V1_CHUNK = 1024;
+// Chunks of a work: of its whole blocks, which are what the stream has offsets for (a size that is not a multiple of a
+// block loses its rest, as it always has).
+__device__ __forceinline__ int v1_chunks(long long n) { return (int)(n / V1_BLOCK_ELEMS) * (V1_BLOCK_ELEMS / V1_CHUNK); }
 struct V1Range {
   int work;          // -1: no such range
   int c0, cnt;       // chunks inside the work
@@ -57,7 +60,7 @@ __device__ __forceinline__ void v1_locate(int r, int part, long long total_block
   w.work = -1;
   for (int i = 0; i < n_works; ++i) {
     const int n = __ldg(n_8 + i);
-    const int nc = n / V1_CHUNK, nr = (nc + per - 1) / per;
+    const int nc = v1_chunks(n), nr = (nc + per - 1) / per;
     if (r < first + nr) {
       const int c0 = (r - first) * per;
       long long cnt = min(per, nc - c0);
@@ -251,9 +254,9 @@ __global__ void __launch_bounds__(128) v1_place_kernel(
   }
   if (blockIdx.x == 0)
     for (int i = tid; i < n_works; i += 128)
-      if (n_8[i] == 0) {
+      if (v1_chunks(n_8[i]) == 0) {
         counts[i] = 0;
-        if (nbytes_8) nbytes_8[i] = 0;
+        if (nbytes_8) nbytes_8[i] = n_8[i] ? (int)align128(v1_det_bytes(n_8[i])) : 0;
       }
   __syncthreads();
   if (sw.work < 0) return;
@@ -267,7 +270,7 @@ __global__ void __launch_bounds__(128) v1_place_kernel(
   int first = 0;
   for (int j = 0; j < sw.work; ++j) {
     const long long n = n_8[j];
-    const int nr = ((int)(n / V1_CHUNK) + 4 * part - 1) / (4 * part);
+    const int nr = (v1_chunks(n) + 4 * part - 1) / (4 * part);
     if ((j & 3) == warp) {
       int t = 0;
 #pragma unroll 4

@@ -200,6 +200,31 @@ def test_v1_outliers_that_leave_an_unfinished_piece(step):
     assert count == countc == int(per.sum()) and torch.equal(det, detc) and torch.equal(esc[:count], escc[:count])
 
 
+def test_v1_works_that_end_inside_a_block_are_coded_up_to_their_last_whole_block():
+    """Sizes that are not a multiple of 4096: the stream has offsets for whole blocks, and the base stands behind the last."""
+    sizes = [6144, 4096, 2048, 10240]
+    x = torch.cat([gauss(s, seed=i) for i, s in enumerate(sizes)])
+    n_8 = torch.tensor(sizes, dtype=torch.int32, device=DEV)
+    bases = torch.full((256,), 118, dtype=torch.int32, device=DEV)
+    at = [0]
+    for s in sizes:
+        at.append(at[-1] + codec.align128(s + s // 8 * 3 + s // 4096 * 4 + 4))
+    det = torch.zeros(at[-1], dtype=torch.uint8, device=DEV)
+    scratch, esc = (torch.zeros(1 << 15, dtype=torch.uint8, device=DEV) for _ in range(2))
+    gc = torch.full((4,), -1, dtype=torch.int32, device=DEV)
+    hz.compress_split_store(x, n_8, bases, det, scratch, esc, gc, 4)
+    start = 0
+    for w, s in enumerate(sizes):
+        whole = s // 4096 * 4096
+        e = (bits(x[start:start + whole]).int() >> 7) & 255
+        out = (e < 118) | (e > 124)
+        assert int(gc[w]) == int(out.sum())
+        offsets = det[at[w] + s + s // 8 * 3:][:s // 4096 * 4 + 4].clone().view(torch.int32).tolist()
+        if whole:
+            assert offsets == [int(out[:4096 * b].sum()) for b in range(s // 4096)] + [118]
+        start += s
+
+
 @pytest.mark.parametrize("n", [1, 7, 4095, 4096, 100_001, 3_000_003])
 def test_v1_base_statistic_sizes(n):
     for scale in (0.02, 3.0):
