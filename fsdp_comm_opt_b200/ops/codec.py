@@ -75,7 +75,8 @@ def _total_blocks_hint(n_8: torch.Tensor, n_works: int, total_padded: int | None
 
 
 def _v1_totals(blocks: int, n_works: int, dev: torch.device) -> torch.Tensor:
-    """Device words for the per-range outlier totals between the two launches of an encode."""
+    """Device words for the per-range outlier totals between the two launches of an encode.  The caller holds them until
+    both are enqueued: freed before, another thread's allocation on the stream could come between."""
     return torch.empty(_lib.cuda().zc_v1_totals_words(blocks, n_works), dtype=torch.int32, device=dev)
 
 
@@ -121,11 +122,11 @@ def v1_compress_split_store(input, n_8, bases_in, output, output1, output_final,
     blocks = padded // ELEMS_PER_BLOCK
     if blocks == 0:
         return
+    totals = _v1_totals(blocks, n_works, dev)
     _lib.check(_lib.cuda().zc_v1_encode_split(
         input.data_ptr(), total_n, n_8.data_ptr(), _lib.ptr(_orig_n_8), n_works,
         bases_in.data_ptr(), output.data_ptr(), output1.data_ptr(), output_final.data_ptr(),
-        global_zero_counter_8.data_ptr(), _v1_totals(blocks, n_works, dev).data_ptr(), blocks, _lib.stream_ptr(dev)),
-        "zc_v1_encode_split")
+        global_zero_counter_8.data_ptr(), totals.data_ptr(), blocks, _lib.stream_ptr(dev)), "zc_v1_encode_split")
 
 
 def v1_compress_split_store_pad(input, n_8, orig_n_8, bases_in, output, output1, output_final,
@@ -224,11 +225,11 @@ def v1_compress_8(input, n_8, nbytes_8, bases_in, output, output_final, global_z
     blocks = padded // ELEMS_PER_BLOCK
     if blocks == 0:
         return
+    totals = _v1_totals(blocks, n_works, dev)
     _lib.check(_lib.cuda().zc_v1_encode_fused(
         input.data_ptr(), total_n, n_8.data_ptr(), n_works, bases_in.data_ptr(), output.data_ptr(),
         output_final.data_ptr(), output_final.numel(), nbytes_8.data_ptr(),
-        global_zero_counter_8.data_ptr(), _v1_totals(blocks, n_works, dev).data_ptr(), blocks, _lib.stream_ptr(dev)),
-        "zc_v1_encode_fused")
+        global_zero_counter_8.data_ptr(), totals.data_ptr(), blocks, _lib.stream_ptr(dev)), "zc_v1_encode_fused")
 
 
 def _v1_decode_fused(compressed_input, n_8, nbytes_8, output, n_works, orig_each=-1,

@@ -284,3 +284,36 @@ def test_v2_nibble_mode_size_and_escapes():
     rec, hdr = codec.v2_encode(y, nibble=True)
     assert int((hdr.view(torch.int32) >> 16).sum()) > 0     # escapes are present
     assert torch.equal(bits(codec.v2_decode(rec, hdr, y.numel(), nibble=True)), bits(y))
+
+
+@pytest.mark.parametrize("layout", ["split", "fused"])
+def test_the_totals_of_an_encode_are_held_until_both_kernels_are_enqueued(layout, monkeypatch):
+    import types
+    import weakref
+
+    held = []
+
+    class Totals(torch.Tensor):
+        pass
+
+    def totals(blocks, n_works, dev):
+        t = torch.zeros(8, dtype=torch.int32).as_subclass(Totals)
+        held.append(weakref.ref(t))
+        return t
+
+    def launch(*args):
+        assert held[-1]() is not None, "the workspace's memory may be given to another thread before the launches"
+        return 0
+
+    monkeypatch.setattr(codec, "_v1_totals", totals)
+    monkeypatch.setattr(codec, "_same_device", lambda *t: types.SimpleNamespace(type="cuda"))
+    monkeypatch.setattr(codec._lib, "stream_ptr", lambda dev: 0)
+    monkeypatch.setattr(codec._lib, "cuda", lambda: types.SimpleNamespace(zc_v1_encode_split=launch, zc_v1_encode_fused=launch))
+    n = 4096
+    x = torch.zeros(n, dtype=torch.bfloat16)
+    ints, buf = torch.full((1,), n, dtype=torch.int32), torch.zeros(4 * n, dtype=torch.uint8)
+    if layout == "split":
+        codec.v1_compress_split_store(x, ints, ints, buf, buf, buf, ints, 1)
+    else:
+        codec.v1_compress_8(x, ints, ints.clone(), ints, buf, buf.clone(), ints.clone(), 1)
+    assert len(held) == 1
