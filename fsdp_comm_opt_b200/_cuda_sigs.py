@@ -30,7 +30,10 @@ def declare(lib) -> None:
     _sig(lib, "zc_v1_encode_fused", P, L, P, I, P, P, P, L, P, P, P, L, P)
     _sig(lib, "zc_v1_decode_split", P, P, P, P, I, L, P, P, P, L, L, P)
     _sig(lib, "zc_v1_decode_fused", P, P, P, I, L, P, L, L, P)
-    _sig(lib, "zc_v1_base_from_std", P, L, P, P)
+    _sig(lib, "zc_v1_base_from_std", P, L, P, P, P)
+    _sig(lib, "zc_v1_moments_bytes")
+    if hasattr(lib, "zc_v1_moments_bytes"):
+        lib.zc_v1_moments_bytes.restype = L
     # elementwise / optimizer
     _sig(lib, "zc_rmsnorm_fwd", P, P, P, P, P, P, L, I, F, P)
     _sig(lib, "zc_rmsnorm_bwd", P, P, P, P, P, P, P, P, L, I, P)

@@ -17,8 +17,6 @@
 // before its first input load, synchronised to place its outliers, and needed a scan launch over all blocks
 // between encode and compaction.  A part finds its work once and has the next chunk's input in flight while
 // it codes the current one.
-#include <mutex>
-
 #include "codec_dev.cuh"
 #include "launch_util.h"
 
@@ -576,29 +574,15 @@ int zc_v1_decode_fused(const void* comp, const int* n_8, const int* nbytes_8, in
                    total_blocks, st);
 }
 
-// Workspaces: MOMENT_SLOTS per device, their counters zeroed once and left at zero by every launch; launches
-// take them in turn, so calls on different streams do not share one.
-int zc_v1_base_from_std(const void* x, long long n, int* bases, cudaStream_t st) {
+// Bytes of the workspace (16-byte aligned) of a base statistic.
+long long zc_v1_moments_bytes() { return sizeof(zc::Moments); }
+
+// `ws`: zero before its first use and left so by every launch; launches that share it have to follow one another.
+int zc_v1_base_from_std(const void* x, long long n, int* bases, void* ws, cudaStream_t st) {
   using namespace zc;
-  constexpr unsigned MOMENT_SLOTS = 256;
-  static Moments* acc[64] = {nullptr};
-  static unsigned turn[64] = {0};
-  static std::mutex mutex;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return ERR_BAD_ARG;
   if (n <= 0) return 0;
-  Moments* slot;
-  {
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!acc[dev]) {
-      if (cudaMalloc(&acc[dev], MOMENT_SLOTS * sizeof(Moments)) != cudaSuccess) return (int)cudaGetLastError();
-      cudaMemset(acc[dev], 0, MOMENT_SLOTS * sizeof(Moments));
-    }
-    slot = acc[dev] + turn[dev]++ % MOMENT_SLOTS;
-  }
   const int grid = (int)std::min<long long>(n / 8 / MOMENT_THREADS + 1, std::min(sm_count(), MOMENT_CTAS));
-  v1_base_kernel<<<grid, MOMENT_THREADS, 0, st>>>((const uint16_t*)x, n, slot, bases);
+  v1_base_kernel<<<grid, MOMENT_THREADS, 0, st>>>((const uint16_t*)x, n, (Moments*)ws, bases);
   return launch_status();
 }
 
@@ -608,6 +592,7 @@ int zc_v1_base_from_std(const void* x, long long n, int* bases, cudaStream_t st)
 // Allocation-free variant (see zc_noalloc.h): the outlier staging area is a static device array.
 // ---------------------------------------------------------------------------------------------
 #include <cstdio>
+#include <mutex>
 
 #include "zc_noalloc.h"
 

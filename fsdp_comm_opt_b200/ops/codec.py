@@ -303,12 +303,32 @@ def v1_decompress_8_padded(compressed_input: torch.Tensor, orig_numel: int, nbyt
     return out
 
 
+_MOMENTS: dict = {}
+
+
+def _moments(dev: torch.device) -> torch.Tensor:
+    """Zeroed workspace of the base statistic's kernel, which leaves it zeroed: one per stream, whose launches follow one
+    another, and one of its own, cleared at every replay, for a launch that is recorded into a graph and may be replayed on
+    any stream.  A stream's is dropped when 64 others have come since."""
+    capturing = torch.cuda.is_current_stream_capturing()
+    key = (dev.index, _lib.stream_ptr(dev))
+    ws = None if capturing else _MOMENTS.get(key)
+    if ws is None:
+        ws = torch.zeros(_lib.cuda().zc_v1_moments_bytes(), dtype=torch.uint8, device=dev)
+        if not capturing:
+            while len(_MOMENTS) >= 64:
+                _MOMENTS.pop(next(iter(_MOMENTS)), None)
+            _MOMENTS[key] = ws
+    return ws
+
+
 def v1_base_from_std(x: torch.Tensor, bases_out: torch.Tensor) -> None:
     """bases_out[0] = clamp(floor(log2(max(std(x), 1e-30)) - 5.35 + 127), 0, 255) without a host
     sync (reference: main/zipccl_comm.py:56-64, which runs six ATen kernels for this)."""
     _req(bases_out, torch.int32, "bases_out", 1)
     if x.device.type == "cuda" and x.dtype == torch.bfloat16 and x.is_contiguous():
-        _lib.check(_lib.cuda().zc_v1_base_from_std(x.data_ptr(), x.numel(), bases_out.data_ptr(),
+        ws = _moments(x.device)
+        _lib.check(_lib.cuda().zc_v1_base_from_std(x.data_ptr(), x.numel(), bases_out.data_ptr(), ws.data_ptr(),
                                                    _lib.stream_ptr(x.device)), "zc_v1_base_from_std")
         return
     std = x.float().std() if x.numel() > 1 else torch.zeros((), device=x.device)

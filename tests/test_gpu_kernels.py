@@ -284,6 +284,31 @@ def test_v1_base_statistic_kernel():
     assert int(bases[0]) == 116
 
 
+def test_v1_base_statistic_on_several_streams_and_replayed():
+    """Launches of different streams, and those of a recorded graph replayed beside them, have workspaces of their own."""
+    xs = [gauss(1 << 22, std=0.02 * 4 ** i, seed=i) for i in range(4)]
+    want = [math.floor(math.log2(x.double().std().item()) - 5.35 + 127.0) for x in xs]
+    outs = [torch.zeros(300, dtype=torch.int32, device=DEV) for _ in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    recorded = torch.zeros(1, dtype=torch.int32, device=DEV)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        codec.v1_base_from_std(xs[3], recorded)
+    torch.cuda.synchronize()
+    replays = []
+    for k in range(300):
+        for x, out, st in zip(xs[:3], outs, streams):
+            with torch.cuda.stream(st):
+                codec.v1_base_from_std(x, out[k:])
+        with torch.cuda.stream(streams[3]):
+            recorded.zero_()
+            graph.replay()
+            replays.append(recorded.clone())
+    torch.cuda.synchronize()
+    for out, w in zip(outs[:3] + [torch.cat(replays)], want):
+        assert bool((out == w).all())
+
+
 # ------------------------------------------------------------------ elementwise
 def test_rmsnorm_fwd_bwd():
     torch.manual_seed(0)
