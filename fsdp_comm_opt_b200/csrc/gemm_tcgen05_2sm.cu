@@ -539,14 +539,10 @@ static bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols
   return r == CUDA_SUCCESS;
 }
 
-// Per-device launch state: how many clusters of two the device runs at once, and the fp32 workspace
-// of the split tail (grown on demand, never shrunk; growing it is the only allocation this file
-// makes and it happens before the launch that needs it).
+// Per-device launch state: how many clusters of two the device runs at once, and the tile counters.
 struct DeviceState {
   bool ready = false;
   int clusters = 0;
-  float* partial = nullptr;
-  size_t partial_elems = 0;
   unsigned* counters = nullptr;  // COUNTER_SLOTS pairs, all zero between launches; launches take slots in turn
   unsigned next_slot = 0;
 };
@@ -587,6 +583,39 @@ static int single_split(int64_t tiles, int64_t k_blocks, int clusters) {
   return (int)((k_blocks + per - 1) / per);  // no empty slice
 }
 
+// How a product's tiles are cut along K: the last `split_tiles` of them into `split` slices each.
+struct Cut {
+  int64_t tiles;
+  int split = 1, split_tiles = 0, grid_clusters;
+  int64_t bytes() const { return split > 1 ? (int64_t)split_tiles * split * BM * BN * sizeof(float) : 0; }
+};
+static Cut cut_of(int64_t M, int64_t N, int64_t K, int device_clusters) {
+  static const int forced_split = getenv("ZC_GEMM_SPLIT") ? atoi(getenv("ZC_GEMM_SPLIT")) : -1;
+  Cut c;
+  c.tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int64_t k_blocks = (K + BK - 1) / BK;
+  const int clusters = c.grid_clusters = (int)std::min<int64_t>(c.tiles, device_clusters);
+  // Tail: the tiles of the last, partial wave are cut into K slices so that every cluster has one
+  // unit of about the same length to finish with.
+  const int64_t rem = c.tiles % clusters;
+  if (rem > 0 && c.tiles > clusters) {
+    int split = (int)std::min<int64_t>(std::min<int64_t>(clusters / rem, MAX_SPLIT), k_blocks / 8);
+    if (forced_split >= 0) split = std::min(forced_split, MAX_SPLIT);
+    if (split >= 2 && rem * 10 <= (int64_t)clusters * 8) {  // a nearly full last wave is left alone
+      c.split = split;
+      c.split_tiles = (int)rem;
+    }
+    return c;
+  }
+  const int single = single_split(c.tiles, k_blocks, device_clusters);
+  if (single > 1) {
+    c.split = single;
+    c.split_tiles = (int)c.tiles;
+    c.grid_clusters = (int)c.tiles * single;
+  }
+  return c;
+}
+
 static int init_state(DeviceState& ds, int smem) {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (!ds.ready) {
@@ -617,8 +646,8 @@ int* zc_gemm_status_word();  // gemm_tcgen05.cu: the current device's GEMM statu
 // (zc_gemm_status_read_and_clear; code 8 = a bounded wait of this kernel expired).
 // `bias`: null, or N bf16 values (16-byte aligned) added to every row of the product before it is rounded
 // (and before the old C is added when `accumulate` is set).
-// `ws`: null, or `ws_bytes` of device memory (16-byte aligned) of the caller's for the fp32 partial sums of a product
-// that zc_gemm_2sm_split_bytes names a size for; without it such a product is not split.
+// `ws`: null, or `ws_bytes` of device memory (16-byte aligned) of the caller's, that no other stream uses meanwhile, for the
+// fp32 partial sums of a product that zc_gemm_2sm_split_bytes names a size for; without it such a product is not split.
 int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
                         int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate, void* ws,
                         int64_t ws_bytes, cudaStream_t st) {
@@ -657,67 +686,31 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   p.bias = (const __nv_bfloat16*)bias;
   p.accumulate = accumulate;
   static const int forced_gm = getenv("ZC_GEMM_GROUP_M") ? atoi(getenv("ZC_GEMM_GROUP_M")) : 0;
-  static const int forced_split = getenv("ZC_GEMM_SPLIT") ? atoi(getenv("ZC_GEMM_SPLIT")) : -1;
   p.group_m = forced_gm > 0 ? forced_gm : 8;
   p.status = status;
-  const int64_t tiles = m_tiles * n_tiles;
-  const int64_t k_blocks = (K + BK - 1) / BK;
-  const int clusters = (int)std::min<int64_t>(tiles, ds.clusters);
-  // Tail: the tiles of the last, partial wave are cut into K slices so that every cluster has one
-  // unit of about the same length to finish with.
-  const int64_t rem = tiles % clusters;
-  int split = 1, grid_clusters = clusters;
-  if (rem > 0 && tiles > clusters) {
-    split = (int)std::min<int64_t>(std::min<int64_t>(clusters / rem, MAX_SPLIT), k_blocks / 8);
-    if (forced_split >= 0) split = std::min(forced_split, MAX_SPLIT);
-    if (split < 2 || rem * 10 > (int64_t)clusters * 8) split = 1;  // a nearly full last wave is left alone
+  Cut cut = cut_of(M, N, K, ds.clusters);
+  if (!ws || ws_bytes < cut.bytes()) {
+    cut.split = 1;
+    cut.grid_clusters = (int)std::min<int64_t>(cut.tiles, ds.clusters);
   }
-  int64_t rem_tiles = rem;
-  const int single = ws ? single_split(tiles, k_blocks, ds.clusters) : 1;
-  if (single > 1 && ws_bytes >= tiles * single * (int64_t)(BM * BN * sizeof(float))) {
-    split = single;
-    rem_tiles = tiles;
-    grid_clusters = (int)(tiles * split);
-  } else {
-    ws = nullptr;
-  }
-  p.split = split;
-  p.full_tiles = (int)(split > 1 ? tiles - rem_tiles : tiles);
+  p.split = cut.split;
+  p.full_tiles = (int)(cut.split > 1 ? cut.tiles - cut.split_tiles : cut.tiles);
+  p.partial = cut.split > 1 ? (float*)ws : nullptr;
   // Counters only where a second round is handed out, and not in a launch that is being recorded: a
   // replayed launch would keep its slot for good, next to launches of other streams that take slots in turn.
   p.counter = nullptr;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (tiles > clusters && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+  if (cut.tiles > ds.clusters && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
     std::lock_guard<std::mutex> lock(g_mutex);
     p.counter = ds.counters + 2 * (ds.next_slot++ % COUNTER_SLOTS);
   }
-  p.partial = nullptr;
-  if (split > 1 && ws) {
-    p.partial = (float*)ws;
-  } else if (split > 1) {
-    const size_t need = (size_t)rem * split * BM * BN;
-    std::lock_guard<std::mutex> lock(g_mutex);
-    if (ds.partial_elems < need) {
-      // earlier launches may still read the old buffer: drain the device before replacing it
-      if (ds.partial) { cudaDeviceSynchronize(); cudaFree(ds.partial); ds.partial = nullptr; ds.partial_elems = 0; }
-      const size_t want = std::max(need, (size_t)ds.clusters * BM * BN);
-      if (cudaMalloc(&ds.partial, want * sizeof(float)) != cudaSuccess) {
-        cudaGetLastError();
-        p.split = 1;
-        p.full_tiles = (int)tiles;
-      } else {
-        ds.partial_elems = want;
-      }
-    }
-    p.partial = ds.partial;
-  }
-  const dim3 grid(2 * grid_clusters);
+  const dim3 grid(2 * cut.grid_clusters);
   if (a_major == MAJOR_K && b_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_K><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   else if (a_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   else gemm_2sm_kernel<MAJOR_MN, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   int rc = launch_status();
   if (rc == 0 && p.split > 1) {
-    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)rem_tiles), 256, 0, st>>>(p, (int)m_tiles, (int)n_tiles);
+    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st>>>(p, (int)m_tiles, (int)n_tiles);
     rc = launch_status();
   }
   return rc;
@@ -736,9 +729,7 @@ int64_t zc_gemm_2sm_split_bytes(int64_t M, int64_t N, int64_t K) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (M <= 0 || N <= 0 || K <= 0 || dev < 0 || dev >= 64 || init_state(g_state[dev], STAGES * STAGE + 1024)) return 0;
-  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int split = single_split(tiles, (K + BK - 1) / BK, g_state[dev].clusters);
-  return split > 1 ? tiles * split * (int64_t)(BM * BN * sizeof(float)) : 0;
+  return cut_of(M, N, K, g_state[dev].clusters).bytes();
 }
 
 int zc_gemm_bf16_2sm_ld(const void* A, const void* B, void* C, int64_t M, int64_t N, int64_t K, int64_t lda,

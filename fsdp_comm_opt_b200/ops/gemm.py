@@ -14,14 +14,12 @@ copy of the weight or the activations is made.  CPU tensors always use ``torch.m
 """
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
 
 from .. import _lib
-
-# above this a product's 256 x 256 tiles occupy more than half of the 74 pairs of SMs: it is not split along K
-_SPLIT_MAX_OUT = 37 * 256 * 256
 
 _BACKEND = os.environ.get("ZC_GEMM_BACKEND", "auto")
 
@@ -42,6 +40,11 @@ def _rows_ok(t: torch.Tensor) -> bool:
     apart (a slice ``buf[:, :n]`` of a padded buffer qualifies), 16-byte aligned base."""
     return (t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1]
             and t.data_ptr() % 16 == 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def _split_bytes(M: int, N: int, K: int, device: int) -> int:
+    return _lib.cuda().zc_gemm_2sm_split_bytes(M, N, K)
 
 
 def _pad8(n: int) -> int:
@@ -91,7 +94,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
             fused_bias = (bias is not None and bias.dtype == torch.bfloat16 and bias.is_contiguous()
                           and bias.numel() == N and bias.data_ptr() % 16 == 0)
             # fp32 partial sums of a product that is split along K: this call's own, so that no other stream shares them
-            ws_bytes = lib.zc_gemm_2sm_split_bytes(M, N, K) if M * N <= _SPLIT_MAX_OUT else 0
+            ws_bytes = _split_bytes(M, N, K, a.device.index)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device) if ws_bytes else None
             _lib.check(lib.zc_gemm_bf16_2sm_ws(
                 a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if fused_bias else None, M, N, K,

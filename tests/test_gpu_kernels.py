@@ -789,6 +789,30 @@ def test_gemm_split_along_k_when_tiles_are_few(M, N, K):
         assert ((acc.double() - (ref + y.double())).norm() / ref.norm()).item() < 2 ** -8 + 1e-5
 
 
+def test_products_split_along_k_on_two_streams_have_partial_sums_of_their_own():
+    """The tail of the last wave is split (4096 x 6144: 384 tiles on 74 clusters), and so is a product of few tiles; the slices
+    are added by a second kernel, which other streams' products may run ahead of."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(5)
+    cases = [[(torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV).bfloat16()) for _ in range(2)]
+             for m, n, k in ((4096, 6144, 1024), (512, 512, 8192))]
+    for m, n, k in ((4096, 6144, 1024), (512, 512, 8192)):
+        assert _lib.cuda().zc_gemm_2sm_split_bytes(m, n, k) > 0
+    for pair in cases:
+        alone = [gemm.gemm(x, w, False, True) for x, w in pair]
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in pair]
+        got = [[], []]
+        for _ in range(20):
+            for st, (x, w), out in zip(streams, pair, got):
+                with torch.cuda.stream(st):
+                    out.append(gemm.gemm(x, w, False, True))
+        torch.cuda.synchronize()
+        for ref, out in zip(alone, got):
+            assert all(torch.equal(ref, y) for y in out)
+
+
 def test_gemm_with_leading_dimensions_and_odd_sizes():
     """Operands and results that are slices of wider buffers, and M / N / K that are not multiples of 8
     (GPT-2's vocabulary): the two-SM kernel takes row strides, zero-fills what lies outside a slice and
