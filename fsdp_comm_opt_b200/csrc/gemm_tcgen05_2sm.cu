@@ -548,6 +548,9 @@ struct DeviceState {
 };
 static DeviceState g_state[64];
 static std::mutex g_mutex;
+// The counters.  Zero from the module's load: a cleared allocation would have to be waited for by the first launch on every
+// stream, which the legacy stream's memset is not ordered with.
+static __device__ unsigned g_counters[2 * COUNTER_SLOTS];
 
 template <int A_MAJOR, int B_MAJOR>
 static int max_clusters(int smem) {
@@ -623,8 +626,7 @@ static int init_state(DeviceState& ds, int smem) {
     c = std::min(c, max_clusters<MAJOR_K, MAJOR_MN>(smem));
     c = std::min(c, max_clusters<MAJOR_MN, MAJOR_MN>(smem));
     ds.clusters = c;
-    if (cudaMalloc(&ds.counters, 2 * COUNTER_SLOTS * sizeof(unsigned)) != cudaSuccess) return ERR_BAD_ARG;
-    cudaMemset(ds.counters, 0, 2 * COUNTER_SLOTS * sizeof(unsigned));
+    if (cudaGetSymbolAddress((void**)&ds.counters, g_counters) != cudaSuccess) return ERR_BAD_ARG;
     ds.ready = true;
   }
   return 0;
