@@ -7,8 +7,9 @@ communication and its tensors stay where they are (parameters and gradients are 
 buffers), so the launches of forward and backward are recorded once per batch shape and replayed.  The
 optimizer runs outside the graph: its learning rate and bias corrections change every step.
 
-A shape is recorded after it has been run ``EAGER_STEPS`` times; up to ``MAX_SHAPES`` shapes are kept, the least
-recently used one is dropped first.  Steps run eagerly, as they would without this module, whenever a
+A shape is recorded after it has been run ``EAGER_STEPS`` times.  Up to ``MAX_SHAPES`` shapes are kept, and one gives way
+to another only after ``IDLE_STEPS`` steps without it: a recording costs more than an eager step, and batches of more
+shapes than are kept would pay for one at every step if the least recently used made room.  Steps run eagerly, as they would without this module, whenever a
 replay could differ from that: hooks added to a module or a parameter, autocast, anomaly detection, a
 capture that is already under way, another GEMM or attention implementation selected since, moved storage.
 """
@@ -23,12 +24,13 @@ from ..ops import attention, gemm, rope
 
 
 class _Recorded:
-    __slots__ = ("graph", "ids", "loss", "key", "keep", "launches")
+    __slots__ = ("graph", "ids", "loss", "key", "keep", "launches", "used")
 
 
 class StepGraphs:
     EAGER_STEPS = 2
-    MAX_SHAPES = 4
+    MAX_SHAPES = 16    # all of one memory pool: they share their activations' memory
+    IDLE_STEPS = 1024
     # A graph's activations live in a pool of their own beside the allocator's: recorded only where that
     # is small against the memory left.
     MAX_BYTES = 8 << 30
@@ -42,6 +44,7 @@ class StepGraphs:
         self._seen: dict = {}
         self._recorded: OrderedDict = OrderedDict()
         self._refused: set = set()
+        self._steps = 0
         self._stream = None
         self._pool = None
 
@@ -88,9 +91,11 @@ class StepGraphs:
             return None
         shape = tuple(ids.shape)
         key = self._key()
+        self._steps += 1
         rec = self._recorded.get(shape)
         if rec is not None and rec.key != key:
             del self._recorded[shape]
+            self._seen[shape] = 0
             rec = None
         if rec is None:
             if shape in self._refused:
@@ -101,6 +106,9 @@ class StepGraphs:
                     self._seen.clear()
                 self._seen[shape] = seen + 1
                 return None
+            full = len(self._recorded) >= self.MAX_SHAPES
+            if full and self._steps - next(iter(self._recorded.values())).used < self.IDLE_STEPS:
+                return None
             free, _ = torch.cuda.mem_get_info(self.flat.device)
             free += torch.cuda.memory_reserved(self.flat.device) - torch.cuda.memory_allocated(self.flat.device)
             if (not self._host_bound(ids.numel())
@@ -109,11 +117,11 @@ class StepGraphs:
                     self._refused.clear()
                 self._refused.add(shape)
                 return None
-            rec = self._record(shape, key)
-            while len(self._recorded) >= self.MAX_SHAPES:
+            if full:
                 self._recorded.popitem(last=False)
-            self._recorded[shape] = rec
+            rec = self._recorded[shape] = self._record(shape, key)
         self._recorded.move_to_end(shape)
+        rec.used = self._steps
         rec.ids.copy_(ids, non_blocking=True)
         rec.graph.replay()
         _lib.add_launches(rec.launches)

@@ -152,3 +152,25 @@ def _many_lengths_worker(rank, world):
 
 def test_steps_of_many_lengths_equal_eager_steps():
     run_ranks(_many_lengths_worker, 1, backend="nccl")
+
+
+def _many_shapes_worker(rank, world):
+    from fsdp_comm_opt_b200.parallel.step_graph import StepGraphs
+
+    StepGraphs.MAX_SHAPES, StepGraphs.IDLE_STEPS = 4, 40
+    recorded, record = [], StepGraphs._record
+
+    def counted(self, shape, *rest):
+        recorded.append(shape)
+        return record(self, shape, *rest)
+
+    StepGraphs._record = counted
+    a, b = _engines()
+    _same_steps(a, b, [(1, 64 + 16 * (i % 6)) for i in range(48)])      # six shapes in turn, room for four
+    assert recorded == [(1, 64 + 16 * i) for i in range(4)]
+    _same_steps(a, b, [(2, 64 + 16 * (i % 2)) for i in range(45)])      # two others replace those that went idle
+    assert recorded[4:] == [(2, 64), (2, 80)] and set(recorded[4:]) < set(a._graphs._recorded)
+
+
+def test_more_shapes_than_are_kept_do_not_record_at_every_step():
+    run_ranks(_many_shapes_worker, 1, backend="nccl")
