@@ -138,6 +138,7 @@ class StepGraphs:
         rec.graph = torch.cuda.CUDAGraph()
         if self._stream is None:
             self._stream = torch.cuda.Stream(dev)
+        if not self._recorded:  # a pool ends with its last graph
             self._pool = torch.cuda.graph_pool_handle()
         cur = torch.cuda.current_stream(dev)
         before = _lib.launch_count()

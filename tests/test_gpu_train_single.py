@@ -174,3 +174,20 @@ def _many_shapes_worker(rank, world):
 
 def test_more_shapes_than_are_kept_do_not_record_at_every_step():
     run_ranks(_many_shapes_worker, 1, backend="nccl")
+
+
+def _key_change_worker(rank, world):
+    from fsdp_comm_opt_b200.ops import gemm
+
+    a, b = _engines()
+    shape = (2, 96)
+    for change in (lambda e: None, lambda e: setattr(e.model, "activation_checkpointing", True), lambda e: e.model.eval(),
+                   lambda e: gemm.set_backend("cublas")):
+        change(a), change(b)
+        graph = next((r.graph for r in a._graphs._recorded.values()), None)
+        _same_steps(a, b, [shape] * 4)
+        assert a._graphs._recorded[shape].graph is not graph
+
+
+def test_the_only_recorded_shape_is_recorded_again_when_an_option_changes():
+    run_ranks(_key_change_worker, 1, backend="nccl")
