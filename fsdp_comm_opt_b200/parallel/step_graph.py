@@ -31,8 +31,8 @@ class StepGraphs:
     EAGER_STEPS = 2
     MAX_SHAPES = 16    # all of one memory pool: they share their activations' memory
     IDLE_STEPS = 1024
-    # A graph's activations live in a pool of their own beside the allocator's: recorded only where that
-    # is small against the memory left.
+    # A graph's activations live in a pool of their own beside the allocator's, which gives none of its cached
+    # blocks back during a recording: recorded only where they are small against the memory that nobody has taken.
     MAX_BYTES = 8 << 30
     MAX_FREE_FRACTION = 0.125
 
@@ -110,7 +110,6 @@ class StepGraphs:
             if full and self._steps - next(iter(self._recorded.values())).used < self.IDLE_STEPS:
                 return None
             free, _ = torch.cuda.mem_get_info(self.flat.device)
-            free += torch.cuda.memory_reserved(self.flat.device) - torch.cuda.memory_allocated(self.flat.device)
             if (not self._host_bound(ids.numel())
                     or self._activation_bytes(ids.numel()) > min(self.MAX_BYTES, self.MAX_FREE_FRACTION * free)):
                 if len(self._refused) > 256:

@@ -191,3 +191,19 @@ def _key_change_worker(rank, world):
 
 def test_the_only_recorded_shape_is_recorded_again_when_an_option_changes():
     run_ranks(_key_change_worker, 1, backend="nccl")
+
+
+def _little_memory_worker(rank, world):
+    import torch
+
+    a, b = _engines()
+    # 4 GB that the allocator has cached and, as the driver is made to say here, little else
+    torch.empty(1 << 32, dtype=torch.uint8, device="cuda")
+    info = torch.cuda.mem_get_info
+    torch.cuda.mem_get_info = lambda *x: (64 << 20, info(*x)[1])
+    _same_steps(a, b, [(2, 512)] * 4)
+    assert not a._graphs._recorded
+
+
+def test_cached_blocks_of_the_allocator_are_no_room_for_a_recording():
+    run_ranks(_little_memory_worker, 1, backend="nccl")
