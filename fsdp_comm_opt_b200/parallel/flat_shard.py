@@ -588,6 +588,13 @@ class FlatShardEngine:
         for g in self.groups:
             self._reshard(g)
 
+    def drop_gradients(self) -> None:
+        """Forget what a backward pass that was given up half way has left (one rank: nothing is in flight)."""
+        for g in self.groups:
+            g.grads_ready = False
+            for s in g.slots:
+                s.param.grad = None
+
     def wait_for_gradients(self) -> None:
         if self.cuda:
             cur = self._current()

@@ -12,9 +12,13 @@ to another only after ``IDLE_STEPS`` steps without it: a recording costs more th
 shapes than are kept would pay for one at every step if the least recently used made room.  Steps run eagerly, as they would without this module, whenever a
 replay could differ from that: hooks added to a module or a parameter, autocast, anomaly detection, a
 capture that is already under way, another GEMM or attention implementation selected since, moved storage.
+A recording that fails (no memory for the graph, a call that no recording may make) is given up, the step runs
+eagerly and so do all later ones.
 """
 from __future__ import annotations
 
+import contextlib
+import warnings
 from collections import OrderedDict
 
 import torch
@@ -45,6 +49,7 @@ class StepGraphs:
         self._recorded: OrderedDict = OrderedDict()
         self._refused: set = set()
         self._steps = 0
+        self._failed = False
         self._stream = None
         self._pool = None
 
@@ -87,7 +92,7 @@ class StepGraphs:
 
     def run(self, ids: torch.Tensor):
         """Forward and backward of ``ids`` by replay; None when this step has to run eagerly."""
-        if ids.dim() != 2 or ids.dtype != torch.int64 or not self._allowed():
+        if self._failed or ids.dim() != 2 or ids.dtype != torch.int64 or not self._allowed():
             return None
         shape = tuple(ids.shape)
         key = self._key()
@@ -118,7 +123,14 @@ class StepGraphs:
                 return None
             if full:
                 self._recorded.popitem(last=False)
-            rec = self._recorded[shape] = self._record(shape, key)
+            try:
+                rec = self._record(shape, key)
+            except Exception as e:
+                warnings.warn(f"training steps run without CUDA graphs from here on: {type(e).__name__}: {e}")
+                self._failed = True
+                self._recorded.clear()
+                return None
+            self._recorded[shape] = rec
         self._recorded.move_to_end(shape)
         rec.used = self._steps
         rec.ids.copy_(ids, non_blocking=True)
@@ -150,8 +162,13 @@ class StepGraphs:
                 self.flat.backward(out.loss)
                 rec.loss = out.loss.detach()
                 del out
-            finally:
-                rec.graph.capture_end()
+            except BaseException:
+                self.flat.drop_gradients()
+                _lib.add_launches(before - _lib.launch_count())
+                with contextlib.suppress(RuntimeError):  # the first error is the one to report
+                    rec.graph.capture_end()
+                raise
+            rec.graph.capture_end()
         cur.wait_stream(self._stream)
         rec.launches = _lib.launch_count() - before
         _lib.add_launches(-rec.launches)  # recorded, not run

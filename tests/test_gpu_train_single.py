@@ -207,3 +207,38 @@ def _little_memory_worker(rank, world):
 
 def test_cached_blocks_of_the_allocator_are_no_room_for_a_recording():
     run_ranks(_little_memory_worker, 1, backend="nccl")
+
+
+def _failed_recording_worker(rank, world, where):
+    import warnings
+
+    import torch
+
+    from fsdp_comm_opt_b200.ops import swiglu
+    from fsdp_comm_opt_b200.parallel.step_graph import StepGraphs
+
+    attempts, record = [], StepGraphs._record
+    StepGraphs._record = lambda self, *x: (attempts.append(x), record(self, *x))[1]
+    a, b = _engines()
+
+    def out_of_memory(*x):
+        if torch.cuda.is_current_stream_capturing():
+            raise torch.OutOfMemoryError("no block for the recording")
+
+    if where == "forward":
+        call = swiglu.swiglu
+        swiglu.swiglu = lambda x: (out_of_memory(x), call(x))[1]
+    else:                                                               # half of the gradients are in place by then
+        pre = a.flat._pre_backward
+        a.flat._pre_backward = lambda g: (out_of_memory(g) if g.name == "layers.0" else None, pre(g))[1]
+    with warnings.catch_warnings(record=True) as caught:
+        warnings.simplefilter("always")
+        _same_steps(a, b, [(2, 96)] * 4 + [(2, 64)] * 4)
+    assert len(attempts) == 1 and not a._graphs._recorded
+    assert sum("no block for the recording" in str(w.message) for w in caught) == 1
+    assert all(p.grad is None for p in a.model.parameters())
+
+
+@pytest.mark.parametrize("where", ["forward", "backward"])
+def test_a_recording_that_fails_leaves_the_step_to_run_eagerly(where):
+    run_ranks(_failed_recording_worker, 1, backend="nccl", args=(where,))
