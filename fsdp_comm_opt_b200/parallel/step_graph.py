@@ -103,7 +103,7 @@ class StepGraphs:
             self._seen[shape] = 0
             rec = None
         if rec is None:
-            if shape in self._refused:
+            if (shape, key) in self._refused:
                 return None
             seen = self._seen.get(shape, 0)
             if seen < self.EAGER_STEPS:
@@ -119,7 +119,7 @@ class StepGraphs:
                     or self._activation_bytes(ids.numel()) > min(self.MAX_BYTES, self.MAX_FREE_FRACTION * free)):
                 if len(self._refused) > 256:
                     self._refused.clear()
-                self._refused.add(shape)
+                self._refused.add((shape, key))
                 return None
             if full:
                 self._recorded.popitem(last=False)

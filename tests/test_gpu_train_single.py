@@ -242,3 +242,25 @@ def _failed_recording_worker(rank, world, where):
 @pytest.mark.parametrize("where", ["forward", "backward"])
 def test_a_recording_that_fails_leaves_the_step_to_run_eagerly(where):
     run_ranks(_failed_recording_worker, 1, backend="nccl", args=(where,))
+
+
+def _refusal_worker(rank, world):
+    import torch
+
+    a, b = _engines(n_layers=16)
+    bytes_of = a._graphs._activation_bytes
+    need = bytes_of(2 * 512)
+    a.model.activation_checkpointing = True
+    room = bytes_of(2 * 512)
+    a.model.activation_checkpointing = False
+    info = torch.cuda.mem_get_info
+    torch.cuda.mem_get_info = lambda *x: (4 * (room + need), info(*x)[1])   # an eighth of it: between the two
+    _same_steps(a, b, [(2, 512)] * 3)
+    assert not a._graphs._recorded
+    a.model.activation_checkpointing = b.model.activation_checkpointing = True
+    _same_steps(a, b, [(2, 512)] * 3)
+    assert len(a._graphs._recorded) == 1
+
+
+def test_a_shape_that_was_too_large_is_recorded_once_it_fits():
+    run_ranks(_refusal_worker, 1, backend="nccl")
