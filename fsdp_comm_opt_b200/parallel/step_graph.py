@@ -10,8 +10,10 @@ optimizer runs outside the graph: its learning rate and bias corrections change 
 A shape is recorded after it has been run ``EAGER_STEPS`` times.  Up to ``MAX_SHAPES`` shapes are kept, and one gives way
 to another only after ``IDLE_STEPS`` steps without it: a recording costs more than an eager step, and batches of more
 shapes than are kept would pay for one at every step if the least recently used made room.  Steps run eagerly, as they would without this module, whenever a
-replay could differ from that: hooks added to a module or a parameter, autocast, anomaly detection, a
-capture that is already under way, another GEMM or attention implementation selected since, moved storage.
+replay could differ from that: hooks added to a module, to a parameter or to all modules, modules or parameters put
+in place of the model's own, a ``forward`` or an epsilon set on one of them, moved storage, saved-tensor hooks, dispatch
+and function modes, autocast, anomaly detection, a capture that is already under way.  A shape is recorded again when
+another GEMM or attention implementation has been selected since.
 A recording that fails (no memory for the graph, a call that no recording may make) is given up, the step runs
 eagerly and so do all later ones.
 """
@@ -22,9 +24,25 @@ import warnings
 from collections import OrderedDict
 
 import torch
+from torch import overrides
+from torch.nn.modules import module
+from torch.utils._device import DeviceContext
 
 from .. import _lib
 from ..ops import attention, gemm, rope
+
+
+def _modes() -> bool:
+    """Whether something watches or replaces every operation or saved tensor of this thread, or every module call."""
+    return bool(torch._C._len_torch_dispatch_stack()
+                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+                or module._has_any_global_hook()
+                # a default device is a function mode too, and changes nothing here
+                or any(not isinstance(m, DeviceContext) for m in overrides._get_current_function_mode_stack()))
+
+
+def _address(t):
+    return None if t is None else t.data_ptr()
 
 
 class _Recorded:
@@ -42,9 +60,15 @@ class StepGraphs:
 
     def __init__(self, model, flat, cfg):
         self.model, self.flat, self.cfg = model, flat, cfg
+        # the model as the engine has built it; the objects are kept, so that no other one can have their identity
         self._modules = list(model.modules())
         self._params = list(model.parameters())
-        self._expected_hooks = self._hooks()
+        self._hook_dicts = [d for m in self._modules for d in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
+                                                               m._backward_pre_hooks)]
+        self._child_dicts = [d for m in self._modules for d in (m._modules, m._parameters) if d]
+        self._attrs = [m.__dict__ for m in self._modules]
+        self._with_eps = [m for m in self._modules if hasattr(m, "eps")]
+        self._built = self._state()
         self._seen: dict = {}
         self._recorded: OrderedDict = OrderedDict()
         self._refused: set = set()
@@ -54,13 +78,16 @@ class StepGraphs:
         self._pool = None
 
     # -- when a replay is the same as running the step ---------------------------------------------
-    def _hooks(self) -> int:
-        n = 0
-        for m in self._modules:
-            n += len(m._forward_hooks) + len(m._forward_pre_hooks) + len(m._backward_hooks) + len(m._backward_pre_hooks)
-        for p in self._params:
-            n += (p._backward_hooks is not None) + (not p.requires_grad) + (p.grad is not None)
-        return n
+    def _state(self) -> list:
+        """What the model is made of, apart from the values of its parameters."""
+        return [
+            [key for d in self._hook_dicts if d for key in d],
+            [id(x) for d in self._child_dicts for x in d.values()],
+            ["forward" in d for d in self._attrs],
+            [m.eps for m in self._with_eps],
+            [(p.data_ptr(), _address(getattr(p, "main_grad", None)), p.requires_grad, p.grad is None,
+              not p._backward_hooks, not p._post_accumulate_grad_hooks) for p in self._params],
+        ]
 
     def _key(self):
         f = self.flat
@@ -69,7 +96,7 @@ class StepGraphs:
 
     def _allowed(self) -> bool:
         return (torch.is_grad_enabled() and not torch.is_anomaly_enabled() and not torch.is_autocast_enabled("cuda")
-                and not torch.cuda.is_current_stream_capturing() and self._hooks() == self._expected_hooks)
+                and not torch.cuda.is_current_stream_capturing() and not _modes() and self._state() == self._built)
 
     def _activation_bytes(self, tokens: int) -> int:
         """What forward and backward hold at once, from the tensors that the blocks save."""

@@ -264,3 +264,81 @@ def _refusal_worker(rank, world):
 
 def test_a_shape_that_was_too_large_is_recorded_once_it_fits():
     run_ranks(_refusal_worker, 1, backend="nccl")
+
+
+def _guard_worker(rank, world):
+    import torch
+
+    from fsdp_comm_opt_b200.parallel.step_graph import StepGraphs
+
+    StepGraphs.MAX_SHAPES = 1
+    a, b = _engines()
+    shape = (2, 96)
+    replayed, run = [], StepGraphs.run
+    StepGraphs.run = lambda self, ids: (replayed.append(run(self, ids)), replayed[-1])[1]
+
+    def steps(eager):
+        replayed.clear()
+        _same_steps(a, b, [shape] * 2)
+        assert all((r is None) == eager for r in replayed) and len(replayed) == 2
+
+    _same_steps(a, b, [shape] * 3)
+    steps(False)
+    seen = []
+    norm, head = a.model.model.norm, a.model.lm_head
+    both = [(e.model.model.norm, e.model.lm_head) for e in (a, b)]
+
+    def called(*x):
+        seen.append(1)
+
+    # what is called, packed or counted at every step has to be so while it is there, and only then
+    for watch in (lambda: norm.weight.register_hook(called),
+                  lambda: norm.weight.register_post_accumulate_grad_hook(called),
+                  lambda: head.register_forward_hook(called),
+                  lambda: torch.nn.modules.module.register_module_forward_hook(called)):
+        handle = watch()
+        seen.clear()
+        steps(True)
+        assert seen
+        handle.remove()
+        seen.clear()
+        steps(False)
+        assert not seen
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (called(), t)[1], lambda t: t):
+        steps(True)
+    assert seen
+    # a hook in the place of another
+    hooks = next(m._forward_hooks for m in a.model.modules() if m._forward_hooks)
+    key, old = next(iter(hooks.items()))
+    del hooks[key]
+    hooks[key + 100_000] = old
+    steps(True)
+    del hooks[key + 100_000]
+    hooks[key] = old
+    steps(False)
+    # other parts in the place of the model's own
+    for n, h in both:
+        n.eps = 0.5
+    steps(True)
+    for n, h in both:
+        n.eps = a.model_config.norm_eps
+        n.weight.data = n.weight.data.clone()
+    steps(True)
+    for n, h in both:
+        e = a if n is norm else b
+        g = e.flat.groups[-1]
+        e.flat._replace_param_storage(g, g.full)
+        own = h.forward
+        h.forward = lambda x, own=own: own(x) * 0.5
+    steps(True)
+    for n, h in both:
+        del h.forward
+    steps(False)
+    for e in (a, b):
+        e.model.model.layers[1] = torch.nn.Identity()                   # x alone: unpacking it as (x, delta) would fail
+        e.model.model.layers[1].forward = lambda x, delta: (x, delta)
+    steps(True)
+
+
+def test_steps_with_hooks_modes_or_replaced_parts_run_eagerly():
+    run_ranks(_guard_worker, 1, backend="nccl")
