@@ -12,12 +12,11 @@ from typing import Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
-from torch.utils.checkpoint import checkpoint
 
 from ..ops import attention as attn_ops
 from ..ops import gemm, gpt2_ops, loss as loss_ops
 from .config import ModelConfig
-from .llama import CausalLMOutput, Embedding
+from .llama import CausalLMOutput, Embedding, recomputed
 
 
 class BiasLinear(nn.Module):
@@ -96,7 +95,7 @@ class GPT2ForCausalLM(nn.Module):
         x, m = t.wte(input_ids), t.wpe(pos)[None].expand(B, S, -1)   # the position add runs in the first norm
         for blk in t.h:
             if self.activation_checkpointing and torch.is_grad_enabled():
-                x, m = checkpoint(blk, x, m, use_reentrant=False, preserve_rng_state=False)
+                x, m = recomputed(blk, x, m)
             else:
                 x, m = blk(x, m)
         x, _ = gpt2_ops.add_layer_norm(x, m, t.ln_f.weight, t.ln_f.bias, t.ln_f.eps)

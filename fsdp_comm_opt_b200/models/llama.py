@@ -115,6 +115,14 @@ class LlamaBackbone(nn.Module):
         self.norm = RMSNorm(cfg.d_model, cfg.norm_eps)
 
 
+def recomputed(block, x, delta):
+    """A block whose activations are computed again in backward, with the random numbers of the first time (a dropout that
+    was added to it keeps its mask).  The generators cannot be read while a CUDA graph is recorded; the engine records
+    models as it has built them only, and those draw none."""
+    capturing = x.is_cuda and torch.cuda.is_current_stream_capturing()
+    return checkpoint(block, x, delta, use_reentrant=False, preserve_rng_state=not capturing)
+
+
 class LlamaForCausalLM(nn.Module):
     def __init__(self, cfg: ModelConfig):
         super().__init__()
@@ -136,7 +144,7 @@ class LlamaForCausalLM(nn.Module):
         x, delta = self.model.embed_tokens(input_ids), None
         for layer in self.model.layers:
             if self.activation_checkpointing and torch.is_grad_enabled():
-                x, delta = checkpoint(layer, x, delta, use_reentrant=False, preserve_rng_state=False)
+                x, delta = recomputed(layer, x, delta)
             else:
                 x, delta = layer(x, delta)
         x = self.model.norm(x, delta)

@@ -195,3 +195,29 @@ def test_gemm_from_codec_records_cpu():
     assert torch.equal(y, ref) and torch.equal(linear_t_plain(x, rec, hdr, N, K), ref)
     with pytest.raises(ValueError):
         RecordLinear(N, K, "cpu", slab_rows=100)
+
+
+@pytest.mark.parametrize("shape", ["tiny", "gpt2-tiny"])
+def test_a_dropout_added_to_a_recomputed_block_keeps_its_mask(shape):
+    import dataclasses
+
+    from fsdp_comm_opt_b200.models import build_model, decoder_layers, get_config
+
+    masks = []
+
+    class Dropout(torch.nn.Dropout):
+        def forward(self, x):
+            y = super().forward(x)
+            masks.append((y != 0).clone())
+            return y
+
+    torch.manual_seed(0)
+    model = build_model(dataclasses.replace(get_config(shape), vocab_size=64, n_layers=1))
+    model.init_weights()
+    model.activation_checkpointing = True
+    block = decoder_layers(model)[0]
+    name = "wo" if shape == "tiny" else "c_proj"
+    setattr(block, name, torch.nn.Sequential(Dropout(0.5), getattr(block, name)))
+    ids = torch.randint(0, 64, (1, 16))
+    model(input_ids=ids, labels=ids).loss.backward()
+    assert len(masks) > 1 and all(torch.equal(m, masks[0]) for m in masks[1:])
