@@ -725,6 +725,60 @@ def test_embedding_gradient_in_the_flat_buffer(n, dim, rows, accumulate):
     hook.remove()
 
 
+@pytest.mark.parametrize("draw", ["equal", "half", "zipf", "nine"])
+@pytest.mark.parametrize("n,dim", [(4096, 4096), (8192, 8192), (4096, 1600), (8192, 200)])
+def test_embedding_gradient_of_frequent_ids(n, dim, draw):
+    """A padded batch, half of one, word frequencies, and ids just frequent enough to be divided over blocks: the sums, and
+    no more time than PyTorch's sorted gradient and its copy take."""
+    from fsdp_comm_opt_b200.ops.embedding import embedding
+
+    torch.manual_seed(dim)
+    rows = 2000
+    ids = torch.randint(0, rows, (n,), device=DEV)
+    if draw == "equal":
+        ids.fill_(7)
+    elif draw == "half":
+        ids[n // 2:] = 7
+    elif draw == "zipf":
+        ids = torch.multinomial(1.0 / torch.arange(1, rows + 1, device=DEV), n, replacement=True)
+    else:
+        ids = torch.arange(n, device=DEV) // 9
+    w = torch.nn.Parameter(torch.zeros(rows, dim, dtype=torch.bfloat16, device=DEV))
+    w.main_grad = torch.ones_like(w)
+    w.main_grad_written = False
+    g = torch.randn(n, dim, device=DEV).bfloat16()
+    out = embedding(ids, w)
+    out.backward(g, retain_graph=True)
+    ref = torch.zeros(rows, dim, dtype=torch.float64, device=DEV).index_add(0, ids, g.double())
+    mag = torch.zeros(rows, dim, dtype=torch.float64, device=DEV).index_add(0, ids, g.double().abs())
+    # m fp32 additions of bf16 terms, rounded once: 2^-9 relative plus m 2^-24 of the terms' magnitudes, m at most n
+    assert ((w.main_grad.double() - ref).abs() <= ref.abs() * 2 ** -8 + mag * n * 2 ** -24 + 1e-30).all()
+
+    def ours():
+        w.main_grad_written = False
+        out.backward(g, retain_graph=True)
+
+    dense = torch.empty_like(w.main_grad)
+
+    def sorted_gradient():
+        dense.copy_(torch.ops.aten.embedding_dense_backward(g, ids, rows, -1, False))
+
+    def best(fn):
+        times = []
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            torch.cuda._sleep(200_000)          # the host is ahead of the device: launches are not what is compared
+            a.record()
+            fn()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert best(ours) < best(sorted_gradient)
+
+
 # ------------------------------------------------------------------ GEMM
 @pytest.mark.parametrize("backend,M,N,K", [
     ("tcgen05", 128, 128, 128), ("tcgen05", 256, 512, 384), ("tcgen05", 4096, 1536, 1024), ("tcgen05", 384, 256, 4096),
