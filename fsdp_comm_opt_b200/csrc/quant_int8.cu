@@ -18,6 +18,7 @@ namespace zc {
 namespace q8 {
 
 constexpr int THREADS = 256;
+constexpr int MAX_GRID_Y = 65535;
 
 __device__ __forceinline__ float widen(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float widen(float v) { return v; }
@@ -238,20 +239,22 @@ int quantise(const void* x, int64_t n, uint8_t* out, cudaStream_t st) {
 }
 
 template <typename T>
-int dequantise(const uint8_t* gathered, int64_t stride, int world, int64_t n, void* out, cudaStream_t st) {
-  if (world > 65535) return ERR_UNSUPPORTED;
+int dequantise(const uint8_t* gathered, int64_t stride, int world, int64_t n, T* out, cudaStream_t st) {
   const bool ok = ((reinterpret_cast<uintptr_t>(gathered) | (uintptr_t)stride) & 15) == 0 &&
                   reinterpret_cast<uintptr_t>(out) % sizeof(T) == 0;
   const int64_t units = (n + 7) / 8;
   // 32 CTAs per SM (four waves): 108 us for the eight ranks above, 121 with one wave, which reads too many pages
   // at a time
   const int64_t most = std::max<int64_t>(1, (int64_t)sm_count() * 32 / world);
-  if (ok) {
-    const dim3 grid((unsigned)std::min<int64_t>((units + THREADS - 1) / THREADS, most), world);
-    dequant_kernel<T><<<grid, THREADS, 0, st>>>(gathered, stride, n, (T*)out);
-  } else {
-    const dim3 grid((unsigned)std::min<int64_t>((n + THREADS - 1) / THREADS, 2 * most), world);
-    dequant_unaligned_kernel<T><<<grid, THREADS, 0, st>>>(gathered, stride, n, (T*)out);
+  for (; world > 0; world -= MAX_GRID_Y, gathered += MAX_GRID_Y * stride, out += MAX_GRID_Y * n) {
+    const int rows = std::min(world, MAX_GRID_Y);
+    if (ok) {
+      const dim3 grid((unsigned)std::min<int64_t>((units + THREADS - 1) / THREADS, most), rows);
+      dequant_kernel<T><<<grid, THREADS, 0, st>>>(gathered, stride, n, out);
+    } else {
+      const dim3 grid((unsigned)std::min<int64_t>((n + THREADS - 1) / THREADS, 2 * most), rows);
+      dequant_unaligned_kernel<T><<<grid, THREADS, 0, st>>>(gathered, stride, n, out);
+    }
   }
   return launch_status();
 }
@@ -280,9 +283,9 @@ int zc_dequant_int8(const void* gathered, int64_t stride, int world, int64_t n, 
   using namespace zc;
   if (world <= 0 || n <= 0) return 0;
   switch (dtype) {
-    case 0: return q8::dequantise<__nv_bfloat16>((const uint8_t*)gathered, stride, world, n, out, st);
-    case 1: return q8::dequantise<float>((const uint8_t*)gathered, stride, world, n, out, st);
-    case 2: return q8::dequantise<__half>((const uint8_t*)gathered, stride, world, n, out, st);
+    case 0: return q8::dequantise<__nv_bfloat16>((const uint8_t*)gathered, stride, world, n, (__nv_bfloat16*)out, st);
+    case 1: return q8::dequantise<float>((const uint8_t*)gathered, stride, world, n, (float*)out, st);
+    case 2: return q8::dequantise<__half>((const uint8_t*)gathered, stride, world, n, (__half*)out, st);
     default: return ERR_UNSUPPORTED;
   }
 }

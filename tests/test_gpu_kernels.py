@@ -433,6 +433,19 @@ def test_int8_vector_paths_and_their_edges(n, world, dt):
         assert not buf[r, 16 + n:].any()
 
 
+@pytest.mark.parametrize("world", [65535, 65536, 140_000])
+def test_int8_contributions_beyond_a_grids_rows(world):
+    n = 11
+    g = torch.Generator(device=DEV).manual_seed(world)
+    buf = torch.randint(0, 256, (world, quant.packed_bytes(n)), generator=g, device=DEV).to(torch.uint8)
+    scale = torch.rand(world, generator=g, device=DEV) + 0.5
+    buf[:, :4] = scale.view(world, 1).view(torch.uint8)
+    out = torch.zeros(world * n, dtype=torch.float32, device=DEV)
+    quant.dequantize_unpack(buf, n, out)
+    ref = buf[:, 16:16 + n].contiguous().view(torch.int8).float() * scale[:, None]
+    assert torch.equal(out.view(world, n), ref)
+
+
 @pytest.mark.parametrize("pdt,sdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
 def test_fused_adamw_kernel(pdt, sdt):
     torch.manual_seed(5)
