@@ -475,7 +475,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CE_THREADS, 3)
   }
   const float scale = inv_count[0], inv_s = 1.f / gs;
   // the CTA that holds the label's logit writes the loss (shared memory, or a tail column that this thread reads before
-  // it overwrites any)
+  // it overwrites any); a label that nobody holds, which the CPU path refuses, makes it NaN
+  if (threadIdx.x == 0 && rank == 0 && (label < 0 || label >= V)) row_loss[row] = CUDART_NAN_F;
   if (threadIdx.x == (int)((label - tail0) & (CE_THREADS - 1)) && tail && label >= tail0 && label < V)
     row_loss[row] = gm + __logf(gs) - __bfloat162float(lr[label]);
   if (threadIdx.x == 0 && label >= (int64_t)v0 * 8 && label < (int64_t)v1 * 8)
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(CE_THREADS, 3) ce_kernel(__nv_bfloat16* __rest
   const float gs = block_sum(s, red);
   const float lse = gm + __logf(gs);
   const float scale = inv_count[0];
-  const float picked = __bfloat162float(lr[label]);
+  const float picked = label >= 0 && label < V ? __bfloat162float(lr[label]) : CUDART_NAN_F;
   __syncthreads();  // everyone has read lr[label] before it is overwritten
   if (threadIdx.x == 0) row_loss[row] = lse - picked;
   const float inv_s = 1.f / gs;

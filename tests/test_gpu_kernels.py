@@ -396,6 +396,28 @@ def test_cross_entropy_at_the_edges_of_its_clusters(V):
     assert (work[:, V:] == 0).all()
 
 
+@pytest.mark.parametrize("V", [8192, 1001, 50257, 100001])
+def test_cross_entropy_of_a_label_outside_the_vocabulary_is_nan(V):
+    """One CTA a row, a ragged row, two CTAs a row and the kernel for long rows: no logit outside the row is read and no row's
+    loss is left unwritten; the other rows are as ever."""
+    from fsdp_comm_opt_b200 import _lib
+
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    logits = torch.randn(6, ld, device=DEV).bfloat16()
+    labels = torch.tensor([3, -1, V, V - 1, 1 << 40, -100], device=DEV)
+    ref = torch.logsumexp(logits[:, :V].double(), 1)
+    want = [ref[0] - logits[0, 3].double(), ref[3] - logits[3, V - 1].double()]
+    rows = torch.full((6,), 7.0, device=DEV)
+    inv = torch.ones(1, device=DEV)
+    _lib.check(_lib.cuda().zc_ce_fwd_bwd_ld(logits.data_ptr(), labels.data_ptr(), rows.data_ptr(), inv.data_ptr(), 6, V, ld, -100,
+                                            _lib.stream_ptr(logits.device)), "zc_ce_fwd_bwd")
+    assert rows.isnan().tolist() == [False, True, True, False, True, False] and rows[5] == 0
+    for got, w in zip((rows[0], rows[3]), want):
+        assert abs(got.item() - w.item()) < 1e-4 * abs(w.item())       # fp32 sums of fast exponentials
+    assert (logits[:, :V].float().sum(1)[[0, 3, 5]].abs() < 0.05).all()     # softmax minus one-hot, in bf16
+
+
 def test_int8_quant_kernels():
     torch.manual_seed(4)
     n, world = 100003, 3
