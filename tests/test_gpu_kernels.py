@@ -849,14 +849,16 @@ def test_tcgen05_gemm_three_forms(backend, M, N, K):
         gemm.set_backend("auto")
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 128, 1792), (128, 128, 1856), (512, 256, 8192), (1024, 1024, 4096), (200, 137, 2056),
+@pytest.mark.parametrize("M,N,K", [(128, 128, 1792), (128, 128, 1856), (128, 128, 1920), (512, 256, 8192), (1024, 1024, 4096), (200, 137, 2056),
                                    (300, 520, 37 * 64), (2048, 1024, 4095), (256, 9472, 2560), (256, 9728, 2560)])
 def test_gemm_split_along_k_when_tiles_are_few(M, N, K):
-    """The longest K that is not split and the shortest that is, slices of 8 K blocks, a K that does not divide into equal
+    """The longest K that is not split (1856) and the shortest that is (1920), slices of 8 K blocks, a K that does not divide into equal
     slices, ragged M / N / K, and the last size that is split (37 tiles) beside the first that is not.  Each is rounded once from fp32 sums: half
     a bf16 unit (2^-9) at most per value, so the relative error in the 2-norm is below 2^-9 plus the sums' 1e-5."""
     from fsdp_comm_opt_b200.ops import gemm
 
+    assert (_lib.cuda().zc_gemm_2sm_split_bytes(M, N, K) > 0) == ((M, N, K) not in [(128, 128, 1792), (128, 128, 1856),
+                                                                                    (256, 9728, 2560)])
     torch.manual_seed(K)
     pad = (K + 7) // 8 * 8
     x = torch.randn(M, pad, device=DEV).bfloat16()[:, :K]
