@@ -22,7 +22,8 @@
 // ring in shared memory), so a cluster that starts late, or not at all for a while, because another
 // kernel (a collective running beside the GEMM) holds its SMs simply takes fewer units; with a
 // static round-robin the whole GEMM would wait for that cluster's share.  (Launches recorded into a CUDA
-// graph, which only a one-rank step makes, and those with no second round use the static order.)
+// graph, which only a one-rank step makes, those with no second round, and those of streams beyond COUNTER_SLOTS use the
+// static order.)
 // Units: whole tiles first, then the tiles of the last, partial wave are split
 // along K into `split` slices each, so that all clusters stay busy to the end.  A slice writes its
 // fp32 partial sums to a workspace and a small second kernel adds the slices and rounds to bf16.
@@ -543,8 +544,9 @@ static bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols
 struct DeviceState {
   bool ready = false;
   int clusters = 0;
-  unsigned* counters = nullptr;  // COUNTER_SLOTS pairs, all zero between launches; launches take slots in turn
-  unsigned next_slot = 0;
+  unsigned* counters = nullptr;  // COUNTER_SLOTS pairs, all zero between launches
+  cudaStream_t owner[COUNTER_SLOTS];  // a stream's launches, which follow one another, share a pair
+  int owners = 0;
 };
 static DeviceState g_state[64];
 static std::mutex g_mutex;
@@ -698,13 +700,17 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   p.split = cut.split;
   p.full_tiles = (int)(cut.split > 1 ? cut.tiles - cut.split_tiles : cut.tiles);
   p.partial = cut.split > 1 ? (float*)ws : nullptr;
-  // Counters only where a second round is handed out, and not in a launch that is being recorded: a
-  // replayed launch would keep its slot for good, next to launches of other streams that take slots in turn.
+  // Counters only where a second round is handed out, and not in a launch that is being recorded, which may be
+  // replayed on any stream, nor on a stream beyond the first COUNTER_SLOTS or one of several under one handle.
   p.counter = nullptr;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cut.tiles > ds.clusters && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+  if (cut.tiles > ds.clusters && st != cudaStreamPerThread && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+      capture == cudaStreamCaptureStatusNone) {
     std::lock_guard<std::mutex> lock(g_mutex);
-    p.counter = ds.counters + 2 * (ds.next_slot++ % COUNTER_SLOTS);
+    int slot = 0;
+    while (slot < ds.owners && ds.owner[slot] != st) ++slot;
+    if (slot == ds.owners && slot < COUNTER_SLOTS) ds.owner[ds.owners++] = st;
+    if (slot < COUNTER_SLOTS) p.counter = ds.counters + 2 * slot;
   }
   const dim3 grid(2 * cut.grid_clusters);
   if (a_major == MAJOR_K && b_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_K><<<grid, THREADS, smem, st>>>(mapA, mapB, p);

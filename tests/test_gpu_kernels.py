@@ -904,6 +904,29 @@ def test_products_split_along_k_on_two_streams_have_partial_sums_of_their_own():
             assert all(torch.equal(ref, y) for y in out)
 
 
+def _first_products_worker(rank, world):
+    from fsdp_comm_opt_b200.ops import gemm
+
+    x, w = torch.randn(4096, 256, device=DEV).bfloat16(), torch.randn(6144, 256, device=DEV).bfloat16()
+    ref = x.double() @ w.double().t()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(8)]
+    got = []
+    for k in range(40):                        # the first of all on a stream that does not wait for the legacy stream
+        with torch.cuda.stream(streams[k % 8]):
+            got.append(gemm.gemm(x, w, False, True))
+    torch.cuda.synchronize()
+    assert all(torch.equal(got[0], y) for y in got)
+    assert ((got[0].double() - ref).norm() / ref.norm()).item() < 2 ** -9 + 1e-5   # rounded once from fp32 sums
+
+
+def test_the_first_products_of_a_process_run_on_side_streams():
+    """Every stream hands out its tiles (384 on 74 clusters) from counters of its own."""
+    from mp_util import run_ranks
+
+    run_ranks(_first_products_worker, 1, init_pg=False, backend="nccl")
+
+
 def test_gemm_with_leading_dimensions_and_odd_sizes():
     """Operands and results that are slices of wider buffers, and M / N / K that are not multiples of 8
     (GPT-2's vocabulary): the two-SM kernel takes row strides, zero-fills what lies outside a slice and
