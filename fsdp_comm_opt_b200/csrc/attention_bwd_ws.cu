@@ -881,8 +881,8 @@ int zc_attn_bwd_ws_status_read_and_clear() {
   return v;
 }
 
-// Same argument list as zc_attn_bwd: `dq_acc` is the fp32 accumulator of dQ, B * Hq * D * (S rounded up to 4)
-// floats that the launcher clears.
+// Same argument list as zc_attn_bwd: `dq_acc` is the fp32 accumulator of dQ, B * S * Hq * D floats that the launcher
+// clears.
 int zc_attn_bwd_ws(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                    float* delta, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv, int D, int64_t qs0,
                    int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1, int64_t ks2, int64_t vs0, int64_t vs1,

@@ -1,8 +1,8 @@
 """Token cross-entropy over bf16 logits with the gradient produced in the same pass.
 
 ``cross_entropy(logits, labels)`` returns the mean loss over labels != ignore_index.  On CUDA one
-kernel per call reads each logits row twice (online max/sum, then gradient) and overwrites the
-row with d(loss)/d(logits); backward only rescales.  HF's loss path, which the reference uses
+kernel per call reads each logits row once (rows too long for two CTAs' shared memory, or unaligned, twice) and overwrites
+the row with d(loss)/d(logits); backward only rescales.  HF's loss path, which the reference uses
 (train.py:252), upcasts the whole ``[T, V]`` logits tensor to fp32 first.
 """
 from __future__ import annotations
