@@ -7,13 +7,17 @@ communication and its tensors stay where they are (parameters and gradients are 
 buffers), so the launches of forward and backward are recorded once per batch shape and replayed.  The
 optimizer runs outside the graph: its learning rate and bias corrections change every step.
 
-A shape is recorded after it has been run ``EAGER_STEPS`` times.  Up to ``MAX_SHAPES`` shapes are kept, and one gives way
-to another only after ``IDLE_STEPS`` steps without it: a recording costs more than an eager step, and batches of more
-shapes than are kept would pay for one at every step if the least recently used made room.  Steps run eagerly, as they would without this module, whenever a
-replay could differ from that: hooks added to a module, to a parameter or to all modules, modules or parameters put
-in place of the model's own, a ``forward`` or an epsilon set on one of them, moved storage, saved-tensor hooks, dispatch
-and function modes, autocast, anomaly detection, a capture that is already under way.  A shape is recorded again when
-another GEMM or attention implementation has been selected since.
+A shape is recorded after it has been run ``EAGER_STEPS`` times.  Up to ``MAX_SHAPES`` shapes are kept, and
+one gives way to another only after ``IDLE_STEPS`` steps without it: a recording costs more than an eager
+step, and batches of more shapes than are kept would pay for one at every step if the least recently used
+made room (ten lengths of the d = 256 model in turn took 3.4 ms a step with four kept so, 2.5 eagerly,
+1.1 to 2.1 now).
+
+Steps run eagerly, as they would without this module, whenever a replay could differ from that: hooks added
+to a module, to a parameter or to all modules, modules or parameters put in place of the model's own, a
+``forward``, an epsilon or an entry of the configuration changed, moved storage, saved-tensor hooks,
+dispatch and function modes, autocast, anomaly detection, a capture that is already under way.  A shape is
+recorded again when another GEMM or attention implementation has been selected since.
 A recording that fails (no memory for the graph, a call that no recording may make) is given up, the step runs
 eagerly and so do all later ones.
 """
@@ -85,6 +89,8 @@ class StepGraphs:
             [id(x) for d in self._child_dicts for x in d.values()],
             ["forward" in d for d in self._attrs],
             [m.eps for m in self._with_eps],
+            [id(d.get("cfg")) for d in self._attrs],
+            list(vars(self.model.config).values()),
             [(p.data_ptr(), _address(getattr(p, "main_grad", None)), p.requires_grad, p.grad is None,
               not p._backward_hooks, not p._post_accumulate_grad_hooks) for p in self._params],
         ]

@@ -334,6 +334,11 @@ def _guard_worker(rank, world):
     for n, h in both:
         del h.forward
     steps(False)
+    theta = a.model_config.rope_theta
+    a.model_config.rope_theta = theta / 100                             # both engines' own configuration object
+    steps(True)
+    a.model_config.rope_theta = theta
+    steps(False)
     for e in (a, b):
         e.model.model.layers[1] = torch.nn.Identity()                   # x alone: unpacking it as (x, delta) would fail
         e.model.model.layers[1].forward = lambda x, delta: (x, delta)
