@@ -8,8 +8,9 @@
 //   warp 0      TMA producer (both CTAs): cp.async.bulk.tensor ... cta_group::2 loads into the CTA's
 //               own stage buffers, transaction bytes counted on the even CTA's `full` barrier
 //   warp 1      even CTA: MMA issuer; commits arrive on the `empty` / `acc_full` barriers of both CTAs
-//   warps 2-5   epilogue (both CTAs): tcgen05.ld the CTA's 128 x 256 accumulator, convert, store;
-//               arrivals of both CTAs' epilogue warps free the accumulator on the even CTA
+//   warps 2-5   epilogue (both CTAs): tcgen05.ld the CTA's 128 x 256 accumulator, convert, turn 64 columns of 32 rows
+//               round in shared memory, store whole 128-byte lines; arrivals of both CTAs' epilogue warps free the
+//               accumulator on the even CTA
 // Every CTA fetches its own tiles with plain per-CTA TMA loads; no load is shared between CTAs.
 //
 // The issuing thread is the scarce resource: one thread has to launch a 128-clock MMA every 128
@@ -27,6 +28,10 @@
 // Units: whole tiles first, then the tiles of the last, partial wave are split
 // along K into `split` slices each, so that all clusters stay busy to the end.  A slice writes its
 // fp32 partial sums to a workspace and a small second kernel adds the slices and rounds to bf16.
+// What a small product costs is fixed: 256 x 256 x 64 took 7.5 us a launch in a graph, of which the epilogue, 16 bytes of 32
+// rows a store, was 4.6, the pair's two barriers with release semantics 1.3, and an arrival with release behind the stores 0.6.
+// It is 5.6 now: 0.45 to the pair's barrier, 0.4 to the first load, 0.4 for it, 0.4 for the MMAs, 2.0 for the epilogue (bound
+// by the four warps' shared memory and store instructions; 32-column boxes stored by TMA took 2.6), 0.4 to leave.
 // Every wait is bounded; on expiry the status word is set and both CTAs reach the teardown.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -59,6 +64,9 @@ constexpr int MAX_SPLIT_SINGLE = 16;  // slices of a product that has fewer tile
 constexpr int SINGLE_MIN_KB = 8;      // K blocks of such a slice at least,
 constexpr int SINGLE_MIN_SAVED = 20;  // and fewer K blocks one after the other than in the whole product
 constexpr int SCHED = 4;       // slots of the unit-index ring
+constexpr int EPI_COLS = 64;   // columns that an epilogue warp turns round in shared memory at a time: 32 rows x 128 bytes
+constexpr int EPI_BYTES = 32 * EPI_COLS * 2;
+constexpr int SHARED_OFF = STAGES * STAGE + 4 * EPI_BYTES;  // struct Shared behind the stages and the epilogue's buffers
 constexpr int COUNTER_SLOTS = 256;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -66,10 +74,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// The pair's barrier in two halves.  Relaxed: what the other CTA has to see of this one's memory is only the initialised
+// mbarriers, which fence.mbarrier_init publishes (with release the two barriers of a launch took 2400 clocks, so 400).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
   uint32_t r;
@@ -78,6 +86,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same without waiting for this thread's earlier stores to be seen: where the arrival publishes nothing in memory, only
+// that tcgen05.ld has read the accumulator (a release took 1100 clocks behind the epilogue's stores).
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load into this CTA's shared memory; the bytes are counted on the barrier at `bar_cluster_addr`
 // (the even CTA's `full` barrier)
@@ -153,10 +166,24 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// Everything is in dynamic shared memory, whose beginning is 1024-byte aligned when there is no static part: 208.2 KB in
+// all, so that two 8 KB CTAs of a collective still fit beside this one.
+struct Shared {
+  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+  uint64_t sched_full[SCHED], sched_empty[SCHED];
+  int sched_u[SCHED];
+  uint32_t tmem_base;
+  int abort;
+};
+constexpr int SMEM_BYTES = SHARED_OFF + (int)sizeof(Shared);
+static_assert(SMEM_BYTES + 1024 + 2 * (8192 + 1024 + 128) <= 228 * 1024, "room for two CTAs of a collective");
+
 struct Params {
   __nv_bfloat16* C;
-  float* partial;      // [tail tiles][split][256][256] fp32, or null when split == 1
-  int64_t M, N, K;
+  float* partial;      // [tail tiles][split] slabs of 256 x 256 fp32 (partial_off), or null when split == 1
+  int64_t M, N;
+  int m_tiles, n_tiles, k_blocks;
+  float inv_band;      // 1 / (group_m * n_tiles)
   int64_t ldc;         // elements between rows of C (>= N rounded up to 8: whole 8-column groups are stored)
   const __nv_bfloat16* bias;  // [N] added to every row before rounding, or null
   int accumulate;
@@ -172,13 +199,21 @@ struct Params {
 // `group_m` m-tiles keeps that set a compact block of the output, so the A rows and B columns it
 // needs together stay in L2 however large K is (a full column of m-tiles does not once M * K
 // outgrows the cache).
-// (32-bit arithmetic: the issuing thread pays for every instruction between two tiles.)
-__device__ __forceinline__ void tile_coords(int t, int m_tiles, int n_tiles, int group_m, int& mi, int& ni) {
-  const int per_band = group_m * n_tiles;
-  const int band = t / per_band, r = t - band * per_band;
-  const int rows = min(group_m, m_tiles - band * group_m);
-  ni = r / rows;
-  mi = band * group_m + (r - ni * rows);
+// (A division by a number whose reciprocal is known, for quotients below 2^24 right after one correction at most: the integer
+// division's thirty instructions lie between two tiles, and before the first.)
+__device__ __forceinline__ int div_by(int t, int d, float inv, int& rem) {
+  int q = (int)((float)t * inv);
+  rem = t - q * d;
+  while (rem < 0) { --q; rem += d; }
+  while (rem >= d) { ++q; rem -= d; }
+  return q;
+}
+__device__ __forceinline__ void tile_coords(int t, const Params& p, int& mi, int& ni) {
+  int r, in_col;
+  const int band = div_by(t, p.group_m * p.n_tiles, p.inv_band, r);
+  const int rows = min(p.group_m, p.m_tiles - band * p.group_m);
+  ni = div_by(r, rows, __frcp_rn((float)rows), in_col);
+  mi = band * p.group_m + in_col;
 }
 
 // One unit of work: a tile and a range of its K blocks.
@@ -187,22 +222,22 @@ struct Unit {
   int kb0, kb1;
   int slice;  // index of the fp32 partial slab, or -1 for a whole tile
 };
-__device__ __forceinline__ Unit unit_of(int u, const Params& p, int m_tiles, int n_tiles, int k_blocks) {
+__device__ __forceinline__ Unit unit_of(int u, const Params& p) {
   Unit w;
   int t = u;
   w.kb0 = 0;
-  w.kb1 = k_blocks;
+  w.kb1 = p.k_blocks;
   w.slice = -1;
   if (u >= p.full_tiles) {
     const int r = u - p.full_tiles;
     t = p.full_tiles + r / p.split;
     const int s = r % p.split;
-    const int per = (k_blocks + p.split - 1) / p.split;
+    const int per = (p.k_blocks + p.split - 1) / p.split;
     w.kb0 = s * per;
-    w.kb1 = min(k_blocks, w.kb0 + per);
+    w.kb1 = min(p.k_blocks, w.kb0 + per);
     w.slice = r;
   }
-  tile_coords(t, m_tiles, n_tiles, p.group_m, w.mi, w.ni);
+  tile_coords(t, p, w.mi, w.ni);
   return w;
 }
 
@@ -224,80 +259,108 @@ __device__ __forceinline__ void add_bias8(const __nv_bfloat16* bias, int64_t col
   }
 }
 
+// f += the eight old bf16 values of C
+__device__ __forceinline__ void add_old8(const uint4& old, float (&f)[8]) {
+  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 o2 = __bfloat1622float2(ob[j]);
+    f[2 * j] += o2.x;
+    f[2 * j + 1] += o2.y;
+  }
+}
+__device__ __forceinline__ uint4 round8(const float (&f)[8]) {
+  uint4 v;
+  __nv_bfloat162 a0 = __floats2bfloat162_rn(f[0], f[1]), a1 = __floats2bfloat162_rn(f[2], f[3]);
+  __nv_bfloat162 a2 = __floats2bfloat162_rn(f[4], f[5]), a3 = __floats2bfloat162_rn(f[6], f[7]);
+  v.x = *reinterpret_cast<uint32_t*>(&a0);
+  v.y = *reinterpret_cast<uint32_t*>(&a1);
+  v.z = *reinterpret_cast<uint32_t*>(&a2);
+  v.w = *reinterpret_cast<uint32_t*>(&a3);
+  return v;
+}
+// Where a slab of partial sums keeps columns 4 c4 .. 4 c4 + 3 of a tile's row, in float4: the rows of a warp, which holds a
+// row a thread, lie next to each other.
+__device__ __forceinline__ int partial_off(int row, int c4) { return ((row >> 5) * (BN / 4) + c4) * 32 + (row & 31); }
+
 template <int A_MAJOR, int B_MAJOR>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     gemm_2sm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Params p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
-  __shared__ uint64_t sched_full[SCHED], sched_empty[SCHED];
-  __shared__ int sched_u[SCHED];
-  __shared__ uint32_t tmem_base;
-  __shared__ volatile int s_abort;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) {  // the same in both CTAs of a pair
+    if (threadIdx.x == 0) atomicExch(p.status, 9);
+    return;
+  }
+  Shared& sh = *reinterpret_cast<Shared*>(smem + SHARED_OFF);
+  uint64_t *full = sh.full, *empty = sh.empty, *acc_full = sh.acc_full, *acc_empty = sh.acc_empty;
+  uint64_t *sched_full = sh.sched_full, *sched_empty = sh.sched_empty;
+  volatile int* sched_u = sh.sched_u;
+  volatile int& s_abort = sh.abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();  // 0: even CTA (issues the MMAs), 1: odd CTA
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 1);    // used on the even CTA: its producer's arrive.expect_tx
-      mbar_init(&empty[s], 1);   // one commit per use, on both CTAs
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&acc_full[a], 1);   // one commit per unit, on both CTAs
-      mbar_init(&acc_empty[a], 8);  // used on the even CTA: four epilogue warps of each CTA
-    }
-    for (int q = 0; q < SCHED; ++q) {
-      mbar_init(&sched_full[q], 1);    // the even CTA's producer publishes a unit index (in both CTAs)
-      mbar_init(&sched_empty[q], 10);  // used on the even CTA: every other role of both CTAs has read it
-    }
+  if (warp == 0) {
+    // A thread per barrier: full (used on the even CTA: its producer's arrive.expect_tx), empty (one commit per use, on
+    // both CTAs), acc_full (one commit per unit, on both CTAs), acc_empty (on the even CTA: four epilogue warps of each CTA),
+    // sched_full (the even CTA's producer publishes a unit index in both CTAs), sched_empty (on the even CTA: every other
+    // role of both CTAs has read it)
+    constexpr int ACC_EMPTY = 2 * STAGES + 2, SCHED_FULL = ACC_EMPTY + 2, SCHED_EMPTY = SCHED_FULL + SCHED;
+    if (lane < SCHED_EMPTY + SCHED)
+      mbar_init(&full[lane], lane >= SCHED_EMPTY ? 10 : lane >= ACC_EMPTY && lane < SCHED_FULL ? 8 : 1);
     mbar_fence_init();
-    s_abort = 0;
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
+    if (lane == 0) s_abort = 0;
+    __syncwarp();
   }
+  cluster_arrive();
   if (warp == 1) {
     // each CTA allocates its own SM's whole TMEM (512 columns, so the base is column 0 in both)
-    tmem_alloc(&tmem_base, 2 * BN);
+    tmem_alloc(&sh.tmem_base, 2 * BN);
     tmem_relinquish();
+  } else if (warp == 2 && lane < 2) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(lane ? &mapB : &mapA) : "memory");
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  cluster_sync_all();  // both CTAs' barriers are initialised before any remote arrival
-  tc_fence_after_sync();
-  const uint32_t tm = tmem_base;
   // edge tiles: rows / columns / K blocks past the matrix read as zeros (TMA fill) and are not stored
-  const int m_tiles = (int)((p.M + BM - 1) / BM), n_tiles = (int)((p.N + BN - 1) / BN);
-  const int k_blocks = (int)((p.K + BK - 1) / BK);
-  const int tiles = m_tiles * n_tiles;
-  const int units = p.full_tiles + (tiles - p.full_tiles) * p.split;
+  const int units = p.full_tiles + (p.m_tiles * p.n_tiles - p.full_tiles) * p.split;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
+  const Unit first = unit_of(cluster_id, p);
+  if (warp != 0) {  // the producer has no use for the accumulators' address
+    tc_fence_before_sync();
+    asm volatile("bar.sync 1, 160;" ::: "memory");
+    tc_fence_after_sync();
+  }
+  cluster_wait();  // both CTAs' barriers are initialised before any remote arrival
+  const uint32_t tm = sh.tmem_base;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t full_base = smem_u32(&full[0]), empty_base = smem_u32(&empty[0]);
   const uint32_t sfull_base = smem_u32(&sched_full[0]);
   const uint32_t sempty_c0 = map_to_cta(smem_u32(&sched_empty[0]), 0);  // the even CTA's sched_empty[0]
   bool ok = true;
-  // Every role walks the same sequence of units, i = 0, 1, ...: slot i % SCHED of the ring holds the
-  // i-th unit of this cluster (an index >= units ends the sequence).
+  // Every role walks the same sequence of units, i = 0, 1, ... (an index >= units ends it).  The first is the cluster's
+  // number, known without waiting for another CTA; with counters slot (i - 1) % SCHED of the ring holds the i-th.
+  auto from_ring = [&](uint32_t i) { return p.counter && i > 0; };
   auto next_unit = [&](uint32_t i, bool& good) -> int {
-    const uint32_t slot = i & (SCHED - 1), sph = (i / SCHED) & 1;
+    if (!from_ring(i)) return cluster_id + (int)i * n_clusters;
+    const uint32_t slot = (i - 1) & (SCHED - 1), sph = ((i - 1) / SCHED) & 1;
     good = rank == 0 ? wait_bar(sfull_base + 8 * slot, sph, &s_abort)
                      : wait_bar_cluster(sfull_base + 8 * slot, sph, &s_abort);
     return good ? sched_u[slot] : 0x7fffffff;
   };
-  auto release_unit = [&](uint32_t i) { mbar_arrive_cluster(sempty_c0 + 8 * (i & (SCHED - 1))); };
+  auto release_unit = [&](uint32_t i) {
+    if (from_ring(i)) mbar_arrive_cluster(sempty_c0 + 8 * ((i - 1) & (SCHED - 1)));
+  };
 
   if (warp == 0) {
     if (lane == 0) {
       const uint32_t full0 = map_to_cta(full_base, 0);  // the even CTA's full[0]; full[s] is 8 s bytes on
       const uint32_t sfull_c1 = map_to_cta(sfull_base, 1);
-      const uint32_t su_c1 = map_to_cta(smem_u32(&sched_u[0]), 1);
+      const uint32_t su_c1 = map_to_cta(smem_u32(sh.sched_u), 1);
       uint32_t s = 0, ph = 0;
       for (uint32_t i = 0; ok; ++i) {
         int u;
-        if (rank == 0) {
+        if (rank == 0 && from_ring(i)) {
           // fetch the i-th unit and publish it to both CTAs
-          const uint32_t slot = i & (SCHED - 1), sph = (i / SCHED) & 1;
+          const uint32_t slot = (i - 1) & (SCHED - 1), sph = ((i - 1) / SCHED) & 1;
           if (!(ok = wait_bar_cluster(smem_u32(&sched_empty[slot]), sph ^ 1, &s_abort))) break;
-          u = (i == 0 || !p.counter) ? cluster_id + (int)i * n_clusters : n_clusters + (int)atomicAdd(p.counter, 1u);
+          u = n_clusters + (int)atomicAdd(p.counter, 1u);
           sched_u[slot] = u;
           st_shared_cluster_u32(su_c1 + 4 * slot, (uint32_t)u);
           mbar_arrive(&sched_full[slot]);
@@ -308,7 +371,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           release_unit(i);
         }
         if (u >= units) break;
-        const Unit w = unit_of(u, p, m_tiles, n_tiles, k_blocks);
+        const Unit w = i == 0 ? first : unit_of(u, p);
         const int m0 = w.mi * BM + (int)rank * BM_CTA;
         const int n0 = w.ni * BN + (int)rank * BN_CTA;
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
@@ -354,7 +417,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         if (!ok) break;
         release_unit(unit_it);
         if (u >= units) break;
-        const Unit w = unit_of(u, p, m_tiles, n_tiles, k_blocks);
+        const Unit w = unit_it == 0 ? first : unit_of(u, p);
         const uint32_t acc = unit_it & 1, acc_ph = (unit_it >> 1) & 1;
         if (!(ok = wait_bar_cluster(acce + 8 * acc, acc_ph ^ 1, &s_abort))) break;
         tc_fence_after_sync();
@@ -384,13 +447,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     const int quarter = warp & 3;
     const uint32_t accf = smem_u32(&acc_full[0]);
     const uint32_t acce_c0 = map_to_cta(smem_u32(&acc_empty[0]), 0);
+    // This warp's buffer: row `lane`, 128 bytes, its 16-byte chunk j at position j ^ lane % 8.  Written a row a thread, read
+    // (and stored) four rows an instruction.
+    uint8_t* epi = smem + STAGES * STAGE + quarter * EPI_BYTES;
+    const int out_row = lane >> 3, out_chunk = lane & 7;
     for (uint32_t unit_it = 0; ok; ++unit_it) {
       const int u = next_unit(unit_it, ok);
       if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
       __syncwarp();
       if (lane == 0) release_unit(unit_it);
       if (u >= units) break;
-      const Unit w = unit_of(u, p, m_tiles, n_tiles, k_blocks);
+      const Unit w = unit_it == 0 ? first : unit_of(u, p);
       const uint32_t acc = unit_it & 1, acc_ph = (unit_it >> 1) & 1;
       ok = wait_bar_cluster(accf + 8 * acc, acc_ph, &s_abort);
       if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
@@ -399,44 +466,79 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       if (w.slice < 0) {
         const int64_t row = (int64_t)w.mi * BM + row_in_tile;
         const int64_t col0 = (int64_t)w.ni * BN;
-        __nv_bfloat16* crow = p.C + row * p.ldc + col0;
-        const bool row_ok = row < p.M;
+        if (p.accumulate) {
+          // the old values come in as they lie, 16 bytes of a row a thread
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c), r);
-          tmem_ld_wait();
+          for (int c = 0; c < BN; c += 32) {
+            uint32_t r[32];
+            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c), r);
+            tmem_ld_wait();
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (!row_ok || col0 + c + q * 8 >= p.N) continue;
-            float f[8];
+            for (int q = 0; q < 4; ++q) {
+              if (row >= p.M || col0 + c + q * 8 >= p.N) continue;
+              float f[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q * 8 + j]);
-            if (p.bias) add_bias8(p.bias, col0 + c + q * 8, p.N, f);
-            uint4* dst = reinterpret_cast<uint4*>(crow + c + q * 8);
-            if (p.accumulate) {
-              const uint4 old = *dst;
-              const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
+              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q * 8 + j]);
+              if (p.bias) add_bias8(p.bias, col0 + c + q * 8, p.N, f);
+              uint4* dst = reinterpret_cast<uint4*>(p.C + row * p.ldc + col0 + c + q * 8);
+              add_old8(*dst, f);
+              *dst = round8(f);
+            }
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(acce_c0 + 8 * acc);
+        } else {
+          const int64_t warp_row = (int64_t)w.mi * BM + rank * BM_CTA + quarter * 32;
+          const int rows_left = (int)min((int64_t)32, p.M - warp_row) - out_row;  // from this thread's first on
+          const int cols_left = (int)min((int64_t)BN, p.N - col0);
+          const __nv_bfloat16* bias = p.bias + col0;
+          __nv_bfloat16* dst = p.C + (warp_row + out_row) * p.ldc + col0 + out_chunk * 8;
+          // No branch in this loop but those on whole chunks: one at every group of eight columns, bias or not, old values
+          // or not, cost more than the work.
+#pragma unroll 1
+          for (int c = 0; c < BN; c += EPI_COLS) {
+            uint32_t r[2][32];
+            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c), r[0]);
+            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c + 32), r[1]);
+            tmem_ld_wait();
+            if (c == BN - EPI_COLS) {  // the accumulator is free
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster_relaxed(acce_c0 + 8 * acc);
+            }
+            if (p.bias) {  // a column's value a lane
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 o2 = __bfloat1622float2(ob[j]);
-                f[2 * j] += o2.x;
-                f[2 * j + 1] += o2.y;
+              for (int h = 0; h < 2; ++h) {
+                const int col = c + h * 32 + lane;
+                const float mine = col < cols_left ? __bfloat162float(bias[col]) : 0.f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) + __shfl_sync(0xffffffffu, mine, j));
               }
             }
-            uint4 v;
-            __nv_bfloat162 a0 = __floats2bfloat162_rn(f[0], f[1]), a1 = __floats2bfloat162_rn(f[2], f[3]);
-            __nv_bfloat162 a2 = __floats2bfloat162_rn(f[4], f[5]), a3 = __floats2bfloat162_rn(f[6], f[7]);
-            v.x = *reinterpret_cast<uint32_t*>(&a0);
-            v.y = *reinterpret_cast<uint32_t*>(&a1);
-            v.z = *reinterpret_cast<uint32_t*>(&a2);
-            v.w = *reinterpret_cast<uint32_t*>(&a3);
-            *dst = v;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              float f[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q >> 2][(q & 3) * 8 + j]);
+              *reinterpret_cast<uint4*>(epi + lane * 128 + ((q ^ (lane & 7)) << 4)) = round8(f);
+            }
+            __syncwarp();
+            uint4 v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              v[q] = *reinterpret_cast<const uint4*>(epi + (4 * q + out_row) * 128 + ((out_chunk ^ ((4 * q + out_row) & 7)) << 4));
+            __syncwarp();
+            if (c + out_chunk * 8 < cols_left) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                if (4 * q < rows_left) *reinterpret_cast<uint4*>(dst + c + (int64_t)(4 * q) * p.ldc) = v[q];
+            }
           }
         }
       } else {
-        // K slice of a tail tile: fp32 partial sums, added up by gemm_2sm_fixup_kernel
-        float* prow = p.partial + ((int64_t)w.slice * BM + row_in_tile) * BN;
+        // K slice of a tail tile: fp32 partial sums, added up by gemm_2sm_fixup_kernel; a warp's store is 512 bytes in a row
+        float4* prow = reinterpret_cast<float4*>(p.partial + (int64_t)w.slice * (BM * BN)) + partial_off(row_in_tile, 0);
 #pragma unroll 1
         for (int c = 0; c < BN; c += 32) {
           uint32_t r[32];
@@ -444,12 +546,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            reinterpret_cast<uint4*>(prow + c)[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+            prow[(c / 4 + q) * 32] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                                 __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
         }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(acce_c0 + 8 * acc);
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acce_c0 + 8 * acc);
     }
     if (!ok) s_abort = 1;
   }
@@ -457,7 +560,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   __syncthreads();
   if (tid == 0 && s_abort) atomicExch(p.status, 8);
   // neither CTA may leave (or free its TMEM) while the pair's MMAs can still touch its memory
-  cluster_sync_all();
+  cluster_arrive();
+  cluster_wait();
   if (warp == 1) tmem_dealloc(tm, 2 * BN);
   if (tid == 0 && rank == 0 && p.counter) {
     // the last cluster to finish puts the counters back to zero for the next launch that uses this slot
@@ -469,42 +573,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 }
 
 // C tile (+)= sum over the K slices of its fp32 partials, rounded once to bf16.
-__global__ void __launch_bounds__(256) gemm_2sm_fixup_kernel(const Params p, int m_tiles, int n_tiles) {
+__global__ void __launch_bounds__(256) gemm_2sm_fixup_kernel(const Params p) {
   const int tail = blockIdx.y;  // index among the split tiles
   int mi, ni;
-  tile_coords(p.full_tiles + tail, m_tiles, n_tiles, p.group_m, mi, ni);
-  const float* base = p.partial + (int64_t)tail * p.split * (BM * BN);
+  tile_coords(p.full_tiles + tail, p, mi, ni);
+  const float4* base = reinterpret_cast<const float4*>(p.partial) + (int64_t)tail * p.split * (BM * BN / 4);
+  // a warp takes eight rows x 32 columns: 128 bytes in a row of every load, 64 of every store
   for (int i = blockIdx.x * 256 + threadIdx.x; i < BM * BN / 8; i += gridDim.x * 256) {
-    const int row = i / (BN / 8), c8 = i % (BN / 8);
+    const int wi = i >> 5, lane = i & 31;
+    const int row = (wi / (BN / 32)) * 8 + (lane & 7), c8 = (wi % (BN / 32)) * 4 + (lane >> 3);
     if ((int64_t)mi * BM + row >= p.M || (int64_t)ni * BN + c8 * 8 >= p.N) continue;
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
     for (int s = 0; s < p.split; ++s) {
-      const float4* src = reinterpret_cast<const float4*>(base + (int64_t)s * (BM * BN) + row * BN + c8 * 8);
-      const float4 x = src[0], y = src[1];
+      const float4* src = base + (int64_t)s * (BM * BN / 4);
+      const float4 x = src[partial_off(row, 2 * c8)], y = src[partial_off(row, 2 * c8 + 1)];
       f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
       f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
     }
     if (p.bias) add_bias8(p.bias, (int64_t)ni * BN + c8 * 8, p.N, f);
     uint4* dst = reinterpret_cast<uint4*>(p.C + ((int64_t)mi * BM + row) * p.ldc + (int64_t)ni * BN + c8 * 8);
-    if (p.accumulate) {
-      const uint4 old = *dst;
-      const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 o2 = __bfloat1622float2(ob[j]);
-        f[2 * j] += o2.x;
-        f[2 * j + 1] += o2.y;
-      }
-    }
-    uint4 v;
-    __nv_bfloat162 a0 = __floats2bfloat162_rn(f[0], f[1]), a1 = __floats2bfloat162_rn(f[2], f[3]);
-    __nv_bfloat162 a2 = __floats2bfloat162_rn(f[4], f[5]), a3 = __floats2bfloat162_rn(f[6], f[7]);
-    v.x = *reinterpret_cast<uint32_t*>(&a0);
-    v.y = *reinterpret_cast<uint32_t*>(&a1);
-    v.z = *reinterpret_cast<uint32_t*>(&a2);
-    v.w = *reinterpret_cast<uint32_t*>(&a3);
-    *dst = v;
+    if (p.accumulate) add_old8(*dst, f);
+    *dst = round8(f);
   }
 }
 
@@ -682,15 +772,17 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   if (b_major == MAJOR_K) ok = ok && make_map(&mapB, B, N, K, ldb, BK, BN_CTA);
   else ok = ok && make_map(&mapB, B, K, N, ldb, 64, BK);
   if (!ok) return ERR_BAD_ARG;
-  const int smem = STAGES * STAGE + 1024;
+  const int smem = SMEM_BYTES;
   DeviceState& ds = g_state[dev];
   if (const int rc = init_state(ds, smem)) return rc;
   Params p;
-  p.C = (__nv_bfloat16*)C; p.M = M; p.N = N; p.K = K; p.ldc = ldc;
+  p.C = (__nv_bfloat16*)C; p.M = M; p.N = N; p.ldc = ldc;
+  p.m_tiles = (int)m_tiles; p.n_tiles = (int)n_tiles; p.k_blocks = (int)((K + BK - 1) / BK);
   p.bias = (const __nv_bfloat16*)bias;
   p.accumulate = accumulate;
   static const int forced_gm = getenv("ZC_GEMM_GROUP_M") ? atoi(getenv("ZC_GEMM_GROUP_M")) : 0;
   p.group_m = forced_gm > 0 ? forced_gm : 8;
+  p.inv_band = 1.f / (float)((int64_t)p.group_m * p.n_tiles);
   p.status = status;
   Cut cut = cut_of(M, N, K, ds.clusters);
   if (!ws || ws_bytes < cut.bytes()) {
@@ -718,7 +810,7 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   else gemm_2sm_kernel<MAJOR_MN, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
   int rc = launch_status();
   if (rc == 0 && p.split > 1) {
-    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st>>>(p, (int)m_tiles, (int)n_tiles);
+    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st>>>(p);
     rc = launch_status();
   }
   return rc;
@@ -736,7 +828,7 @@ int64_t zc_gemm_2sm_split_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace zc::g2;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (M <= 0 || N <= 0 || K <= 0 || dev < 0 || dev >= 64 || init_state(g_state[dev], STAGES * STAGE + 1024)) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || dev < 0 || dev >= 64 || init_state(g_state[dev], SMEM_BYTES)) return 0;
   return cut_of(M, N, K, g_state[dev].clusters).bytes();
 }
 
