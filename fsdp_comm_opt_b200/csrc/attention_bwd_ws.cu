@@ -17,6 +17,8 @@
 #include <cuda_bf16.h>
 #include <math_constants.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <type_traits>
 
@@ -83,6 +85,7 @@ struct BwdParams {
   int64_t dks0, dks1, dks2, dvs0, dvs1, dvs2;
   float scale;
   int* status;
+  int parts;  // CTAs that share a key block's query blocks (the key-row kernel)
 };
 
 template <int D>
@@ -507,12 +510,26 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t tmem_a, uint32_t b, 
       "}\n" ::"r"(d), "r"(tmem_a), "r"(b), "r"(idesc), "r"(accumulate), "n"(DESC_HI)
       : "memory");
 }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// four floats at the shared-memory address `at` of CTA `rank` of the cluster
+__device__ __forceinline__ float4 ld_cluster(uint32_t at, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(at), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-template <int D>
+// SHARED: a cluster of p.parts CTAs works on one key block.  (The kernel of its own without it: the few instructions more
+// before a CTA's first load cost 3 % where CTAs are short.)
+template <int D, bool SHARED>
 __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_constant__ CUtensorMap mapQ,
                                                              const __grid_constant__ CUtensorMap mapK,
                                                              const __grid_constant__ CUtensorMap mapV,
@@ -537,12 +554,25 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
   volatile int* s_abort = &m.abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per_jb = p.Hkv * p.B;
-  const int jb = blockIdx.x / per_jb;
-  const int hk = (blockIdx.x % per_jb) % p.Hkv, b = (blockIdx.x % per_jb) / p.Hkv;
+  const int parts = SHARED ? p.parts : 1;
+  const int part = SHARED ? blockIdx.x % parts : 0, unit = SHARED ? blockIdx.x / parts : blockIdx.x;
+  const int jb = unit / per_jb;
+  const int hk = (unit % per_jb) % p.Hkv, b = (unit % per_jb) / p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int k0 = jb * 128;
   const int nqb = (p.S + 127) / 128;
-  const int iters = group * (nqb - jb);  // query blocks at or below this key block's diagonal
+  const int all_iters = group * (nqb - jb);  // query blocks at or below this key block's diagonal
+  const int iters = SHARED ? (all_iters - part + parts - 1) / parts : all_iters;  // this CTA's: the part-th, (part + parts)-th, ...
+  // the query head and block of an iteration, and from it to the CTA's next
+  auto skip = [&](int& h, int& ib, int by) {
+    ib += by;
+    while (ib >= nqb) { ib -= nqb - jb; ++h; }
+  };
+  auto start = [&](int& h, int& ib) { if (SHARED) skip(h, ib, part); };
+  auto next = [&](int& h, int& ib) {
+    if (SHARED) skip(h, ib, parts);
+    else if (++ib == nqb) { ib = jb; ++h; }
+  };
   if (tid == 0) {
     mbar_init(&m.kv_full, 1);
     for (int i = 0; i < 2; ++i) {
@@ -586,6 +616,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         tma_load_4d(sV + sl * 16384, &mapV, &m.kv_full, sl * 64, hk, k0, b);
       }
       int h = hk * group, ib = jb;
+      start(h, ib);
       for (int i = 0; i < iters; ++i) {
         const int sq = i & 1, sd = i % C::DO_STAGES;
         if (!role_wait(&m.q_empty[sq], ((i >> 1) & 1) ^ 1)) { *s_abort = 1; break; }
@@ -598,7 +629,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
 #pragma unroll
         for (int sl = 0; sl < D / 64; ++sl)
           tma_load_4d(sdO + sd * C::TILE + sl * 16384, &mapdO, &m.do_full[sd], sl * 64, h, ib * 128, b);
-        if (++ib == nqb) { ib = jb; ++h; }
+        next(h, ib);
       }
     } else if (warp == 1 && lane == 0) {
       const uint32_t id_s = idesc_bf16(128, 128, MAJOR_K, MAJOR_K);    // S^T, dP^T
@@ -625,7 +656,12 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         mma_commit(&m.dp_full);
       };
       auto run = [&]() -> bool {
-        if (!role_wait(&m.kv_full, 0) || !role_wait(&m.q_full[0], 0)) return false;
+        if (!role_wait(&m.kv_full, 0)) return false;
+        if (SHARED && iters == 0) {  // fewer query blocks than CTAs share them
+          mma_commit(&m.all_done);
+          return true;
+        }
+        if (!role_wait(&m.q_full[0], 0)) return false;
         tc_fence_after_sync();
         issue_s(0);
         if (!role_wait(&m.do_full[0], 0)) return false;
@@ -673,6 +709,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
       if (!run()) *s_abort = 1;
     } else if (warp == 2) {
       int h = hk * group, ib = jb;
+      start(h, ib);
       for (int i = 0; i < iters; ++i) {
         const int st = i & 1;
         const int64_t row = ((int64_t)b * p.Hq + h) * p.S;
@@ -691,7 +728,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         dst[32 + lane] = make_float4(vd[0], vd[1], vd[2], vd[3]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&m.stat_full[st]);
-        if (++ib == nqb) { ib = jb; ++h; }
+        next(h, ib);
       }
     }
   } else if (warp < 12) {
@@ -702,7 +739,8 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
     const uint32_t lane_base = (uint32_t)(quarter * 32);
     const int c0 = half * 64;
     const uint64_t sl22 = pack2(p.scale * LOG2E, p.scale * LOG2E), scale2 = pack2(p.scale, p.scale);
-    int ib = jb;
+    int h = 0, ib = jb;
+    if (SHARED) skip(h, ib, part);
     bool fail = false;
     for (int i = 0; i < iters; ++i) {
       const int st = i & 1;
@@ -775,11 +813,31 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         mbar_arrive(&m.stat_empty[st]);
       }
       __syncwarp();
-      if (++ib == nqb) ib = jb;
+      next(h, ib);
     }
     if (!fail) fail = !mbar_wait_parked(&m.all_done, 0, s_abort);
     if (__any_sync(0xffffffffu, fail)) {
       *s_abort = 1;
+    } else if (SHARED) {
+      // fp32 sums of this CTA's share into its own shared memory (K, V, Q and dO are done with), four columns of 128 rows
+      // after each other; nothing where it had no share
+      tc_fence_after_sync();
+      if (iters > 0) {
+#pragma unroll 1
+        for (int which = 0; which < 2; ++which) {
+          float4* dst = reinterpret_cast<float4*>(smem) + which * (D / 4) * 128 + r;
+#pragma unroll 1
+          for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
+            uint32_t rr[32];
+            tmem_ld32(tmem_addr(tm + (which ? C::TM_DV : C::TM_DK), lane_base, c), rr);
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              dst[(c / 4 + q) * 128] = make_float4(__uint_as_float(rr[4 * q]), __uint_as_float(rr[4 * q + 1]),
+                                                   __uint_as_float(rr[4 * q + 2]), __uint_as_float(rr[4 * q + 3]));
+          }
+        }
+      }
     } else {
       tc_fence_after_sync();
       const int key = k0 + r;
@@ -813,6 +871,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
     const int r = quarter * 32 + lane;     // query row of the tile == TMEM lane
     const uint32_t lane_base = (uint32_t)(quarter * 32);
     int h = hk * group, ib = jb;
+    start(h, ib);
     bool fail = false;
     for (int i = 0; i < iters; ++i) {
       fail = !mbar_wait_parked(&m.dq_full, i & 1, s_abort) || *s_abort;
@@ -844,24 +903,93 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         }
       }
       __syncwarp();
-      if (++ib == nqb) { ib = jb; ++h; }
+      next(h, ib);
     }
     if (tid == 384) bulk_wait0();
     if (fail) *s_abort = 1;
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if (SHARED) {
+    __syncwarp();
+    cluster_sync();
+    if (warp >= 4 && warp < 12) {
+      // Each CTA of the cluster adds up its share of the columns, in the order of the parts, eight of a row a thread.
+      const int filled = min(parts, all_iters), groups = 2 * (D / 8) / parts;
+      for (int u = tid - 128; u < groups * 128; u += 256) {
+        const int g = part * groups + (u >> 7), row = u & 127, key = k0 + row;  // g: dK's groups of eight columns, then dV's
+        const uint32_t at = smem_u32(smem) + (uint32_t)(2 * g * 128 + row) * 16;
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int c = 0; c < filled; ++c) {
+          const float4 x = ld_cluster(at, c), y = ld_cluster(at + 128 * 16, c);
+          f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
+          f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
+        }
+        if (key < p.S) {
+          const int col = (g % (D / 8)) * 8;
+          __nv_bfloat16* dst = g >= D / 8 ? p.dv + b * p.dvs0 + (int64_t)key * p.dvs1 + hk * p.dvs2
+                                          : p.dk + b * p.dks0 + (int64_t)key * p.dks1 + hk * p.dks2;
+          *reinterpret_cast<uint4*>(dst + col) =
+              make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        }
+      }
+    }
+    cluster_sync();  // the others have read this CTA's sums
+  } else {
+    __syncthreads();
+  }
   if (tid == 0 && *s_abort) atomicExch(p.status, 6);
   if (warp == 1) tmem_dealloc(tm, 512);
 }
 
+// How many CTAs (a cluster) share the query blocks of a key block.  A key block's iterations follow one another, so with
+// few key blocks, batches and KV heads the chip waits for the longest of them: 1024 keys, 8 / 2 heads of 128 are 16 CTAs of up to
+// 32 iterations, 83 us; shared by eight 27.  Counted in iterations (2.3 us at head dimension 128, 2 at 64): the longest CTA
+// or the average of all SMs, and for every wave of CTAs what one costs beside its iterations, 4 alone and a few more for
+// adding up the shares.  (us, alone and shared) 2048 keys, 32 / 8 heads: 166, by two 106; 4096, 8 / 2: 308, by eight 111;
+// 4096, 32 / 8: 337, by two 353, so alone; 1024, 64 / 8: 167, by four 75; head dimension 64, 2048 keys, 8 heads: 40, by two 36.
+static int parts_of(int S, int Hq, int Hkv, int B, int D) {
+  const int sms = sm_count(), nqb = (S + 127) / 128, group = Hq / Hkv;
+  const double alone = 4.0, shared = D == 128 ? 7.0 : 5.5;
+  const double ctas = (double)nqb * Hkv * B, longest = (double)group * nqb, all = ctas * group * (nqb + 1) / 2;
+  int best = 1;
+  double least = 0;
+  for (int c = 1; c <= 8; c *= 2) {
+    const double slots = c == 8 ? sms * 0.875 : sms;  // clusters of eight leave SMs of every GPC over
+    const double t = std::max(std::ceil(longest / c), all / sms) + std::ceil(ctas * c / slots) * (c > 1 ? shared : alone);
+    if (c == 1 || t < least) { best = c; least = t; }
+  }
+  return best;
+}
+
 template <int D>
 static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                  const CUtensorMap& mdq, const BwdParams& p, cudaStream_t st) {
+                  const CUtensorMap& mdq, BwdParams p, cudaStream_t st) {
   using C = Cfg<D>;
-  if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+  static_assert(2 * 128 * D * 4 <= C::DS, "the shares' sums take the place of K, V, Q and dO");
+  p.parts = parts_of(p.S, p.Hq, p.Hkv, p.B, D);
+  const int units = (p.S + 127) / 128 * p.Hkv * p.B;
+  if (p.parts == 1) {
+    if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+      return launch_status();
+    attn_bwd_kt_kernel<D, false><<<units, 512, C::SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
     return launch_status();
-  attn_bwd_kt_kernel<D><<<(p.S + 127) / 128 * p.Hkv * p.B, 512, C::SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+  }
+  if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    return launch_status();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(units * p.parts);
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.parts;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, attn_bwd_kt_kernel<D, true>, mq, mk, mv, mdo, mdq, (const BwdParams)p);
   return launch_status();
 }
 

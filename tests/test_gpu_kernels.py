@@ -564,6 +564,25 @@ def test_attention_at_the_edges_of_key_and_query_tiles(B, S, Hq, Hkv, D):
     assert ((dqkv - dref).norm() / dref.norm()).item() < 1e-2
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(1, 2048, 32, 8, 128), (1, 1920, 8, 8, 64), (2, 1000, 8, 2, 128), (1, 1100, 8, 2, 128),
+                                          (1, 700, 2, 1, 64)])
+def test_attention_backward_shared_by_a_cluster(B, S, Hq, Hkv, D):
+    """Two, four and eight CTAs to a key block's query blocks, shares that are not equal and shares that are empty (the last
+    key blocks have one block a head).  The bound of the test above: bf16 probabilities and score gradients."""
+    torch.manual_seed(S)
+    qkv = (torch.randn(B, S, Hq + 2 * Hkv, D, device=DEV) * 0.5).bfloat16().requires_grad_()
+    o = attention.causal_attention(qkv, Hq, Hkv)
+    g = torch.randn_like(o)
+    (dqkv,) = torch.autograd.grad(o, qkv, g)
+    torch.cuda.synchronize()
+    assert attention.status_read_and_clear() == 0
+    qf = qkv.detach().float().requires_grad_()
+    (dref,) = torch.autograd.grad(_attn_ref(qf, Hq, Hkv), qf, g.float())
+    for part in (slice(0, Hq), slice(Hq, Hq + Hkv), slice(Hq + Hkv, None)):
+        d, r = dqkv[:, :, part].float(), dref[:, :, part]
+        assert ((d - r).norm() / r.norm()).item() < 1e-2
+
+
 @pytest.mark.parametrize("impl", ["2q+kt", "ws+ws"])
 def test_attention_rising_scores_rescale_the_accumulator(impl, monkeypatch):
     """Keys whose scores grow along the sequence raise the running row maximum again and again, so
