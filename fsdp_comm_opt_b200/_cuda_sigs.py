@@ -77,9 +77,10 @@ def declare(lib) -> None:
     _sig(lib, "zc_gemm_bf16_2sm_ld", P, P, P, L, L, L, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm_bias", P, P, P, P, L, L, L, L, L, L, I, I, I, P)
     _sig(lib, "zc_gemm_bf16_2sm_ws", P, P, P, P, L, L, L, L, L, L, I, I, I, P, L, P)
-    _sig(lib, "zc_gemm_2sm_split_bytes", L, L, L)
-    if hasattr(lib, "zc_gemm_2sm_split_bytes"):
-        lib.zc_gemm_2sm_split_bytes.restype = L
+    for name in ("zc_gemm_2sm_split_bytes", "zc_gemm_ws_bytes"):
+        _sig(lib, name, L, L, L)
+        if hasattr(lib, name):
+            getattr(lib, name).restype = L
     _sig(lib, "zc_gemm_status_read_and_clear")
     # fused collectives
     from ctypes import c_double, c_uint

@@ -41,6 +41,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "gemm_common.cuh"
 #include "launch_util.h"
 #include "nvtx_util.h"
 #include "umma.cuh"
@@ -241,44 +242,6 @@ __device__ __forceinline__ Unit unit_of(int u, const Params& p) {
   return w;
 }
 
-// f[j] += bias[col + j], j = 0..7 (col is a multiple of 8; the last group of a ragged N is read element-wise)
-__device__ __forceinline__ void add_bias8(const __nv_bfloat16* bias, int64_t col, int64_t N, float (&f)[8]) {
-  if (col + 8 <= N) {
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + col));
-    const __nv_bfloat162* bb = reinterpret_cast<const __nv_bfloat162*>(&b);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 t = __bfloat1622float2(bb[j]);
-      f[2 * j] += t.x;
-      f[2 * j + 1] += t.y;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (col + j < N) f[j] += __bfloat162float(bias[col + j]);
-  }
-}
-
-// f += the eight old bf16 values of C
-__device__ __forceinline__ void add_old8(const uint4& old, float (&f)[8]) {
-  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 o2 = __bfloat1622float2(ob[j]);
-    f[2 * j] += o2.x;
-    f[2 * j + 1] += o2.y;
-  }
-}
-__device__ __forceinline__ uint4 round8(const float (&f)[8]) {
-  uint4 v;
-  __nv_bfloat162 a0 = __floats2bfloat162_rn(f[0], f[1]), a1 = __floats2bfloat162_rn(f[2], f[3]);
-  __nv_bfloat162 a2 = __floats2bfloat162_rn(f[4], f[5]), a3 = __floats2bfloat162_rn(f[6], f[7]);
-  v.x = *reinterpret_cast<uint32_t*>(&a0);
-  v.y = *reinterpret_cast<uint32_t*>(&a1);
-  v.z = *reinterpret_cast<uint32_t*>(&a2);
-  v.w = *reinterpret_cast<uint32_t*>(&a3);
-  return v;
-}
 // Where a slab of partial sums keeps columns 4 c4 .. 4 c4 + 3 of a tile's row, in float4: the rows of a warp, which holds a
 // row a thread, lie next to each other.
 __device__ __forceinline__ int partial_off(int row, int c4) { return ((row >> 5) * (BN / 4) + c4) * 32 + (row & 31); }
@@ -598,38 +561,6 @@ __global__ void __launch_bounds__(256) gemm_2sm_fixup_kernel(const Params p) {
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-// 2-D bf16 row-major tensor [rows][cols] with rows `ld` elements apart; box = (box_cols inner, box_rows),
-// 128B swizzle.  Elements past `cols` in a row (padding up to ld) are outside the map and read as zeros.
-static bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t el[2] = {1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, el,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    fprintf(stderr, "[zc_gemm_2sm] cuTensorMapEncodeTiled failed (%d): ptr=%p rows=%lld cols=%lld box=(%d,%d)\n",
-            (int)r, ptr, (long long)rows, (long long)cols, box_cols, box_rows);
-  return r == CUDA_SUCCESS;
-}
-
 // Per-device launch state: how many clusters of two the device runs at once, and the tile counters.
 struct DeviceState {
   bool ready = false;
@@ -711,6 +642,15 @@ static Cut cut_of(int64_t M, int64_t N, int64_t K, int device_clusters) {
   return c;
 }
 
+// In how many parts along K the kernel of small products takes a product, 0 where this kernel is expected to be faster: with
+// many tiles, or where K is so long that 256 x 256 tiles, which read half as much an FMA, cut into more slices win.  In us: what
+// a launch costs beside its K blocks, a K block, the fix-up.
+static int small_parts(int64_t M, int64_t N, int64_t K, bool cut_k, int clusters) {
+  const Cut cut = cut_of(M, N, K, clusters);
+  const int split = cut_k ? cut.split : 1;
+  return gemm_small_parts(M, N, K, cut_k, 5.6 + 0.28 * (double)((K + BK - 1) / BK) / split + (split > 1 ? 4.0 : 0.0));
+}
+
 static int init_state(DeviceState& ds, int smem) {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (!ds.ready) {
@@ -742,9 +682,9 @@ int* zc_gemm_status_word();  // gemm_tcgen05.cu: the current device's GEMM statu
 // (and before the old C is added when `accumulate` is set).
 // `ws`: null, or `ws_bytes` of device memory (16-byte aligned) of the caller's, that no other stream uses meanwhile, for the
 // fp32 partial sums of a product that zc_gemm_2sm_split_bytes names a size for; without it such a product is not split.
-int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
-                        int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate, void* ws,
-                        int64_t ws_bytes, cudaStream_t st) {
+static int gemm_2sm(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K, int64_t lda,
+                    int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate, bool cut_k, void* ws, int64_t ws_bytes,
+                    cudaStream_t st) {
   ZC_NVTX_RANGE("zc_gemm_bf16_2sm");
   if (reinterpret_cast<uintptr_t>(bias) & 15) return zc::ERR_UNSUPPORTED;
   using namespace zc;
@@ -765,6 +705,11 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   const int a_major = trans_a ? MAJOR_MN : MAJOR_K;
   const int b_major = trans_b ? MAJOR_K : MAJOR_MN;
   if (a_major == MAJOR_MN && b_major == MAJOR_K) return ERR_UNSUPPORTED;  // no layer GEMM has this form
+  const int smem = SMEM_BYTES;
+  DeviceState& ds = g_state[dev];
+  if (const int rc = init_state(ds, smem)) return rc;
+  if (const int parts = small_parts(M, N, K, cut_k, ds.clusters))
+    return gemm_small_launch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_major, b_major, accumulate, parts, status, st);
   CUtensorMap mapA, mapB;
   bool ok;
   if (a_major == MAJOR_K) ok = make_map(&mapA, A, M, K, lda, BK, BM_CTA);
@@ -772,9 +717,6 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   if (b_major == MAJOR_K) ok = ok && make_map(&mapB, B, N, K, ldb, BK, BN_CTA);
   else ok = ok && make_map(&mapB, B, K, N, ldb, 64, BK);
   if (!ok) return ERR_BAD_ARG;
-  const int smem = SMEM_BYTES;
-  DeviceState& ds = g_state[dev];
-  if (const int rc = init_state(ds, smem)) return rc;
   Params p;
   p.C = (__nv_bfloat16*)C; p.M = M; p.N = N; p.ldc = ldc;
   p.m_tiles = (int)m_tiles; p.n_tiles = (int)n_tiles; p.k_blocks = (int)((K + BK - 1) / BK);
@@ -816,10 +758,17 @@ int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias,
   return rc;
 }
 
+int zc_gemm_bf16_2sm_ws(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
+                        int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate, void* ws,
+                        int64_t ws_bytes, cudaStream_t st) {
+  return gemm_2sm(A, B, C, bias, M, N, K, lda, ldb, ldc, trans_a, trans_b, accumulate, true, ws, ws_bytes, st);
+}
+
+// The same with every sum along K in one piece.
 int zc_gemm_bf16_2sm_bias(const void* A, const void* B, void* C, const void* bias, int64_t M, int64_t N, int64_t K,
                           int64_t lda, int64_t ldb, int64_t ldc, int trans_a, int trans_b, int accumulate,
                           cudaStream_t st) {
-  return zc_gemm_bf16_2sm_ws(A, B, C, bias, M, N, K, lda, ldb, ldc, trans_a, trans_b, accumulate, nullptr, 0, st);
+  return gemm_2sm(A, B, C, bias, M, N, K, lda, ldb, ldc, trans_a, trans_b, accumulate, false, nullptr, 0, st);
 }
 
 // Bytes of the workspace with which zc_gemm_bf16_2sm_ws splits an M x N x K product along K; 0 when it does not.
@@ -830,6 +779,16 @@ int64_t zc_gemm_2sm_split_bytes(int64_t M, int64_t N, int64_t K) {
   cudaGetDevice(&dev);
   if (M <= 0 || N <= 0 || K <= 0 || dev < 0 || dev >= 64 || init_state(g_state[dev], SMEM_BYTES)) return 0;
   return cut_of(M, N, K, g_state[dev].clusters).bytes();
+}
+
+// Bytes of the workspace that zc_gemm_bf16_2sm_ws wants for an M x N x K product: those, or 0 for one that the kernel of
+// small products takes.
+int64_t zc_gemm_ws_bytes(int64_t M, int64_t N, int64_t K) {
+  using namespace zc::g2;
+  const int64_t bytes = zc_gemm_2sm_split_bytes(M, N, K);  // (makes the device's state)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return bytes && small_parts(M, N, K, true, g_state[dev].clusters) ? 0 : bytes;
 }
 
 int zc_gemm_bf16_2sm_ld(const void* A, const void* B, void* C, int64_t M, int64_t N, int64_t K, int64_t lda,

@@ -4,7 +4,9 @@ Backends (``set_backend``):
   ``"tcgen05_2sm"``  the hand-written sm_100a kernel in ``csrc/gemm_tcgen05_2sm.cu``: clusters of two
                  CTAs, ``tcgen05.mma.cta_group::2`` on 256 x 256 tiles with the B operand split between
                  the pair, TMA loads into 128B-swizzled shared memory, TMEM accumulators, persistent
-                 over tiles with a split-K tail.  Any M, N, K; rows a multiple of 8 elements apart.
+                 over tiles with a split-K tail; products that do not fill the chip with such tiles run on
+                 ``csrc/gemm_small.cu`` (128 x 128 tiles on one SM, K over a cluster).  Any M, N, K; rows a
+                 multiple of 8 elements apart.
   ``"tcgen05"``  the one-SM kernel in ``csrc/gemm_tcgen05.cu`` (128 x 256 tiles; M % 128, N % 128,
                  K % 64).
   ``"cublas"``   ``torch.matmul`` (cuBLASLt), kept as the comparison column of the benchmarks.
@@ -43,8 +45,8 @@ def _rows_ok(t: torch.Tensor) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
-def _split_bytes(M: int, N: int, K: int, device: int) -> int:
-    return _lib.cuda().zc_gemm_2sm_split_bytes(M, N, K)
+def _ws_bytes(M: int, N: int, K: int, device: int) -> int:
+    return _lib.cuda().zc_gemm_ws_bytes(M, N, K)
 
 
 def _pad8(n: int) -> int:
@@ -66,7 +68,8 @@ def _kernel_for(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int, trans_
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
-         out: torch.Tensor | None = None, accumulate: bool = False, bias: torch.Tensor | None = None) -> torch.Tensor:
+         out: torch.Tensor | None = None, accumulate: bool = False, bias: torch.Tensor | None = None,
+         whole_k: bool = False) -> torch.Tensor:
     """C[M,N] (+)= op(A) @ op(B) for row-major 2-D bf16 tensors.
 
     op(A) is A ``[M,K]`` (or A^T of a stored ``[K,M]`` when ``trans_a``); op(B) is B ``[K,N]`` (or
@@ -75,7 +78,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
     multiple of 8 (GPT-2's vocabulary of 50257) the result allocated here is a ``[:, :N]`` view of a
     buffer whose rows are padded to the next multiple of 8, so that the next GEMM and the loss kernel
     can read it with aligned rows; its padding columns hold zeros.  ``bias`` ([N]) is added to every
-    row in the kernel's epilogue (the two-SM kernel), else by a separate add.
+    row in the kernel's epilogue (the two-SM kernel), else by a separate add.  ``whole_k``: every value is one
+    sum along K, whatever M and N are, so that the rows of a product have the same bits when they are computed apart.
     """
     M, K = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
     N = b.shape[0] if trans_b else b.shape[1]
@@ -94,12 +98,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
             fused_bias = (bias is not None and bias.dtype == torch.bfloat16 and bias.is_contiguous()
                           and bias.numel() == N and bias.data_ptr() % 16 == 0)
             # fp32 partial sums of a product that is split along K: this call's own, so that no other stream shares them
-            ws_bytes = _split_bytes(M, N, K, a.device.index)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device) if ws_bytes else None
-            _lib.check(lib.zc_gemm_bf16_2sm_ws(
-                a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if fused_bias else None, M, N, K,
-                a.stride(0), b.stride(0), out.stride(0), int(trans_a), int(trans_b), int(accumulate),
-                ws.data_ptr() if ws is not None else None, ws_bytes, _lib.stream_ptr(a.device)), "zc_gemm_bf16_2sm")
+            args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if fused_bias else None, M, N, K,
+                    a.stride(0), b.stride(0), out.stride(0), int(trans_a), int(trans_b), int(accumulate))
+            if whole_k:
+                rc = lib.zc_gemm_bf16_2sm_bias(*args, _lib.stream_ptr(a.device))
+            else:
+                ws_bytes = _ws_bytes(M, N, K, a.device.index)
+                ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device) if ws_bytes else None
+                rc = lib.zc_gemm_bf16_2sm_ws(*args, ws.data_ptr() if ws is not None else None, ws_bytes,
+                                             _lib.stream_ptr(a.device))
+            _lib.check(rc, "zc_gemm_bf16_2sm")
             if bias is not None and not fused_bias:
                 out.add_(bias.to(out.dtype))
         else:

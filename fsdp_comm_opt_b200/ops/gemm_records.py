@@ -85,7 +85,7 @@ class RecordLinear:
                 decode(s + self.ring - 1)
             slot = s % self.ring
             main.wait_event(self._decoded[slot])
-            gemm(self.buf[slot], x, False, True, out=out[s * R:(s + 1) * R])
+            gemm(self.buf[slot], x, False, True, out=out[s * R:(s + 1) * R], whole_k=True)
             ev = torch.cuda.Event()
             ev.record(main)
             self._free[slot] = ev
@@ -102,4 +102,4 @@ def linear_t_plain(x: torch.Tensor, records: torch.Tensor, headers: torch.Tensor
             out.copy_(y)
             return out
         return y
-    return gemm(w, x, False, True, out=out)
+    return gemm(w, x, False, True, out=out, whole_k=True)

@@ -899,6 +899,29 @@ def test_gemm_split_along_k_when_tiles_are_few(M, N, K):
         assert ((acc.double() - (ref + y.double())).norm() / ref.norm()).item() < 2 ** -8 + 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 128, 128), (129, 136, 136), (300, 1000, 1000), (512, 256, 1024), (256, 129, 2040), (1024, 1024, 4096),
+                                   (1536, 1500, 192), (128, 18944, 128), (128, 18945, 128)])
+def test_products_of_few_tiles_run_on_one_sm_a_tile(M, N, K):
+    """One tile, a row and a few columns more, ragged edges in every direction, K in two, four and eight parts, all SMs busy
+    (148 tiles) and one tile more than that.  Rounded once from fp32 sums: 2^-9 and the sums' 1e-5."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(M + N + K)
+    mk = lambda r, c: torch.randn(r, (c + 7) // 8 * 8, device=DEV).bfloat16()[:, :c]
+    x, w, dy, bias = mk(M, K), mk(N, K), mk(M, N), torch.randn(N, device=DEV).bfloat16()
+    ref = x.double() @ w.double().t()
+    y = gemm.gemm(x, w, False, True, bias=bias)
+    whole = gemm.gemm(x, w, False, True, whole_k=True)
+    acc = torch.empty(M, (N + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :N].copy_(dy)
+    gemm.gemm(x, w, False, True, out=acc, accumulate=True)
+    results = [(y, ref + bias.double()), (whole, ref), (acc, ref + dy.double()),
+               (gemm.gemm(dy, w, False, False), dy.double() @ w.double()), (gemm.gemm(dy, x, True, False), dy.double().t() @ x.double())]
+    torch.cuda.synchronize()
+    assert _lib.cuda().zc_gemm_status_read_and_clear() == 0
+    for got, want in results:
+        assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -9 + 1e-5
+
+
 def test_products_split_along_k_on_two_streams_have_partial_sums_of_their_own():
     """The tail of the last wave is split (4096 x 6144: 384 tiles on 74 clusters), and so is a product of few tiles; the slices
     are added by a second kernel, which other streams' products may run ahead of."""
