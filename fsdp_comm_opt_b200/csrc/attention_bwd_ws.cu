@@ -85,7 +85,7 @@ struct BwdParams {
   int64_t dks0, dks1, dks2, dvs0, dvs1, dvs2;
   float scale;
   int* status;
-  int parts;  // CTAs that share a key block's query blocks (the key-row kernel)
+  int parts;  // CTAs that share a key block's query heads (the key-row kernel)
 };
 
 template <int D>
@@ -558,21 +558,11 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
   const int part = SHARED ? blockIdx.x % parts : 0, unit = SHARED ? blockIdx.x / parts : blockIdx.x;
   const int jb = unit / per_jb;
   const int hk = (unit % per_jb) % p.Hkv, b = (unit % per_jb) / p.Hkv;
-  const int group = p.Hq / p.Hkv;
+  const int group = p.Hq / p.Hkv / parts;  // query heads of this CTA
+  const int h0 = hk * (p.Hq / p.Hkv) + part * group;
   const int k0 = jb * 128;
   const int nqb = (p.S + 127) / 128;
-  const int all_iters = group * (nqb - jb);  // query blocks at or below this key block's diagonal
-  const int iters = SHARED ? (all_iters - part + parts - 1) / parts : all_iters;  // this CTA's: the part-th, (part + parts)-th, ...
-  // the query head and block of an iteration, and from it to the CTA's next
-  auto skip = [&](int& h, int& ib, int by) {
-    ib += by;
-    while (ib >= nqb) { ib -= nqb - jb; ++h; }
-  };
-  auto start = [&](int& h, int& ib) { if (SHARED) skip(h, ib, part); };
-  auto next = [&](int& h, int& ib) {
-    if (SHARED) skip(h, ib, parts);
-    else if (++ib == nqb) { ib = jb; ++h; }
-  };
+  const int iters = group * (nqb - jb);  // query blocks at or below this key block's diagonal
   if (tid == 0) {
     mbar_init(&m.kv_full, 1);
     for (int i = 0; i < 2; ++i) {
@@ -615,8 +605,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         tma_load_4d(sK + sl * 16384, &mapK, &m.kv_full, sl * 64, hk, k0, b);
         tma_load_4d(sV + sl * 16384, &mapV, &m.kv_full, sl * 64, hk, k0, b);
       }
-      int h = hk * group, ib = jb;
-      start(h, ib);
+      int h = h0, ib = jb;
       for (int i = 0; i < iters; ++i) {
         const int sq = i & 1, sd = i % C::DO_STAGES;
         if (!role_wait(&m.q_empty[sq], ((i >> 1) & 1) ^ 1)) { *s_abort = 1; break; }
@@ -629,7 +618,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
 #pragma unroll
         for (int sl = 0; sl < D / 64; ++sl)
           tma_load_4d(sdO + sd * C::TILE + sl * 16384, &mapdO, &m.do_full[sd], sl * 64, h, ib * 128, b);
-        next(h, ib);
+        if (++ib == nqb) { ib = jb; ++h; }
       }
     } else if (warp == 1 && lane == 0) {
       const uint32_t id_s = idesc_bf16(128, 128, MAJOR_K, MAJOR_K);    // S^T, dP^T
@@ -656,12 +645,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         mma_commit(&m.dp_full);
       };
       auto run = [&]() -> bool {
-        if (!role_wait(&m.kv_full, 0)) return false;
-        if (SHARED && iters == 0) {  // fewer query blocks than CTAs share them
-          mma_commit(&m.all_done);
-          return true;
-        }
-        if (!role_wait(&m.q_full[0], 0)) return false;
+        if (!role_wait(&m.kv_full, 0) || !role_wait(&m.q_full[0], 0)) return false;
         tc_fence_after_sync();
         issue_s(0);
         if (!role_wait(&m.do_full[0], 0)) return false;
@@ -708,8 +692,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
       };
       if (!run()) *s_abort = 1;
     } else if (warp == 2) {
-      int h = hk * group, ib = jb;
-      start(h, ib);
+      int h = h0, ib = jb;
       for (int i = 0; i < iters; ++i) {
         const int st = i & 1;
         const int64_t row = ((int64_t)b * p.Hq + h) * p.S;
@@ -728,7 +711,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         dst[32 + lane] = make_float4(vd[0], vd[1], vd[2], vd[3]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&m.stat_full[st]);
-        next(h, ib);
+        if (++ib == nqb) { ib = jb; ++h; }
       }
     }
   } else if (warp < 12) {
@@ -739,8 +722,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
     const uint32_t lane_base = (uint32_t)(quarter * 32);
     const int c0 = half * 64;
     const uint64_t sl22 = pack2(p.scale * LOG2E, p.scale * LOG2E), scale2 = pack2(p.scale, p.scale);
-    int h = 0, ib = jb;
-    if (SHARED) skip(h, ib, part);
+    int ib = jb;
     bool fail = false;
     for (int i = 0; i < iters; ++i) {
       const int st = i & 1;
@@ -813,29 +795,27 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         mbar_arrive(&m.stat_empty[st]);
       }
       __syncwarp();
-      next(h, ib);
+      if (++ib == nqb) ib = jb;
     }
     if (!fail) fail = !mbar_wait_parked(&m.all_done, 0, s_abort);
     if (__any_sync(0xffffffffu, fail)) {
       *s_abort = 1;
     } else if (SHARED) {
-      // fp32 sums of this CTA's share into its own shared memory (K, V, Q and dO are done with), four columns of 128 rows
-      // after each other; nothing where it had no share
+      // fp32 sums of this CTA's heads into its own shared memory (K, V, Q and dO are done with), four columns of 128 rows
+      // after each other
       tc_fence_after_sync();
-      if (iters > 0) {
 #pragma unroll 1
-        for (int which = 0; which < 2; ++which) {
-          float4* dst = reinterpret_cast<float4*>(smem) + which * (D / 4) * 128 + r;
+      for (int which = 0; which < 2; ++which) {
+        float4* dst = reinterpret_cast<float4*>(smem) + which * (D / 4) * 128 + r;
 #pragma unroll 1
-          for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
-            uint32_t rr[32];
-            tmem_ld32(tmem_addr(tm + (which ? C::TM_DV : C::TM_DK), lane_base, c), rr);
-            tmem_ld_wait();
+        for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
+          uint32_t rr[32];
+          tmem_ld32(tmem_addr(tm + (which ? C::TM_DV : C::TM_DK), lane_base, c), rr);
+          tmem_ld_wait();
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-              dst[(c / 4 + q) * 128] = make_float4(__uint_as_float(rr[4 * q]), __uint_as_float(rr[4 * q + 1]),
-                                                   __uint_as_float(rr[4 * q + 2]), __uint_as_float(rr[4 * q + 3]));
-          }
+          for (int q = 0; q < 8; ++q)
+            dst[(c / 4 + q) * 128] = make_float4(__uint_as_float(rr[4 * q]), __uint_as_float(rr[4 * q + 1]),
+                                                 __uint_as_float(rr[4 * q + 2]), __uint_as_float(rr[4 * q + 3]));
         }
       }
     } else {
@@ -870,8 +850,7 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;     // query row of the tile == TMEM lane
     const uint32_t lane_base = (uint32_t)(quarter * 32);
-    int h = hk * group, ib = jb;
-    start(h, ib);
+    int h = h0, ib = jb;
     bool fail = false;
     for (int i = 0; i < iters; ++i) {
       fail = !mbar_wait_parked(&m.dq_full, i & 1, s_abort) || *s_abort;
@@ -903,24 +882,24 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         }
       }
       __syncwarp();
-      next(h, ib);
+      if (++ib == nqb) { ib = jb; ++h; }
     }
     if (tid == 384) bulk_wait0();
     if (fail) *s_abort = 1;
   }
   tc_fence_before_sync();
-  if (SHARED) {
+  if constexpr (SHARED) {
     __syncwarp();
     cluster_sync();
     if (warp >= 4 && warp < 12) {
       // Each CTA of the cluster adds up its share of the columns, in the order of the parts, eight of a row a thread.
-      const int filled = min(parts, all_iters), groups = 2 * (D / 8) / parts;
+      const int groups = 2 * (D / 8) / parts;
       for (int u = tid - 128; u < groups * 128; u += 256) {
         const int g = part * groups + (u >> 7), row = u & 127, key = k0 + row;  // g: dK's groups of eight columns, then dV's
         const uint32_t at = smem_u32(smem) + (uint32_t)(2 * g * 128 + row) * 16;
         float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
-        for (int c = 0; c < filled; ++c) {
+        for (int c = 0; c < parts; ++c) {
           const float4 x = ld_cluster(at, c), y = ld_cluster(at + 128 * 16, c);
           f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
           f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
@@ -942,21 +921,23 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
   if (warp == 1) tmem_dealloc(tm, 512);
 }
 
-// How many CTAs (a cluster) share the query blocks of a key block.  A key block's iterations follow one another, so with
-// few key blocks, batches and KV heads the chip waits for the longest of them: 1024 keys, 8 / 2 heads of 128 are 16 CTAs of up to
-// 32 iterations, 83 us; shared by eight 27.  Counted in iterations (2.3 us at head dimension 128, 2 at 64): the longest CTA
-// or the average of all SMs, and for every wave of CTAs what one costs beside its iterations, 4 alone and a few more for
-// adding up the shares.  (us, alone and shared) 2048 keys, 32 / 8 heads: 166, by two 106; 4096, 8 / 2: 308, by eight 111;
-// 4096, 32 / 8: 337, by two 353, so alone; 1024, 64 / 8: 167, by four 75; head dimension 64, 2048 keys, 8 heads: 40, by two 36.
+// How many CTAs (a cluster) share the query heads of a key block.  A key block's iterations follow one another, so with few
+// key blocks, batches and KV heads the chip waits for the longest of them: 1024 keys, 8 / 2 heads of 128 are 16 CTAs of up to
+// 32 iterations, 83 us.  By heads and not by query blocks: a query block's dQ then still gets its key blocks' tiles an
+// iteration after each other, in the same order from run to run where all CTAs run at once.  Counted in iterations (2.3 us at head
+// dimension 128, 2 at 64): the longest CTA or the average of all SMs, and for every wave of CTAs what one costs beside its
+// iterations, 4 alone and a few more for adding up the shares.  (us, alone and
+// shared) 1024 keys, 8 / 2 heads: 83, by four 31; 2048, 32 / 8: 166, by two 100; 4096, 8 / 2: 308, by four 108; 1024, 64 / 8: 167, by
+// four 72; 4096, 64 / 8: 713, by two 683; 4096, 32 / 8: 337, by two 353, so alone.
 static int parts_of(int S, int Hq, int Hkv, int B, int D) {
   const int sms = sm_count(), nqb = (S + 127) / 128, group = Hq / Hkv;
   const double alone = 4.0, shared = D == 128 ? 7.0 : 5.5;
   const double ctas = (double)nqb * Hkv * B, longest = (double)group * nqb, all = ctas * group * (nqb + 1) / 2;
   int best = 1;
   double least = 0;
-  for (int c = 1; c <= 8; c *= 2) {
+  for (int c = 1; c <= 8 && group % c == 0; c *= 2) {
     const double slots = c == 8 ? sms * 0.875 : sms;  // clusters of eight leave SMs of every GPC over
-    const double t = std::max(std::ceil(longest / c), all / sms) + std::ceil(ctas * c / slots) * (c > 1 ? shared : alone);
+    const double t = std::max(longest / c, all / sms) + std::ceil(ctas * c / slots) * (c > 1 ? shared : alone);
     if (c == 1 || t < least) { best = c; least = t; }
   }
   return best;
