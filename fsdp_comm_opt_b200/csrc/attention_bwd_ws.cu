@@ -395,6 +395,7 @@ template <int D>
 __global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
                                                          float* __restrict__ delta, float4* __restrict__ dq_acc, int S,
                                                          int Hq, int64_t total) {
+  chain();
   constexpr int T = D / 8;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   float acc = 0.f;
@@ -423,6 +424,7 @@ __global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict
 template <int D>
 __global__ void __launch_bounds__(256) dq_convert8_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
                                                           int64_t units, uint32_t Hq, int64_t s_bs, int64_t s_h) {
+  chain();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= units) return;
   const float4 a = __ldcs(acc + 2 * i), c = __ldcs(acc + 2 * i + 1);
@@ -592,6 +594,8 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tm = m.tmem_base;
+  chain_wait();
+  if (warp == 1) chain_next();  // which has its TMEM
   // bounded wait: parked in hardware, woken when the phase completes, given up after two seconds or when another role
   // raised the abort flag
   auto role_wait = [&](uint64_t* bar, uint32_t parity) -> bool { return mbar_wait_parked(bar, parity, s_abort); };
@@ -953,24 +957,12 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
   if (p.parts == 1) {
     if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
       return launch_status();
-    attn_bwd_kt_kernel<D, false><<<units, 512, C::SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+    zc::launch_chained(attn_bwd_kt_kernel<D, false>, units, 512, C::SMEM, st, mq, mk, mv, mdo, mdq, p);
     return launch_status();
   }
   if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
     return launch_status();
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(units * p.parts);
-  cfg.blockDim = dim3(512);
-  cfg.dynamicSmemBytes = C::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = p.parts;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, attn_bwd_kt_kernel<D, true>, mq, mk, mv, mdo, mdq, (const BwdParams)p);
+  zc::launch_chained_cluster(p.parts, attn_bwd_kt_kernel<D, true>, units * p.parts, 512, C::SMEM, st, mq, mk, mv, mdo, mdq, p);
   return launch_status();
 }
 
@@ -1086,18 +1078,18 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
     delta_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                      delta, B, S, Hq, D);
   } else if (D == 128) {
-    delta_zero_kernel<128><<<ugrid, 256, 0, st>>>((const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
+    zc::launch_chained(delta_zero_kernel<128>, ugrid, 256, 0, st, (const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
   } else {
-    delta_zero_kernel<64><<<ugrid, 256, 0, st>>>((const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
+    zc::launch_chained(delta_zero_kernel<64>, ugrid, 256, 0, st, (const uint4*)o, (const uint4*)dout, delta, (float4*)dq_acc, S, Hq, rows);
   }
   const int rc = D == 128 ? bkt::launch<128>(mq, mk, mv, mdo, mdq, p, st) : bkt::launch<64>(mq, mk, mv, mdo, mdq, p, st);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(dq) & 15) || rows >= (1ll << 32))
     dq_convert_kernel<<<(unsigned)(sm_count() * 16), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, (int64_t)B * S, Hq, D, dqs1, dqs2);
   else if (D == 128)
-    dq_convert8_kernel<128><<<ugrid, 256, 0, st>>>((const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
+    zc::launch_chained(dq_convert8_kernel<128>, ugrid, 256, 0, st, (const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
   else
-    dq_convert8_kernel<64><<<ugrid, 256, 0, st>>>((const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
+    zc::launch_chained(dq_convert8_kernel<64>, ugrid, 256, 0, st, (const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
   return launch_status();
 }
 

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_fwd_2q_kernel(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tm = tmem_base;
+  chain_wait();
+  if (warp == 1) chain_next();  // which has its TMEM
 
   if (warp == 0) {
     if (lane == 0) {
@@ -399,7 +401,7 @@ int zc_attn_fwd_2q(const void* q, const void* k, const void* v, void* o, float* 
   const int smem = 65536 + STAGES * 32768 + 1024;
   static bool attr = false;
   if (!attr) { cudaFuncSetAttribute(attn_fwd_2q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr = true; }
-  attn_fwd_2q_kernel<<<p.ncb * Hq * B, THREADS, smem, st>>>(mq, mk, mv, p);
+  zc::launch_chained(attn_fwd_2q_kernel, p.ncb * Hq * B, THREADS, smem, st, mq, mk, mv, p);
   return launch_status();
 }
 

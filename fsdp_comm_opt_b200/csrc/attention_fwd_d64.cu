@@ -84,6 +84,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_fwd_d64_kernel(const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tm_s = tmem_base, tm_o = tm_s + 128, tm_p = tm_s + 192;
+  chain_wait();
+  if (warp == 1) chain_next();  // which has its TMEM
 
   if (warp < 4) {
     regs_dec<48>();  // 48 + 208 = the launch's 2 x 128
@@ -278,7 +280,7 @@ int attn_fwd_d64(const void* q, const void* k, const void* v, void* o, float* ls
   p.nqb = (S + 127) / 128;
   if (cudaFuncSetAttribute(attn_fwd_d64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
     return launch_status();
-  attn_fwd_d64_kernel<<<p.nqb * Hq * B, THREADS, SMEM, st>>>(mq, mk, mv, p);
+  zc::launch_chained(attn_fwd_d64_kernel, p.nqb * Hq * B, THREADS, SMEM, st, mq, mk, mv, p);
   return launch_status();
 }
 

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
     const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ rstd_out, int cols, float eps) {
+  chain();
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
   const int nvec = cols / 8;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
     const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
+  chain();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(
     const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
     const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw32,
     float* __restrict__ partials, int64_t rows, int cols) {
+  chain();
   __shared__ float red[32];
   const int nvec = cols / 8;
   float wv[MAXV][8], dwacc[MAXV][8];
@@ -267,6 +270,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(
 // latency: 1024 columns are 32 blocks of a few loads each (3.0 us; 8 blocks of 32 x 32 threads took 5.1).
 __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __restrict__ partials, int nblocks,
                                                                 int cols, float* __restrict__ dw) {
+  chain();
   __shared__ float4 acc[8][33];
   const int c4 = blockIdx.x * 8 + threadIdx.x;  // float4 column
   const int lane = (threadIdx.y * 8 + threadIdx.x) & 31, warp = threadIdx.y >> 2;
@@ -301,6 +305,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __
 __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
                                                    const float* __restrict__ sinT, int64_t T, int S, int n_rot,
                                                    int total_heads, int D, float sign) {
+  chain();
   const int vph = D / 16;  // 8-element vectors per half head
   const int64_t total = T * n_rot * vph;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -334,6 +339,7 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ q
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                                          __nv_bfloat16* __restrict__ out, int64_t T, int F) {
+  chain();
   const int vpr = F / 8;
   const int64_t total = T * vpr;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -352,6 +358,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                                          const __nv_bfloat16* __restrict__ dy,
                                                          __nv_bfloat16* __restrict__ dgu, int64_t T, int F) {
+  chain();
   const int vpr = F / 8;
   const int64_t total = T * vpr;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -413,6 +420,7 @@ template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CE_THREADS, 3)
     ce_row_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ row_loss,
                   const float* __restrict__ inv_count, int V, int64_t ld, int ignore_index) {
+  chain();
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) uint8_t ce_smem[];
   BF8* part = reinterpret_cast<BF8*>(ce_smem);
@@ -503,7 +511,7 @@ static int ce_rows(__nv_bfloat16* logits, const int64_t* labels, float* row_loss
   const int smem = ((V / 8 + CL - 1) / CL) * 16;
   if (cudaFuncSetAttribute(ce_row_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, CE_SMEM) != cudaSuccess)
     return launch_status();
-  ce_row_kernel<CL><<<(unsigned)(T * CL), CE_THREADS, smem, st>>>(logits, labels, row_loss, inv_count, V, ld, ignore_index);
+  zc::launch_chained(ce_row_kernel<CL>, (unsigned)(T * CL), CE_THREADS, smem, st, logits, labels, row_loss, inv_count, V, ld, ignore_index);
   return launch_status();
 }
 
@@ -517,6 +525,7 @@ __global__ void __launch_bounds__(CE_THREADS, 3) ce_kernel(__nv_bfloat16* __rest
                                                   const int64_t* __restrict__ labels,
                                                   float* __restrict__ row_loss, const float* __restrict__ inv_count,
                                                   int V, int64_t ld, int ignore_index) {
+  chain();
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
@@ -635,6 +644,7 @@ __global__ void __launch_bounds__(256) adamw_vec_kernel(TP* __restrict__ p, TG* 
                                                         TS* __restrict__ v, int64_t nvec, float lr, float b1, float b2,
                                                         float eps, float wd, float bc1, float rsqrt_bc2,
                                                         int zero_grad, const int* __restrict__ guard) {
+  chain();
   if (guard && *guard) return;  // a collective of this step gave up: leave parameters and moments alone
   const float decay = 1.f - lr * wd, step = lr / bc1;
   auto update = [&](float (&pf)[8], const float (&gf)[8], float (&mf)[8], float (&vf)[8]) {
@@ -697,7 +707,7 @@ int adamw_launch(void* p, void* g, void* m, void* v, int64_t n, float lr, float 
     // a few dozen CTAs per SM that follow one another in address order: 10^9 elements take 2301 us, 2424 with one
     // wave whose CTAs stride through seven buffers at their own pace
     const int grid = (int)std::min<int64_t>((nvec + 511) / 512, (int64_t)sm_count() * 64);
-    adamw_vec_kernel<TP, TG, TS><<<grid, 256, 0, st>>>((TP*)p, (TG*)g, (TS*)m, (TS*)v, nvec, lr, b1, b2, eps, wd,
+    zc::launch_chained(adamw_vec_kernel<TP, TG, TS>, grid, 256, 0, st, (TP*)p, (TG*)g, (TS*)m, (TS*)v, nvec, lr, b1, b2, eps, wd,
                                                         bc1, rs, zg, guard);
   } else {
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 16);
@@ -732,7 +742,7 @@ int zc_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
   if (nvec <= 32 * 20) {  // one warp per row (wider rows do not fit a warp's registers)
     const unsigned grid = (unsigned)((rows + 3) / 4);
 #define ZC_RN_FWDW(V)                                                                                             \
-  zc::rmsnorm_fwd_warp_kernel<V><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, \
+  zc::launch_chained(zc::rmsnorm_fwd_warp_kernel<V>, grid, 128, 0, st, (const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, \
                                                        (bf16*)h_out, rstd, rows, cols, eps)
     if (nvec <= 32 * 4) ZC_RN_FWDW(4);
     else if (nvec <= 32 * 16) ZC_RN_FWDW(16);
@@ -741,7 +751,7 @@ int zc_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
     return zc::launch_status();
   }
 #define ZC_RN_FWD(V)                                                                                              \
-  zc::rmsnorm_fwd_kernel<V><<<(unsigned)rows, zc::RN_THREADS, 0, st>>>((const bf16*)x, (const bf16*)res,          \
+  zc::launch_chained(zc::rmsnorm_fwd_kernel<V>, (unsigned)rows, zc::RN_THREADS, 0, st, (const bf16*)x, (const bf16*)res,          \
                                                                        (const bf16*)w, (bf16*)y, (bf16*)h_out,    \
                                                                        rstd, cols, eps)
   if (nvec <= zc::RN_THREADS) ZC_RN_FWD(1);
@@ -763,7 +773,7 @@ int zc_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
   const int grid = zc_rmsnorm_bwd_ctas(rows);
   const int nvec = cols / 8;
 #define ZC_RN_BWD(V)                                                                                             \
-  zc::rmsnorm_bwd_kernel<V><<<grid, zc::RN_THREADS, 0, st>>>((const bf16*)dy, (const bf16*)h, (const bf16*)w,    \
+  zc::launch_chained(zc::rmsnorm_bwd_kernel<V>, grid, zc::RN_THREADS, 0, st, (const bf16*)dy, (const bf16*)h, (const bf16*)w,    \
                                                              rstd, (const bf16*)dh, (bf16*)dx, dw32, partials,   \
                                                              rows, cols)
   if (nvec <= zc::RN_THREADS) ZC_RN_BWD(1);
@@ -771,7 +781,7 @@ int zc_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
   else ZC_RN_BWD(4);
 #undef ZC_RN_BWD
   if (partials)
-    zc::rmsnorm_dw_reduce_kernel<<<(cols / 4 + 7) / 8, dim3(8, 128), 0, st>>>(partials, grid, cols, dw32);
+    zc::launch_chained(zc::rmsnorm_dw_reduce_kernel, (cols / 4 + 7) / 8, dim3(8, 128), 0, st, partials, grid, cols, dw32);
   return zc::launch_status();
 }
 
@@ -781,7 +791,7 @@ int zc_rope_inplace(void* qkv, const float* cosT, const float* sinT, int64_t T, 
   const int64_t total = T * n_rot * (D / 16);
   if (total == 0) return 0;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
-  zc::rope_kernel<<<grid, 256, 0, st>>>((bf16*)qkv, cosT, sinT, T, S, n_rot, total_heads, D, sign);
+  zc::launch_chained(zc::rope_kernel, grid, 256, 0, st, (bf16*)qkv, cosT, sinT, T, S, n_rot, total_heads, D, sign);
   return zc::launch_status();
 }
 
@@ -790,7 +800,7 @@ int zc_swiglu_fwd(const void* gu, void* out, int64_t T, int F, cudaStream_t st) 
   const int64_t total = T * (F / 8);
   if (total == 0) return 0;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 128);
-  zc::swiglu_fwd_kernel<<<grid, 256, 0, st>>>((const bf16*)gu, (bf16*)out, T, F);
+  zc::launch_chained(zc::swiglu_fwd_kernel, grid, 256, 0, st, (const bf16*)gu, (bf16*)out, T, F);
   return zc::launch_status();
 }
 
@@ -799,7 +809,7 @@ int zc_swiglu_bwd(const void* gu, const void* dy, void* dgu, int64_t T, int F, c
   const int64_t total = T * (F / 8);
   if (total == 0) return 0;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 128);
-  zc::swiglu_bwd_kernel<<<grid, 256, 0, st>>>((const bf16*)gu, (const bf16*)dy, (bf16*)dgu, T, F);
+  zc::launch_chained(zc::swiglu_bwd_kernel, grid, 256, 0, st, (const bf16*)gu, (const bf16*)dy, (bf16*)dgu, T, F);
   return zc::launch_status();
 }
 
@@ -815,7 +825,7 @@ int zc_ce_fwd_bwd_ld(void* logits, const int64_t* labels, float* row_loss, const
     if (bytes <= zc::CE_SMEM) return zc::ce_rows<1>(lg, labels, row_loss, inv_count, T, V, ld, ignore_index, st);
     return zc::ce_rows<2>(lg, labels, row_loss, inv_count, T, V, ld, ignore_index, st);
   }
-  zc::ce_kernel<<<(unsigned)T, zc::CE_THREADS, 0, st>>>((bf16*)logits, labels, row_loss, inv_count, V, ld, ignore_index);
+  zc::launch_chained(zc::ce_kernel, (unsigned)T, zc::CE_THREADS, 0, st, (bf16*)logits, labels, row_loss, inv_count, V, ld, ignore_index);
   return zc::launch_status();
 }
 

@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(THREADS, 3) embedding_grad_kernel(const int64_
                                                                  const __nv_bfloat16* __restrict__ dout,
                                                                  __nv_bfloat16* __restrict__ grad, int n, int dim,
                                                                  int64_t rows, int accumulate) {
+  chain();
   __shared__ uint32_t match[MAX_N / 32];
   __shared__ uint32_t any[MAX_N / 1024];   // which words of `match` are not zero
   __shared__ uint32_t count;               // positions with this id: all, and in the upper half those before this block's
@@ -153,7 +154,7 @@ int zc_embedding_grad(const void* ids, const void* dout, void* grad, int64_t n, 
   if (n < 1 || n > emb::MAX_N || dim < 8 || dim % 8 || dim > (1 << 24) || rows < 1) return ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(grad)) & 15) return ERR_UNSUPPORTED;
   if (!accumulate) cudaMemsetAsync(grad, 0, (size_t)rows * dim * 2, st);
-  emb::embedding_grad_kernel<<<(unsigned)n, emb::THREADS, 0, st>>>((const int64_t*)ids, (const __nv_bfloat16*)dout,
+  zc::launch_chained(emb::embedding_grad_kernel, (unsigned)n, emb::THREADS, 0, st, (const int64_t*)ids, (const __nv_bfloat16*)dout,
                                                                    (__nv_bfloat16*)grad, (int)n, (int)dim, rows, accumulate);
   return launch_status();
 }

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     fence_proxy_async_smem();
     if (lane == 0) s_abort = 0;
     __syncwarp();
+    chain_wait();
     if (lane == 0) {
       if (PARTS > 1) mbar_expect_tx(&sh.received, TILE_BYTES - SHARE);
       for (int i = 0; i < min(kbs, STAGES); ++i) load(i, i);
@@ -121,6 +122,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tm = sh.tmem_base;
+  if (warp != 0) chain_wait();
+  if (warp == 1) chain_next();  // which has its TMEM
 
   if (warp == 0) {
     if (lane == 0) {
@@ -294,14 +297,7 @@ static int launch(cudaLaunchConfig_t cfg, const CUtensorMap& mapA, const CUtenso
   const auto kernel = gemm_small_kernel<A_MAJOR, B_MAJOR, PARTS>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_STAGES * STAGE + (int)sizeof(Shared)) != cudaSuccess)
     return launch_status();
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = PARTS;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = PARTS > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, p);
+  launch_chained_cluster(PARTS, kernel, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes, cfg.stream, mapA, mapB, p);
   return launch_status();
 }
 template <int PARTS>

@@ -291,6 +291,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     tc_fence_after_sync();
   }
   cluster_wait();  // both CTAs' barriers are initialised before any remote arrival
+  chain_wait();
+  if (warp == 1) chain_next();  // which has its TMEM
   const uint32_t tm = sh.tmem_base;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t full_base = smem_u32(&full[0]), empty_base = smem_u32(&empty[0]);
@@ -537,6 +539,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
 
 // C tile (+)= sum over the K slices of its fp32 partials, rounded once to bf16.
 __global__ void __launch_bounds__(256) gemm_2sm_fixup_kernel(const Params p) {
+  chain();
   const int tail = blockIdx.y;  // index among the split tiles
   int mi, ni;
   tile_coords(p.full_tiles + tail, p, mi, ni);
@@ -747,12 +750,12 @@ static int gemm_2sm(const void* A, const void* B, void* C, const void* bias, int
     if (slot < COUNTER_SLOTS) p.counter = ds.counters + 2 * slot;
   }
   const dim3 grid(2 * cut.grid_clusters);
-  if (a_major == MAJOR_K && b_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_K><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
-  else if (a_major == MAJOR_K) gemm_2sm_kernel<MAJOR_K, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
-  else gemm_2sm_kernel<MAJOR_MN, MAJOR_MN><<<grid, THREADS, smem, st>>>(mapA, mapB, p);
+  if (a_major == MAJOR_K && b_major == MAJOR_K) zc::launch_chained(gemm_2sm_kernel<MAJOR_K, MAJOR_K>, grid, THREADS, smem, st, mapA, mapB, p);
+  else if (a_major == MAJOR_K) zc::launch_chained(gemm_2sm_kernel<MAJOR_K, MAJOR_MN>, grid, THREADS, smem, st, mapA, mapB, p);
+  else zc::launch_chained(gemm_2sm_kernel<MAJOR_MN, MAJOR_MN>, grid, THREADS, smem, st, mapA, mapB, p);
   int rc = launch_status();
   if (rc == 0 && p.split > 1) {
-    gemm_2sm_fixup_kernel<<<dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st>>>(p);
+    zc::launch_chained(gemm_2sm_fixup_kernel, dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st, p);
     rc = launch_status();
   }
   return rc;

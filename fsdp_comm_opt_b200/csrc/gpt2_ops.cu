@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(LN_THREADS) layernorm_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
     const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ mean_out, float* __restrict__ rstd_out, int cols, float eps) {
+  chain();
   __shared__ float2 red[32];
   const int64_t row = blockIdx.x;
   const int nvec = cols / 8;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(LN_THREADS) layernorm_bwd_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dh,
     __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int64_t rows, int cols) {
+  chain();
   __shared__ float2 red[32];
   const int nvec = cols / 8;
   float wv[MAXV][8], dwacc[MAXV][8], dbacc[MAXV][8];
@@ -204,6 +206,7 @@ __global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* _
                                                                   int seg, void* __restrict__ outA,
                                                                   void* __restrict__ outB, int out_bf16, int accA,
                                                                   int accB) {
+  chain();
   __shared__ float4 acc[32][32];
   const int c4 = blockIdx.x * 32 + threadIdx.x;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -243,6 +246,7 @@ __global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* _
 // 256 columns; blockIdx.y strides over the rows; partials[blockIdx.y][cols] fp32
 __global__ void __launch_bounds__(256) bf16_column_partials_kernel(const __nv_bfloat16* __restrict__ in, int64_t rows,
                                                                    int cols, int64_t ld, float* __restrict__ partials) {
+  chain();
   __shared__ float red[8][32][8];
   const int v = blockIdx.x * 32 + threadIdx.x;  // 8-column vector
   float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -278,6 +282,7 @@ constexpr float GELU_C = 0.044715f;
 __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ bias,
                                                             __nv_bfloat16* __restrict__ y, int64_t rows, int cols) {
+  chain();
   const int vpr = cols / 8;
   const int64_t total = rows * vpr;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
@@ -299,6 +304,7 @@ __global__ void __launch_bounds__(256) bias_gelu_bwd_kernel(const __nv_bfloat16*
                                                             const __nv_bfloat16* __restrict__ bias,
                                                             const __nv_bfloat16* __restrict__ dy,
                                                             __nv_bfloat16* __restrict__ dx, int64_t rows, int cols) {
+  chain();
   const int vpr = cols / 8;
   const int64_t total = rows * vpr;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
@@ -334,7 +340,7 @@ int zc_layernorm_fwd(const void* x, const void* res, const void* w, const void* 
   if (rows == 0) return 0;
   const int nvec = cols / 8;
 #define ZC_LN_FWD(V)                                                                                              \
-  layernorm_fwd_kernel<V><<<(unsigned)rows, LN_THREADS, 0, st>>>((const bf16*)x, (const bf16*)res, (const bf16*)w,  \
+  zc::launch_chained(layernorm_fwd_kernel<V>, (unsigned)rows, LN_THREADS, 0, st, (const bf16*)x, (const bf16*)res, (const bf16*)w,  \
                                                                  (const bf16*)b, (bf16*)y, (bf16*)h_out, mean, rstd, \
                                                                  cols, eps)
   if (nvec <= LN_THREADS) ZC_LN_FWD(1);
@@ -358,13 +364,13 @@ int zc_layernorm_bwd(const void* dy, const void* x, const void* w, const float* 
   const int grid = zc_layernorm_bwd_ctas(rows);
   const int nvec = cols / 8;
 #define ZC_LN_BWD(V)                                                                                          \
-  layernorm_bwd_kernel<V><<<grid, LN_THREADS, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd, \
+  zc::launch_chained(layernorm_bwd_kernel<V>, grid, LN_THREADS, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd, \
                                                        (const bf16*)dh, (bf16*)dx, partials, rows, cols)
   if (nvec <= LN_THREADS) ZC_LN_BWD(1);
   else if (nvec <= 2 * LN_THREADS) ZC_LN_BWD(2);
   else ZC_LN_BWD(4);
 #undef ZC_LN_BWD
-  column_sum_deliver_kernel<<<(2 * cols / 4 + 31) / 32, dim3(32, 32), 0, st>>>(partials, grid, 2 * cols, cols, dw, db,
+  zc::launch_chained(column_sum_deliver_kernel, (2 * cols / 4 + 31) / 32, dim3(32, 32), 0, st, partials, grid, 2 * cols, cols, dw, db,
                                                                                 out_bf16, acc_w, acc_b);
   return zc::launch_status();
 }
@@ -380,9 +386,9 @@ int zc_bf16_column_sum(const void* in, int64_t rows, int cols, int64_t ld, void*
   if (cols % 8 || ld % 8 || (reinterpret_cast<uintptr_t>(in) & 15)) return ERR_UNSUPPORTED;
   if (rows == 0 || cols == 0) return 0;
   const int rb = zc_bf16_column_sum_blocks(rows);
-  bf16_column_partials_kernel<<<dim3((cols / 8 + 31) / 32, rb), dim3(32, 8), 0, st>>>((const bf16*)in, rows, cols, ld,
+  zc::launch_chained(bf16_column_partials_kernel, dim3((cols / 8 + 31) / 32, rb), dim3(32, 8), 0, st, (const bf16*)in, rows, cols, ld,
                                                                                        partials);
-  column_sum_deliver_kernel<<<(cols / 4 + 31) / 32, dim3(32, 32), 0, st>>>(partials, rb, cols, cols, out, nullptr,
+  zc::launch_chained(column_sum_deliver_kernel, (cols / 4 + 31) / 32, dim3(32, 32), 0, st, partials, rb, cols, cols, out, nullptr,
                                                                             out_bf16, accumulate, 0);
   return zc::launch_status();
 }
@@ -392,7 +398,7 @@ int zc_bias_gelu_fwd(const void* x, const void* bias, void* y, int64_t rows, int
   const int64_t total = rows * (cols / 8);
   if (total == 0) return 0;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
-  zc::gpt2::bias_gelu_fwd_kernel<<<grid, 256, 0, st>>>((const bf16*)x, (const bf16*)bias, (bf16*)y, rows, cols);
+  zc::launch_chained(zc::gpt2::bias_gelu_fwd_kernel, grid, 256, 0, st, (const bf16*)x, (const bf16*)bias, (bf16*)y, rows, cols);
   return zc::launch_status();
 }
 
@@ -402,7 +408,7 @@ int zc_bias_gelu_bwd(const void* x, const void* bias, const void* dy, void* dx, 
   const int64_t total = rows * (cols / 8);
   if (total == 0) return 0;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)zc::sm_count() * 16);
-  zc::gpt2::bias_gelu_bwd_kernel<<<grid, 256, 0, st>>>((const bf16*)x, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
+  zc::launch_chained(zc::gpt2::bias_gelu_bwd_kernel, grid, 256, 0, st, (const bf16*)x, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
                                                         rows, cols);
   return zc::launch_status();
 }

@@ -46,6 +46,50 @@ inline int launch_status() {
   return e == cudaSuccess ? 0 : (int)e;
 }
 
+// Kernels of a recorded step that follow one another on a stream.  A kernel that begins with chain() (or calls chain_wait()
+// before any thread's first access to global memory, and chain_next() once its CTA has what it needs of the SM) may be
+// launched by launch_chained: in a launch that is being recorded its CTAs then come up while the kernel before it still runs and
+// wait there until that has completed and its results are seen.  Not in launches that run at once: beside collectives, whose
+// CTAs need the slots that the waiting ones would hold.  Step of the tiny model (110 kernels)
+// 355 -> 334 us, of the small one (190) 1647 -> 1609.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain() {
+  chain_wait();
+  chain_next();
+}
+template <typename... P, typename... A>
+inline void launch_chained_cluster(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                   A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusActive) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster;
+    at[n].val.clusterDim.y = 1;
+    at[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  launch_chained_cluster(1, kernel, grid, block, smem, st, args...);
+}
+#endif
+
 constexpr int ERR_BAD_ARG = -1;
 constexpr int ERR_UNSUPPORTED = -2;
 
