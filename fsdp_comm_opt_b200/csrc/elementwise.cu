@@ -192,67 +192,97 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
 // dw = sum_rows dy * xhat: every CTA keeps partial sums in registers over its rows and writes them
 // to its row of `partials` ([gridDim.x, cols] fp32), which rmsnorm_dw_reduce_kernel then sums
 // (one fp32 atomic per column and CTA instead was 2.4 M atomics on 4096 addresses per call and
-// took most of the kernel's time); with partials == nullptr the atomics into dw32 remain
-template <int MAXV>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(
+// took most of the kernel's time); with partials == nullptr the atomics into dw32 remain.
+// A CTA of NT threads, V vectors of eight columns each, walks its rows with the next row's operands on their way (kept as
+// they are stored, 16 bytes a vector) and one barrier a row.  Bound by HBM: 4096 rows of 4096 columns 41.6 -> 31.3 us (the
+// bytes take 20.5), of 5120 91.8 -> 47.3, of 8192 120.5 -> 61.8 (41.0) against loads that begin after the row before.
+template <int NT, int V, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) rmsnorm_bwd_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
     const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
     const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw32,
     float* __restrict__ partials, int64_t rows, int cols) {
   chain();
-  __shared__ float red[32];
-  const int nvec = cols / 8;
-  float wv[MAXV][8], dwacc[MAXV][8];
+  __shared__ float red[2][NT / 32];
+  const int nvec = cols / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  BF8 wv[V], d[V], x[V], e[V];  // e: the residual path's gradient
+  float dwacc[V][8], rstd = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * RN_THREADS;
+  for (int i = 0; i < V; ++i) {
+    const int v = threadIdx.x + i * NT;
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-    if (v < nvec) unpack8(ld8(w + v * 8), wv[i]);
+    if (v < nvec) wv[i] = ld8(w + v * 8);
   }
-  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float rstd = rstd_in[row];
-    float g[MAXV][8], xh[MAXV][8];
-    BF8 eh[MAXV];  // the residual-path gradient, fetched with the other operands: one memory round trip per row
+  auto fetch = [&](int64_t row) {
+    rstd = rstd_in[row];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int v = threadIdx.x + i * NT;
+      if (v < nvec) {
+        d[i] = ld8(dy + row * cols + v * 8);
+        x[i] = ld8(h + row * cols + v * 8);
+        if (dh) e[i] = ld8(dh + row * cols + v * 8);
+      }
+    }
+  };
+  int64_t row = blockIdx.x;
+  if (row < rows) fetch(row);
+  for (int k = 0; row < rows; ++k) {
+    BF8 cd[V], cx[V], ce[V];
+    const float r = rstd;
+    const int64_t here = row;
     float dot = 0.f;
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = threadIdx.x + i * RN_THREADS;
-      if (v < nvec) {
-        float d[8];
-        unpack8(ld8(dy + row * cols + v * 8), d);
-        unpack8(ld8(h + row * cols + v * 8), xh[i]);
-        if (dh) eh[i] = ld8(dh + row * cols + v * 8);
+    for (int i = 0; i < V; ++i) {
+      cd[i] = d[i];
+      cx[i] = x[i];
+      ce[i] = e[i];
+    }
+    row += gridDim.x;
+    if (row < rows) fetch(row);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      if ((int)threadIdx.x + i * NT < nvec) {
+        float df[8], xh[8], wf[8];
+        unpack8(cd[i], df);
+        unpack8(cx[i], xh);
+        unpack8(wv[i], wf);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] *= rstd;
-          g[i][j] = d[j] * wv[i][j];
-          dot += g[i][j] * xh[i][j];
-          dwacc[i][j] += d[j] * xh[i][j];
+          xh[j] *= r;
+          dot += (df[j] * wf[j]) * xh[j];
+          dwacc[i][j] += df[j] * xh[j];
         }
       }
     }
-    dot = block_sum(dot, red) / (float)cols;
+    dot = warp_sum(dot);
+    if (lane == 0) red[k & 1][warp] = dot;
+    __syncthreads();  // the only one: a warp writes this half of `red` again after the next row's
+    dot = warp_sum(lane < NT / 32 ? red[k & 1][lane] : 0.f) / (float)cols;
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = threadIdx.x + i * RN_THREADS;
+    for (int i = 0; i < V; ++i) {
+      const int v = threadIdx.x + i * NT;
       if (v < nvec) {
-        float o[8];
+        float df[8], xh[8], wf[8], o[8];
+        unpack8(cd[i], df);
+        unpack8(cx[i], xh);
+        unpack8(wv[i], wf);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * dot);
+        for (int j = 0; j < 8; ++j) o[j] = r * (df[j] * wf[j] - xh[j] * r * dot);
         if (dh) {
-          float e[8];
-          unpack8(eh[i], e);
+          float ef[8];
+          unpack8(ce[i], ef);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += e[j];
+          for (int j = 0; j < 8; ++j) o[j] += ef[j];
         }
-        st8(dx + row * cols + v * 8, pack8(o));
+        st8(dx + here * cols + v * 8, pack8(o));
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * RN_THREADS;
+  for (int i = 0; i < V; ++i) {
+    const int v = threadIdx.x + i * NT;
     if (v < nvec) {
       if (partials) {
         float4* dst = reinterpret_cast<float4*>(partials + (int64_t)blockIdx.x * cols + v * 8);
@@ -760,7 +790,7 @@ int zc_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
   return zc::launch_status();
 }
 
-// CTAs the backward launches for `rows` rows: the number of rows `partials` must have
+// CTAs that the backward launches for `rows` rows at most: the number of rows `partials` must have
 int zc_rmsnorm_bwd_ctas(int64_t rows) { return (int)std::min<int64_t>(rows, (int64_t)zc::sm_count() * 4); }
 
 // dw32: [cols] fp32.  With partials ([zc_rmsnorm_bwd_ctas(rows), cols] fp32) it is overwritten with
@@ -769,15 +799,15 @@ int zc_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
                    float* dw32, float* partials, int64_t rows, int cols, cudaStream_t st) {
   if (cols % 8 || cols > zc::RN_MAX_COLS) return ERR_UNSUPPORTED;
   if (rows == 0) return 0;
-  const int grid = zc_rmsnorm_bwd_ctas(rows);
-  const int nvec = cols / 8;
-#define ZC_RN_BWD(V)                                                                                             \
-  zc::launch_chained(zc::rmsnorm_bwd_kernel<V>, grid, zc::RN_THREADS, 0, st, (const bf16*)dy, (const bf16*)h, (const bf16*)w,    \
-                                                             rstd, (const bf16*)dh, (bf16*)dx, dw32, partials,   \
-                                                             rows, cols)
-  if (nvec <= zc::RN_THREADS) ZC_RN_BWD(1);
-  else if (nvec <= 2 * zc::RN_THREADS) ZC_RN_BWD(2);
-  else ZC_RN_BWD(4);
+  // as many CTAs as run at once; narrow rows do not hold a thread's loads long enough for that to matter
+  int grid = 0;
+#define ZC_RN_BWD(NT, V, PER_SM)                                                                                       \
+  grid = (int)std::min<int64_t>(rows, (int64_t)zc::sm_count() * PER_SM);                                               \
+  zc::launch_chained(zc::rmsnorm_bwd_kernel<NT, V, PER_SM>, grid, NT, 0, st, (const bf16*)dy, (const bf16*)h,          \
+                     (const bf16*)w, rstd, (const bf16*)dh, (bf16*)dx, dw32, partials, rows, cols)
+  if (cols <= 128 * 8) { ZC_RN_BWD(128, 1, 4); }
+  else if (cols <= 256 * 2 * 8) { ZC_RN_BWD(256, 2, 2); }
+  else { ZC_RN_BWD(512, 2, 1); }
 #undef ZC_RN_BWD
   if (partials)
     zc::launch_chained(zc::rmsnorm_dw_reduce_kernel, (cols / 4 + 7) / 8, dim3(8, 128), 0, st, partials, grid, cols, dw32);
