@@ -66,124 +66,86 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// RMSNorm.  One CTA (256 threads) per row, row cached in registers (cols <= 8192, cols % 8 == 0).
+// RMSNorm (cols <= 8192, cols % 8 == 0).
 //   h = x (+ residual, rounded to bf16);  rstd = rsqrt(mean(h^2) + eps);  y = h * rstd * w
+// A CTA of NT threads, V vectors of eight columns each, walks its rows with the next row's operands on their way (kept as
+// they are stored) and one barrier a row.  Bound by HBM: with the residual 4096 rows of 4096 columns take 24.9 us (the bytes
+// 20.5; a warp a row 36.9, a CTA a row 29.8), of 5120 32.9 (25.6; 43.2), of 8192 46.7 (41.0; 62.8); 1024 rows of 1024 columns 4.4.
 // ---------------------------------------------------------------------------------------------
-constexpr int RN_THREADS = 256;
-constexpr int RN_MAX_COLS = RN_THREADS * 4 * 8;  // MAXV (vectors of 8 per thread) is 1, 2 or 4
+constexpr int RN_MAX_COLS = 8192;
 
-template <int MAXV>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
-    float* __restrict__ rstd_out, int cols, float eps) {
-  chain();
-  __shared__ float red[32];
-  const int64_t row = blockIdx.x;
-  const int nvec = cols / 8;
-  float h[MAXV][8];
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * RN_THREADS;
-    if (v < nvec) {
-      unpack8(ld8(x + row * cols + v * 8), h[i]);
-      if (res) {
-        float r[8];
-        unpack8(ld8(res + row * cols + v * 8), r);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) h[i][j] += r[j];
-        const BF8 hb = pack8(h[i]);
-        st8(h_out + row * cols + v * 8, hb);
-        unpack8(hb, h[i]);  // normalise the rounded sum, as the unfused op order would
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += h[i][j] * h[i][j];
-    }
-  }
-  ss = block_sum(ss, red);
-  const float rstd = rsqrtf(ss / (float)cols + eps);
-  if (threadIdx.x == 0) rstd_out[row] = rstd;
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = threadIdx.x + i * RN_THREADS;
-    if (v < nvec) {
-      float wv[8], o[8];
-      unpack8(ld8(w + v * 8), wv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = h[i][j] * rstd * wv[j];
-      st8(y + row * cols + v * 8, pack8(o));
-    }
-  }
-}
-
-// The same forward with one WARP per row (cols <= NV * 256): no block-wide synchronisation, all of a
-// row's loads issued before the first use, and the row kept packed (bf16) in registers between the
-// sum of squares and the scaling.  One row per CTA leaves the kernel waiting on two barriers per row
-// with a single load batch in flight (0.44 of the copy bandwidth); independent warps keep many rows'
-// loads in flight per SM.
-template <int NV>
-__global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
+template <int NT, int V, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
     const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
   chain();
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int nvec = cols / 8;
-  const __nv_bfloat16* xr = x + row * cols;
-  BF8 hv[NV];
+  __shared__ float red[2][NT / 32];
+  const int nvec = cols / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  BF8 wv[V], a[V], b[V];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int v = lane + 32 * i;
-    if (v < nvec) hv[i] = ld8(xr + v * 8);
+  for (int i = 0; i < V; ++i) {
+    const int v = threadIdx.x + i * NT;
+    if (v < nvec) wv[i] = ld8(w + v * 8);
   }
-  if (res) {
-    const __nv_bfloat16* rr = res + row * cols;
-    BF8 rv[NV];
+  auto fetch = [&](int64_t row) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = lane + 32 * i;
-      if (v < nvec) rv[i] = ld8(rr + v * 8);
-    }
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = lane + 32 * i;
+    for (int i = 0; i < V; ++i) {
+      const int v = threadIdx.x + i * NT;
       if (v < nvec) {
-        float a[8], b[8];
-        unpack8(hv[i], a);
-        unpack8(rv[i], b);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] += b[j];
-        hv[i] = pack8(a);  // the rounded sum is what gets normalised, as the unfused op order would
-        st8(h_out + row * cols + v * 8, hv[i]);
+        a[i] = ld8(x + row * cols + v * 8);
+        if (res) b[i] = ld8(res + row * cols + v * 8);
       }
     }
-  }
-  float ss = 0.f;
+  };
+  int64_t row = blockIdx.x;
+  if (row < rows) fetch(row);
+  for (int k = 0; row < rows; ++k) {
+    const int64_t here = row;
+    BF8 hv[V];
+    float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    if (lane + 32 * i < nvec) {
-      float a[8];
-      unpack8(hv[i], a);
+    for (int i = 0; i < V; ++i) {
+      hv[i] = a[i];
+      if (res) {
+        float f[8], r[8];
+        unpack8(a[i], f);
+        unpack8(b[i], r);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss += a[j] * a[j];
+        for (int j = 0; j < 8; ++j) f[j] += r[j];
+        hv[i] = pack8(f);  // the rounded sum is what gets normalised, as the unfused op order would
+      }
     }
-  }
-  ss = warp_sum(ss);
-  const float rstd = rsqrtf(ss / (float)cols + eps);
-  if (lane == 0) rstd_out[row] = rstd;
+    row += gridDim.x;
+    if (row < rows) fetch(row);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int v = lane + 32 * i;
-    if (v < nvec) {
-      float a[8], wv[8], o[8];
-      unpack8(hv[i], a);
-      unpack8(ld8(w + v * 8), wv);
+    for (int i = 0; i < V; ++i) {
+      const int v = threadIdx.x + i * NT;
+      if (v < nvec) {
+        if (res) st8(h_out + here * cols + v * 8, hv[i]);
+        float f[8];
+        unpack8(hv[i], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = a[j] * rstd * wv[j];
-      st8(y + row * cols + v * 8, pack8(o));
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) red[k & 1][warp] = ss;
+    __syncthreads();  // the only one: a warp writes this half of `red` again after the next row's
+    ss = warp_sum(lane < NT / 32 ? red[k & 1][lane] : 0.f);
+    const float rstd = rsqrtf(ss / (float)cols + eps);
+    if (threadIdx.x == 0) rstd_out[here] = rstd;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int v = threadIdx.x + i * NT;
+      if (v < nvec) {
+        float f[8], wf[8];
+        unpack8(hv[i], f);
+        unpack8(wv[i], wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * wf[j];
+        st8(y + here * cols + v * 8, pack8(f));
+      }
     }
   }
 }
@@ -767,25 +729,13 @@ int zc_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
                    int cols, float eps, cudaStream_t st) {
   if (cols % 8 || cols > zc::RN_MAX_COLS) return ERR_UNSUPPORTED;
   if (rows == 0) return 0;
-  const int nvec = cols / 8;
-  if (nvec <= 32 * 20) {  // one warp per row (wider rows do not fit a warp's registers)
-    const unsigned grid = (unsigned)((rows + 3) / 4);
-#define ZC_RN_FWDW(V)                                                                                             \
-  zc::launch_chained(zc::rmsnorm_fwd_warp_kernel<V>, grid, 128, 0, st, (const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, \
-                                                       (bf16*)h_out, rstd, rows, cols, eps)
-    if (nvec <= 32 * 4) ZC_RN_FWDW(4);
-    else if (nvec <= 32 * 16) ZC_RN_FWDW(16);
-    else ZC_RN_FWDW(20);
-#undef ZC_RN_FWDW
-    return zc::launch_status();
-  }
-#define ZC_RN_FWD(V)                                                                                              \
-  zc::launch_chained(zc::rmsnorm_fwd_kernel<V>, (unsigned)rows, zc::RN_THREADS, 0, st, (const bf16*)x, (const bf16*)res,          \
-                                                                       (const bf16*)w, (bf16*)y, (bf16*)h_out,    \
-                                                                       rstd, cols, eps)
-  if (nvec <= zc::RN_THREADS) ZC_RN_FWD(1);
-  else if (nvec <= 2 * zc::RN_THREADS) ZC_RN_FWD(2);
-  else ZC_RN_FWD(4);
+#define ZC_RN_FWD(NT, V, PER_SM)                                                                                       \
+  zc::launch_chained(zc::rmsnorm_fwd_kernel<NT, V, PER_SM>,                                                            \
+                     (unsigned)std::min<int64_t>(rows, (int64_t)zc::sm_count() * PER_SM), NT, 0, st, (const bf16*)x,   \
+                     (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)h_out, rstd, rows, cols, eps)
+  if (cols <= 128 * 8) ZC_RN_FWD(128, 1, 8);
+  else if (cols <= 256 * 2 * 8) ZC_RN_FWD(256, 2, 3);
+  else ZC_RN_FWD(512, 2, 2);
 #undef ZC_RN_FWD
   return zc::launch_status();
 }

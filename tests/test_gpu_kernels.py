@@ -331,6 +331,45 @@ def test_rmsnorm_fwd_bwd():
         assert torch.allclose(y2.float(), F.rms_norm(x.detach().float(), (cols,), w.detach().float(), 1e-5), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 8), (700, 1024), (1300, 1024), (5, 1032), (461, 4096), (3, 4104), (301, 8192)])
+def test_rmsnorm_walks_rows_of_every_width(rows, cols):
+    """The widths at which the CTA changes, one vector more, and more rows than CTAs run at once.  Every result is rounded once
+    from fp32 to eight bits: 2^-8 of a value at most (2^-8.6 of a norm of many), and the fp32 sums' 1e-5."""
+    torch.manual_seed(rows + cols)
+    x, r, g = (torch.randn(rows, cols, device=DEV).bfloat16() for _ in range(3))
+    gh = torch.randn(rows, cols, device=DEV).bfloat16()
+    w = (1 + 0.1 * torch.randn(cols, device=DEV)).bfloat16().requires_grad_()
+    x.requires_grad_()
+    y, h = norm.add_rms_norm(x, r, w, 1e-5)
+    dx, dw = torch.autograd.grad([y, h], [x, w], [g, gh])
+    assert torch.equal(h, (x.detach().float() + r.float()).bfloat16())
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    yd = hd * (hd.pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt() * wd
+    dhd, dwd = torch.autograd.grad(yd, [hd, wd], g.double())
+    for got, want in [(y, yd), (dx, dhd + gh.double()), (dw, dwd)]:
+        assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
+
+
+@pytest.mark.parametrize("n", [8, 2048, 2056, 4096, 4104, 100_000])
+def test_adamw_updates_every_vector_once(n):
+    """Around a thread's second vector and a CTA's 512; elements are independent, so each size has the bits of the largest.
+    Rounded once to eight bits: 2^-8 of a value at most."""
+    torch.manual_seed(3)
+    whole = [(torch.randn(100_000, device=DEV) * s).bfloat16() for s in (1.0, 0.1, 0.01)] + [torch.rand(100_000, device=DEV).bfloat16()]
+    run = lambda t: _lib.check(_lib.cuda().zc_adamw(*(v.data_ptr() for v in t), t[0].numel(), 0, 0, 0, 1e-3, 0.9, 0.95, 1e-8, 0.01, 0.1,
+                                                    0.05, 0, _lib.stream_ptr(t[0].device)), "zc_adamw")
+    part = [v[:n].clone() for v in whole]
+    p, g, m, v = (t.double() for t in part)
+    run(part)
+    run(whole)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b[:n]) for a, b in zip(part, whole))
+    m, v = 0.9 * m + 0.1 * g, 0.95 * v + 0.05 * g * g
+    p = p * (1 - 1e-3 * 0.01) - 1e-3 / 0.1 * m / (v.sqrt() / 0.05 ** 0.5 + 1e-8)
+    for got, want in zip((part[0], part[2], part[3]), (p, m, v)):
+        assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
+
+
 def test_swiglu_fwd_bwd():
     torch.manual_seed(1)
     gu = torch.randn(257, 2 * 1024, device=DEV).bfloat16().requires_grad_()
