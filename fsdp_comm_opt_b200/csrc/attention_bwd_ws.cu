@@ -823,30 +823,24 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         }
       }
     } else {
+      // half of the warps dK, half dV; K, V, Q and dO are done with
       tc_fence_after_sync();
-      const int key = k0 + r;
+      const uint32_t tmx = tm + (half ? C::TM_DV : C::TM_DK);
+      const int key = k0 + quarter * 32;
+      const int64_t stride = half ? p.dvs1 : p.dks1;
+      __nv_bfloat16* dst = half ? p.dv + b * p.dvs0 + hk * p.dvs2 : p.dk + b * p.dks0 + hk * p.dks2;
 #pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        const uint32_t tmx = tm + (which ? C::TM_DV : C::TM_DK);
-        __nv_bfloat16* dst = which ? p.dv + b * p.dvs0 + (int64_t)key * p.dvs1 + hk * p.dvs2
-                                   : p.dk + b * p.dks0 + (int64_t)key * p.dks1 + hk * p.dks2;
-#pragma unroll 1
-        for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 32) {
-          uint32_t rr[32];
-          tmem_ld32(tmem_addr(tmx, lane_base, c), rr);
-          tmem_ld_wait();
-          if (key < p.S) {
+      for (int c = 0; c < D; c += 64) {
+        uint32_t pk[32];
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 u;
-              u.x = pack_bf16(__uint_as_float(rr[i]), __uint_as_float(rr[i + 1]));
-              u.y = pack_bf16(__uint_as_float(rr[i + 2]), __uint_as_float(rr[i + 3]));
-              u.z = pack_bf16(__uint_as_float(rr[i + 4]), __uint_as_float(rr[i + 5]));
-              u.w = pack_bf16(__uint_as_float(rr[i + 6]), __uint_as_float(rr[i + 7]));
-              *reinterpret_cast<uint4*>(dst + c + i) = u;
-            }
-          }
+        for (int k = 0; k < 64; k += 32) {
+          uint32_t rr[32];
+          tmem_ld32(tmem_addr(tmx, lane_base, c + k), rr);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 16; ++q) pk[k / 2 + q] = pack_bf16(__uint_as_float(rr[2 * q]), __uint_as_float(rr[2 * q + 1]));
         }
+        store_rows64(smem + (warp - 4) * 4096, pk, dst + key * stride + c, stride, p.S - key);
       }
     }
   } else {
@@ -896,10 +890,12 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
     __syncwarp();
     cluster_sync();
     if (warp >= 4 && warp < 12) {
-      // Each CTA of the cluster adds up its share of the columns, in the order of the parts, eight of a row a thread.
-      const int groups = 2 * (D / 8) / parts;
-      for (int u = tid - 128; u < groups * 128; u += 256) {
-        const int g = part * groups + (u >> 7), row = u & 127, key = k0 + row;  // g: dK's groups of eight columns, then dV's
+      // Each CTA of the cluster adds up its share of the columns, in the order of the parts, eight of a row a thread; a warp
+      // has up to four such groups next to each other, of eight rows or more.
+      const int groups = 2 * (D / 8) / parts, wide = min(groups, 4), high = 32 / wide;
+      for (int w = warp - 4; w < groups / wide * (128 / high); w += 8) {
+        const int row = (w % (128 / high)) * high + lane % high, key = k0 + row;
+        const int g = part * groups + w / (128 / high) * wide + lane / high;  // dK's groups of eight columns, then dV's
         const uint32_t at = smem_u32(smem) + (uint32_t)(2 * g * 128 + row) * 16;
         float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2

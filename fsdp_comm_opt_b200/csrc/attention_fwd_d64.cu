@@ -237,24 +237,19 @@ __global__ void __launch_bounds__(THREADS, 2) attn_fwd_d64_kernel(const __grid_c
     } else {
       tc_fence_after_sync();
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* dst = p.o + ((int64_t)(b * p.S + row) * p.Hq + h) * D;
-#pragma unroll 1
+      uint32_t pk[32];
+#pragma unroll
       for (int c = 0; c < D; c += 32) {
         uint32_t rr[32];
         tmem_ld32(tmem_addr(tm_o, lane_base, c), rr);
         tmem_ld_wait();
-        if (row < p.S) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 u;
-            u.x = pack_bf16(__uint_as_float(rr[i]) * inv, __uint_as_float(rr[i + 1]) * inv);
-            u.y = pack_bf16(__uint_as_float(rr[i + 2]) * inv, __uint_as_float(rr[i + 3]) * inv);
-            u.z = pack_bf16(__uint_as_float(rr[i + 4]) * inv, __uint_as_float(rr[i + 5]) * inv);
-            u.w = pack_bf16(__uint_as_float(rr[i + 6]) * inv, __uint_as_float(rr[i + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c + i) = u;
-          }
-        }
+        for (int i = 0; i < 16; ++i)
+          pk[c / 2 + i] = pack_bf16(__uint_as_float(rr[2 * i]) * inv, __uint_as_float(rr[2 * i + 1]) * inv);
       }
+      // Q's place: the MMAs that read it have completed
+      store_rows64(sQ + (warp & 3) * 4096, pk, p.o + ((int64_t)(b * p.S + row - lane) * p.Hq + h) * D, (int64_t)p.Hq * D,
+                   p.S - (row - lane));
       if (row < p.S) p.lse[((int64_t)b * p.Hq + h) * p.S + row] = (l > 0.f) ? (m_ref + log2f(l)) * LN2 : -CUDART_INF_F;
     }
   }

@@ -73,4 +73,24 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
   return r != 0;
 }
 
+// 64 columns of a warp's 32 rows, a row a lane (bf16 pairs), through `buf` (4 KB of shared memory of the warp's) to global
+// memory: whole 128-byte lines, four rows an instruction.  `dst` is row 0's first column, rows lie `stride` elements apart;
+// the first `rows` of them are stored.  (16 bytes of 32 rows an instruction, as the lanes hold them, take 60 clocks each.)
+__device__ __forceinline__ void store_rows64(uint8_t* buf, const uint32_t (&pk)[32], __nv_bfloat16* dst, int64_t stride, int rows) {
+  const int lane = threadIdx.x & 31, row = lane >> 3, chunk = lane & 7;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<uint4*>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+        make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+  __syncwarp();
+  uint4 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = *reinterpret_cast<const uint4*>(buf + (4 * q + row) * 128 + ((chunk ^ ((4 * q + row) & 7)) << 4));
+  __syncwarp();
+  dst += row * stride + chunk * 8;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (4 * q + row < rows) *reinterpret_cast<uint4*>(dst + (int64_t)(4 * q) * stride) = v[q];
+}
+
 }  // namespace zc
