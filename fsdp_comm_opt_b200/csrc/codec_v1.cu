@@ -465,19 +465,25 @@ __global__ void __launch_bounds__(MOMENT_THREADS) v1_base_kernel(const uint16_t*
   const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const long long nv = vec ? n / 8 : 0;
   const uint4* xv = reinterpret_cast<const uint4*>(x);
-  long long i = t;
-  for (; i + 3 * nt < nv; i += 4 * nt) {
-    uint4 v[4];
+  // The next trip's loads are in flight while this one's values are added, the last trip's together like the others'
+  // (an encode of 27 264 000 elements with its statistic: 53.5 -> 51.5 us).
+  uint4 v[4];
+  auto fetch = [&](long long i) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __ldg(xv + i + k * nt);
+    for (int k = 0; k < 4; ++k)
+      if (i + k * nt < nv) v[k] = __ldg(xv + i + k * nt);
+  };
+  fetch(t);
+  for (long long i = t; i < nv; i += 4 * nt) {
+    uint4 c[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { add2(v[k].x); add2(v[k].y); add2(v[k].z); add2(v[k].w); }
+    for (int k = 0; k < 4; ++k) c[k] = v[k];
+    fetch(i + 4 * nt);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * nt < nv) { add2(c[k].x); add2(c[k].y); add2(c[k].z); add2(c[k].w); }
   }
-  for (; i < nv; i += nt) {
-    const uint4 v = __ldg(xv + i);
-    add2(v.x); add2(v.y); add2(v.z); add2(v.w);
-  }
-  for (i = nv * 8 + t; i < n; i += nt) add2((uint32_t)__ldg(x + i));
+  for (long long i = nv * 8 + t; i < n; i += nt) add2((uint32_t)__ldg(x + i));
   __shared__ bool last;
   double2 t2 = block_sum2(s, q);
   if (threadIdx.x == 0) {
