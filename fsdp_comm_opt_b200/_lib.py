@@ -78,24 +78,22 @@ _LAUNCHES = 0
 
 
 class _CountingLib:
-    """Proxy over the CDLL that counts kernel launches made through the C launchers."""
+    """Proxy over the CDLL that counts kernel launches made through the C launchers.  A launcher becomes an attribute when it
+    is first asked for, so that later calls find it without coming here."""
 
     def __init__(self, lib):
         self._lib = lib
-        self._cache = {}
 
     def __getattr__(self, name):
-        fn = self._cache.get(name)
-        if fn is None:
-            raw = getattr(self._lib, name)
-            n = _KERNELS_PER_CALL.get(name, 1)
+        raw = getattr(self._lib, name)
+        n = _KERNELS_PER_CALL.get(name, 1)
 
-            def fn(*args, _raw=raw, _n=n):
-                global _LAUNCHES
-                _LAUNCHES += _n
-                return _raw(*args)
+        def fn(*args, _raw=raw, _n=n):
+            global _LAUNCHES
+            _LAUNCHES += _n
+            return _raw(*args)
 
-            self._cache[name] = fn
+        setattr(self, name, fn)
         return fn
 
 

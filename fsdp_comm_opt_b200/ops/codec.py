@@ -43,6 +43,9 @@ def v1_det_bytes(padded_numel: int) -> int:
 # --------------------------------------------------------------------------------------------
 
 def _req(t: torch.Tensor, dtype, name: str, numel_min: int = 0) -> torch.Tensor:
+    # what a small call passes three times, in as few steps as there are conditions
+    if type(t) is torch.Tensor and t.dtype is dtype and t.is_contiguous() and t.numel() >= numel_min:
+        return t
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a tensor")
     if t.dtype != dtype:
@@ -366,7 +369,7 @@ def v2_encode(x: torch.Tensor, records: torch.Tensor | None = None,
     _req(headers, torch.int32, "headers", nc)
     if nc == 0:
         return records, headers
-    if dev.type == "cpu":
+    if x.is_cpu:
         fn = _lib.cpu().zc_cpu_v2_encode_nibble if nibble else _lib.cpu().zc_cpu_v2_encode
         fn(x.data_ptr(), n, records.data_ptr(), headers.data_ptr())
     else:
@@ -386,7 +389,7 @@ def v2_decode(records: torch.Tensor, headers: torch.Tensor, numel: int,
     _req(out, torch.bfloat16, "out", numel)
     if nc == 0:
         return out
-    if dev.type == "cpu":
+    if records.is_cpu:
         fn = _lib.cpu().zc_cpu_v2_decode_nibble if nibble else _lib.cpu().zc_cpu_v2_decode
         fn(records.data_ptr(), headers.data_ptr(), numel, out.data_ptr())
     else:
