@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(256) dq_convert8_kernel(const float4* __restri
 // What bounds it: the issue of the MMAs, which take 70 to 110 clocks each whatever their width (an operand's bytes
 // move at about 70 B per clock from shared memory), 40 of them an iteration at head dimension 128 and 32 at 64.  With 64
 // queries an iteration and P^T in shared memory it was 64 for the same work.  16384 keys, 32 / 8 heads of 128: 7200 ->
-// 4884 us; 8 x 1024 keys, 25 heads of 64: 259 -> 180.
+// 4884 us; 8 x 1024 keys, 25 heads of 64: 259 -> 180, and 175 -> 168 since dK and dV are stored in whole lines.
 // CTAs are numbered heaviest first (key block 0 has the most query blocks below the diagonal).
 namespace bkt {
 using namespace bws;
