@@ -75,8 +75,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// The pair's barrier in two halves.  Relaxed: what the other CTA has to see of this one's memory is only the initialised
-// mbarriers, which fence.mbarrier_init publishes (with release the two barriers of a launch took 2400 clocks, so 400).
+// The pair's barrier in two halves.  Relaxed (with release the two barriers of a launch took 2400 clocks, so 400): at the start
+// the other CTA has to see the initialised mbarriers, which fence.mbarrier_init publishes, and to come after the allocation
+// of tensor memory, which has returned when its warp arrives.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of the cluster
@@ -273,14 +274,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     if (lane == 0) s_abort = 0;
     __syncwarp();
   }
-  cluster_arrive();
   if (warp == 1) {
-    // each CTA allocates its own SM's whole TMEM (512 columns, so the base is column 0 in both)
+    // each CTA allocates its own SM's whole TMEM (512 columns, so the base is column 0 in both), and arrives at the pair's
+    // barrier behind that: the even CTA's MMAs write the odd one's tensor memory
     tmem_alloc(&sh.tmem_base, 2 * BN);
     tmem_relinquish();
+    tc_fence_before_sync();
   } else if (warp == 2 && lane < 2) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(lane ? &mapB : &mapA) : "memory");
   }
+  __syncwarp();
+  cluster_arrive();
   // edge tiles: rows / columns / K blocks past the matrix read as zeros (TMA fill) and are not stored
   const int units = p.full_tiles + (p.m_tiles * p.n_tiles - p.full_tiles) * p.split;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
@@ -290,7 +294,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     asm volatile("bar.sync 1, 160;" ::: "memory");
     tc_fence_after_sync();
   }
-  cluster_wait();  // both CTAs' barriers are initialised before any remote arrival
+  cluster_wait();  // both CTAs have their barriers, before any remote arrival, and their tensor memory
+  tc_fence_after_sync();
   chain_wait();
   if (warp == 1) chain_next();  // which has its TMEM
   const uint32_t tm = sh.tmem_base;

@@ -985,6 +985,31 @@ def test_products_split_along_k_on_two_streams_have_partial_sums_of_their_own():
             assert all(torch.equal(ref, y) for y in out)
 
 
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (1000, 3000, 200), (4096, 6144, 256)])
+def test_products_beside_kernels_that_hold_tensor_memory_keep_their_bits(M, N, K):
+    """Products of single SMs, of 48 pairs and of all, while other streams' attention and products take and free tensor memory."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(M)
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    qkv = torch.randn(2, 700, 12, 64, device=DEV).bfloat16()
+    ref = x.double() @ w.double().t()
+    alone = gemm.gemm(x, w, False, True)
+    other = attention.causal_attention(qkv, 8, 2)
+    torch.cuda.synchronize()
+    assert ((alone.double() - ref).norm() / ref.norm()).item() < 2 ** -9 + 1e-5
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    got = [[], [], []]
+    for _ in range(30):
+        for st, out in zip(streams, got):
+            with torch.cuda.stream(st):
+                out.append(attention.causal_attention(qkv, 8, 2) if st is streams[0] else gemm.gemm(x, w, False, True))
+    torch.cuda.synchronize()
+    assert _lib.cuda().zc_gemm_status_read_and_clear() == 0 and attention.status_read_and_clear() == 0
+    assert all(torch.equal(other, o) for o in got[0])
+    assert all(torch.equal(alone, y) for out in got[1:] for y in out)
+
+
 def _first_products_worker(rank, world):
     from fsdp_comm_opt_b200.ops import gemm
 
