@@ -77,8 +77,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 }
 // The pair's barrier in two halves.  Relaxed (with release the two barriers of a launch took 2400 clocks, so 400): at the start
 // the other CTA has to see the initialised mbarriers, which fence.mbarrier_init publishes, and to come after the allocation
-// of tensor memory, which has returned when its warp arrives.
+// of tensor memory, which has returned when its warp arrives; at the end every arrival at a CTA's mbarriers has been waited
+// for there.  With release where a wait was given up, and arrivals may be on their way.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
@@ -323,8 +325,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
       const uint32_t full0 = map_to_cta(full_base, 0);  // the even CTA's full[0]; full[s] is 8 s bytes on
       const uint32_t sfull_c1 = map_to_cta(sfull_base, 1);
       const uint32_t su_c1 = map_to_cta(smem_u32(sh.sched_u), 1);
-      uint32_t s = 0, ph = 0;
-      for (uint32_t i = 0; ok; ++i) {
+      uint32_t s = 0, ph = 0, i = 0;
+      for (; ok; ++i) {
         int u;
         if (rank == 0 && from_ring(i)) {
           // fetch the i-th unit and publish it to both CTAs
@@ -365,6 +367,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
+      // What the other CTA still sends to this one's barriers: the releases of the last slots, i of which have been published
+      // (here on the even CTA), and the commits of the last stages.
+      if (rank == 0 && p.counter)
+        for (uint32_t k = i > SCHED ? i - SCHED : 0; ok && k < i; ++k)
+          ok = wait_bar_cluster(smem_u32(&sched_empty[k & (SCHED - 1)]), (k / SCHED) & 1, &s_abort);
+      for (int k = 0; ok && k < STAGES; ++k) {
+        ok = wait_bar(empty_base + 8 * s, ph ^ 1, &s_abort);
+        if (++s == STAGES) { s = 0; ph ^= 1; }
+      }
       if (!ok) s_abort = 1;
     }
   } else if (warp == 1) {
@@ -381,8 +392,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
       const uint32_t empty_c0 = map_to_cta(empty_base, 0), empty_c1 = map_to_cta(empty_base, 1);
       const uint32_t accf_c0 = map_to_cta(smem_u32(&acc_full[0]), 0), accf_c1 = map_to_cta(smem_u32(&acc_full[0]), 1);
       const uint32_t acce = smem_u32(&acc_empty[0]);
-      uint32_t s = 0, ph = 0;
-      for (uint32_t unit_it = 0; ok; ++unit_it) {
+      uint32_t s = 0, ph = 0, unit_it = 0;
+      for (; ok; ++unit_it) {
         const int u = next_unit(unit_it, ok);
         if (!ok) break;
         release_unit(unit_it);
@@ -411,6 +422,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
           mma_commit_pair(accf_c1 + 8 * acc);
         }
       }
+      // both CTAs' epilogue warps have let go of the last accumulators
+      for (uint32_t k = unit_it > 2 ? unit_it - 2 : 0; ok && k < unit_it; ++k)
+        ok = wait_bar_cluster(acce + 8 * (k & 1), (k >> 1) & 1, &s_abort);
       if (!ok) s_abort = 1;
     }
   } else {
@@ -529,8 +543,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
   tc_fence_before_sync();
   __syncthreads();
   if (tid == 0 && s_abort) atomicExch(p.status, 8);
-  // neither CTA may leave (or free its TMEM) while the pair's MMAs can still touch its memory
-  cluster_arrive();
+  // Neither CTA may leave (or free its TMEM) while the pair's MMAs or the other CTA's arrivals can still touch its memory.  Both
+  // have come by now (the producers and the MMA issuer have waited for the last of them) unless a wait was given up.
+  __syncwarp();
+  if (s_abort) cluster_arrive_release();
+  else cluster_arrive();
   cluster_wait();
   if (warp == 1) tmem_dealloc(tm, 2 * BN);
   if (tid == 0 && rank == 0 && p.counter) {

@@ -1010,6 +1010,35 @@ def test_products_beside_kernels_that_hold_tensor_memory_keep_their_bits(M, N, K
     assert all(torch.equal(alone, y) for out in got[1:] for y in out)
 
 
+@pytest.mark.parametrize("M,N,K", [(1000, 3000, 64), (4096, 5120, 64), (2048, 1600, 4800), (128, 128, 16384), (8192, 8192, 64)])
+def test_products_that_end_on_an_arrival_of_the_other_cta_repeat(M, N, K):
+    """Pairs of one tile and of many (with the ring of tile numbers and without: a recorded launch), whole tiles, old values and
+    slices of K, whose last arrivals at the even CTA are followed by its end; hundreds of launches have no time in between."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(K)
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    c = torch.randn(M, N, device=DEV).bfloat16()
+    run = lambda out, acc: gemm.gemm(x, w, False, True, out=out, accumulate=acc)
+    ref = [run(torch.empty_like(c), False), run(c.clone(), True)]
+    out = [torch.empty_like(c), c.clone()]
+    for _ in range(100):
+        run(out[0], False)
+        run(out[1].copy_(c), True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        recorded = [run(torch.empty_like(c), False), run(c.clone(), True)]
+    for _ in range(20):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert _lib.cuda().zc_gemm_status_read_and_clear() == 0
+    want = x.double() @ w.double().t()
+    for got, whole in zip(ref, (want, want + c.double())):
+        assert ((got.double() - whole).norm() / whole.norm()).item() < 2 ** -9 + 1e-5
+    for got in (out, recorded):
+        assert all(torch.equal(a, b) for a, b in zip(ref, got))
+
+
 def _first_products_worker(rank, world):
     from fsdp_comm_opt_b200.ops import gemm
 
