@@ -254,11 +254,12 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc_fence_before_sync();
   if (PARTS > 1 && warp < 2) cluster_wait();
   __syncthreads();
+  if (tid == 0 && s_abort) atomicExch(p.status, 10);
   if (warp == 1) tmem_dealloc(tm, BN);
   if (PARTS > 1) {
     if (warp >= 2) {
       const bool ok = mbar_wait(&sh.received, 0);
-      if (!__all_sync(0xffffffffu, ok)) s_abort = 1;
+      if (!__all_sync(0xffffffffu, ok) && lane == 0) atomicExch(p.status, 10);  // the flag's reader does not wait for this warp
       // a warp has 32 columns, eight rows a round: 128 bytes in a row of every load, 64 of every store
       const int c8 = (warp - 2) * 4 + (lane >> 3), cols_left = (int)min((int64_t)BN, p.N - n0);
       const int64_t row0 = m0 + part * ROWS + (lane & 7);
@@ -289,7 +290,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     cluster_arrive();
     cluster_wait();  // the others have what this CTA sent them
   }
-  if (tid == 0 && s_abort) atomicExch(p.status, 10);
 }
 
 template <int A_MAJOR, int B_MAJOR, int PARTS>

@@ -291,9 +291,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
   const int units = p.full_tiles + (p.m_tiles * p.n_tiles - p.full_tiles) * p.split;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
   const Unit first = unit_of(cluster_id, p);
-  if (warp != 0) {  // the producer has no use for the accumulators' address
+  // This CTA's abort flag is clear and its accumulators' address known.  The producer, which cleared the one and has no use for
+  // the other, does not wait here.
+  if (warp == 0) {
+    asm volatile("bar.arrive 1, 192;" ::: "memory");
+  } else {
     tc_fence_before_sync();
-    asm volatile("bar.sync 1, 160;" ::: "memory");
+    asm volatile("bar.sync 1, 192;" ::: "memory");
     tc_fence_after_sync();
   }
   cluster_wait();  // both CTAs have their barriers, before any remote arrival, and their tensor memory

@@ -1039,6 +1039,24 @@ def test_products_that_end_on_an_arrival_of_the_other_cta_repeat(M, N, K):
         assert all(torch.equal(a, b) for a, b in zip(ref, got))
 
 
+def test_products_behind_kernels_that_fill_shared_memory_report_no_failure():
+    """Attention's backward leaves gradients and probabilities all over shared memory, where the products keep their abort flags: a
+    flag that is read before it is cleared would end a wait and be reported."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    torch.manual_seed(2)
+    qkv = torch.randn(1, 2048, 24, 128, device=DEV).bfloat16().requires_grad_()
+    o = attention.causal_attention(qkv, 16, 4)
+    cases = [(torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV).bfloat16())
+             for m, n, k in ((4096, 5120, 64), (512, 256, 1024), (256, 512, 256))]
+    ref = [gemm.gemm(x, w, False, True) for x, w in cases]
+    for _ in range(20):
+        torch.autograd.grad(o, qkv, torch.ones_like(o), retain_graph=True)
+        got = [gemm.gemm(x, w, False, True) for x, w in cases]
+        assert _lib.cuda().zc_gemm_status_read_and_clear() == 0
+        assert all(torch.equal(a, b) for a, b in zip(ref, got))
+
+
 def _first_products_worker(rank, world):
     from fsdp_comm_opt_b200.ops import gemm
 
