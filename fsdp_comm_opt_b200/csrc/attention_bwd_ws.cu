@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
 // bytes of each input and 32 of the accumulator a thread.  Bound by HBM; 4096 x 32 x 128: 20.5 us, with a warp a
 // (row, head), four-byte loads and a memset 28.5 + 12.2.
 template <int D>
-__global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
+__global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* o, const uint4* dout,
                                                          float* __restrict__ delta, float4* __restrict__ dq_acc, int S,
                                                          int Hq, int64_t total) {
   chain();
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   float acc = 0.f;
   if (i < total * T) {
-    const uint4 a = __ldg(o + i), g = __ldg(dout + i);
+    const uint4 a = o[i], g = dout[i];
     dq_acc[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
     dq_acc[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
@@ -422,12 +422,12 @@ __global__ void __launch_bounds__(256) delta_zero_kernel(const uint4* __restrict
 // acc [rows, Hq, D] fp32 -> dq bf16 (16-byte aligned, element strides multiples of 8): eight elements a thread.
 // Bound by HBM; 4096 x 32 x 128: 24 us with four elements and 64-bit divisions a thread, 13 so.
 template <int D>
-__global__ void __launch_bounds__(256) dq_convert8_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+__global__ void __launch_bounds__(256) dq_convert8_kernel(const float4* acc, __nv_bfloat16* __restrict__ dq,
                                                           int64_t units, uint32_t Hq, int64_t s_bs, int64_t s_h) {
   chain();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= units) return;
-  const float4 a = __ldcs(acc + 2 * i), c = __ldcs(acc + 2 * i + 1);
+  const float4 a = ld_once(acc + 2 * i), c = ld_once(acc + 2 * i + 1);
   const uint32_t rh = (uint32_t)(i / (D / 8)), r = rh / Hq, h = rh - r * Hq;
   uint4 v;
   __nv_bfloat162 p0 = __floats2bfloat162_rn(a.x, a.y), p1 = __floats2bfloat162_rn(a.z, a.w);
@@ -705,8 +705,8 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
         for (int k = 0; k < 4; ++k) {
           // queries past the end: P = exp2(0 - inf) = 0
           const int q = ib * 128 + lane * 4 + k;
-          vl[k] = q < p.S ? -__ldg(p.lse + row + q) * LOG2E : -CUDART_INF_F;
-          vd[k] = q < p.S ? -__ldg(p.delta + row + q) * p.scale : 0.f;
+          vl[k] = q < p.S ? -p.lse[row + q] * LOG2E : -CUDART_INF_F;
+          vd[k] = q < p.S ? -p.delta[row + q] * p.scale : 0.f;
         }
         const bool ok = role_wait(&m.stat_empty[st], ((i >> 1) & 1) ^ 1);
         if (!__all_sync(0xffffffffu, ok)) { *s_abort = 1; break; }

@@ -76,8 +76,8 @@ constexpr int RN_MAX_COLS = 8192;
 
 template <int NT, int V, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
+    const __nv_bfloat16* x, const __nv_bfloat16* res,
+    const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
   chain();
   __shared__ float red[2][NT / 32];
@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
 // bytes take 20.5), of 5120 91.8 -> 47.3, of 8192 120.5 -> 61.8 (41.0) against loads that begin after the row before.
 template <int NT, int V, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_bwd_kernel(
-    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
-    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
-    const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw32,
+    const __nv_bfloat16* dy, const __nv_bfloat16* h,
+    const __nv_bfloat16* w, const float* rstd_in,
+    const __nv_bfloat16* dh, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw32,
     float* __restrict__ partials, int64_t rows, int cols) {
   chain();
   __shared__ float red[2][NT / 32];
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_bwd_kernel(
 
 // dw[c] = sum over the CTAs' partial rows; block (8, 128): 8 float4 columns (128 bytes of a row) x 128 row groups.  A
 // latency: 1024 columns are 32 blocks of a few loads each (3.0 us; 8 blocks of 32 x 32 threads took 5.1).
-__global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __restrict__ partials, int nblocks,
+__global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* partials, int nblocks,
                                                                 int cols, float* __restrict__ dw) {
   chain();
   __shared__ float4 acc[8][33];
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __
   if (c4 * 4 < cols) {
 #pragma unroll 4
     for (int r = threadIdx.y; r < nblocks; r += 128) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(partials + (int64_t)r * cols) + c4);
+      const float4 v = reinterpret_cast<const float4*>(partials + (int64_t)r * cols)[c4];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
   }
@@ -294,8 +294,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __
 // ---------------------------------------------------------------------------------------------
 // RoPE in place on the first n_rot heads of a packed [T, total_heads * D] tensor
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
-                                                   const float* __restrict__ sinT, int64_t T, int S, int n_rot,
+__global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* cosT,
+                                                   const float* sinT, int64_t T, int S, int n_rot,
                                                    int total_heads, int D, float sign) {
   chain();
   const int vph = D / 16;  // 8-element vectors per half head
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ q
 // ---------------------------------------------------------------------------------------------
 // SwiGLU on packed [T, 2F] = [gate | up]
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* gu,
                                                          __nv_bfloat16* __restrict__ out, int64_t T, int F) {
   chain();
   const int vpr = F / 8;
@@ -347,8 +347,8 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
   }
 }
 
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
-                                                         const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* gu,
+                                                         const __nv_bfloat16* dy,
                                                          __nv_bfloat16* __restrict__ dgu, int64_t T, int F) {
   chain();
   const int vpr = F / 8;
@@ -410,8 +410,8 @@ __device__ __forceinline__ BF8 ce_grad8(const BF8& q, float gm, float inv_s, flo
 
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CE_THREADS, 3)
-    ce_row_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ row_loss,
-                  const float* __restrict__ inv_count, int V, int64_t ld, int ignore_index) {
+    ce_row_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* labels, float* __restrict__ row_loss,
+                  const float* inv_count, int V, int64_t ld, int ignore_index) {
   chain();
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) uint8_t ce_smem[];
@@ -514,8 +514,8 @@ static int ce_rows(__nv_bfloat16* logits, const int64_t* labels, float* row_loss
 // logits the GEMM writes into rows padded to an aligned stride); the pad columns come out as zeros.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(CE_THREADS, 3) ce_kernel(__nv_bfloat16* __restrict__ logits,
-                                                  const int64_t* __restrict__ labels,
-                                                  float* __restrict__ row_loss, const float* __restrict__ inv_count,
+                                                  const int64_t* labels,
+                                                  float* __restrict__ row_loss, const float* inv_count,
                                                   int V, int64_t ld, int ignore_index) {
   chain();
   __shared__ float red[32];
@@ -635,7 +635,7 @@ template <typename TP, typename TG, typename TS>
 __global__ void __launch_bounds__(256) adamw_vec_kernel(TP* __restrict__ p, TG* __restrict__ g, TS* __restrict__ m,
                                                         TS* __restrict__ v, int64_t nvec, float lr, float b1, float b2,
                                                         float eps, float wd, float bc1, float rsqrt_bc2,
-                                                        int zero_grad, const int* __restrict__ guard) {
+                                                        int zero_grad, const int* guard) {
   chain();
   if (guard && *guard) return;  // a collective of this step gave up: leave parameters and moments alone
   const float decay = 1.f - lr * wd, step = lr / bc1;

@@ -28,8 +28,8 @@ constexpr int IDS_AHEAD = 8;   // ids in flight per thread
 constexpr int AHEAD = 8;       // rows in flight per thread
 constexpr int MIN_COLS = 64, MAX_COLS = THREADS * 8;   // columns of a block at least and at most
 
-__global__ void __launch_bounds__(THREADS, 3) embedding_grad_kernel(const int64_t* __restrict__ ids,
-                                                                 const __nv_bfloat16* __restrict__ dout,
+__global__ void __launch_bounds__(THREADS, 3) embedding_grad_kernel(const int64_t* ids,
+                                                                 const __nv_bfloat16* dout,
                                                                  __nv_bfloat16* __restrict__ grad, int n, int dim,
                                                                  int64_t rows, int accumulate) {
   chain();
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(THREADS, 3) embedding_grad_kernel(const int64_
 #pragma unroll
     for (int k = 0; k < IDS_AHEAD; ++k) {
       const int j = (w0 + k * WARPS) * 32 + lane;
-      other[k] = j < n ? __ldg(ids + j) : -1;
+      other[k] = j < n ? ids[j] : -1;
     }
 #pragma unroll
     for (int k = 0; k < IDS_AHEAD; ++k) {
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(THREADS, 3) embedding_grad_kernel(const int64_
         uint4 v[AHEAD];
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
-          if (a < m) v[a] = __ldg(reinterpret_cast<const uint4*>(dout + (int64_t)pos[a] * dim + c));
+          if (a < m) v[a] = *reinterpret_cast<const uint4*>(dout + (int64_t)pos[a] * dim + c);
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
           if (a < m) {

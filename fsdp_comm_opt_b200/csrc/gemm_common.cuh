@@ -11,7 +11,7 @@ namespace zc {
 // f[j] += bias[col + j], j = 0..7 (col is a multiple of 8; the last group of a ragged N is read element-wise)
 __device__ __forceinline__ void add_bias8(const __nv_bfloat16* bias, int64_t col, int64_t N, float (&f)[8]) {
   if (col + 8 <= N) {
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + col));
+    const uint4 b = *reinterpret_cast<const uint4*>(bias + col);
     const __nv_bfloat162* bb = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -63,8 +63,8 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float2* red) {
 // ---------------------------------------------------------------------------------------------
 template <int MAXV>
 __global__ void __launch_bounds__(LN_THREADS) layernorm_fwd_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
-    const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
+    const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w,
+    const __nv_bfloat16* b, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
     float* __restrict__ mean_out, float* __restrict__ rstd_out, int cols, float eps) {
   chain();
   __shared__ float2 red[32];
@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(LN_THREADS) layernorm_fwd_kernel(
 // partials[cta][0 | 1][cols] and summed by column_sum_deliver_kernel (no atomics)
 template <int MAXV>
 __global__ void __launch_bounds__(LN_THREADS) layernorm_bwd_kernel(
-    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-    const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dh,
+    const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
+    const float* mean_in, const float* rstd_in, const __nv_bfloat16* dh,
     __nv_bfloat16* __restrict__ dx, float* __restrict__ partials, int64_t rows, int cols) {
   chain();
   __shared__ float2 red[32];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(LN_THREADS) layernorm_bwd_kernel(
 // [seg, 2 seg) to outB (null: a single segment), as fp32 or bf16, overwriting or adding to what is
 // there.  Used for LayerNorm's weight / bias gradients and the linear layers' bias gradients, which
 // can then be written straight into the flat gradient buffer of a sharded engine.
-__global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* __restrict__ in, int nrows, int ncols,
+__global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* in, int nrows, int ncols,
                                                                   int seg, void* __restrict__ outA,
                                                                   void* __restrict__ outB, int out_bf16, int accA,
                                                                   int accB) {
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* _
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c4 * 4 < ncols) {
     for (int r = threadIdx.y; r < nrows; r += 32) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(in + (int64_t)r * ncols) + c4);
+      const float4 v = reinterpret_cast<const float4*>(in + (int64_t)r * ncols)[c4];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
   }
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* _
 
 // partial column sums of a bf16 matrix [rows, cols] (rows `ld` elements apart): block (32, 8) covers
 // 256 columns; blockIdx.y strides over the rows; partials[blockIdx.y][cols] fp32
-__global__ void __launch_bounds__(256) bf16_column_partials_kernel(const __nv_bfloat16* __restrict__ in, int64_t rows,
+__global__ void __launch_bounds__(256) bf16_column_partials_kernel(const __nv_bfloat16* in, int64_t rows,
                                                                    int cols, int64_t ld, float* __restrict__ partials) {
   chain();
   __shared__ float red[8][32][8];
@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(256) bf16_column_partials_kernel(const __nv_bf
 constexpr float GELU_K = 0.7978845608028654f;
 constexpr float GELU_C = 0.044715f;
 
-__global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                            const __nv_bfloat16* __restrict__ bias,
+__global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const __nv_bfloat16* x,
+                                                            const __nv_bfloat16* bias,
                                                             __nv_bfloat16* __restrict__ y, int64_t rows, int cols) {
   chain();
   const int vpr = cols / 8;
@@ -300,9 +300,9 @@ __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const __nv_bfloat16*
   }
 }
 
-__global__ void __launch_bounds__(256) bias_gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                            const __nv_bfloat16* __restrict__ bias,
-                                                            const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(256) bias_gelu_bwd_kernel(const __nv_bfloat16* x,
+                                                            const __nv_bfloat16* bias,
+                                                            const __nv_bfloat16* dy,
                                                             __nv_bfloat16* __restrict__ dx, int64_t rows, int cols) {
   chain();
   const int vpr = cols / 8;

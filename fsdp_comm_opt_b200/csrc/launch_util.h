@@ -52,12 +52,21 @@ inline int launch_status() {
 // wait there until that has completed and its results are seen.  Not in launches that run at once: beside collectives, whose
 // CTAs need the slots that the waiting ones would hold.  Step of the tiny model (110 kernels)
 // 355 -> 334 us, of the small one (190) 1647 -> 1609.
+// Such a kernel is on the chip while its inputs are still written, so it reads them with ordinary loads, which stay behind the
+// wait: the read-only path (__ldg, or a const __restrict__ parameter, of which the compiler makes the same) is for data that do
+// not change while a kernel runs, and its loads may be moved ahead of the wait.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain() {
   chain_wait();
   chain_next();
+}
+// an ordinary load of what nobody reads again
+__device__ __forceinline__ float4 ld_once(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
 }
 template <typename... P, typename... A>
 inline void launch_chained_cluster(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

@@ -1263,3 +1263,74 @@ def test_gemm_from_codec_records_matches_fp32_matmul(N, K, M, slab_rows, ring):
     ref = w.float() @ x.float().t()
     assert torch.equal(y1, y2) and torch.equal(y1, plain)
     assert torch.allclose(y1.float(), ref, rtol=2e-2, atol=2e-2 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("heads,kv,D", [(4, 2, 128), (8, 2, 64)])
+def test_recorded_launches_have_the_bits_of_launches_one_after_the_other(heads, kv, D):
+    """Recorded kernels come up while the one before them still writes what they read.  Every kind of them behind another, behind a
+    copy, behind a library kernel and on a branch that joins again, forward and backward, with other inputs at every replay:
+    a value of the replay before would differ.  (Two key blocks: dQ has the same bits in either order.)"""
+    from fsdp_comm_opt_b200.ops import embedding, gemm
+
+    B, S, C, F_, V = 2, 256, 512, 1024, 1000
+    T = B * S
+    torch.manual_seed(D)
+    mk = lambda *shape: (torch.randn(*shape, device=DEV) * shape[-1] ** -0.5).bfloat16().requires_grad_()
+    table, w_qkv, w_o, w_gu, w_down, w_up, w_back, w_head = (
+        mk(64, C), mk((heads + 2 * kv) * D, C), mk(C, heads * D), mk(2 * F_, C), mk(C, F_), mk(F_, C), mk(C, F_), mk(V, C))
+    n1, n2, n3, nb, b_up, b_back = (torch.randn(n, device=DEV).bfloat16().requires_grad_() for n in (C, C, C, C, F_, C))
+    weights = [w_qkv, w_o, w_gu, w_down, w_up, w_back, w_head, n1, n2, n3, nb, b_up, b_back]
+    table.main_grad = torch.zeros_like(table)
+    cos, sin = rope.rope_tables(S, D, 10000.0, torch.device(DEV, 0))
+    side = torch.cuda.Stream()
+
+    def step(ids, labels, extra, moments):
+        table.main_grad_written = False
+        x = embedding.embedding(ids, table) + extra
+        q = gemm.linear(norm.rms_norm(x, n1), w_qkv).view(T, -1)
+        q = rope.apply_rope(q, cos, sin, heads + kv, D, S) if D == 64 else q
+        a = gemm.linear(attention.causal_attention(q.view(B, S, heads + 2 * kv, D), heads, kv).reshape(T, heads * D), w_o)
+        y, h = norm.add_rms_norm(a, x.reshape(T, C), n2, 1e-5)
+        m = gemm.linear(swiglu.swiglu(gemm.linear(y, w_gu)), w_down)
+        z, h2 = gpt2_ops.add_layer_norm(m, h, n3, nb)
+        g = gemm.linear(gpt2_ops.bias_gelu(gemm.linear(z, w_up), b_up), w_back, b_back) + h2
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            branch = gemm.gemm(z.detach(), w_up.detach(), False, True)
+        value = loss.cross_entropy(gemm.linear(g, w_head), labels)
+        grads = torch.autograd.grad(value, weights + [table], allow_unused=True)[:-1]
+        main.wait_stream(side)
+        p, mean, sq = (t.clone() for t in moments)
+        grad = grads[2].clone()
+        _lib.check(_lib.cuda().zc_adamw(p.data_ptr(), grad.data_ptr(), mean.data_ptr(), sq.data_ptr(), p.numel(), 0, 0, 0, 1e-3, 0.9, 0.95,
+                                        1e-8, 0.01, 0.1, 0.05, 0, _lib.stream_ptr(p.device)), "zc_adamw")
+        return [value, branch, table.main_grad.clone(), p, mean, sq, *grads]
+
+    def inputs(k):
+        g = torch.Generator(DEV).manual_seed(k)
+        return [torch.randint(0, 64, (B, S), device=DEV, generator=g), torch.randint(0, V, (T,), device=DEV, generator=g),
+                torch.randn(B, S, C, device=DEV, generator=g).bfloat16(),
+                [torch.rand(2 * F_, C, device=DEV, generator=g).bfloat16() for _ in range(3)]]
+
+    def put(k):
+        for a, b in zip(fixed[:3] + fixed[3], (lambda i: i[:3] + i[3])(inputs(k))):
+            a.copy_(b)
+
+    stream = torch.cuda.Stream()  # of all steps, recorded or not
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        fixed = inputs(0)
+        want = [[t.detach() for t in step(*inputs(k))] for k in range(12)]
+        again = [[t.detach() for t in step(*inputs(k))] for k in range(12)]
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for x, y in zip(want, again) for a, b in zip(x, y))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ids, labels, extra = (t.clone() for t in fixed[:3])
+            recorded = [t.detach() for t in step(ids, labels, extra, fixed[3])]
+        for k in [*range(12), *range(12)]:
+            put(k)
+            graph.replay()
+            assert all(torch.equal(a, b) for a, b in zip(want[k], recorded)), k
+    assert _lib.cuda().zc_gemm_status_read_and_clear() == 0 and attention.status_read_and_clear() == 0

@@ -1,10 +1,13 @@
 """CPU paths of the ops against plain PyTorch fp32 references (values and gradients)."""
 import math
+import re
+from pathlib import Path
 
 import pytest
 import torch
 import torch.nn.functional as F
 
+from fsdp_comm_opt_b200 import _lib
 from fsdp_comm_opt_b200.ops import adamw, attention, gemm, loss, norm, quant, rope, swiglu
 
 
@@ -221,3 +224,33 @@ def test_a_dropout_added_to_a_recomputed_block_keeps_its_mask(shape):
     ids = torch.randint(0, 64, (1, 16))
     model(input_ids=ids, labels=ids).loss.backward()
     assert len(masks) > 1 and all(torch.equal(m, masks[0]) for m in masks[1:])
+
+
+def _global_functions(src):
+    """(signature, body) of every ``__global__`` function of a CUDA source."""
+    for m in re.finditer("__global__", src):
+        at = src.index("{", m.end())
+        depth, end = 1, at + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(src[end], 0)
+            end += 1
+        yield src[m.start():at], src[at:end]
+
+
+def test_chained_kernels_read_what_others_write_with_ordinary_loads():
+    """A kernel that waits for the one before it while that still writes may not read through the read-only path: neither with
+    __ldg nor through a const __restrict__ parameter, whose loads the compiler turns into the same.  The headers that these
+    kernels share have no such load either."""
+    csrc = Path(_lib.__file__).parent / "csrc"
+    chained = []
+    for f in sorted(csrc.glob("*.cu")):
+        src = f.read_text()
+        for sig, body in _global_functions(src):
+            if not re.search(r"\bchain(_wait)?\(\)", body):
+                continue
+            chained.append(sig)
+            assert not re.search(r"__ldg|__ldcs|ld\.global\.nc", body), f"{f.name}: {sig}"
+            assert not re.search(r"const \w+\* ?__restrict__", sig), f"{f.name}: {sig}"
+    assert len(chained) >= 20
+    for header in ("gemm_common.cuh", "attn_sm100.cuh", "attn_common.cuh", "umma.cuh"):
+        assert "__ldg" not in (csrc / header).read_text()
