@@ -146,6 +146,7 @@ class ShardGroup:
         self.shard = None         # view of the master tensor
         self.shard_c = None       # the same shard in the compute dtype (what the all-gather sends)
         self.grad_shard = None    # view of the gradient tensor
+        self.grad_shard_c = None  # on one rank: the same in the compute dtype, which backward writes
         self.ag_hook = None
         self.rs_hook = None
         self.grads_ready = False  # gradient buffer handed out for this backward
@@ -234,14 +235,16 @@ class FlatShardEngine:
         # ---- persistent storage: one tensor per role over all groups --------------------------
         total = sum(g.shard_numel for g in self.groups)
         self.master = torch.zeros(total, dtype=plan.master_dtype, device=device)
-        grad_dtype = cd if (self.world == 1 or plan.master_dtype == cd) else torch.float32
-        self.grad_master = torch.zeros(total, dtype=grad_dtype, device=device)
+        self.grad_master = torch.zeros(total, dtype=cd if plan.master_dtype == cd else torch.float32, device=device)
+        # what backward writes on one rank: the optimizer's gradients, unless it wants them in fp32
+        grad_c = self.grad_master if plan.master_dtype == cd or self.world > 1 else torch.zeros(total, dtype=cd, device=device)
         self.master_c = self.master if plan.master_dtype == cd else torch.zeros(total, dtype=cd, device=device)
         off = 0
         for g in self.groups:
             g.shard = self.master[off:off + g.shard_numel]
             g.shard_c = self.master_c[off:off + g.shard_numel]
             g.grad_shard = self.grad_master[off:off + g.shard_numel]
+            g.grad_shard_c = grad_c[off:off + g.shard_numel]
             off += g.shard_numel
             g.ag_hook = plan.ag_hook_factory() if plan.ag_hook_factory else PlainAllGather()
             g.rs_hook = plan.rs_hook_factory() if plan.rs_hook_factory else PlainReduceScatter()
@@ -326,7 +329,7 @@ class FlatShardEngine:
         self._sync_compute_copy()
         for g in self.groups:
             if self.world == 1:
-                g.full, g.full_grad, g.state = g.shard_c, g.grad_shard, UNSHARDED
+                g.full, g.full_grad, g.state = g.shard_c, g.grad_shard_c, UNSHARDED
                 self._replace_param_storage(g, g.full)
                 self._set_main_grads(g)
             else:
@@ -473,6 +476,8 @@ class FlatShardEngine:
         self._collect_grads(g)
         g.grads_ready = False
         if self.world == 1:
+            if g.grad_shard_c.dtype != g.grad_shard.dtype:
+                g.grad_shard.copy_(g.grad_shard_c)
             return
         self._reshard(g)
         if self.cuda:

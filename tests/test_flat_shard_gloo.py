@@ -62,6 +62,29 @@ def test_flat_engine_gpt2_family_and_fp32_master(tmp_path):
     assert len(lb) == 4 and lb[-1] < lb[0]
 
 
+def _fp32_master_on_one_rank(rank, world):
+    from fsdp_comm_opt_b200.engine import EngineConfig, TrainEngine
+
+    eng = TrainEngine(EngineConfig(model="tiny", lr=1e-3, master_dtype=torch.float32), torch.device("cpu"))
+    flat, losses = eng.flat, []
+    for b in _batches(0, 4, eng.model_config.vocab_size):
+        before = flat.master.clone()
+        losses.append(eng.step(b))
+        # what backward left in bf16 is what the optimizer sees in fp32, and the layers compute with the rounded weights
+        assert flat.master_param.grad is flat.grad_master and flat.grad_master.dtype == torch.float32
+        for g in flat.groups:
+            for s in g.slots:
+                assert s.param.main_grad.dtype == torch.bfloat16
+                assert torch.equal(g.grad_shard[s.offset:s.offset + s.numel], s.param.main_grad.reshape(-1).float())
+        assert flat.grad_master.abs().max() > 0 and not torch.equal(before, flat.master)
+        assert torch.equal(flat.master_c, flat.master.bfloat16()) and not torch.equal(flat.master_c.float(), flat.master)
+    assert losses[-1] < losses[0]
+
+
+def test_fp32_master_weights_on_one_rank():
+    run_ranks(_fp32_master_on_one_rank, 1)
+
+
 def _one_vs_two(rank, world, out_path):
     """World size 2 against a single process that sees both ranks' batches as one batch."""
     from fsdp_comm_opt_b200.engine import EngineConfig, TrainEngine

@@ -82,6 +82,31 @@ def test_replayed_steps_equal_eager_steps(family):
     run_ranks(_graph_worker, 1, backend="nccl", args=(family,))
 
 
+def _fp32_master_worker(rank, world, family):
+    import torch
+
+    from fsdp_comm_opt_b200.engine import EngineConfig, TrainEngine
+
+    model, dev = "gpt2-tiny" if family == "gpt2" else "tiny", torch.device("cuda", 0)
+    a, b = (TrainEngine(EngineConfig(model=model, lr=1e-3, seed=3, step_graphs=g, master_dtype=torch.float32), dev) for g in (True, False))
+    ids = torch.randint(0, a.model_config.vocab_size, (2, 96), generator=torch.Generator().manual_seed(1)).pin_memory()
+    losses = []
+    for _ in range(8):
+        la, lb = a.step(ids), b.step(ids)
+        assert abs(la - lb) < 2e-3 * abs(lb), (la, lb)                  # dQ is summed in any order
+        losses.append(la)
+    assert a._graphs._recorded and losses[-1] < losses[0]
+    assert a.flat.master.dtype == a.flat.grad_master.dtype == torch.float32
+    assert all(torch.equal(g.grad_shard, g.grad_shard_c.float()) and g.grad_shard.any() for g in a.flat.groups)
+    d = (a.flat.master - b.flat.master).norm() / b.flat.master.norm()
+    assert d < 5e-3
+
+
+@pytest.mark.parametrize("family", ["llama", "gpt2"])
+def test_fp32_master_weights_on_one_gpu(family):
+    run_ranks(_fp32_master_worker, 1, backend="nccl", args=(family,))
+
+
 def _finished_worker(rank, world, graphs):
     import dataclasses
 
