@@ -81,6 +81,8 @@ def declare(lib) -> None:
         _sig(lib, name, L, L, L)
         if hasattr(lib, name):
             getattr(lib, name).restype = L
+    _sig(lib, "zc_gemm_small_best_parts", L, L, L)
+    _sig(lib, "zc_gemm_small_tiles_at_once", I)
     _sig(lib, "zc_gemm_status_read_and_clear")
     # fused collectives
     from ctypes import c_double, c_uint

@@ -310,18 +310,32 @@ static int launch_forms(int a_major, int b_major, const cudaLaunchConfig_t& cfg,
 
 }  // namespace gs
 
+// Tiles whose `parts` CTAs each, a cluster, run at once.
+static int tiles_at_once(int parts) {
+  using namespace gs;
+  constexpr int SMEM = MAX_STAGES * STAGE + (int)sizeof(Shared);
+  static int two[64], four[64], eight[64];
+  switch (parts) {
+    case 1: return sm_count();
+    case 2: return clusters_at_once(gemm_small_kernel<MAJOR_K, MAJOR_K, 2>, 2, THREADS, SMEM, two);
+    case 4: return clusters_at_once(gemm_small_kernel<MAJOR_K, MAJOR_K, 4>, 4, THREADS, SMEM, four);
+    default: return clusters_at_once(gemm_small_kernel<MAJOR_K, MAJOR_K, 8>, 8, THREADS, SMEM, eight);
+  }
+}
+
 // us that a product of these sizes is expected to take here, and in how many parts along K; 0 where there are more tiles than
-// SMs.  Measured: 3.2 a launch and 0.27 a K block (500 clocks: the operands' way into shared memory and out of it, which two
-// CTAs to an SM share, so that 256 tiles of 4 K blocks took 8.1 us, 7.2 with the two-SM kernel), 1.9 to 2.8 for what the CTAs
-// of a cluster send each other.  512 x 256 x 256: 6.7 -> 4.3, 512 x 256 x 1024: 10.3 -> 7.0, 1024^3: 10.4 -> 7.4.
+// SMs.  Measured: 3.2 a launch and 0.27 a K block (500 clocks: the operands' way into shared memory and out of it), 1.9 to 2.8
+// for what the CTAs of a cluster send each other.  512 x 256 x 256: 6.7 -> 4.3, 512 x 256 x 1024: 10.3 -> 7.0, 1024^3:
+// 10.4 -> 7.4.  Only as many parts as let all clusters run at once (74 of two, 33 of four, 15 of eight on 148 SMs): with a second
+// wave 16 tiles of K 1024 by eight took 11.8 us, 6.0 by four, and 36 tiles by four 11.2, 6.3 by two.
 static double expected_us(int64_t M, int64_t N, int64_t K, bool cut_k, int& parts) {
   using namespace gs;
-  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kbs = (K + BK - 1) / BK, sms = sm_count();
+  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kbs = (K + BK - 1) / BK;
   static const double sent[4] = {0.0, 1.9, 2.5, 2.8};
   double least = 0;
   parts = 0;
-  if (tiles > sms) return 0;
-  for (int i = 0; i < 4 && (i == 0 || (cut_k && (tiles << i) <= sms && kbs >= 2LL << i)); ++i) {
+  if (tiles > sm_count()) return 0;
+  for (int i = 0; i < 4 && (i == 0 || (cut_k && tiles <= tiles_at_once(1 << i) && kbs >= 2LL << i)); ++i) {
     const double us = 3.2 + 0.27 * (double)((kbs + (1 << i) - 1) >> i) + sent[i];
     if (i == 0 || us < least) { least = us; parts = 1 << i; }
   }
@@ -357,3 +371,12 @@ int gemm_small_launch(const void* A, const void* B, void* C, const void* bias, i
 }
 
 }  // namespace zc
+
+// For a look at the rule: in how many parts along K the kernel of small products would take a product at best (0: more tiles
+// than SMs), and how many tiles in so many parts run at once.
+extern "C" int zc_gemm_small_best_parts(int64_t M, int64_t N, int64_t K) {
+  int parts;
+  zc::expected_us(M, N, K, true, parts);
+  return parts;
+}
+extern "C" int zc_gemm_small_tiles_at_once(int parts) { return zc::tiles_at_once(parts); }

@@ -39,6 +39,36 @@ inline int resident_ctas(K kernel, int threads, int dyn_smem, int (&cached)[64])
   return cached[dev];
 }
 
+// Clusters of `cluster` CTAs of `kernel` that run at once on the whole device: fewer than its SMs would hold one by one, since a
+// cluster lies within a GPC (of 148, 74 clusters of two, 33 of four or 15 of eight CTAs an SM each).  Kept by the caller, as above.
+template <typename K>
+inline int clusters_at_once(K kernel, int cluster, int threads, int dyn_smem, int (&cached)[64]) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (cached[dev] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = dyn_smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 1;
+    }
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
 // 0 on success, else the cudaError_t of the launch (configuration errors are reported here;
 // execution errors surface at the next synchronisation).
 inline int launch_status() {

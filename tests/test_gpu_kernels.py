@@ -961,6 +961,27 @@ def test_products_of_few_tiles_run_on_one_sm_a_tile(M, N, K):
         assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -9 + 1e-5
 
 
+@pytest.mark.parametrize("K", [1000, 1024, 2048, 4096])
+def test_products_are_cut_into_no_more_clusters_than_run_at_once(K):
+    """A cluster lies within a GPC, so fewer fit than CTAs alone: the last number of tiles that is cut into so many parts and the
+    first that is not.  Rounded once from fp32 sums: 2^-9 and the sums' 1e-5."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    lib = _lib.cuda()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    fit = {parts: lib.zc_gemm_small_tiles_at_once(parts) for parts in (1, 2, 4, 8)}
+    assert fit[1] == sms and all(0 < parts * fit[parts] <= sms for parts in fit) and fit[8] < fit[4] < fit[2]
+    chosen = {tiles: lib.zc_gemm_small_best_parts(128, 128 * tiles, K) for tiles in range(1, sms + 2)}
+    assert chosen[sms + 1] == 0 and all(chosen[t] >= 1 and t <= fit[chosen[t]] for t in range(1, sms + 1))
+    torch.manual_seed(K)
+    x = torch.randn(128, K, device=DEV).bfloat16()
+    for tiles in sorted({t for parts in (2, 4, 8) for t in (fit[parts], fit[parts] + 1)}):
+        w = torch.randn(128 * tiles, K, device=DEV).bfloat16()
+        ref = x.double() @ w.double().t()
+        assert ((gemm.gemm(x, w, False, True).double() - ref).norm() / ref.norm()).item() < 2 ** -9 + 1e-5
+    assert lib.zc_gemm_status_read_and_clear() == 0
+
+
 def test_products_split_along_k_on_two_streams_have_partial_sums_of_their_own():
     """The tail of the last wave is split (4096 x 6144: 384 tiles on 74 clusters), and so is a product of few tiles; the slices
     are added by a second kernel, which other streams' products may run ahead of."""
