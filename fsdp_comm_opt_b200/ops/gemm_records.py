@@ -17,13 +17,24 @@ all-gather output and lets cuBLAS read that, ``main/zipccl_comm.py:134-152``.)
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
+from .. import _lib
 from . import codec
 from .gemm import gemm
 
 _CHUNK = codec.V2_CHUNK
 _SLOT = codec.V2_SLOT
+
+
+@functools.lru_cache(maxsize=4096)
+def _whole_k(N: int, M: int, K: int, device: int) -> bool:
+    """One sum along K a value, so that slabs have the bits of the whole product, except where the two-SM kernel has an
+    almost empty wave or few tiles to cut along K: there the cut is worth more (us, cut and not: 14336 x 4096 x 4096 319 / 335,
+    6144 x 4096 x 4096 141 / 152, 4096 x 128 x 4096 13 / 24)."""
+    return _lib.cuda().zc_gemm_2sm_split_bytes(N, M, K) == 0
 
 
 class RecordLinear:
@@ -85,7 +96,7 @@ class RecordLinear:
                 decode(s + self.ring - 1)
             slot = s % self.ring
             main.wait_event(self._decoded[slot])
-            gemm(self.buf[slot], x, False, True, out=out[s * R:(s + 1) * R], whole_k=True)
+            gemm(self.buf[slot], x, False, True, out=out[s * R:(s + 1) * R], whole_k=_whole_k(R, M, K, x.device.index))
             ev = torch.cuda.Event()
             ev.record(main)
             self._free[slot] = ev
@@ -102,4 +113,4 @@ def linear_t_plain(x: torch.Tensor, records: torch.Tensor, headers: torch.Tensor
             out.copy_(y)
             return out
         return y
-    return gemm(w, x, False, True, out=out, whole_k=True)
+    return gemm(w, x, False, True, out=out, whole_k=_whole_k(N, x.shape[0], K, x.device.index))

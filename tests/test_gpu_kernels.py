@@ -1355,3 +1355,34 @@ def test_recorded_launches_have_the_bits_of_launches_one_after_the_other(heads, 
             graph.replay()
             assert all(torch.equal(a, b) for a, b in zip(want[k], recorded)), k
     assert _lib.cuda().zc_gemm_status_read_and_clear() == 0 and attention.status_read_and_clear() == 0
+
+
+@pytest.mark.parametrize("N,K,M,slab_rows", [(4096, 1000, 520, 256), (2048, 1024, 2048, 128)])
+def test_slabs_and_whole_products_of_different_kernels_have_the_same_bits(N, K, M, slab_rows):
+    """A slab's few tiles run on one SM each, the whole product on pairs of SMs; both are one sum along K."""
+    from fsdp_comm_opt_b200.ops import gemm_records
+
+    lib = _lib.cuda()
+    assert gemm_records._whole_k(N, M, K, 0) and gemm_records._whole_k(slab_rows, M, K, 0)
+    assert lib.zc_gemm_small_best_parts(slab_rows, M, K) > 0 and lib.zc_gemm_small_best_parts(N, M, K) == 0
+    g = torch.Generator().manual_seed(N)
+    w, x = (torch.randn(n, K, generator=g).bfloat16().cuda() for n in (N, M))
+    rec, hdr = codec.v2_encode(w.view(-1))
+    slabs = gemm_records.RecordLinear(N, K, "cuda", slab_rows=slab_rows, ring=3)(x, rec, hdr)
+    plain = gemm_records.linear_t_plain(x, rec, hdr, N, K)
+    ref = w.double() @ x.double().t()
+    assert torch.equal(slabs, plain)
+    assert ((plain.double() - ref).norm() / ref.norm()).item() < 2 ** -9 + 1e-5
+
+
+@pytest.mark.parametrize("N,K,M", [(4096, 4096, 128), (6144, 4096, 4096)])
+def test_products_from_records_are_cut_along_k_where_other_products_are(N, K, M):
+    """Few tiles, and a last wave of ten: the product of a decoded weight is the same launch as any other's."""
+    from fsdp_comm_opt_b200.ops import gemm, gemm_records
+
+    g = torch.Generator().manual_seed(M)
+    w, x = (torch.randn(n, K, generator=g).bfloat16().cuda() for n in (N, M))
+    rec, hdr = codec.v2_encode(w.view(-1))
+    cut, whole = gemm.gemm(w, x, False, True), gemm.gemm(w, x, False, True, whole_k=True)
+    assert not torch.equal(cut, whole)          # fp32 sums of other parts
+    assert torch.equal(gemm_records.linear_t_plain(x, rec, hdr, N, K), cut)
