@@ -1386,3 +1386,69 @@ def test_products_from_records_are_cut_along_k_where_other_products_are(N, K, M)
     cut, whole = gemm.gemm(w, x, False, True), gemm.gemm(w, x, False, True, whole_k=True)
     assert not torch.equal(cut, whole)          # fp32 sums of other parts
     assert torch.equal(gemm_records.linear_t_plain(x, rec, hdr, N, K), cut)
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 128, 16384), (200, 137, 16390), (384, 512, 16384), (256, 2304, 4096), (256, 2290, 4090), (256, 9472, 3328),
+                                   (2048, 1024, 4095)])
+def test_products_whose_slices_of_k_a_second_kernel_adds(M, N, K):
+    """Sixteen slices, a last slice of two K blocks, slices of eight, ragged edges, 37 tiles in two: sizes that still take the two-SM
+    kernel and its workspace, alone and on two streams at once.  Rounded once from fp32 sums: 2^-9 and the sums' 1e-5."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    lib = _lib.cuda()
+    assert lib.zc_gemm_ws_bytes(M, N, K) == lib.zc_gemm_2sm_split_bytes(M, N, K) > 0
+    torch.manual_seed(K)
+    mk = lambda r, c: torch.randn(r, (c + 7) // 8 * 8, device=DEV).bfloat16()[:, :c]
+    pairs, old = [(mk(M, K), mk(N, K)) for _ in range(2)], mk(M, N)
+    bias = torch.randn(N, device=DEV).bfloat16()
+    alone = []
+    for x, w in pairs:
+        ref = x.double() @ w.double().t()
+        acc = torch.empty(M, (N + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :N].copy_(old)
+        alone.append(gemm.gemm(x, w, False, True))
+        gemm.gemm(x, w, False, True, out=acc, accumulate=True)
+        for got, want in ((alone[-1], ref), (gemm.gemm(x, w, False, True, bias=bias), ref + bias.double()), (acc, ref + old.double())):
+            assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -9 + 1e-5
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in pairs], [[], []]
+    for _ in range(20):
+        for st, (x, w), out in zip(streams, pairs, got):
+            with torch.cuda.stream(st):
+                out.append(gemm.gemm(x, w, False, True))
+    torch.cuda.synchronize()
+    assert lib.zc_gemm_status_read_and_clear() == 0
+    assert all(torch.equal(ref, y) for ref, out in zip(alone, got) for y in out)
+
+
+@pytest.mark.parametrize("M,N,K,parts", [(129, 136, 136, 1), (300, 1001, 200, 1), (769, 650, 2040, 2), (129, 137, 900, 4), (130, 250, 2040, 8),
+                                         (1100, 4301, 200, 0), (200, 137, 16390, 0), (4000, 6100, 1030, 0)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_products_into_a_part_of_a_buffer_leave_the_rest_alone(M, N, K, parts, accumulate):
+    """Every element of a result in a buffer with longer rows and more of them, both kernels, K in one and in several parts.  An
+    element is rounded once, by 2^-8 of itself at most, from a sum of K products, whose fp32 errors are below K 2^-22 of the sum of
+    their sizes.  The columns up to the next multiple of eight are zeros (or what they were, when added to); all else is untouched."""
+    from fsdp_comm_opt_b200.ops import gemm
+
+    lib = _lib.cuda()
+    if parts:
+        assert lib.zc_gemm_small_best_parts(M, N, K) == parts and lib.zc_gemm_ws_bytes(M, N, K) == 0
+    else:
+        assert lib.zc_gemm_small_best_parts(M, N, K) == 0 or lib.zc_gemm_ws_bytes(M, N, K) > 0
+    torch.manual_seed(M + K)
+    pad = (N + 7) // 8 * 8
+    mk = lambda r, c: torch.randn(r, (c + 7) // 8 * 8, device=DEV).bfloat16()[:, :c]
+    x, w, bias = mk(M, K), mk(N, K), torch.randn(N, device=DEV).bfloat16()
+    ref, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    for b in (None, bias):
+        buf = torch.randn(M + 9, pad + 24, device=DEV).bfloat16()
+        before = buf.clone()
+        gemm.gemm(x, w, False, True, out=buf[4:4 + M, 8:8 + N], accumulate=accumulate, bias=b)
+        torch.cuda.synchronize()
+        assert lib.zc_gemm_status_read_and_clear() == 0
+        want = ref + (before[4:4 + M, 8:8 + N].double() if accumulate else 0) + (b.double() if b is not None else 0)
+        bound = want.abs() * 2 ** -8 + (size + want.abs() + 8) * K * 2 ** -22
+        assert ((buf[4:4 + M, 8:8 + N].double() - want).abs() <= bound).all()
+        padding = buf[4:4 + M, 8 + N:8 + pad]
+        assert torch.equal(padding, before[4:4 + M, 8 + N:8 + pad]) if accumulate else not padding.any()
+        buf[4:4 + M, 8:8 + pad] = before[4:4 + M, 8:8 + pad]
+        assert torch.equal(buf, before)
