@@ -921,23 +921,45 @@ __global__ void __launch_bounds__(512, 1) attn_bwd_kt_kernel(const __grid_consta
   if (warp == 1) tmem_dealloc(tm, 512);
 }
 
+// Key blocks whose `parts` CTAs each, a cluster, run at once.
+template <int D>
+static int blocks_at_once(int parts) {
+  static int two[64], four[64], eight[64];
+  const auto kernel = attn_bwd_kt_kernel<D, true>;
+  switch (parts) {
+    case 1: return sm_count();
+    case 2: return clusters_at_once(kernel, 2, 512, Cfg<D>::SMEM, two);
+    case 4: return clusters_at_once(kernel, 4, 512, Cfg<D>::SMEM, four);
+    default: return clusters_at_once(kernel, 8, 512, Cfg<D>::SMEM, eight);
+  }
+}
+
 // How many CTAs (a cluster) share the query heads of a key block.  A key block's iterations follow one another, so with few
 // key blocks, batches and KV heads the chip waits for the longest of them: 1024 keys, 8 / 2 heads of 128 are 16 CTAs of up to
-// 32 iterations, 83 us.  By heads and not by query blocks: a query block's dQ then still gets its key blocks' tiles an
-// iteration after each other, in the same order from run to run where all CTAs run at once.  Counted in iterations (2.3 us at head
-// dimension 128, 2 at 64): the longest CTA or the average of all SMs, and for every wave of CTAs what one costs beside its
-// iterations, 4 alone and a few more for adding up the shares.  (us, alone and
-// shared) 1024 keys, 8 / 2 heads: 83, by four 31; 2048, 32 / 8: 166, by two 100; 4096, 8 / 2: 308, by four 108; 1024, 64 / 8: 167, by
-// four 72; 4096, 64 / 8: 713, by two 683; 4096, 32 / 8: 337, by two 353, so alone.
-static int parts_of(int S, int Hq, int Hkv, int B, int D) {
+// 32 iterations, 83 us.  Counted in iterations (2.3 us at head dimension 128, 2 at 64): the longest CTA or the average of all
+// SMs, and for every wave of clusters (74 of two, 33 of four, 15 of eight run at once) what one costs beside its iterations, 4 alone
+// and a few more for adding up the shares.  (us, alone and shared) 1024 keys, 8 / 2 heads: 83, by four 31; 2048, 32 / 8: 166, by
+// two 100; 4096, 8 / 2: 308, by four 108; 1024, 64 / 8: 167, by two 97; 4096, 64 / 8: 713, by two 683; 4096, 32 / 8: 337, by two 353,
+// so alone.
+// A query block's dQ gets its key blocks' tiles in the order of time.  By heads and not by query blocks the tiles come an
+// iteration after each other, and where all CTAs run at once they come in the same order at every run; in a second wave they do not
+// (1920 keys, 16 / 8 heads of 64: alone none of 2998 runs differed from the first, by two all of 39).  So where dQ repeats without
+// sharing, key blocks are shared only as far as all clusters run at once.  What that costs: 1024 keys, 64 / 8 heads of 128, 97 us
+// where four would take 75; 1280 keys, 212 where they would take 115.  Without sharing it repeats in one wave, at head dimension 128 up to twelve key blocks (of
+// 2340 runs in 60 places of memory none differed from the first at 1536 keys, 8 / 2 heads, 323 at 1920, 16 / 8: a CTA's 2.3 us an iteration
+// drift further apart than that).
+template <int D>
+static int parts_of(int S, int Hq, int Hkv, int B) {
   const int sms = sm_count(), nqb = (S + 127) / 128, group = Hq / Hkv;
   const double alone = 4.0, shared = D == 128 ? 7.0 : 5.5;
   const double ctas = (double)nqb * Hkv * B, longest = (double)group * nqb, all = ctas * group * (nqb + 1) / 2;
+  const bool repeats = ctas <= sms && (D == 64 || nqb <= 12);
   int best = 1;
   double least = 0;
   for (int c = 1; c <= 8 && group % c == 0; c *= 2) {
-    const double slots = c == 8 ? sms * 0.875 : sms;  // clusters of eight leave SMs of every GPC over
-    const double t = std::max(longest / c, all / sms) + std::ceil(ctas * c / slots) * (c > 1 ? shared : alone);
+    const double waves = std::ceil(ctas / blocks_at_once<D>(c));
+    if (c > 1 && repeats && waves > 1) break;
+    const double t = std::max(longest / c, all / sms) + waves * (c > 1 ? shared : alone);
     if (c == 1 || t < least) { best = c; least = t; }
   }
   return best;
@@ -948,7 +970,7 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
                   const CUtensorMap& mdq, BwdParams p, cudaStream_t st) {
   using C = Cfg<D>;
   static_assert(2 * 128 * D * 4 <= C::DS, "the shares' sums take the place of K, V, Q and dO");
-  p.parts = parts_of(p.S, p.Hq, p.Hkv, p.B, D);
+  p.parts = parts_of<D>(p.S, p.Hq, p.Hkv, p.B);
   const int units = (p.S + 127) / 128 * p.Hkv * p.B;
   if (p.parts == 1) {
     if (cudaFuncSetAttribute(attn_bwd_kt_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)

@@ -622,6 +622,25 @@ def test_attention_backward_shared_by_a_cluster(B, S, Hq, Hkv, D):
         assert ((d - r).norm() / r.norm()).item() < 1e-2
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(1, 700, 16, 2, 64), (1, 1100, 16, 2, 128), (1, 1536, 8, 2, 128), (1, 1024, 64, 8, 128),
+                                          (2, 1100, 8, 2, 128), (1, 1024, 32, 8, 128), (1, 900, 32, 8, 64), (1, 1920, 16, 8, 64)])
+def test_attention_backward_repeats_its_bits_when_shared(B, S, Hq, Hkv, D):
+    """dQ is added up in the order in which key blocks come to it, which is the same at every run while all clusters run at once:
+    by eight, by four, by two and alone, where more CTAs to a key block would take a second wave.
+    Against fp32 within the bound of the test above."""
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, Hq + 2 * Hkv, D, device=DEV).bfloat16().requires_grad_()
+    o = attention.causal_attention(qkv, Hq, Hkv)
+    g = torch.randn_like(o)
+    (first,) = torch.autograd.grad(o, qkv, g, retain_graph=True)
+    differ = [(torch.autograd.grad(o, qkv, g, retain_graph=True)[0] != first).any() for _ in range(20)]
+    assert not torch.stack(differ).any()
+    assert attention.status_read_and_clear() == 0
+    qf = qkv.detach().float().requires_grad_()
+    (dref,) = torch.autograd.grad(_attn_ref(qf, Hq, Hkv), qf, g.float())
+    assert ((first.float() - dref).norm() / dref.norm()).item() < 1e-2
+
+
 @pytest.mark.parametrize("impl", ["2q+kt", "ws+ws"])
 def test_attention_rising_scores_rescale_the_accumulator(impl, monkeypatch):
     """Keys whose scores grow along the sequence raise the running row maximum again and again, so
