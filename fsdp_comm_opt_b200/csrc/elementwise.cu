@@ -70,7 +70,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 //   h = x (+ residual, rounded to bf16);  rstd = rsqrt(mean(h^2) + eps);  y = h * rstd * w
 // A CTA of NT threads, V vectors of eight columns each, walks its rows with the next row's operands on their way (kept as
 // they are stored) and one barrier a row.  Bound by HBM: with the residual 4096 rows of 4096 columns take 24.9 us (the bytes
-// 20.5; a warp a row 36.9, a CTA a row 29.8), of 5120 32.9 (25.6; 43.2), of 8192 46.7 (41.0; 62.8); 1024 rows of 1024 columns 4.4.
+// 20.5; a warp a row 36.9, a CTA a row 29.8), of 5120 32.9 (25.6; 43.2), of 8192 46.7 (41.0; 62.8); 512 rows of 1024 columns 2.3.
 // ---------------------------------------------------------------------------------------------
 constexpr int RN_MAX_COLS = 8192;
 
@@ -150,6 +150,72 @@ __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
   }
 }
 
+// The same with a warp a row of up to NV vectors a lane, four rows a CTA: no barrier, a row's loads all in flight and the row
+// kept as it is stored.  The next kernel's CTAs come up as these end: among many short CTAs they are in the way (recorded one behind
+// the other, 4096 rows of 1024 columns take 6.7 us, 8.9 with the next one's on the chip from the start).
+template <int NV>
+__global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
+    const __nv_bfloat16* x, const __nv_bfloat16* res,
+    const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
+    float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
+  chain_wait();
+  const int lane = threadIdx.x & 31, nvec = cols / 8;
+  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  BF8 hv[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = lane + 32 * i;
+    if (v < nvec) hv[i] = ld8(x + row * cols + v * 8);
+  }
+  if (res) {
+    BF8 rv[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = lane + 32 * i;
+      if (v < nvec) rv[i] = ld8(res + row * cols + v * 8);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = lane + 32 * i;
+      if (v < nvec) {
+        float f[8], r[8];
+        unpack8(hv[i], f);
+        unpack8(rv[i], r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += r[j];
+        hv[i] = pack8(f);
+        st8(h_out + row * cols + v * 8, hv[i]);
+      }
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    if (lane + 32 * i < nvec) {
+      float f[8];
+      unpack8(hv[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+  }
+  ss = warp_sum(ss);
+  const float rstd = rsqrtf(ss / (float)cols + eps);
+  if (lane == 0) rstd_out[row] = rstd;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = lane + 32 * i;
+    if (v < nvec) {
+      float f[8], wf[8];
+      unpack8(hv[i], f);
+      unpack8(ld8(w + v * 8), wf);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * wf[j];
+      st8(y + row * cols + v * 8, pack8(f));
+    }
+  }
+}
+
 // dx = rstd * (g - xhat * mean(g * xhat)) (+ dh),  g = dy * w,  xhat = h * rstd
 // dw = sum_rows dy * xhat: every CTA keeps partial sums in registers over its rows and writes them
 // to its row of `partials` ([gridDim.x, cols] fp32), which rmsnorm_dw_reduce_kernel then sums
@@ -157,7 +223,9 @@ __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
 // took most of the kernel's time); with partials == nullptr the atomics into dw32 remain.
 // A CTA of NT threads, V vectors of eight columns each, walks its rows with the next row's operands on their way (kept as
 // they are stored, 16 bytes a vector) and one barrier a row.  Bound by HBM: 4096 rows of 4096 columns 41.6 -> 31.3 us (the
-// bytes take 20.5), of 5120 91.8 -> 47.3, of 8192 120.5 -> 61.8 (41.0) against loads that begin after the row before.
+// bytes take 20.5), of 5120 91.8 -> 47.3, of 8192 120.5 -> 61.8 (41.0) against loads that begin after the row before.  Up to 2048
+// columns smaller CTAs, four to an SM (65536 rows of 2048: 263 -> 176), or where an SM has ten rows at most one vector a thread, of
+// fewer partial sums (1000 rows: 10.4 -> 9.1).
 template <int NT, int V, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_bwd_kernel(
     const __nv_bfloat16* dy, const __nv_bfloat16* h,
@@ -729,13 +797,24 @@ int zc_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
                    int cols, float eps, cudaStream_t st) {
   if (cols % 8 || cols > zc::RN_MAX_COLS) return ERR_UNSUPPORTED;
   if (rows == 0) return 0;
-#define ZC_RN_FWD(NT, V, PER_SM)                                                                                       \
-  zc::launch_chained(zc::rmsnorm_fwd_kernel<NT, V, PER_SM>,                                                            \
-                     (unsigned)std::min<int64_t>(rows, (int64_t)zc::sm_count() * PER_SM), NT, 0, st, (const bf16*)x,   \
-                     (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)h_out, rstd, rows, cols, eps)
-  if (cols <= 128 * 8) ZC_RN_FWD(128, 1, 8);
-  else if (cols <= 256 * 2 * 8) ZC_RN_FWD(256, 2, 3);
-  else ZC_RN_FWD(512, 2, 2);
+#define ZC_RN_FWD(kernel, grid, threads)                                                                               \
+  zc::launch_chained(kernel, (unsigned)(grid), threads, 0, st, (const bf16*)x, (const bf16*)res, (const bf16*)w,       \
+                     (bf16*)y, (bf16*)h_out, rstd, rows, cols, eps)
+  const int64_t sms = zc::sm_count(), quads = (rows + 3) / 4;
+  // From six rows an SM on, a warp a row where a lane holds it in few registers: (us, a CTA a row and a warp a row) 65536 rows of 64
+  // columns 33.5 and 17.7, of 512 57 and 30, of 2048 152 and 110, with the residual 218 and 182; 1000 rows of 1024 3.1 and 2.8, 700 2.1 and
+  // 2.7; without the residual 16384 of 3072 51.5 and 45.3, with it 76.0 and 77.4.
+  if (rows > 6 * sms && (cols <= 2048 || (cols <= 3072 && !res))) {
+    if (cols <= 1024) ZC_RN_FWD(zc::rmsnorm_fwd_warp_kernel<4>, quads, 128);
+    else if (cols <= 2048) ZC_RN_FWD(zc::rmsnorm_fwd_warp_kernel<8>, quads, 128);
+    else ZC_RN_FWD(zc::rmsnorm_fwd_warp_kernel<12>, quads, 128);
+  } else if (cols <= 128 * 8) {
+    ZC_RN_FWD((zc::rmsnorm_fwd_kernel<128, 1, 8>), std::min(rows, sms * 8), 128);
+  } else if (cols <= 256 * 2 * 8) {
+    ZC_RN_FWD((zc::rmsnorm_fwd_kernel<256, 2, 3>), std::min(rows, sms * 3), 256);
+  } else {
+    ZC_RN_FWD((zc::rmsnorm_fwd_kernel<512, 2, 2>), std::min(rows, sms * 2), 512);
+  }
 #undef ZC_RN_FWD
   return zc::launch_status();
 }
@@ -756,6 +835,8 @@ int zc_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
   zc::launch_chained(zc::rmsnorm_bwd_kernel<NT, V, PER_SM>, grid, NT, 0, st, (const bf16*)dy, (const bf16*)h,          \
                      (const bf16*)w, rstd, (const bf16*)dh, (bf16*)dx, dw32, partials, rows, cols)
   if (cols <= 128 * 8) { ZC_RN_BWD(128, 1, 4); }
+  else if (cols <= 256 * 8 && rows <= 10 * (int64_t)zc::sm_count()) { ZC_RN_BWD(256, 1, 2); }
+  else if (cols <= 256 * 8) { ZC_RN_BWD(128, 2, 4); }
   else if (cols <= 256 * 2 * 8) { ZC_RN_BWD(256, 2, 2); }
   else { ZC_RN_BWD(512, 2, 1); }
 #undef ZC_RN_BWD

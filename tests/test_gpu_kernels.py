@@ -350,6 +350,25 @@ def test_rmsnorm_walks_rows_of_every_width(rows, cols):
         assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
 
 
+@pytest.mark.parametrize("rows,cols", [(888, 2048), (1480, 2048), (1481, 2048), (1481, 1032), (889, 8), (889, 1024), (890, 1032), (891, 2048), (1500, 2056), (1501, 3072), (889, 3080)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_of_many_rows_at_every_width(rows, cols, residual):
+    """Either side of six and ten rows an SM of 148, of the widths at which a lane's vectors change and of the last one of a warp a row,
+    with rows that do not fill a CTA.  The bounds of the test above."""
+    torch.manual_seed(rows + cols)
+    x, r, g = (torch.randn(rows, cols, device=DEV).bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(cols, device=DEV)).bfloat16().requires_grad_()
+    x.requires_grad_()
+    y, h = norm.add_rms_norm(x, r, w, 1e-5) if residual else (norm.rms_norm(x, w, 1e-5), x)
+    dx, dw = torch.autograd.grad(y, [x, w], g)
+    if residual:
+        assert torch.equal(h, (x.detach().float() + r.float()).bfloat16())
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    yd = hd * (hd.pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt() * wd
+    for got, want in zip((y, dx, dw), (yd, *torch.autograd.grad(yd, [hd, wd], g.double()))):
+        assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
+
+
 @pytest.mark.parametrize("n", [8, 2048, 2056, 4096, 4104, 100_000])
 def test_adamw_updates_every_vector_once(n):
     """Around a thread's second vector and a CTA's 512; elements are independent, so each size has the bits of the largest.
