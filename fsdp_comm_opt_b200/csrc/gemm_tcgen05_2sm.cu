@@ -96,6 +96,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// 16 bytes of global memory into shared memory, and the wait for all of this thread's
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // TMA load into this CTA's shared memory; the bytes are counted on the barrier at `bar_cluster_addr`
 // (the even CTA's `full` barrier)
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
@@ -249,7 +254,9 @@ __device__ __forceinline__ Unit unit_of(int u, const Params& p) {
 // row a thread, lie next to each other.
 __device__ __forceinline__ int partial_off(int row, int c4) { return ((row >> 5) * (BN / 4) + c4) * 32 + (row & 31); }
 
-template <int A_MAJOR, int B_MAJOR>
+// ADD: to the old values of C.  Three CTAs of registers for
+// one to an SM: the 96 a thread leave room for a collective's CTAs beside it.
+template <int A_MAJOR, int B_MAJOR, bool ADD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     gemm_2sm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -447,86 +454,72 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
       if (u >= units) break;
       const Unit w = unit_it == 0 ? first : unit_of(u, p);
       const uint32_t acc = unit_it & 1, acc_ph = (unit_it >> 1) & 1;
+      const int64_t warp_row = (int64_t)w.mi * BM + rank * BM_CTA + quarter * 32, col0 = (int64_t)w.ni * BN;
+      const int rows_left = (int)min((int64_t)32, p.M - warp_row) - out_row;  // from this thread's first on
+      const int cols_left = (int)min((int64_t)BN, p.N - col0);
+      __nv_bfloat16* dst = p.C + (warp_row + out_row) * p.ldc + col0 + out_chunk * 8;
+      auto whole = [&](int q) { return reinterpret_cast<uint4*>(epi + (4 * q + out_row) * 128 + ((out_chunk ^ ((4 * q + out_row) & 7)) << 4)); };
+      // Old values come into the buffer as new ones go out, in whole lines, the first while the products are still computed (16 bytes
+      // of 32 rows a load, behind them: 7424 x 1536 x 320 took 59 us, 19 now).
+      auto fetch_old = [&](int c) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (c + out_chunk * 8 < cols_left && 4 * q < rows_left) copy16_async(whole(q), dst + c + (int64_t)(4 * q) * p.ldc);
+      };
+      if (ADD && w.slice < 0) fetch_old(0);
       ok = wait_bar_cluster(accf + 8 * acc, acc_ph, &s_abort);
       if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
       tc_fence_after_sync();
-      const int row_in_tile = (int)rank * BM_CTA + quarter * 32 + lane;
       if (w.slice < 0) {
-        const int64_t row = (int64_t)w.mi * BM + row_in_tile;
-        const int64_t col0 = (int64_t)w.ni * BN;
-        if (p.accumulate) {
-          // the old values come in as they lie, 16 bytes of a row a thread
+        // No branch in this loop but those on whole chunks: one at every group of eight columns, bias or not, old values
+        // or not, cost more than the work.  32 columns at a time in registers: with 64 some were kept in local memory.
 #pragma unroll 1
-          for (int c = 0; c < BN; c += 32) {
-            uint32_t r[32];
-            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c), r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (row >= p.M || col0 + c + q * 8 >= p.N) continue;
-              float f[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q * 8 + j]);
-              if (p.bias) add_bias8(p.bias, col0 + c + q * 8, p.N, f);
-              uint4* dst = reinterpret_cast<uint4*>(p.C + row * p.ldc + col0 + c + q * 8);
-              add_old8(*dst, f);
-              *dst = round8(f);
-            }
+        for (int c = 0; c < BN; c += EPI_COLS) {
+          if (ADD) {
+            copies_done();
+            __syncwarp();
           }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster_relaxed(acce_c0 + 8 * acc);
-        } else {
-          const int64_t warp_row = (int64_t)w.mi * BM + rank * BM_CTA + quarter * 32;
-          const int rows_left = (int)min((int64_t)32, p.M - warp_row) - out_row;  // from this thread's first on
-          const int cols_left = (int)min((int64_t)BN, p.N - col0);
-          const __nv_bfloat16* bias = p.bias + col0;
-          __nv_bfloat16* dst = p.C + (warp_row + out_row) * p.ldc + col0 + out_chunk * 8;
-          // No branch in this loop but those on whole chunks: one at every group of eight columns, bias or not, old values
-          // or not, cost more than the work.
-#pragma unroll 1
-          for (int c = 0; c < BN; c += EPI_COLS) {
-            uint32_t r[2][32];
-            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c), r[0]);
-            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c + 32), r[1]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tmem_ld32(tmem_addr(tm + acc * BN, quarter * 32, c + h * 32), r);
             tmem_ld_wait();
-            if (c == BN - EPI_COLS) {  // the accumulator is free
+            if (h == 1 && c == BN - EPI_COLS) {  // the accumulator is free
               tc_fence_before_sync();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster_relaxed(acce_c0 + 8 * acc);
             }
             if (p.bias) {  // a column's value a lane
+              const int col = c + h * 32 + lane;
+              const float mine = col < cols_left ? __bfloat162float(p.bias[col0 + col]) : 0.f;
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int col = c + h * 32 + lane;
-                const float mine = col < cols_left ? __bfloat162float(bias[col]) : 0.f;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) + __shfl_sync(0xffffffffu, mine, j));
-              }
+              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __shfl_sync(0xffffffffu, mine, j));
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < 4; ++q) {
+              uint4* at = reinterpret_cast<uint4*>(epi + lane * 128 + (((4 * h + q) ^ (lane & 7)) << 4));
               float f[8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q >> 2][(q & 3) * 8 + j]);
-              *reinterpret_cast<uint4*>(epi + lane * 128 + ((q ^ (lane & 7)) << 4)) = round8(f);
+              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[q * 8 + j]);
+              if (ADD) add_old8(*at, f);
+              *at = round8(f);
             }
-            __syncwarp();
-            uint4 v[8];
+          }
+          __syncwarp();
+          uint4 v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = *whole(q);
+          __syncwarp();
+          if (ADD && c + EPI_COLS < BN) fetch_old(c + EPI_COLS);
+          if (c + out_chunk * 8 < cols_left) {
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-              v[q] = *reinterpret_cast<const uint4*>(epi + (4 * q + out_row) * 128 + ((out_chunk ^ ((4 * q + out_row) & 7)) << 4));
-            __syncwarp();
-            if (c + out_chunk * 8 < cols_left) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (4 * q < rows_left) *reinterpret_cast<uint4*>(dst + c + (int64_t)(4 * q) * p.ldc) = v[q];
-            }
+              if (4 * q < rows_left) *reinterpret_cast<uint4*>(dst + c + (int64_t)(4 * q) * p.ldc) = v[q];
           }
         }
       } else {
         // K slice of a tail tile: fp32 partial sums, added up by gemm_2sm_fixup_kernel; a warp's store is 512 bytes in a row
-        float4* prow = reinterpret_cast<float4*>(p.partial + (int64_t)w.slice * (BM * BN)) + partial_off(row_in_tile, 0);
+        float4* prow = reinterpret_cast<float4*>(p.partial + (int64_t)w.slice * (BM * BN)) + partial_off((int)rank * BM_CTA + quarter * 32 + lane, 0);
 #pragma unroll 1
         for (int c = 0; c < BN; c += 32) {
           uint32_t r[32];
@@ -604,9 +597,9 @@ static std::mutex g_mutex;
 // stream, which the legacy stream's memset is not ordered with.
 static __device__ unsigned g_counters[2 * COUNTER_SLOTS];
 
-template <int A_MAJOR, int B_MAJOR>
+template <int A_MAJOR, int B_MAJOR, bool ADD>
 static int max_clusters(int smem) {
-  cudaFuncSetAttribute(gemm_2sm_kernel<A_MAJOR, B_MAJOR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(gemm_2sm_kernel<A_MAJOR, B_MAJOR, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (sm_count() / 2));
   cfg.blockDim = dim3(THREADS);
@@ -619,7 +612,7 @@ static int max_clusters(int smem) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_2sm_kernel<A_MAJOR, B_MAJOR>, &cfg) != cudaSuccess || n <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_2sm_kernel<A_MAJOR, B_MAJOR, ADD>, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
     n = sm_count() / 2;
   }
@@ -683,9 +676,9 @@ static int small_parts(int64_t M, int64_t N, int64_t K, bool cut_k, int clusters
 static int init_state(DeviceState& ds, int smem) {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (!ds.ready) {
-    int c = max_clusters<MAJOR_K, MAJOR_K>(smem);
-    c = std::min(c, max_clusters<MAJOR_K, MAJOR_MN>(smem));
-    c = std::min(c, max_clusters<MAJOR_MN, MAJOR_MN>(smem));
+    int c = std::min(max_clusters<MAJOR_K, MAJOR_K, false>(smem), max_clusters<MAJOR_K, MAJOR_K, true>(smem));
+    c = std::min({c, max_clusters<MAJOR_K, MAJOR_MN, false>(smem), max_clusters<MAJOR_K, MAJOR_MN, true>(smem)});
+    c = std::min({c, max_clusters<MAJOR_MN, MAJOR_MN, false>(smem), max_clusters<MAJOR_MN, MAJOR_MN, true>(smem)});
     ds.clusters = c;
     if (cudaGetSymbolAddress((void**)&ds.counters, g_counters) != cudaSuccess) return ERR_BAD_ARG;
     ds.ready = true;
@@ -776,9 +769,10 @@ static int gemm_2sm(const void* A, const void* B, void* C, const void* bias, int
     if (slot < COUNTER_SLOTS) p.counter = ds.counters + 2 * slot;
   }
   const dim3 grid(2 * cut.grid_clusters);
-  if (a_major == MAJOR_K && b_major == MAJOR_K) zc::launch_chained(gemm_2sm_kernel<MAJOR_K, MAJOR_K>, grid, THREADS, smem, st, mapA, mapB, p);
-  else if (a_major == MAJOR_K) zc::launch_chained(gemm_2sm_kernel<MAJOR_K, MAJOR_MN>, grid, THREADS, smem, st, mapA, mapB, p);
-  else zc::launch_chained(gemm_2sm_kernel<MAJOR_MN, MAJOR_MN>, grid, THREADS, smem, st, mapA, mapB, p);
+  const auto launch = [&](auto kernel) { zc::launch_chained(kernel, grid, THREADS, smem, st, mapA, mapB, p); };
+  if (a_major == MAJOR_K && b_major == MAJOR_K) launch(accumulate ? gemm_2sm_kernel<MAJOR_K, MAJOR_K, true> : gemm_2sm_kernel<MAJOR_K, MAJOR_K, false>);
+  else if (a_major == MAJOR_K) launch(accumulate ? gemm_2sm_kernel<MAJOR_K, MAJOR_MN, true> : gemm_2sm_kernel<MAJOR_K, MAJOR_MN, false>);
+  else launch(accumulate ? gemm_2sm_kernel<MAJOR_MN, MAJOR_MN, true> : gemm_2sm_kernel<MAJOR_MN, MAJOR_MN, false>);
   int rc = launch_status();
   if (rc == 0 && p.split > 1) {
     zc::launch_chained(gemm_2sm_fixup_kernel, dim3(BM * BN / 8 / 256, (unsigned)cut.split_tiles), 256, 0, st, p);
