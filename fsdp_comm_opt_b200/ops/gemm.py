@@ -97,16 +97,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool,
         if kind == "2sm":
             fused_bias = (bias is not None and bias.dtype == torch.bfloat16 and bias.is_contiguous()
                           and bias.numel() == N and bias.data_ptr() % 16 == 0)
-            # fp32 partial sums of a product that is split along K: this call's own, so that no other stream shares them
-            args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if fused_bias else None, M, N, K,
-                    a.stride(0), b.stride(0), out.stride(0), int(trans_a), int(trans_b), int(accumulate))
+            bias_ptr = bias.data_ptr() if fused_bias else None
             if whole_k:
-                rc = lib.zc_gemm_bf16_2sm_bias(*args, _lib.stream_ptr(a.device))
+                rc = lib.zc_gemm_bf16_2sm_bias(
+                    a.data_ptr(), b.data_ptr(), out.data_ptr(), bias_ptr, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                    int(trans_a), int(trans_b), int(accumulate), _lib.stream_ptr(a.device))
             else:
+                # fp32 partial sums of a product that is split along K: this call's own, so that no other stream shares them
                 ws_bytes = _ws_bytes(M, N, K, a.device.index)
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device) if ws_bytes else None
-                rc = lib.zc_gemm_bf16_2sm_ws(*args, ws.data_ptr() if ws is not None else None, ws_bytes,
-                                             _lib.stream_ptr(a.device))
+                rc = lib.zc_gemm_bf16_2sm_ws(
+                    a.data_ptr(), b.data_ptr(), out.data_ptr(), bias_ptr, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                    int(trans_a), int(trans_b), int(accumulate), ws.data_ptr() if ws is not None else None, ws_bytes,
+                    _lib.stream_ptr(a.device))
             _lib.check(rc, "zc_gemm_bf16_2sm")
             if bias is not None and not fused_bias:
                 out.add_(bias.to(out.dtype))
