@@ -474,7 +474,17 @@ __global__ void __launch_bounds__(MOMENT_THREADS) v1_base_kernel(const uint16_t*
       if (i + k * nt < nv) v[k] = __ldg(xv + i + k * nt);
   };
   fetch(t);
-  for (long long i = t; i < nv; i += 4 * nt) {
+  long long i = t;
+  for (; i + 7 * nt < nv; i += 4 * nt) {  // all of the next trip is there: no checks (27 264 000 elements in L2 15.7 -> 14.6 us, 2 x 10^8 78 -> 64)
+    uint4 c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = v[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = __ldg(xv + i + (4 + k) * nt);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { add2(c[k].x); add2(c[k].y); add2(c[k].z); add2(c[k].w); }
+  }
+  for (; i < nv; i += 4 * nt) {
     uint4 c[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) c[k] = v[k];
@@ -483,7 +493,7 @@ __global__ void __launch_bounds__(MOMENT_THREADS) v1_base_kernel(const uint16_t*
     for (int k = 0; k < 4; ++k)
       if (i + k * nt < nv) { add2(c[k].x); add2(c[k].y); add2(c[k].z); add2(c[k].w); }
   }
-  for (long long i = nv * 8 + t; i < n; i += nt) add2((uint32_t)__ldg(x + i));
+  for (i = nv * 8 + t; i < n; i += nt) add2((uint32_t)__ldg(x + i));
   __shared__ bool last;
   double2 t2 = block_sum2(s, q);
   if (threadIdx.x == 0) {

@@ -284,6 +284,24 @@ def test_v1_base_statistic_kernel():
     assert int(bases[0]) == 116
 
 
+@pytest.mark.parametrize("trips,more", [(4, 0), (7, 0), (7, 8), (8, -8), (8, 0), (8, 24), (11, 8), (12, 5)])
+def test_v1_base_statistic_adds_every_element_once(trips, more):
+    """One value among zeros, at the ends of the CTAs' trips and in between, around the last trip that is loaded without checks (of 148 SMs).
+    Its logarithm lies three quarters of the way between two bases: without the value the base is another, with it twice the next."""
+    nt = 8 * 148 * 1024
+    n = nt * trips + more
+    want = 60
+    value = 2.0 ** (want - 127 + 5.35 + 0.75) * n ** 0.5
+    x = torch.zeros(n, device=DEV, dtype=torch.bfloat16)
+    got = torch.zeros(64, dtype=torch.int32, device=DEV)
+    places = sorted({0, 7, n // 3, n - 1, n - 8, n - 9, n - n % 8 - 1, *(min(k * nt + d, n - 1) for k in range(trips + 1) for d in (-1, 0))} - {-1})
+    for i, at in enumerate(places):
+        x[at] = value
+        codec.v1_base_from_std(x, got[i:])
+        x[at] = 0
+    assert got[:len(places)].tolist() == [want] * len(places)
+
+
 def test_v1_base_statistic_on_several_streams_and_replayed():
     """Launches of different streams, and those of a recorded graph replayed beside them, have workspaces of their own."""
     xs = [gauss(1 << 22, std=0.02 * 4 ** i, seed=i) for i in range(4)]
