@@ -716,8 +716,10 @@ __global__ void __launch_bounds__(256) adamw_vec_kernel(TP* __restrict__ p, TG* 
     }
   };
   const float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  // two vectors a thread, eight 16-byte loads (or more) in flight before the first use
-  const int64_t i = (int64_t)blockIdx.x * 512 + threadIdx.x, k = i + 256;
+  // two vectors a thread, eight 16-byte loads (or more) in flight before the first use: 512 in a row a CTA, or half the buffer apart
+  // where all four streams are 32 bits (below)
+  constexpr bool APART = sizeof(TP) + sizeof(TG) + sizeof(TS) == 12;
+  const int64_t i = (int64_t)blockIdx.x * (APART ? 256 : 512) + threadIdx.x, k = i + (APART ? (int64_t)gridDim.x * 256 : 256);
   if (k < nvec) {
     float pf[8], gf[8], mf[8], vf[8], pf2[8], gf2[8], mf2[8], vf2[8];
     load8<TP>(p + i * 8, pf);
@@ -764,6 +766,7 @@ int adamw_launch(void* p, void* g, void* m, void* v, int64_t n, float lr, float 
     // A CTA to 512 vectors in a row: 8 KB of every stream, and CTAs that follow one another in address order.  4 x 10^8
     // elements: 803 us (6.98 TB/s; a copy 6.48); CTAs that stride through the buffers, a few dozen per SM, with the
     // second vector of a trip a whole grid further, took 920, the same with 8 KB in a row 839.
+    // All in 32 bits the second vector is a grid further: 5 x 10^7 elements 209 us, 213 with 16 KB in a row; 3.4 x 10^6 in L2 12.4 and 14.5.
     const int64_t grid = (nvec + 511) / 512;
     if (grid > 0x7fffffff) return ERR_BAD_ARG;
     zc::launch_chained(adamw_vec_kernel<TP, TG, TS>, (unsigned)grid, 256, 0, st, (TP*)p, (TG*)g, (TS*)m, (TS*)v, nvec, lr, b1, b2, eps, wd,

@@ -407,6 +407,26 @@ def test_adamw_updates_every_vector_once(n):
         assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
 
 
+@pytest.mark.parametrize("n", [8, 2048, 2056, 4096, 4104, 6152, 100_000])
+def test_adamw_in_32_bits_updates_every_vector_once(n):
+    """Streams of 32 bits, whose threads' second vectors are a grid further: each size has the bits of the largest.  A few roundings to
+    24 bits, of sums of two terms with a difference in one of them."""
+    torch.manual_seed(4)
+    whole = [torch.randn(100_000, device=DEV) * s for s in (1.0, 0.1, 0.01)] + [torch.rand(100_000, device=DEV)]
+    run = lambda t: _lib.check(_lib.cuda().zc_adamw(*(v.data_ptr() for v in t), t[0].numel(), 1, 1, 1, 1e-3, 0.9, 0.95, 1e-8, 0.01, 0.1,
+                                                    0.05, 0, _lib.stream_ptr(t[0].device)), "zc_adamw")
+    part = [v[:n].clone() for v in whole]
+    p, g, m, v = (t.double() for t in part)
+    run(part)
+    run(whole)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b[:n]) for a, b in zip(part, whole))
+    m, v = 0.9 * m + 0.1 * g, 0.95 * v + 0.05 * g * g
+    p = p * (1 - 1e-3 * 0.01) - 1e-3 / 0.1 * m / (v.sqrt() / 0.05 ** 0.5 + 1e-8)
+    for got, want in zip((part[0], part[2], part[3]), (p, m, v)):
+        assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -20
+
+
 def test_swiglu_fwd_bwd():
     torch.manual_seed(1)
     gu = torch.randn(257, 2 * 1024, device=DEV).bfloat16().requires_grad_()
