@@ -83,6 +83,8 @@ def declare(lib) -> None:
             getattr(lib, name).restype = L
     _sig(lib, "zc_gemm_small_best_parts", L, L, L)
     _sig(lib, "zc_gemm_small_tiles_at_once", I)
+    _sig(lib, "zc_attn_bwd_parts", I, I, I, I, I)
+    _sig(lib, "zc_attn_bwd_blocks_at_once", I, I)
     _sig(lib, "zc_gemm_status_read_and_clear")
     # fused collectives
     from ctypes import c_double, c_uint

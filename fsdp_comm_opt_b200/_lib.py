@@ -73,7 +73,7 @@ def cuda_lib_path() -> Path:
 _KERNELS_PER_CALL = {
     "zc_v1_encode_split": 2, "zc_v1_encode_fused": 2, "zc_v1_totals_words": 0, "zc_v1_moments_bytes": 0, "zc_quant_int8": 2,
     "zc_health_word": 0, "zc_health_read_and_clear": 0, "zc_health_set": 0, "zc_attn_bwd": 3, "zc_attn_bwd_ws": 3, "zc_attn_bwd_ws_status_read_and_clear": 0, "zc_attn_status_read_and_clear": 0, "zc_attn_ws_status_read_and_clear": 0, "zc_gemm_status_read_and_clear": 0, "zc_gemm_2sm_split_bytes": 0, "zc_gemm_ws_bytes": 0,
-    "zc_gemm_small_best_parts": 0, "zc_gemm_small_tiles_at_once": 0,
+    "zc_gemm_small_best_parts": 0, "zc_gemm_small_tiles_at_once": 0, "zc_attn_bwd_parts": 0, "zc_attn_bwd_blocks_at_once": 0,
 }
 _LAUNCHES = 0
 

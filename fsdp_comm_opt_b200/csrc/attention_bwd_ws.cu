@@ -945,15 +945,16 @@ static int blocks_at_once(int parts) {
 // iteration after each other, and where all CTAs run at once they come in the same order at every run; in a second wave they do not
 // (1920 keys, 16 / 8 heads of 64: alone none of 2998 runs differed from the first, by two all of 39).  So where dQ repeats without
 // sharing, key blocks are shared only as far as all clusters run at once.  What that costs: 1024 keys, 64 / 8 heads of 128, 97 us
-// where four would take 75; 1280 keys, 212 where they would take 115.  Without sharing it repeats in one wave, at head dimension 128 up to twelve key blocks (of
-// 2340 runs in 60 places of memory none differed from the first at 1536 keys, 8 / 2 heads, 323 at 1920, 16 / 8: a CTA's 2.3 us an iteration
-// drift further apart than that).
+// where four would take 75; 1280 keys, 212 where they would take 115.  Without sharing it repeats in one wave while
+// CTAs do not drift apart by an iteration, with few key blocks or few CTAs (of 174 to 2340 runs in several places of memory that
+// differed: head dimension 128, none at 1536 keys, 8 / 2 heads, nor at 2048, 323 at 1920, 16 / 8; 64, none up to 3584 keys with any heads or
+// 7168 with 8 / 1, 116 of 174 at 4096, 32 / 4).
 template <int D>
 static int parts_of(int S, int Hq, int Hkv, int B) {
   const int sms = sm_count(), nqb = (S + 127) / 128, group = Hq / Hkv;
   const double alone = 4.0, shared = D == 128 ? 7.0 : 5.5;
   const double ctas = (double)nqb * Hkv * B, longest = (double)group * nqb, all = ctas * group * (nqb + 1) / 2;
-  const bool repeats = ctas <= sms && (D == 64 || nqb <= 12);
+  const bool repeats = ctas <= sms && (D == 128 ? nqb <= 12 || ctas <= 32 : nqb <= 28 || ctas <= 56);
   int best = 1;
   double least = 0;
   for (int c = 1; c <= 8 && group % c == 0; c *= 2) {
@@ -1110,5 +1111,11 @@ int zc_attn_bwd_kt(const void* q, const void* k, const void* v, const void* o, c
     zc::launch_chained(dq_convert8_kernel<64>, ugrid, 256, 0, st, (const float4*)dq_acc, (__nv_bfloat16*)dq, units, Hq, dqs1, dqs2);
   return launch_status();
 }
+
+// For a look at the rule: how many CTAs share a key block's query heads, and how many key blocks so shared run at once.
+int zc_attn_bwd_parts(int S, int Hq, int Hkv, int B, int D) {
+  return D == 128 ? zc::bkt::parts_of<128>(S, Hq, Hkv, B) : zc::bkt::parts_of<64>(S, Hq, Hkv, B);
+}
+int zc_attn_bwd_blocks_at_once(int parts, int D) { return D == 128 ? zc::bkt::blocks_at_once<128>(parts) : zc::bkt::blocks_at_once<64>(parts); }
 
 }  // extern "C"
