@@ -150,9 +150,33 @@ __global__ void __launch_bounds__(NT, PER_SM) rmsnorm_fwd_kernel(
   }
 }
 
-// The same with a warp a row of up to NV vectors a lane, four rows a CTA: no barrier, a row's loads all in flight and the row
-// kept as it is stored.  The next kernel's CTAs come up as these end: among many short CTAs they are in the way (recorded one behind
-// the other, 4096 rows of 1024 columns take 6.7 us, 8.9 with the next one's on the chip from the start).
+// The sum of 32 W values, s[w] of lane l that of thread 32 w + l, in the order in which a CTA of W warps adds them up above: over the
+// lanes of each warp, then over the warps.  A lane passes on half of its values at each of the first steps.
+template <int W>
+__device__ __forceinline__ float cta_sum(float (&s)[W]) {
+  static_assert(W == 4 || W == 8, "the CTAs above");
+  const int lane = threadIdx.x & 31;
+  int step = 16;
+#pragma unroll
+  for (int n = W / 2; n > 0; n /= 2, step /= 2) {
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const bool hi = lane & step;
+      const float mine = hi ? s[i + n] : s[i], other = hi ? s[i] : s[i + n];
+      s[i] = mine + __shfl_xor_sync(FULLM, other, step);
+    }
+  }
+  float v = s[0];
+#pragma unroll
+  for (int o = 16 / W; o > 0; o >>= 1) v += __shfl_xor_sync(FULLM, v, o);
+#pragma unroll
+  for (int o = 16; o >= 32 / W; o >>= 1) v += __shfl_xor_sync(FULLM, v, o);
+  return v;
+}
+
+// The same as the kernel above, in the same bits, with a warp a row of up to NV vectors a lane, four rows a CTA: no barrier, a row's
+// loads all in flight and the row kept as it is stored.  The next kernel's CTAs come up as these end: among many short CTAs they are in the
+// way (recorded one behind the other, 4096 rows of 1024 columns take 6.7 us, 8.9 with the next one's on the chip from the start).
 template <int NV>
 __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
     const __nv_bfloat16* x, const __nv_bfloat16* res,
@@ -189,17 +213,18 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(
       }
     }
   }
-  float ss = 0.f;
+  constexpr int W = NV > 4 ? 8 : 4;
+  float part[W] = {};
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     if (lane + 32 * i < nvec) {
       float f[8];
       unpack8(hv[i], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      for (int j = 0; j < 8; ++j) part[i % W] += f[j] * f[j];
     }
   }
-  ss = warp_sum(ss);
+  const float ss = cta_sum(part);
   const float rstd = rsqrtf(ss / (float)cols + eps);
   if (lane == 0) rstd_out[row] = rstd;
 #pragma unroll

@@ -387,6 +387,17 @@ def test_rmsnorm_of_many_rows_at_every_width(rows, cols, residual):
         assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8 + 1e-5
 
 
+@pytest.mark.parametrize("cols", [8, 264, 1024, 1032, 2048, 2056, 3072])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_of_a_row_has_the_same_bits_among_few_and_many(cols, residual):
+    """A warp adds a row's squares up in the order of the CTA that takes it where rows are few."""
+    torch.manual_seed(cols)
+    x, r = (torch.randn(3000, cols, device=DEV).bfloat16() for _ in range(2))
+    w = torch.randn(cols, device=DEV).bfloat16()
+    f = lambda a, b: norm.add_rms_norm(a, b, w, 1e-5)[0] if residual else norm.rms_norm(a, w, 1e-5)
+    assert torch.equal(f(x, r), torch.cat([f(a, b) for a, b in zip(x.split(750), r.split(750))]))
+
+
 @pytest.mark.parametrize("n", [8, 2048, 2056, 4096, 4104, 100_000])
 def test_adamw_updates_every_vector_once(n):
     """Around a thread's second vector and a CTA's 512; elements are independent, so each size has the bits of the largest.
