@@ -361,10 +361,14 @@ __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* pa
   const int lane = (threadIdx.y * 8 + threadIdx.x) & 31, warp = threadIdx.y >> 2;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c4 * 4 < cols) {
-#pragma unroll 4
-    for (int r = threadIdx.y; r < nblocks; r += 128) {
-      const float4 v = reinterpret_cast<const float4*>(partials + (int64_t)r * cols)[c4];
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    for (int r = threadIdx.y; r < nblocks; r += 512) {  // four rows' loads in flight
+      float4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (r + 128 * k < nblocks) v[k] = reinterpret_cast<const float4*>(partials + (int64_t)(r + 128 * k) * cols)[c4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (r + 128 * k < nblocks) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
     }
   }
   auto add_lanes = [&](int k) {

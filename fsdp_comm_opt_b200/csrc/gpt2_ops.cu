@@ -211,9 +211,14 @@ __global__ void __launch_bounds__(1024) column_sum_deliver_kernel(const float* i
   const int c4 = blockIdx.x * 32 + threadIdx.x;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c4 * 4 < ncols) {
-    for (int r = threadIdx.y; r < nrows; r += 32) {
-      const float4 v = reinterpret_cast<const float4*>(in + (int64_t)r * ncols)[c4];
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    for (int r = threadIdx.y; r < nrows; r += 128) {  // four rows' loads in flight
+      float4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (r + 32 * k < nrows) v[k] = reinterpret_cast<const float4*>(in + (int64_t)(r + 32 * k) * ncols)[c4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (r + 32 * k < nrows) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
     }
   }
   acc[threadIdx.y][threadIdx.x] = s;
