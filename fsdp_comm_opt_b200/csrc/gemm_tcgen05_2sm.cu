@@ -254,8 +254,9 @@ __device__ __forceinline__ Unit unit_of(int u, const Params& p) {
 // row a thread, lie next to each other.
 __device__ __forceinline__ int partial_off(int row, int c4) { return ((row >> 5) * (BN / 4) + c4) * 32 + (row & 31); }
 
-// ADD: to the old values of C.  Three CTAs of registers for
-// one to an SM: the 96 a thread leave room for a collective's CTAs beside it.
+// ADD: to the old values of C.
+// Shared memory allows one CTA to an SM; the registers are bounded as for three, which is 96 a thread, so that a collective's CTAs fit
+// beside it.
 template <int A_MAJOR, int B_MAJOR, bool ADD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 3)
     gemm_2sm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Params p) {

@@ -82,6 +82,8 @@ inline int launch_status() {
 // wait there until that has completed and its results are seen.  Not in launches that run at once: beside collectives, whose
 // CTAs need the slots that the waiting ones would hold.  Step of the tiny model (110 kernels)
 // 355 -> 334 us, of the small one (190) 1647 -> 1609.
+// CTAs that wait have taken the first slots that came free, which may be many to an SM on a few SMs: a kernel of several waves of short
+// CTAs does without chain_next(), and the next one's come up as its own end.
 // Such a kernel is on the chip while its inputs are still written, so it reads them with ordinary loads, which stay behind the
 // wait: the read-only path (__ldg, or a const __restrict__ parameter, of which the compiler makes the same) is for data that do
 // not change while a kernel runs, and its loads may be moved ahead of the wait.
